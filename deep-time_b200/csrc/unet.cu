@@ -120,39 +120,54 @@ __global__ void k_upsample(int nimg, int h, int w, Tensor4 in, Tensor4 out) {
 }
 
 // gradient through upsampling and the producing ReLU: g[p][c] = (sum of the 2 x 2 children's
-// gradients) where act > 0, else 0
+// gradients) where act > 0, else 0. Bound by HBM: eight channels (16 bytes) a thread, 32-bit
+// indices; one channel a thread with 64-bit divisions took 418 us for a 16 x 512 x 256 batch's three
+// levels, this 125 us.
 __global__ void k_upsample_bwd_mask(int nimg, int h, int w, Tensor4 gup, Tensor4 act, Tensor4 g) {
   // (h, w): the coarse level's shape; children at 2y.., 2x..
-  size_t total = (size_t)nimg * h * w * g.c;
-  int hf = 2 * h, wf = 2 * w;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
-    int c = (int)(k % g.c);
-    size_t p = k / g.c;
-    int x = (int)(p % w), y = (int)((p / w) % h);
-    size_t n = p / ((size_t)w * h);
-    float s = 0.f;
+  const int hf = 2 * h, wf = 2 * w, c8 = g.c / 8;
+  const unsigned total = (unsigned)nimg * h * w * c8;
+  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
+    unsigned c = k % c8, p = k / c8;
+    unsigned x = p % w, r = p / w, y = r % h, n = r / h;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, a[8];
+#pragma unroll
     for (int dy = 0; dy < 2; ++dy)
-      for (int dx = 0; dx < 2; ++dx)
-        s += __bfloat162float(gup.p[(((n * hf) + 2 * y + dy) * wf + 2 * x + dx) * gup.stride + gup.off + c]);
-    float a = __bfloat162float(act.p[p * act.stride + act.off + c]);
-    g.p[p * g.stride + g.off + c] = __float2bfloat16(a > 0.f ? s : 0.f);
+#pragma unroll
+      for (int dx = 0; dx < 2; ++dx) {
+        float f[8];
+        bf8_to_f(*reinterpret_cast<const uint4*>(gup.p + ((size_t)(n * hf + 2 * y + dy) * wf + 2 * x + dx) * gup.stride +
+                                                 gup.off + c * 8),
+                 f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += f[e];
+      }
+    bf8_to_f(*reinterpret_cast<const uint4*>(act.p + (size_t)p * act.stride + act.off + c * 8), a);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = a[e] > 0.f ? s[e] : 0.f;
+    *reinterpret_cast<uint4*>(g.p + (size_t)p * g.stride + g.off + c * 8) = f_to_bf8(s);
   }
 }
 
 // gradient of an encoder level's output: its skip gradient plus the pooling's (1/4 of the parent
-// cell's), through the ReLU; written over the skip slice
+// cell's), through the ReLU; written over the skip slice. Eight channels a thread as above (748 us
+// to 168 us for the three levels of a 16 x 512 x 256 batch).
 __global__ void k_skip_pool_bwd_mask(int nimg, int h, int w, Tensor4 gskip, Tensor4 gpool, Tensor4 act) {
-  size_t total = (size_t)nimg * h * w * act.c;
-  int hc = h / 2, wc = w / 2;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
-    int c = (int)(k % act.c);
-    size_t p = k / act.c;
-    int x = (int)(p % w), y = (int)((p / w) % h);
-    size_t n = p / ((size_t)w * h);
-    float s = __bfloat162float(gskip.p[p * gskip.stride + gskip.off + c]) +
-              0.25f * __bfloat162float(gpool.p[(((n * hc) + y / 2) * wc + x / 2) * gpool.stride + gpool.off + c]);
-    float a = __bfloat162float(act.p[p * act.stride + act.off + c]);
-    gskip.p[p * gskip.stride + gskip.off + c] = __float2bfloat16(a > 0.f ? s : 0.f);
+  const int hc = h / 2, wc = w / 2, c8 = act.c / 8;
+  const unsigned total = (unsigned)nimg * h * w * c8;
+  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
+    unsigned c = k % c8, p = k / c8;
+    unsigned x = p % w, r = p / w, y = r % h, n = r / h;
+    uint4* gs = reinterpret_cast<uint4*>(gskip.p + (size_t)p * gskip.stride + gskip.off + c * 8);
+    float s[8], q[8], a[8];
+    bf8_to_f(*gs, s);
+    bf8_to_f(*reinterpret_cast<const uint4*>(gpool.p + ((size_t)(n * hc + y / 2) * wc + x / 2) * gpool.stride + gpool.off +
+                                             c * 8),
+             q);
+    bf8_to_f(*reinterpret_cast<const uint4*>(act.p + (size_t)p * act.stride + act.off + c * 8), a);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = a[e] > 0.f ? s[e] + 0.25f * q[e] : 0.f;
+    *gs = f_to_bf8(s);
   }
 }
 
@@ -189,29 +204,42 @@ __global__ void k_mse(size_t npix, const float* __restrict__ pred, const float* 
 }
 
 // head backward: g[p][c] = dpred[p] W[c] where act > 0 (the last conv's ReLU); partial weight
-// and bias gradients per block: part[block][0..C-1] = sum dpred * act, part[block][C] = sum dpred
+// and bias gradients per block: part[block][0..C-1] = sum dpred * act, part[block][C] = sum dpred.
+// Bound by HBM: a pixel's 32 channels as four 16-byte words (2 bytes at a time: 489 us for
+// 16 x 512 x 256 pixels, this 57 us).
 __global__ void k_head_bwd(size_t npix, Tensor4 act, const float* __restrict__ Wh, const float* __restrict__ dpred, Tensor4 g,
                            float* __restrict__ part) {
   __shared__ float red[64][33];
-  const int C = act.c;  // 32
-  float accw[32];
+  constexpr int C = 32;  // act.c
+  float accw[C], wh[C];
   float accb = 0.f;
-  for (int c = 0; c < 32; ++c) accw[c] = 0.f;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    accw[c] = 0.f;
+    wh[c] = Wh[c];
+  }
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < npix; p += (size_t)gridDim.x * blockDim.x) {
     float dp = dpred[p];
-    const bf16* a = act.p + p * act.stride + act.off;
-    bf16* gg = g.p + p * g.stride + g.off;
-    for (int c = 0; c < C; ++c) {
-      float av = __bfloat162float(a[c]);
-      gg[c] = __float2bfloat16(av > 0.f ? dp * Wh[c] : 0.f);
-      accw[c] += dp * av;
+    const uint4* a = reinterpret_cast<const uint4*>(act.p + p * act.stride + act.off);
+    uint4* gg = reinterpret_cast<uint4*>(g.p + p * g.stride + g.off);
+#pragma unroll
+    for (int c = 0; c < 32; c += 8) {
+      float av[8], gv[8];
+      bf8_to_f(a[c / 8], av);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        gv[e] = av[e] > 0.f ? dp * wh[c + e] : 0.f;
+        accw[c + e] += dp * av[e];
+      }
+      gg[c / 8] = f_to_bf8(gv);
     }
     accb += dp;
   }
   // reduce over the block in a fixed order: warp shuffles then the warps in order
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
   for (int c = 0; c <= C; ++c) {
-    float v = c < C ? accw[c] : accb;
+    float v = c < C ? accw[c < C ? c : 0] : accb;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (lane == 0) red[warp][c] = v;
   }
@@ -223,13 +251,42 @@ __global__ void k_head_bwd(size_t npix, Tensor4 act, const float* __restrict__ W
   }
 }
 
-// bias gradient partials: part[block][c] = sum over the block's pixels of g[p][c]
-__global__ void k_bias_grad(size_t npix, Tensor4 g, float* __restrict__ part) {
-  // blockDim = C (<= 256 channels, one thread a channel), pixels strided over blocks
-  int c = threadIdx.x;
-  float s = 0.f;
-  for (size_t p = blockIdx.x; p < npix; p += gridDim.x) s += __bfloat162float(g.p[p * g.stride + g.off + c]);
-  part[(size_t)blockIdx.x * g.c + c] = s;
+// bias gradient partials: part[block][c] = sum over the block's pixels of g[p][c]. Bound by HBM
+// (each gradient read once): a thread takes eight channels (16 bytes) of a pixel, a block of 256
+// threads 256 / (C / 8) pixels at a time, four of them in flight a thread; the block's rows are
+// then added in order. One channel a thread and one pixel at a time took 3.66 ms at 32 channels
+// of 16 x 512 x 256 pixels (0.04 TB/s), this 34 us (3.9 TB/s). C divides 2048 and is a multiple of 8.
+constexpr int BIAS_THREADS = 256, BIAS_BLOCKS = 592;
+__global__ void __launch_bounds__(BIAS_THREADS) k_bias_grad(unsigned npix, Tensor4 g, float* __restrict__ part) {
+  __shared__ float red[BIAS_THREADS][9];
+  const unsigned c8 = g.c / 8, lane = threadIdx.x % c8, row = threadIdx.x / c8, rows = BIAS_THREADS / c8;
+  const bf16* src = g.p + g.off + lane * 8;
+  const unsigned step = gridDim.x * rows;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (size_t p = blockIdx.x * rows + row; p < npix; p += (size_t)4 * step) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const size_t q = p + (size_t)u * step;
+      v[u] = q < npix ? *reinterpret_cast<const uint4*>(src + q * g.stride) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float f[8];
+      bf8_to_f(v[u], f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] += f[e];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) red[threadIdx.x][e] = s[e];
+  __syncthreads();
+  if (threadIdx.x < g.c) {
+    const unsigned l = threadIdx.x / 8, e = threadIdx.x % 8;
+    float t = 0.f;
+    for (unsigned r = 0; r < rows; ++r) t += red[r * c8 + l][e];
+    part[(size_t)blockIdx.x * g.c + threadIdx.x] = t;
+  }
 }
 
 // sum of `parts` partial arrays of length n (in order) into out
@@ -238,6 +295,26 @@ __global__ void k_sum_parts(size_t n, int parts, const float* __restrict__ part,
     float s = 0.f;
     for (int q = 0; q < parts; ++q) s += part[(size_t)q * n + k];
     out[k] = s;
+  }
+}
+
+// The same for a short array of many partials (a layer's biases, the head): a block takes 8 of
+// the n values, 32 threads a value each every 32nd partial, their sums added in order. A walk of 256
+// partials a thread was a chain of dependent loads, 24 us; this 3 us.
+__global__ void __launch_bounds__(256) k_sum_many(unsigned n, int parts, const float* __restrict__ part, float* __restrict__ out) {
+  __shared__ float red[256];
+  const unsigned k = blockIdx.x * 8 + (threadIdx.x & 7);
+  float s = 0.f;
+  if (k < n) {
+#pragma unroll 8
+    for (int q = threadIdx.x >> 3; q < parts; q += 32) s += part[(size_t)q * n + k];
+  }
+  red[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x < 8 && k < n) {
+    float t = 0.f;
+    for (int r = 0; r < 32; ++r) t += red[r * 8 + threadIdx.x];
+    out[k] = t;
   }
 }
 
@@ -476,9 +553,9 @@ static void conv_wgrad(dt_unet* u, const ConvLayer& L, int B, int h, int w, Tens
   k_sum_parts<<<ugrid(u, nw), 256, 0, st>>>(nw, chunks, u->part, u->grad + L.w_off);
   // bias: per-block partials over pixels, then their sum
   size_t npix = (size_t)B * h * w;
-  int bparts = 256;
-  k_bias_grad<<<bparts, L.cout, 0, st>>>(npix, g, u->part);
-  k_sum_parts<<<1, 256, 0, st>>>((size_t)L.cout, bparts, u->part, u->grad + L.b_off);
+  int bparts = std::min<int>(BIAS_BLOCKS, (int)ceil_div(npix, 64));
+  k_bias_grad<<<bparts, BIAS_THREADS, 0, st>>>((unsigned)npix, T4(g.p, g.stride, g.off, L.cout), u->part);
+  k_sum_many<<<ceil_div(L.cout, 8), 256, 0, st>>>((unsigned)L.cout, bparts, u->part, u->grad + L.b_off);
   count_launch();
   count_launch();
   count_launch();
@@ -538,9 +615,9 @@ static void unet_backward(dt_unet* u, cudaStream_t st) {
   LevelBufs& b0 = u->lv[0];
   int c0 = u->base;
   // head
-  int hparts = std::min<int>(256, (int)ceil_div(npix, 256));
+  int hparts = std::min<int>(BIAS_BLOCKS, (int)ceil_div(npix, 256));
   k_head_bwd<<<hparts, 256, 0, st>>>(npix, T4(b0.DB, c0, 0, c0), u->prm + u->head_w, u->dpred, T4(b0.gDB, c0, 0, c0), u->part);
-  k_sum_parts<<<1, 64, 0, st>>>((size_t)c0 + 1, hparts, u->part, u->grad + u->head_w);  // head_b follows head_w
+  k_sum_many<<<ceil_div(c0 + 1, 8), 256, 0, st>>>((unsigned)c0 + 1, hparts, u->part, u->grad + u->head_w);  // head_b follows head_w
   count_launch();
   count_launch();
   // decoder, finest to coarsest
@@ -652,7 +729,7 @@ static dt_status unet_make(dt_unet* u, unsigned long long seed) {
   DT_CUDA(cudaMemcpy(u->prm, h.data(), u->n_params * sizeof(float), cudaMemcpyHostToDevice));
   DT_CUDA(cudaMemset(u->m, 0, u->n_params * sizeof(float)));
   DT_CUDA(cudaMemset(u->v, 0, u->n_params * sizeof(float)));
-  // wgrad partials: 64 chunks x the largest layer, or the head/bias partials
+  // wgrad partials: 64 chunks x the largest layer, or the head/bias partials (BIAS_BLOCKS x 256)
   size_t mx = 0;
   for (auto& L : u->conv) mx = std::max(mx, (size_t)9 * L.cin * L.cout);
   u->part_cap = std::max(mx * 64, (size_t)256 * 512);
