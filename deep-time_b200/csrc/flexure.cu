@@ -1232,42 +1232,48 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS / 2, 3) k_cols_fused(int N, cp
 // The column pass on the sphere's row metric (RowSolve::solve, flexure.rs:1012-1099): no
 // transform along y; per wavenumber k the pentadiagonal d L_k^2 + c (L_k: diagonal
 // (a_j lx_k - b_j - b_(j+1)) / dx^2, off the diagonal b_(j+1) / dx^2) is factored as L D L^T
-// and solved, with the reference's recurrences and order of operations. The factors depend only
-// on the level's (d, c) and k, so k_row_factor makes them once per solve (dd, l1, l2: h x (N + 1)
-// each, row-major, wavenumber fastest) and k_row_solve does the substitutions at every
-// application. One thread per wavenumber q = 0 .. N; column q of the packed half spectrum holds
-// wavenumber q (both parts) for 0 < q < N, and column 0 wavenumbers 0 (real part) and N
-// (imaginary part), which threads 0 and N solve part by part.
+// and solved. The factors depend only on the level's (d, c) and k, so k_row_factor makes them once
+// per solve for every level (blockIdx.y; rd = 1 / dd, l1, l2: h x (N + 1) each, row-major,
+// wavenumber fastest) and k_row_solve does the substitutions at every application. Column q of
+// the packed half spectrum holds wavenumber q (both parts) for 0 < q < N, and column 0 wavenumbers
+// 0 (real part) and N (imaginary part), which wavenumbers 0 and N solve part by part.
+//
+// The factorisation is one serial chain down the rows, bound by its latency: with m2 = d e(j-1)
+// e(j) and n1 = m1 - m2 l1(j-1) the row's chain is l1 = n1 rd, dd = m0 - l1 n1 - l2 m2 and one
+// reciprocal (the reference's carried value l2 dd(j-2) l1 is m2 l1). With two divisions a row and a
+// launch a level it took 90 us a level at 513 wavenumbers x 328 rows (FP64), three in sequence.
 template <class T>
-__global__ void __launch_bounds__(128) k_row_factor(int N, int h, const T* __restrict__ lx, const T* __restrict__ ma,
-                                                    const T* __restrict__ mb, T inv_dx2, const Scalars* S, int level,
-                                                    T* __restrict__ dds, T* __restrict__ l1s, T* __restrict__ l2s) {
+__device__ __forceinline__ T row_recip(T x);
+template <>
+__device__ __forceinline__ float row_recip(float x) { return recip(x); }
+template <>
+__device__ __forceinline__ double row_recip(double x) { return recip_fast(x); }
+
+template <class T>
+__global__ void __launch_bounds__(64) k_row_factor(int N, int h, const T* __restrict__ lx, const T* __restrict__ ma,
+                                                   const T* __restrict__ mb, T inv_dx2, const Scalars* S, T* __restrict__ fac) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q > N) return;
-  const T d = (T)S->node_d[level], c = (T)S->c_ref;
+  const T d = (T)S->node_d[blockIdx.y], c = (T)S->c_ref;
   const T lxk = lx[q];
-  const size_t stride = (size_t)N + 1;
-  T dd1 = 0, dd2 = 0, l1p = 0;  // dd[j-1], dd[j-2], l1[j-1]
-  T t1 = 0, e1 = 0, e2 = 0;     // t(j-1), e(j-1), e(j-2)
+  const size_t stride = (size_t)N + 1, plane = (size_t)h * stride;
+  fac += (size_t)blockIdx.y * 3 * plane + q;
+  T r1 = 0, r2 = 0, l1p = 0;  // 1 / dd[j-1], 1 / dd[j-2], l1[j-1]
+  T t1 = 0, e1 = 0, e2 = 0;   // t(j-1), e(j-1), e(j-2)
 #pragma unroll 4
   for (int j = 0; j < h; ++j) {
     const T tj = (ma[j] * lxk - mb[j] - mb[j + 1]) * inv_dx2;
     const T ej = j + 1 < h ? mb[j + 1] * inv_dx2 : (T)0;
-    T p1 = 0, p2 = 0;
-    if (j >= 2) p2 = d * e2 * e1 / dd2;  // m2(j-2) / dd[j-2]
-    if (j >= 1) {
-      T carried = j >= 2 ? p2 * dd2 * l1p : (T)0;
-      p1 = (d * e1 * (t1 + tj) - carried) / dd1;  // (m1(j-1) - carried) / dd[j-1]
-    }
-    const T up = j > 0 ? e1 : (T)0;
-    T dj = d * (tj * tj + up * up + ej * ej) + c;  // m0(j)
-    if (j >= 1) dj -= p1 * p1 * dd1;
-    if (j >= 2) dj -= p2 * p2 * dd2;
-    dds[(size_t)j * stride + q] = dj;
-    l1s[(size_t)j * stride + q] = p1;
-    l2s[(size_t)j * stride + q] = p2;
-    dd2 = dd1;
-    dd1 = dj;
+    const T m2 = d * e2 * e1;                    // 0 for j < 2
+    const T n1 = d * e1 * (t1 + tj) - m2 * l1p;  // 0 for j < 1
+    const T p1 = n1 * r1, p2 = m2 * r2;
+    const T dj = (d * (tj * tj + e1 * e1 + ej * ej) + c - p2 * m2) - p1 * n1;
+    const T rj = row_recip<T>(dj);
+    fac[(size_t)j * stride] = rj;
+    fac[plane + (size_t)j * stride] = p1;
+    fac[2 * plane + (size_t)j * stride] = p2;
+    r2 = r1;
+    r1 = rj;
     l1p = p1;
     e2 = e1;
     e1 = ej;
@@ -1275,115 +1281,166 @@ __global__ void __launch_bounds__(128) k_row_factor(int N, int h, const T* __res
   }
 }
 
-// The substitutions: x[j] -= x[j-1] l1[j] + ... going down, x[j] /= dd[j], x[j] -= x[j+1] l1[j+1]
-// + ... going up, in place on the level's spectrum. A thread's recurrence waits on nothing but
-// its own arithmetic: it loads RB rows (spectrum and factors) at a time before walking them.
-template <class T>
-__global__ void __launch_bounds__(128) k_row_solve(int N, int h, cplx<T>* __restrict__ half, const T* __restrict__ dds,
-                                                   const T* __restrict__ l1s, const T* __restrict__ l2s, const Scalars* S) {
-  using C = cplx<T>;
-  constexpr int RB = 8;
-  if (S->stop) return;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q > N) return;
-  const int col = q == N ? 0 : q;
-  const bool re = q != N, im = q != 0;  // the parts this thread owns
-  const size_t stride = (size_t)N + 1;
-  auto store = [&](int j, C v) {
-    // column 0's parts belong to two threads: each stores only its own
-    if (re && im) {
-      half[(size_t)j * N + col] = v;
-    } else if (re) {
-      half[(size_t)j * N + col].x = v.x;
-    } else {
-      half[(size_t)j * N + col].y = v.y;
-    }
-  };
-  C x1 = mk<C>((T)0, (T)0), x2 = x1;  // x'[j-1], x'[j-2] (before the division)
-  for (int j0 = 0; j0 < h; j0 += RB) {
-    C v[RB];
-    T a1[RB], a2[RB], dv[RB];
-#pragma unroll
-    for (int u = 0; u < RB; ++u) {
-      const int j = min(j0 + u, h - 1);
-      v[u] = half[(size_t)j * N + col];
-      a1[u] = l1s[(size_t)j * stride + q];
-      a2[u] = l2s[(size_t)j * stride + q];
-      dv[u] = dds[(size_t)j * stride + q];
-    }
-#pragma unroll
-    for (int u = 0; u < RB; ++u) {
-      const int j = j0 + u;
-      if (j >= h) break;
-      C x = v[u];
-      if (j >= 1) {
-        x.x -= x1.x * a1[u];
-        x.y -= x1.y * a1[u];
-      }
-      if (j >= 2) {
-        x.x -= x2.x * a2[u];
-        x.y -= x2.y * a2[u];
-      }
-      x2 = x1;
-      x1 = x;
-      store(j, mk<C>(x.x / dv[u], x.y / dv[u]));
-    }
-  }
-  // the walk up: x[j] -= x[j+1] l1[j+1]; x[j] -= x[j+2] l2[j+2]
-  C y1 = mk<C>((T)0, (T)0), y2 = y1;  // x[j+1], x[j+2]
-  T l1n = 0, l2n = 0, l2nn = 0;       // l1[j+1], l2[j+1], l2[j+2]
-  for (int j0 = h - 1; j0 >= 0; j0 -= RB) {
-    C v[RB];
-    T a1[RB], a2[RB];
-#pragma unroll
-    for (int u = 0; u < RB; ++u) {
-      const int j = max(j0 - u, 0);
-      v[u] = half[(size_t)j * N + col];
-      a1[u] = l1s[(size_t)j * stride + q];
-      a2[u] = l2s[(size_t)j * stride + q];
-    }
-#pragma unroll
-    for (int u = 0; u < RB; ++u) {
-      const int j = j0 - u;
-      if (j < 0) break;
-      C x = v[u];
-      if (j + 1 < h) {
-        x.x -= y1.x * l1n;
-        x.y -= y1.y * l1n;
-      }
-      if (j + 2 < h) {
-        x.x -= y2.x * l2nn;
-        x.y -= y2.y * l2nn;
-      }
-      store(j, x);
-      y2 = y1;
-      y1 = x;
-      l2nn = l2n;
-      l1n = a1[u];
-      l2n = a2[u];
-    }
-  }
-}
-
-// The row solve in chunks: the down and up recurrences of k_row_solve are linear in their two
-// carried values, so each column is cut into chunks of ROW_CHUNK rows that run in parallel from a
-// zero carry, a short pass per column composes the chunks' 2 x 2 carry transfers (made once per
-// solve, from the factors alone), and a second parallel pass reruns each chunk from its true
-// carry. The same sums as the sequential solve, differently rounded; (chunk, wavenumber)
-// threads, wavenumber fastest, so every row step reads contiguous words.
-constexpr int ROW_CHUNK = 64;
-
-// one row of the down recurrence: x = v - s1 l1 - s2 l2, then (s2, s1) <- (s1, x)
+// one row of a substitution: x = v - s1 a1 - s2 a2, then (s2, s1) <- (s1, x)
 template <class C, class T>
-__device__ __forceinline__ void row_down(C v, T a1, T a2, C& s1, C& s2) {
+__device__ __forceinline__ void row_step(C v, T a1, T a2, C& s1, C& s2) {
   C x = v;
-  x.x -= s1.x * a1;
-  x.y -= s1.y * a1;
   x.x -= s2.x * a2;
   x.y -= s2.y * a2;
+  x.x -= s1.x * a1;
+  x.y -= s1.y * a1;
   s2 = s1;
   s1 = x;
 }
+
+// The substitutions of G = 2^lg consecutive wavenumbers a block (level blockIdx.y), every row of
+// their spectrum in the block's registers and every factor in its shared memory, so that each is
+// read once and the spectrum written once. Both recurrences (down: x[j] = v[j] - l1[j] x[j-1] -
+// l2[j] x[j-2]; then z = x rd and up with l1[j+1], l2[j+2]) are linear in their two carried values,
+// so a thread takes a chunk of ROW_CH rows: a walk from a zero carry and from the two unit carries
+// gives the chunk's end state and its 2 x 2 carry transfer, the chunks' carries are composed in
+// order through shared memory, and a second walk starts from the true carry. Bound by latency:
+// 4 ROW_CH + 2 (chunks) dependent steps after one round of loads. Sixteen rows are 64 registers of
+// FP64 values; G = 8 makes a row's segment 64 to 128 bytes. Factor rows are spaced by one row of G
+// after every 16, so that the chunks of a warp fall in distinct banks. Against the passes over
+// 64-row chunks below (a launch list of five a level), the bank's three levels after an L2 flush:
+// FP64 1024 x 328 21 us (162 a level), FP32 2048 x 1024 48 (151 a level), FP32 4096 x 2047 210 (184
+// a level). With the factors read from global memory at each walk the same three took 36, 72, 302.
+constexpr int ROW_CH = 16;
+constexpr int ROW_THREADS = 512;
+// factor rows held: the chunks' and two more (zeros past the last row), spaced
+__host__ __device__ constexpr int row_slot(int j) { return j + j / ROW_CH; }
+__host__ __device__ constexpr int row_slots(int P) { return row_slot(P * ROW_CH + 1) + 1; }
+template <class T>
+static size_t row_smem(int P, int lg) {
+  return ((size_t)row_slots(P) * 3 << lg) * sizeof(T) + (size_t)ceil_div((size_t)P << lg, 32) * 32 * 8 * sizeof(T);
+}
+
+template <class T>
+__global__ void __launch_bounds__(ROW_THREADS, 1) k_row_solve(int N, int h, int P, int lg, cplx<T>* __restrict__ half,
+                                                              const T* __restrict__ fac, const Scalars* S) {
+  using C = cplx<T>;
+  if (S->stop) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int tid = threadIdx.x, nt = blockDim.x, G = 1 << lg, chunk = tid >> lg, g = tid & (G - 1);
+  C* st1 = reinterpret_cast<C*>(smem_raw);  // end states, then carries
+  C* st2 = st1 + nt;
+  C* f1 = st2 + nt;  // carry transfers: the new first value's and the new second value's
+  C* f2 = f1 + nt;
+  const int slots = row_slots(P) << lg;
+  T* srd = reinterpret_cast<T*>(f2 + nt);
+  const int stride = N + 1;  // h (N + 1) < 2^31 (h <= 8192, N <= 32768): 32-bit offsets in a level
+  const int q0 = blockIdx.x * G;
+  {
+    const T* src = fac + (size_t)blockIdx.y * 3 * h * stride;
+    const int rows = P * ROW_CH + 2;
+    for (int e = tid; e < rows << lg; e += nt) {
+      const int j = e >> lg, ge = e & (G - 1);
+      T* dst = srd + ((row_slot(j) << lg) + ge);
+      const T* from = src + (size_t)j * stride + min(q0 + ge, N);
+#pragma unroll
+      for (int k = 0; k < 3; ++k, dst += slots, from += (size_t)h * stride) {
+        if (j < h)
+          __pipeline_memcpy_async(dst, from, sizeof(T));
+        else
+          *dst = (T)0;
+      }
+    }
+    __pipeline_commit();
+  }
+  const int q = q0 + g, col = q >= N ? 0 : q, a = chunk * ROW_CH;
+  C* x = half + (size_t)blockIdx.y * h * N + col;
+  C v[ROW_CH];
+#pragma unroll
+  for (int r = 0; r < ROW_CH; ++r) v[r] = a + r < h ? x[(a + r) * N] : mk<C>((T)0, (T)0);
+  __pipeline_wait_prior(0);
+  __syncthreads();
+  // threads past the last chunk (the block is whole warps) walk the last chunk's factors
+  const T* rd = srd + ((row_slot(min(chunk, P - 1) * ROW_CH) << lg) + g);
+  const T *l1 = rd + slots, *l2 = l1 + slots;
+
+  // the chunks' carries in order (first to last, or last to first): two threads a wavenumber, its
+  // real and imaginary parts; each chunk's carry replaces its end state
+  auto compose = [&](C s1, C s2, C u1, C u2, bool up) {
+    st1[tid] = s1;
+    st2[tid] = s2;
+    f1[tid] = mk<C>(u1.x, u1.y);
+    f2[tid] = mk<C>(u2.x, u2.y);
+    __syncthreads();
+    if (tid < 2 * G) {
+      T* w1 = reinterpret_cast<T*>(st1) + (tid & 1);
+      T* w2 = reinterpret_cast<T*>(st2) + (tid & 1);
+      T c1 = 0, c2 = 0;
+#pragma unroll 4
+      for (int i = 0; i < P; ++i) {
+        const int t = ((up ? P - 1 - i : i) << lg) + (tid >> 1);
+        const T p1 = w1[2 * t], p2 = w2[2 * t];
+        const C g1 = f1[t], g2 = f2[t];
+        w1[2 * t] = c1;
+        w2[2 * t] = c2;
+        const T n1 = p1 + g1.x * c1 + g1.y * c2;
+        const T n2 = p2 + g2.x * c1 + g2.y * c2;
+        c1 = n1;
+        c2 = n2;
+      }
+    }
+    __syncthreads();
+  };
+
+  const C zero = mk<C>((T)0, (T)0);
+  {
+    C s1 = zero, s2 = zero, u1 = mk<C>((T)1, (T)0), u2 = mk<C>((T)0, (T)1);  // u: the unit carries as .x and .y
+#pragma unroll
+    for (int r = 0; r < ROW_CH; ++r) {
+      const T a1 = l1[r << lg], a2 = l2[r << lg];
+      row_step(v[r], a1, a2, s1, s2);
+      row_step(zero, a1, a2, u1, u2);
+    }
+    compose(s1, s2, u1, u2, false);
+  }
+  {
+    C s1 = st1[tid], s2 = st2[tid];
+#pragma unroll
+    for (int r = 0; r < ROW_CH; ++r) {
+      row_step(v[r], l1[r << lg], l2[r << lg], s1, s2);
+      v[r] = cscale(s1, rd[r << lg]);
+    }
+  }
+  __syncthreads();  // the carries are read before the next states replace them
+  {
+    C s1 = zero, s2 = zero, u1 = mk<C>((T)1, (T)0), u2 = mk<C>((T)0, (T)1);
+#pragma unroll
+    for (int r = ROW_CH - 1; r >= 0; --r) {
+      const T a1 = l1[row_slot(r + 1) << lg], a2 = l2[row_slot(r + 2) << lg];
+      row_step(v[r], a1, a2, s1, s2);
+      row_step(zero, a1, a2, u1, u2);
+    }
+    compose(s1, s2, u1, u2, true);
+  }
+  if (q > N) return;
+  const bool re = q != N, im = q != 0;  // column 0's parts belong to two wavenumbers: each stores only its own
+  C s1 = st1[tid], s2 = st2[tid];
+#pragma unroll
+  for (int r = ROW_CH - 1; r >= 0; --r) {
+    row_step(v[r], l1[row_slot(r + 1) << lg], l2[row_slot(r + 2) << lg], s1, s2);
+    if (a + r >= h) continue;
+    C* o = x + (a + r) * N;
+    if (re && im) {
+      *o = s1;
+    } else if (re) {
+      o->x = s1.x;
+    } else {
+      o->y = s1.y;
+    }
+  }
+}
+
+// The same solve for rasters too tall for k_row_solve's block (row_groups below): each column cut
+// into chunks of ROW_CHUNK rows, (chunk, wavenumber) threads in global-memory passes: zero-carry
+// chunk walks, a carry pass per wavenumber through the chunks' transfers (k_row_transfer, once per
+// solve), and walks from the true carry. The spectrum is read three times and written twice.
+constexpr int ROW_CHUNK = 64;
+
 // the up recurrence's coefficients at row j: l1[j + 1] and l2[j + 2] (0 past the last row)
 template <class T>
 __device__ __forceinline__ void up_coeffs(const T* __restrict__ l1s, const T* __restrict__ l2s, int j, int h, size_t q,
@@ -1407,7 +1464,7 @@ __global__ void __launch_bounds__(128) k_row_transfer(int N, int h, int P, const
   // the two unit carries as one complex pair: .x from (1, 0), .y from (0, 1)
   C s1 = mk<C>((T)1, (T)0), s2 = mk<C>((T)0, (T)1);
   for (int j = a; j < b; ++j)
-    row_down(mk<C>((T)0, (T)0), l1s[(size_t)j * stride + q], l2s[(size_t)j * stride + q], s1, s2);
+    row_step(mk<C>((T)0, (T)0), l1s[(size_t)j * stride + q], l2s[(size_t)j * stride + q], s1, s2);
   tf[0 * plane + t] = s1.x;
   tf[1 * plane + t] = s2.x;
   tf[2 * plane + t] = s1.y;
@@ -1416,7 +1473,7 @@ __global__ void __launch_bounds__(128) k_row_transfer(int N, int h, int P, const
   for (int j = b - 1; j >= a; --j) {
     T a1, a2;
     up_coeffs(l1s, l2s, j, h, q, stride, a1, a2);
-    row_down(mk<C>((T)0, (T)0), a1, a2, t1, t2);
+    row_step(mk<C>((T)0, (T)0), a1, a2, t1, t2);
   }
   tb[0 * plane + t] = t1.x;
   tb[1 * plane + t] = t2.x;
@@ -1439,7 +1496,7 @@ __global__ void __launch_bounds__(128) k_row_down_part(int N, int h, int P, cons
   const int c = (int)(t / stride), a = c * ROW_CHUNK, b = min(h, a + ROW_CHUNK);
   C s1 = mk<C>((T)0, (T)0), s2 = s1;
 #pragma unroll 4
-  for (int j = a; j < b; ++j) row_down(half[(size_t)j * N + col], l1s[(size_t)j * stride + q], l2s[(size_t)j * stride + q], s1, s2);
+  for (int j = a; j < b; ++j) row_step(half[(size_t)j * N + col], l1s[(size_t)j * stride + q], l2s[(size_t)j * stride + q], s1, s2);
   part[t] = s1;
   part[plane + t] = s2;
 }
@@ -1471,11 +1528,11 @@ __global__ void __launch_bounds__(128) k_row_carry(int N, int P, bool up, const 
   }
 }
 
-// The chunk's down recurrence from its true carry, y = x' / dd into the spectrum; then the up
+// The chunk's down recurrence from its true carry, y = x' rd into the spectrum; then the up
 // recurrence over the chunk from a zero carry, its end state (z[a], z[a+1]) into part
 template <class T>
 __global__ void __launch_bounds__(128) k_row_down_final(int N, int h, int P, cplx<T>* __restrict__ half,
-                                                        const T* __restrict__ dds, const T* __restrict__ l1s,
+                                                        const T* __restrict__ rds, const T* __restrict__ l1s,
                                                         const T* __restrict__ l2s, const cplx<T>* __restrict__ carry,
                                                         cplx<T>* __restrict__ part, const Scalars* S) {
   using C = cplx<T>;
@@ -1490,22 +1547,22 @@ __global__ void __launch_bounds__(128) k_row_down_final(int N, int h, int P, cpl
   C s1 = carry[t], s2 = carry[plane + t];
 #pragma unroll 4
   for (int j = a; j < b; ++j) {
-    row_down(half[(size_t)j * N + col], l1s[(size_t)j * stride + q], l2s[(size_t)j * stride + q], s1, s2);
-    const T dv = dds[(size_t)j * stride + q];
+    row_step(half[(size_t)j * N + col], l1s[(size_t)j * stride + q], l2s[(size_t)j * stride + q], s1, s2);
+    const T dv = rds[(size_t)j * stride + q];
     C* o = half + (size_t)j * N + col;
     if (re && im) {
-      *o = mk<C>(s1.x / dv, s1.y / dv);
+      *o = mk<C>(s1.x * dv, s1.y * dv);
     } else if (re) {
-      o->x = s1.x / dv;
+      o->x = s1.x * dv;
     } else {
-      o->y = s1.y / dv;
+      o->y = s1.y * dv;
     }
   }
   C t1 = mk<C>((T)0, (T)0), t2 = t1;
   for (int j = b - 1; j >= a; --j) {
     T a1, a2;
     up_coeffs(l1s, l2s, j, h, q, stride, a1, a2);
-    row_down(half[(size_t)j * N + col], a1, a2, t1, t2);
+    row_step(half[(size_t)j * N + col], a1, a2, t1, t2);
   }
   part[t] = t1;
   part[plane + t] = t2;
@@ -1530,7 +1587,7 @@ __global__ void __launch_bounds__(128) k_row_up_final(int N, int h, int P, cplx<
   for (int j = b - 1; j >= a; --j) {
     T a1, a2;
     up_coeffs(l1s, l2s, j, h, q, stride, a1, a2);
-    row_down(half[(size_t)j * N + col], a1, a2, t1, t2);
+    row_step(half[(size_t)j * N + col], a1, a2, t1, t2);
     C* o = half + (size_t)j * N + col;
     if (re && im) {
       *o = t1;
@@ -1991,8 +2048,8 @@ struct Lane {
   // spectra are consecutive (half + k h N), as are the three weights (wt[k] = wt[0] + k n)
   cplx<T>* half_side[2] = {nullptr, nullptr};
   int bank_blocks = 0;  // k_rows_inv_bank's persistent grid (0: not yet known)
-  // the row metric's L D L^T factors per bank level: dd, l1, l2 (h x (N + 1) each); when the
-  // rows make more than one chunk, per level the chunks' carry transfers (8 x chunks x (N + 1))
+  // the row metric's L D L^T factors per bank level: 1 / dd, l1, l2 (h x (N + 1) each); for
+  // rasters too tall for k_row_solve, per level the chunks' carry transfers (8 x chunks x (N + 1))
   // and the chunk states and carries (4 complex x chunks x (N + 1))
   T* row_factors = nullptr;
   T* row_transfer = nullptr;
@@ -2230,6 +2287,17 @@ static dt_status make_any_tables(dt_flex* s, Lane<T>& L) {
   return DT_OK;
 }
 
+// log2 of the wavenumbers a k_row_solve block takes for rasters of h rows: 8, or 4 where that keeps
+// the block within ROW_THREADS threads and the SM's shared memory; -1 (the chunk passes) where even
+// 4 do not fit, h > 2048 in FP32 and h > 1936 in FP64.
+template <class T>
+static int row_groups(int h) {
+  const int P = (int)ceil_div(h, ROW_CH);
+  for (int lg = 3; lg >= 2; --lg)
+    if ((P << lg) <= ROW_THREADS && row_smem<T>(P, lg) <= 227 * 1024) return lg;
+  return -1;
+}
+
 template <class T>
 static dt_status make_lane(dt_flex* s, Lane<T>& L) {
   size_t n = s->n;
@@ -2243,8 +2311,8 @@ static dt_status make_lane(dt_flex* s, Lane<T>& L) {
   L.half_side[1] = L.half + 2 * hn;
   if (s->row_solve) {
     DT_TRY(dalloc(s, &L.row_factors, 9 * (size_t)s->h * (s->N + 1)));
-    const size_t P = ceil_div(s->h, ROW_CHUNK);
-    if (P > 1) {
+    if (row_groups<T>(s->h) < 0) {
+      const size_t P = ceil_div(s->h, ROW_CHUNK);
       DT_TRY(dalloc(s, &L.row_transfer, 3 * 8 * P * (s->N + 1)));
       DT_TRY(dalloc(s, &L.row_state, 3 * 4 * P * (s->N + 1)));
     }
@@ -2514,6 +2582,7 @@ static RowsInvFn<T> rows_inv_for(int mode, int logn) {
 template <class T>
 static void transform_smem_attributes() {
   int big = 200 * 1024;
+  cudaFuncSetAttribute(k_row_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   for (int l = 0; l < FFT_LOGS; ++l) {
     cudaFuncSetAttribute(rows_fwd_fn<T, true>(l, LogSeq{}), cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(rows_fwd_fn<T, false>(l, LogSeq{}), cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -2632,35 +2701,42 @@ static void launch_rows_fwd(dt_flex* s, Lane<T>& L, const T* in, const T* wt, cp
                                                                                    L.tab.post, S);
   counted();
 }
+// The column pass of `levels` consecutive bank levels from `level` on, their spectra consecutive
+// from `half`.
 template <class T>
-static void launch_cols(dt_flex* s, Lane<T>& L, cplx<T>* half, const FftGeo& g, int level, Scalars* S, cudaStream_t st) {
+static void launch_cols(dt_flex* s, Lane<T>& L, cplx<T>* half, const FftGeo& g, int level, Scalars* S, cudaStream_t st,
+                        int levels = 1) {
   if (s->row_solve) {
-    // the row solve per wavenumber with the level's factors (made by setup_precond): in chunks
-    // of rows when there is more than one, else one walk per wavenumber
+    // the row solve per wavenumber with the levels' factors (made by setup_precond)
     const size_t fac = (size_t)s->h * (s->N + 1);
-    const T* dd = L.row_factors + (size_t)level * 3 * fac;
-    const T *l1 = dd + fac, *l2 = dd + 2 * fac;
-    const int P = (int)ceil_div(s->h, ROW_CHUNK);
-    if (P == 1) {
-      k_row_solve<T><<<ceil_div(s->N + 1, 128), 128, 0, st>>>(s->N, s->h, half, dd, l1, l2, S);
+    if (const int lg = row_groups<T>(s->h); lg >= 0) {
+      const int P = (int)ceil_div(s->h, ROW_CH);
+      const int threads = (int)ceil_div((size_t)P << lg, 32) * 32;
+      k_row_solve<T><<<dim3(ceil_div(s->N + 1, 1 << lg), levels), threads, row_smem<T>(P, lg), st>>>(
+          s->N, s->h, P, lg, half, L.row_factors + (size_t)level * 3 * fac, S);
       counted();
       return;
     }
+    const int P = (int)ceil_div(s->h, ROW_CHUNK);
     const size_t plane = (size_t)P * (s->N + 1);
-    const T* tf = L.row_transfer + (size_t)level * 8 * plane;
-    const T* tb = tf + 4 * plane;
-    cplx<T>* part = L.row_state + (size_t)level * 4 * plane;
-    cplx<T>* carry = part + 2 * plane;
     const unsigned gp = ceil_div(plane, 128), gq = ceil_div(s->N + 1, 128);
-    k_row_down_part<T><<<gp, 128, 0, st>>>(s->N, s->h, P, half, l1, l2, part, S);
-    k_row_carry<T><<<gq, 128, 0, st>>>(s->N, P, false, tf, part, carry, S);
-    k_row_down_final<T><<<gp, 128, 0, st>>>(s->N, s->h, P, half, dd, l1, l2, carry, part, S);
-    k_row_carry<T><<<gq, 128, 0, st>>>(s->N, P, true, tb, part, carry, S);
-    k_row_up_final<T><<<gp, 128, 0, st>>>(s->N, s->h, P, half, l1, l2, carry, S);
-    for (int k = 0; k < 5; ++k) counted();
+    for (int k = level; k < level + levels; ++k, half += (size_t)s->h * s->N) {
+      const T* rd = L.row_factors + (size_t)k * 3 * fac;
+      const T *l1 = rd + fac, *l2 = rd + 2 * fac;
+      const T* tf = L.row_transfer + (size_t)k * 8 * plane;
+      const T* tb = tf + 4 * plane;
+      cplx<T>* part = L.row_state + (size_t)k * 4 * plane;
+      cplx<T>* carry = part + 2 * plane;
+      k_row_down_part<T><<<gp, 128, 0, st>>>(s->N, s->h, P, half, l1, l2, part, S);
+      k_row_carry<T><<<gq, 128, 0, st>>>(s->N, P, false, tf, part, carry, S);
+      k_row_down_final<T><<<gp, 128, 0, st>>>(s->N, s->h, P, half, rd, l1, l2, carry, part, S);
+      k_row_carry<T><<<gq, 128, 0, st>>>(s->N, P, true, tb, part, carry, S);
+      k_row_up_final<T><<<gp, 128, 0, st>>>(s->N, s->h, P, half, l1, l2, carry, S);
+      for (int q = 0; q < 5; ++q) counted();
+    }
     return;
   }
-  cols_fn<T>(ilog2(s->h), LogSeq{}, s->cols_fused)<<<g.cgrid, g.cthreads, g.csmem, st>>>(
+  cols_fn<T>(ilog2(s->h), LogSeq{}, s->cols_fused)<<<dim3(g.cgrid, levels), g.cthreads, g.csmem, st>>>(
       s->N, half, L.tab.tw_col, L.tab.omega, L.tab.omega2, L.tab.lx, L.tab.ly, (T)(1.0 / (s->dx * s->dx)), S, level);
   counted();
 }
@@ -2704,6 +2780,13 @@ static void launch_spectral(dt_flex* s, Lane<T>& L, const T* in, const T* wt, T*
   launch_rows_inv<T>(s, L, inv_mode, half, out, wt, inv_mode == INV_STORE_DOT ? in : nullptr, g, S, st);
 }
 
+// Whether the bank's levels share a launch a pass: where each pass is one kernel (the power-of-two
+// transforms, and along y the cosine transform or k_row_solve).
+template <class T>
+static bool bank_batched(const dt_flex* s) {
+  return s->bank_one_launch && !s->any && !(s->row_solve && row_groups<T>(s->h) < 0);
+}
+
 // z = M^-1 r with r.z and max|z| reduced into S (finish_precond). levels 1: one spectral solve at
 // node_d[0]; levels 3: the reference's bank inside damped Jacobi sweeps (flexure.rs:1630-1651).
 template <class T>
@@ -2718,14 +2801,12 @@ static void launch_precondition(dt_flex* s, Lane<T>& L, const T* r, T* z, int le
   // (their spectra and weights are consecutive); otherwise levels 1 and 2 run on side streams
   // (parallel branches when captured into the loop graph). One inverse pass then takes the
   // three spectra to the weighted sum.
-  if (s->bank_one_launch && !s->any && !s->row_solve) {
+  if (bank_batched<T>(s)) {
     FftGeo g = fft_geometry<T>(s);
     rows_fwd_fn<T, true>(ilog2(s->N), LogSeq{})<<<dim3(g.rgrid, 3), g.rthreads, g.rsmem, st>>>(
         s->w, s->h, L.left, L.wt[0], L.half, L.tab.tw_row, L.tab.post, L.S);
     counted();
-    cols_fn<T>(ilog2(s->h), LogSeq{}, s->cols_fused)<<<dim3(g.cgrid, 3), g.cthreads, g.csmem, st>>>(
-        s->N, L.half, L.tab.tw_col, L.tab.omega, L.tab.omega2, L.tab.lx, L.tab.ly, (T)(1.0 / (s->dx * s->dx)), L.S, 0);
-    counted();
+    launch_cols<T>(s, L, L.half, g, 0, L.S, st, 3);
     launch_rows_inv<T>(s, L, INV_BANK, L.half, L.part, L.wt[0], nullptr, g, L.S, st);
     launch_apply<T>(s, JAC_FINAL, nullptr, L.J, L.part, L.d, L.c, r, z, L.S, st);  // z = u + J(r - A u)
     return;
@@ -2888,19 +2969,19 @@ static dt_status setup_precond(dt_flex* s, Lane<T>& L, int precond, int* levels)
     counted();
   }
   if (s->row_solve) {
-    // the row solve's factors of each level (its d, the bank's c_ref)
-    const size_t fac = (size_t)s->h * (s->N + 1);
-    for (int k = 0; k < lv; ++k) {
-      T* dd = L.row_factors + (size_t)k * 3 * fac;
-      k_row_factor<T><<<ceil_div(s->N + 1, 128), 128, 0, st>>>(s->N, s->h, L.tab.lx, metric_a<T>(s), metric_b<T>(s),
-                                                             (T)(1.0 / (s->dx * s->dx)), L.S, k, dd, dd + fac, dd + 2 * fac);
-      counted();
+    // the row solve's factors of the levels (their d, the bank's c_ref)
+    k_row_factor<T><<<dim3(ceil_div(s->N + 1, 64), lv), 64, 0, st>>>(s->N, s->h, L.tab.lx, metric_a<T>(s), metric_b<T>(s),
+                                                                     (T)(1.0 / (s->dx * s->dx)), L.S, L.row_factors);
+    counted();
+    if (row_groups<T>(s->h) < 0) {
+      // the chunks' carry transfers, from the factors alone
+      const size_t fac = (size_t)s->h * (s->N + 1);
       const int P = (int)ceil_div(s->h, ROW_CHUNK);
-      if (P > 1) {
-        // the chunks' carry transfers, from the factors alone
-        const size_t plane = (size_t)P * (s->N + 1);
+      const size_t plane = (size_t)P * (s->N + 1);
+      for (int k = 0; k < lv; ++k) {
+        const T* l1 = L.row_factors + (size_t)k * 3 * fac + fac;
         T* tf = L.row_transfer + (size_t)k * 8 * plane;
-        k_row_transfer<T><<<ceil_div(plane, 128), 128, 0, st>>>(s->N, s->h, P, dd + fac, dd + 2 * fac, tf, tf + 4 * plane);
+        k_row_transfer<T><<<ceil_div(plane, 128), 128, 0, st>>>(s->N, s->h, P, l1, l1 + fac, tf, tf + 4 * plane);
         counted();
       }
     }
@@ -3789,7 +3870,7 @@ static dt_status profile_lane(dt_flex* s, Lane<T>& L, int reps, double* ms, doub
   };
   // the bank's column passes and weighted forward row passes as the solve launches them: the
   // three levels in one launch (each level's bytes again) where it does so
-  const bool bank1 = s->bank_one_launch && !s->any && !s->row_solve;
+  const bool bank1 = bank_batched<T>(s);
   const double bank_levels = bank1 ? 3.0 : 1.0;
   cudaEvent_t a, b;
   DT_CUDA(cudaEventCreate(&a));
@@ -3805,13 +3886,7 @@ static dt_status profile_lane(dt_flex* s, Lane<T>& L, int reps, double* ms, doub
         case 2: k_direction<T><<<ew_grid(s), 256, 0, st>>>(s->n, L.p, L.z, L.S); break;
         case 3: launch_rows_fwd<T>(s, L, L.r, nullptr, L.half, g, L.S, st); break;
         case 4:
-          if (bank1) {
-            cols_fn<T>(ilog2(s->h), LogSeq{}, s->cols_fused)<<<dim3(g.cgrid, 3), g.cthreads, g.csmem, st>>>(
-                s->N, L.half, L.tab.tw_col, L.tab.omega, L.tab.omega2, L.tab.lx, L.tab.ly, (T)(1.0 / (s->dx * s->dx)), L.S, 0);
-            counted();
-          } else {
-            launch_cols<T>(s, L, L.half, g, 0, L.S, st);
-          }
+          launch_cols<T>(s, L, L.half, g, 0, L.S, st, bank1 ? 3 : 1);
           break;
         case 5: launch_rows_inv<T>(s, L, INV_STORE_DOT, L.half, L.z, nullptr, L.r, g, L.S, st); break;
         case 6: launch_apply<T>(s, JAC_LEFT, nullptr, L.J, nullptr, L.d, L.c, L.r, L.left, L.S, st); break;
