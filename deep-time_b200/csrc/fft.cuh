@@ -281,9 +281,10 @@ struct StagesAdj {
   }
 };
 
-// The radix the stages above give a length-2^LOGN transform's last stage.
-__host__ __device__ constexpr int last_radix(int logn) {
-  return logn % 4 == 0 ? 16 : (1 << (logn % 4));
+// The radix the stages above give a length-2^LOGN transform's last stage (8 values a thread: radix
+// 8 while three factors of two remain).
+__host__ __device__ constexpr int last_radix(int logn, int ept = 16) {
+  return ept == 16 ? (logn % 4 == 0 ? 16 : (1 << (logn % 4))) : (logn % 3 == 0 ? 8 : (1 << (logn % 3)));
 }
 
 // Full transform of length 2^LOGN. The caller synchronises before (data in s) and may read s

@@ -618,7 +618,7 @@ __global__ void k_fill(size_t n, T* __restrict__ a, T v) {
 
 // reduce a.b (and max |b| when MAXB) into S->dot_out / S->max_out
 template <class T>
-__global__ void __launch_bounds__(256) k_dot(size_t n, const T* __restrict__ a, const T* __restrict__ b, double* partials, Scalars* S,
+__global__ void __launch_bounds__(256, 8) k_dot(size_t n, const T* __restrict__ a, const T* __restrict__ b, double* partials, Scalars* S,
                                              int site) {
   Acc<2> acc;
   acc.v[0] = 0.0;
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(256) k_dot(size_t n, const T* __restrict__ a, 
 // Preconditioner set-up (flexure.rs:1361-1401 and :1426-1460).
 
 template <class T>
-__global__ void __launch_bounds__(256) k_stats(size_t n, const T* __restrict__ d, const T* __restrict__ c, double dx, int mean_d,
+__global__ void __launch_bounds__(256, 6) k_stats(size_t n, const T* __restrict__ d, const T* __restrict__ c, double dx, int mean_d,
                                                double* partials, Scalars* S) {
   const double RHO_MANTLE = 3300.0;
   // ln(alpha) rises with d, so its extremes are those of the least and the greatest d: two
@@ -707,26 +707,33 @@ __global__ void __launch_bounds__(256) k_bank_weights(int w, int h, const T* __r
 // INV_BANK: the bank's three levels in one pass, out = sum_k wt_k x_k, the levels' spectra and
 // weights consecutive (half + k h N, wt + k w h)
 enum { INV_STORE = 0, INV_STORE_DOT = 2, INV_STORE_W = 3, INV_BANK = 4 };
-// Correctly rounded reciprocals (double: one division; float: the intrinsic).
-__device__ __forceinline__ double recip(double x) { return 1.0 / x; }
-__device__ __forceinline__ float recip(float x) { return __frcp_rn(x); }
-// Reciprocals with no slow-path call, for code that keeps many values in registers around them:
-// float, the hardware's approximate reciprocal (__fdividef, at most 2 ulp for |x| in
-// [2^-126, 2^126]); double, that estimate refined by two Newton-Raphson steps r <- r + r (1 - x r)
-// (each squares the relative error: 2^-22 -> 2^-44 -> 2^-88). Used for the spectral divisors
-// d lambda^2 + c_ref, which lie in (c_ref, 1e36) for any raster this solver takes.
-__device__ __forceinline__ float recip_fast(float x) { return __fdividef(1.0f, x); }
-__device__ __forceinline__ double recip_fast(double x) {
-  double r = (double)__fdividef(1.0f, (float)x);
+// Reciprocals of the spectral divisors d lambda^2 + c_ref, with no slow-path call: float, the
+// correctly rounded intrinsic; double, of a normal number m 2^e, the hardware's float estimate of 1 / m, m in [1, 2),
+// scaled by 2^-e in the exponent bits and refined by two Newton-Raphson steps r <- r + r (1 - x r)
+// (each squares the relative error: 2^-22 -> 2^-44 -> 2^-88, so the last rounding is what is left).
+__device__ __forceinline__ double recip(double x) {
+  const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
+  const double m = __hiloint2double(hi - (e << 20), __double2loint(x));
+  double r = (double)__fdividef(1.0f, (float)m);
+  r = __hiloint2double(__double2hiint(r) - (e << 20), __double2loint(r));
   r = fma(r, fma(-x, r, 1.0), r);
   return fma(r, fma(-x, r, 1.0), r);
 }
+__device__ __forceinline__ float recip(float x) { return __frcp_rn(x); }
+// float, the hardware's approximate reciprocal (__fdividef, at most 2 ulp for |x| in
+// [2^-126, 2^126]), for the divisors of the fused column pass, which lie in (c_ref, 1e36)
+__device__ __forceinline__ float recip_fast(float x) { return __fdividef(1.0f, x); }
 constexpr int FFT_EPT = 16;
+// Small rasters (transforms_small below) take half as many values a thread: twice the warps, one
+// more stage.
+constexpr int FFT_EPT_SMALL = 8;
+constexpr size_t SMALL_CELLS = 1u << 19;
+constexpr int FFT_SMALL_LOG = 10;  // the longest row or column transform with that form
 constexpr int FFT_BATCH = 8;  // global loads a thread of a transform kernel keeps in flight
 constexpr int FFT_MAX_THREADS = 512;
 
 // Rows per block so that a block has at least one warp.
-__host__ __device__ constexpr int rows_per_block(int logn) { return (32 * FFT_EPT >> logn) > 1 ? (32 * FFT_EPT >> logn) : 1; }
+__host__ __device__ constexpr int rows_per_block(int logn, int ept = FFT_EPT) { return (32 * ept >> logn) > 1 ? (32 * ept >> logn) : 1; }
 // Columns per block of the column pass: at least one warp, at most FFT_MAX_THREADS threads,
 // 100 KB of padded shared memory, 8 columns.
 // Column pitch of the column pass: the padded length rounded up to 4 (mod 16), so that the first
@@ -742,8 +749,14 @@ __host__ __device__ constexpr int cols_per_block(int logh, int elem) {
   while (cpb < 8 && cpb * 2 * h <= FFT_MAX_THREADS * FFT_EPT && cpb * 2 * plen * elem <= 102400) cpb *= 2;
   return cpb;
 }
+// The same for small rasters: as few columns as make a row's segment a whole 32-byte sector and a
+// block a warp, so that the blocks reach more SMs (512 x 256 in FP64: 128 blocks instead of 32).
+__host__ __device__ constexpr int cols_per_block_small(int logh, int elem) {
+  int cpb = (32 * FFT_EPT_SMALL >> logh) > 1 ? (32 * FFT_EPT_SMALL >> logh) : 1;
+  return cpb < 32 / elem ? 32 / elem : cpb;
+}
 
-template <class T, bool WEIGHT, int LOGN>
+template <class T, bool WEIGHT, int LOGN, int EPT = FFT_EPT>
 __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_rows_fwd(int w, int h, const T* __restrict__ v, const T* __restrict__ wt,
                                                              cplx<T>* __restrict__ half, const cplx<T>* __restrict__ tw,
                                                              const cplx<T>* __restrict__ post, const Scalars* S) {
@@ -754,19 +767,19 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
   C* s = reinterpret_cast<C*>(smem_raw);
   constexpr int N = 1 << LOGN, NP = P::len(N);
   constexpr int logN = LOGN;
-  constexpr int RB = rows_per_block(LOGN);
+  constexpr int RB = rows_per_block(LOGN, EPT);
   // the bank's levels in one launch: level blockIdx.y's weights and spectrum, both consecutive
   if (WEIGHT) wt += (size_t)blockIdx.y * (2 * N) * h;
   half += (size_t)blockIdx.y * h * N;
   const int row0 = blockIdx.x * RB;
   const int tid = threadIdx.x;
   // load rows as complex pairs (v[2n], v[2n+1]): one 2-wide vector load per pair. The block has
-  // NT threads (fft_geometry), FFT_EPT pairs each; loads go out in batches before the shared
+  // NT threads (fft_geometry), EPT pairs each; loads go out in batches before the shared
   // stores so that a thread keeps FFT_BATCH of them in flight.
-  constexpr int NT = RB * N / FFT_EPT;
-  static_assert(NT * FFT_EPT == RB * N, "rows: whole pairs per thread");
+  constexpr int NT = RB * N / EPT;
+  static_assert(NT * EPT == RB * N, "rows: whole pairs per thread");
   // the raster's width w is 2 N: row offsets use the compile-time 2 N
-  if constexpr (RB == 1 && LOGN >= 4) {
+  if constexpr (EPT == 16 && RB == 1 && LOGN >= 4) {
     // one row per block: the first stage (radix 16, span 1) straight from global memory, thread
     // j taking pairs n = j + r N/16 (consecutive threads, consecutive pairs)
     const int j = tid;
@@ -788,10 +801,10 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
 #pragma unroll
     for (int r = 0; r < 16; ++r) s[17 * j + r] = z[r];  // pad(16 j + r) = 17 j + r
     __syncthreads();
-    Stages<C, FFT_EPT, false, LOGN, 16, LOGN - 4, 0, NT>::run(s, tw);
+    Stages<C, EPT, false, LOGN, 16, LOGN - 4, 0, NT>::run(s, tw);
   } else {
 #pragma unroll 1
-    for (int q0 = 0; q0 < FFT_EPT; q0 += FFT_BATCH) {
+    for (int q0 = 0; q0 < EPT; q0 += FFT_BATCH) {
       C zb[FFT_BATCH];
 #pragma unroll
       for (int u = 0; u < FFT_BATCH; ++u) {
@@ -817,21 +830,20 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
       }
     }
     __syncthreads();
-    smem_fft<C, FFT_EPT, false, LOGN, NT>(s, tw);
+    smem_fft<C, EPT, false, LOGN, NT>(s, tw);
   }
   // split: X[k] = E[k] + W^k O[k], E = (Z[k] + conj Z[N-k]) / 2, O = (Z[k] - conj Z[N-k]) / 2i
-  constexpr int half_n = N / 2 + 1;
-#pragma unroll 2
-  for (int idx = tid; idx < RB * half_n; idx += NT) {
-    int rb = idx / half_n, kk = idx - rb * half_n;
+  // pairs (k, N - k), k = 0 .. N/2 - 1 (EPT / 2 a thread); k = 0's holds the entries 0 and N / 2
+  auto split = [&](int rb, int kk) {
     int j = row0 + rb;
-    if (j >= h) continue;
+    if (j >= h) return;
     const C* row = s + rb * NP;
     C* out = half + (size_t)j * N;
     if (kk == 0) {
       C z0 = row[0];
       out[0] = mk<C>(z0.x + z0.y, z0.x - z0.y);  // (X[0], X[N]) both real
-      continue;
+      if (N == 1) return;
+      kk = N / 2;
     }
     C zk = row[P::at(kk)], zn = row[P::at(N - kk)];
     C E = mk<C>((zk.x + zn.x) * (T)0.5, (zk.y - zn.y) * (T)0.5);
@@ -839,12 +851,21 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
     C wo = cmul(post[kk], O);
     out[kk] = cadd(E, wo);
     if (kk != N - kk) out[N - kk] = cconj(csub(E, wo));
+  };
+  if constexpr (N == 1) {
+    for (int rb = tid; rb < RB; rb += NT) split(rb, 0);
+  } else {
+#pragma unroll 2
+    for (int q = 0; q < EPT / 2; ++q) {
+      int idx = tid + q * NT;
+      split(idx >> (logN - 1), idx & (N / 2 - 1));
+    }
   }
 }
 
 // The column pass: DCT-II along y (Makhoul), divide by d lambda^2 + c_ref, inverse DCT.
 // lx[k] = 2 cos(2 pi k / w) - 2 for k = 0..N; ly[m] = 2 cos(pi m / h) - 2.
-template <class T, int LOGH>
+template <class T, int LOGH, int EPT = FFT_EPT>
 __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_cols(int N, cplx<T>* __restrict__ half, const cplx<T>* __restrict__ tw,
                                                          const cplx<T>* __restrict__ omega, const cplx<T>* __restrict__ omega2, const T* __restrict__ lx,
                                                          const T* __restrict__ ly, T inv_dx2, const Scalars* S, int level) {
@@ -855,7 +876,7 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_col
   C* s = reinterpret_cast<C*>(smem_raw);
   constexpr int h = 1 << LOGH;
   constexpr int HP = col_pitch(h);
-  constexpr int CPB = cols_per_block(LOGH, (int)sizeof(C));
+  constexpr int CPB = EPT == FFT_EPT ? cols_per_block(LOGH, (int)sizeof(C)) : cols_per_block_small(LOGH, (int)sizeof(C));
   constexpr int logc = CPB == 1 ? 0 : CPB == 2 ? 1 : CPB == 4 ? 2 : CPB == 8 ? 3 : CPB == 16 ? 4 : CPB == 32 ? 5 : CPB == 64 ? 6 : CPB == 128 ? 7 : 8;
   // the bank's levels in one launch: level + blockIdx.y, its spectrum consecutive
   half += (size_t)blockIdx.y * h * N;
@@ -863,14 +884,14 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_col
   const int k0 = blockIdx.x * CPB;
   const int tid = threadIdx.x;
   const T dref = (T)S->node_d[level], cref = (T)S->c_ref;
-  // NT threads (fft_geometry), FFT_EPT values each
-  constexpr int NT = CPB * h / FFT_EPT;
-  static_assert(NT * FFT_EPT == CPB * h, "columns: whole values per thread");
+  // NT threads (fft_geometry), EPT values each
+  constexpr int NT = CPB * h / EPT;
+  static_assert(NT * EPT == CPB * h, "columns: whole values per thread");
   // Makhoul's order: v[p] = x[2p] for p < h/2, x[2(h - 1 - p) + 1] after
-  if constexpr (LOGH < 4) {
-    // short columns: gather in Makhoul's order (consecutive threads: consecutive columns)
+  if constexpr (LOGH < 4 || EPT < 16) {
+    // short columns (and small rasters): gather in Makhoul's order (consecutive threads: consecutive columns)
 #pragma unroll 1
-    for (int q0 = 0; q0 < FFT_EPT; q0 += FFT_BATCH) {
+    for (int q0 = 0; q0 < EPT; q0 += FFT_BATCH) {
       C xb[FFT_BATCH];
 #pragma unroll
       for (int u = 0; u < FFT_BATCH; ++u) {
@@ -887,7 +908,7 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_col
       }
     }
     __syncthreads();
-    Stages<C, FFT_EPT, false, LOGH, 1, LOGH, HP, NT>::run(s, tw);
+    Stages<C, EPT, false, LOGH, 1, LOGH, HP, NT>::run(s, tw);
   } else {
     // The forward transform's first stage (radix 16, span 1) straight from global memory: thread
     // tid takes butterfly j = tid / CPB of column tid % CPB, i.e. v[j + r h/16], r = 0 .. 15; a
@@ -905,22 +926,18 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_col
 #pragma unroll
     for (int r = 0; r < 16; ++r) col[17 * j + r] = v[r];  // pad(16 j + r) = 17 j + r
     __syncthreads();
-    Stages<C, FFT_EPT, false, LOGH, 16, LOGH - 4, HP, NT>::run(s, tw);
+    Stages<C, EPT, false, LOGH, 16, LOGH - 4, HP, NT>::run(s, tw);
   }
   // per column and pair (m, h - m): C[m] = (w_m V[m] + i w_(h-m) V[h-m]) / 2, divide, and back
-  constexpr int half_h = h / 2 + 1;
-#pragma unroll 1
-  for (int idx = tid; idx < CPB * half_h; idx += NT) {
-    int cc = idx / half_h, m = idx - cc * half_h;
-    int k = k0 + cc;
-    if (k >= N) continue;
+  // divisors: column 0 is packed (real part k = 0, imaginary part k = N)
+  auto rden = [&](int kx, T lyv) {  // 1 / (d lambda^2 + c): one reciprocal per divisor, then products
+    T l = (lx[kx] + lyv) * inv_dx2;
+    return recip(dref * (l * l) + cref);
+  };
+  auto pair = [&](int cc, int m) {
+    const int k = k0 + cc;
+    if (k >= N) return;
     C* col = s + cc * HP;
-    // divisors: column 0 is packed (real part k = 0, imaginary part k = N)
-    // 1 / (d lambda^2 + c): one reciprocal per divisor, then products
-    auto rden = [&](int kx, T lyv) {
-      T l = (lx[kx] + lyv) * inv_dx2;
-      return recip(dref * (l * l) + cref);
-    };
     const T lym = ly[m];
     if (m == 0) {
       C v0 = col[0];
@@ -933,7 +950,7 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_col
         v0.y *= dd;
       }
       col[0] = v0;
-      continue;
+      return;
     }
     int mm = h - m;
     int pm = P::at(m), pn = P::at(mm);
@@ -961,6 +978,17 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_col
     C vn = cmul(cconj(wn), csub(cn, cmuli(cm)));
     col[pm] = vm;
     if (mm != m) col[pn] = vn;
+  };
+  if constexpr (h == 1) {
+    for (int cc = tid; cc < CPB; cc += NT) pair(cc, 0);
+  } else {
+    // m = 0 .. h/2 - 1, EPT / 2 a thread; the one with m = 0 takes h / 2 too
+#pragma unroll 1
+    for (int q = 0; q < EPT / 2; ++q) {
+      const int idx = tid + q * NT, cc = idx >> (LOGH - 1), m = idx & (h / 2 - 1);
+      pair(cc, m);
+      if (m == 0) pair(cc, h / 2);
+    }
   }
   __syncthreads();
   // the same table through a pointer the compiler cannot prove equal to `tw`: otherwise it keeps
@@ -968,8 +996,8 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_col
   const C* tw_inv;
   asm volatile("mov.b64 %0, %1;" : "=l"(tw_inv) : "l"(tw));
   const T inv_h = (T)1 / (T)h;
-  if constexpr (LOGH < 4) {
-    Stages<C, FFT_EPT, true, LOGH, 1, LOGH, HP, NT>::run(s, tw_inv);
+  if constexpr (LOGH < 4 || EPT < 16) {
+    Stages<C, EPT, true, LOGH, 1, LOGH, HP, NT>::run(s, tw_inv);
 #pragma unroll 4
     for (int idx = tid; idx < CPB * h; idx += NT) {
       int j = idx >> logc, cc = idx & (CPB - 1);
@@ -985,7 +1013,7 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_col
     constexpr int RL = last_radix(LOGH);
     constexpr int LOGRL = RL == 16 ? 4 : RL == 8 ? 3 : RL == 4 ? 2 : 1;
     constexpr int NSL = h / RL;
-    Stages<C, FFT_EPT, true, LOGH, 1, LOGH - LOGRL, HP, NT>::run(s, tw_inv);
+    Stages<C, EPT, true, LOGH, 1, LOGH - LOGRL, HP, NT>::run(s, tw_inv);
 #pragma unroll
     for (int q = 0; q < FFT_EPT / RL; ++q) {
       const int u = tid + q * NT;
@@ -1243,13 +1271,6 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS / 2, 3) k_cols_fused(int N, cp
 // reciprocal (the reference's carried value l2 dd(j-2) l1 is m2 l1). With two divisions a row and a
 // launch a level it took 90 us a level at 513 wavenumbers x 328 rows (FP64), three in sequence.
 template <class T>
-__device__ __forceinline__ T row_recip(T x);
-template <>
-__device__ __forceinline__ float row_recip(float x) { return recip(x); }
-template <>
-__device__ __forceinline__ double row_recip(double x) { return recip_fast(x); }
-
-template <class T>
 __global__ void __launch_bounds__(64) k_row_factor(int N, int h, const T* __restrict__ lx, const T* __restrict__ ma,
                                                    const T* __restrict__ mb, T inv_dx2, const Scalars* S, T* __restrict__ fac) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1268,7 +1289,7 @@ __global__ void __launch_bounds__(64) k_row_factor(int N, int h, const T* __rest
     const T n1 = d * e1 * (t1 + tj) - m2 * l1p;  // 0 for j < 1
     const T p1 = n1 * r1, p2 = m2 * r2;
     const T dj = (d * (tj * tj + e1 * e1 + ej * ej) + c - p2 * m2) - p1 * n1;
-    const T rj = row_recip<T>(dj);
+    const T rj = recip(dj);
     fac[(size_t)j * stride] = rj;
     fac[plane + (size_t)j * stride] = p1;
     fac[2 * plane + (size_t)j * stride] = p2;
@@ -1601,7 +1622,7 @@ __global__ void __launch_bounds__(128) k_row_up_final(int N, int h, int P, cplx<
 
 // Inverse rows: Z[k] = E[k] + i O[k] with E = (X[k] + conj X[N-k]) / 2,
 // O = (X[k] - conj X[N-k]) conj(W^k) / 2; x = IFFT_N(Z) / N de-interleaved.
-template <class T, int MODE, int LOGN>
+template <class T, int MODE, int LOGN, int EPT = FFT_EPT>
 __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_rows_inv(int w, int h, const cplx<T>* __restrict__ half, T* __restrict__ out,
                                                              const T* __restrict__ wt, const T* __restrict__ r,
                                                              const cplx<T>* __restrict__ tw, const cplx<T>* __restrict__ post,
@@ -1616,11 +1637,10 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
   C* s = reinterpret_cast<C*>(smem_raw);
   constexpr int N = 1 << LOGN, NP = P::len(N);
   constexpr int logN = LOGN;
-  constexpr int RB = rows_per_block(LOGN);
+  constexpr int RB = rows_per_block(LOGN, EPT);
   const int row0 = blockIdx.x * RB;
   const int tid = threadIdx.x;
-  constexpr int half_n = N / 2 + 1;
-  constexpr int NT = RB * N / FFT_EPT;  // the block's threads (fft_geometry)
+  constexpr int NT = RB * N / EPT;  // the block's threads (fft_geometry)
   constexpr int IB = FFT_BATCH / 2;     // pairs (X[k], X[N-k]) loaded per batch
   constexpr int LEVELS = MODE == INV_BANK ? 3 : 1;
   const T inv_n = (T)1 / (T)N;
@@ -1634,48 +1654,45 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
   half = half0 + (size_t)lv * h * N;
   wt = wt0 + (size_t)lv * (2 * N) * h;
   if (lv > 0) __syncthreads();  // the previous level's last reads of s are done
+  // pairs (k, N - k), k = 0 .. N/2 - 1 (EPT / 2 a thread, IB loaded at a time); k = 0's holds the
+  // packed entry 0 and entry N / 2
 #pragma unroll 1
-  for (int base = tid; base < RB * half_n; base += IB * NT) {
+  for (int q0 = 0; q0 < (N == 1 ? EPT : EPT / 2); q0 += IB) {
     C xkb[IB], xnb[IB];
 #pragma unroll
     for (int u = 0; u < IB; ++u) {
-      int idx = base + u * NT;
-      int rb = idx / half_n, kk = idx - rb * half_n;
+      int idx = tid + (q0 + u) * NT;
+      int rb = N == 1 ? idx : idx >> (N == 1 ? 0 : LOGN - 1), kk = N == 1 ? 0 : idx & (N / 2 - 1);
       int j = row0 + rb;
       xkb[u] = xnb[u] = mk<C>((T)0, (T)0);
-      if (idx < RB * half_n && j < h) {
+      if (j < h) {
         const C* in = half + (size_t)j * N;
         xkb[u] = in[kk];
-        if (kk > 0) xnb[u] = in[N - kk];
+        xnb[u] = kk > 0 ? in[N - kk] : in[N / 2];
       }
     }
 #pragma unroll
     for (int u = 0; u < IB; ++u) {
-    int idx = base + u * NT;
-    if (idx >= RB * half_n) break;
-    int rb = idx / half_n, kk = idx - rb * half_n;
-    int j = row0 + rb;
-    C* row = s + rb * NP;
-    if (j >= h) {
-      row[P::at(kk)] = mk<C>((T)0, (T)0);
-      if (kk > 0 && kk < N) row[P::at(N - kk)] = mk<C>((T)0, (T)0);
-      continue;
-    }
-    if (kk == 0) {
-      C p = xkb[u];  // (X[0], X[N])
-      row[0] = mk<C>((p.x + p.y) * (T)0.5, (p.x - p.y) * (T)0.5);
-      continue;
-    }
-    C xk = xkb[u], xn = xnb[u];
-    C E = mk<C>((xk.x + xn.x) * (T)0.5, (xk.y - xn.y) * (T)0.5);
-    C D = mk<C>((xk.x - xn.x) * (T)0.5, (xk.y + xn.y) * (T)0.5);
-    C O = cmul(D, cconj(post[kk]));
-    row[P::at(kk)] = cadd(E, cmuli(O));
-    if (kk != N - kk) {
-      // index N - kk: E' = conj E, D' = -conj D, conj(W^(N-k)) = -W^k  =>  O' = conj(D) W^k
-      C O2 = cmul(cconj(D), post[kk]);
-      row[P::at(N - kk)] = cadd(cconj(E), cmuli(O2));
-    }
+      int idx = tid + (q0 + u) * NT;
+      int rb = N == 1 ? idx : idx >> (N == 1 ? 0 : LOGN - 1), kk = N == 1 ? 0 : idx & (N / 2 - 1);
+      C* row = s + rb * NP;
+      C xk = xkb[u], xn = xnb[u];  // zeros past the last row: their transforms are not stored
+      if (kk == 0) {
+        row[0] = mk<C>((xk.x + xk.y) * (T)0.5, (xk.x - xk.y) * (T)0.5);  // (X[0], X[N])
+        if (N == 1) continue;
+        xk = xn;
+        kk = N / 2;
+      }
+      C E = mk<C>((xk.x + xn.x) * (T)0.5, (xk.y - xn.y) * (T)0.5);
+      C D = mk<C>((xk.x - xn.x) * (T)0.5, (xk.y + xn.y) * (T)0.5);
+      C pk = post[kk];
+      C O = cmul(D, cconj(pk));
+      row[P::at(kk)] = cadd(E, cmuli(O));
+      if (kk != N - kk) {
+        // index N - kk: E' = conj E, D' = -conj D, conj(W^(N-k)) = -W^k  =>  O' = conj(D) W^k
+        C O2 = cmul(cconj(D), pk);
+        row[P::at(N - kk)] = cadd(cconj(E), cmuli(O2));
+      }
     }
   }
   __syncthreads();
@@ -1703,12 +1720,12 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
   if constexpr (RB == 1 && LOGN >= 4) {
     // one row per block: all stages but the last through shared memory; the last (radix RL,
     // span N / RL, twiddles w^(r j)) hands each output to the mode's epilogue
-    constexpr int RL = last_radix(LOGN);
+    constexpr int RL = last_radix(LOGN, EPT);
     constexpr int LOGRL = RL == 16 ? 4 : RL == 8 ? 3 : RL == 4 ? 2 : 1;
     constexpr int NSL = N / RL;
-    Stages<C, FFT_EPT, true, LOGN, 1, LOGN - LOGRL, 0, NT>::run(s, tw);
+    Stages<C, EPT, true, LOGN, 1, LOGN - LOGRL, 0, NT>::run(s, tw);
 #pragma unroll
-    for (int q = 0; q < FFT_EPT / RL; ++q) {
+    for (int q = 0; q < EPT / RL; ++q) {
       const int j = tid + q * NT;
       C z[RL];
 #pragma unroll
@@ -1726,7 +1743,7 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
       }
     }
   } else {
-    smem_fft<C, FFT_EPT, true, LOGN, NT>(s, tw);
+    smem_fft<C, EPT, true, LOGN, NT>(s, tw);
 #pragma unroll 4
     for (int idx = tid; idx < RB * N; idx += NT) {
       int rb = idx >> logN, nn = idx & (N - 1);
@@ -1739,6 +1756,80 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS, sizeof(T) == 4 ? 2 : 1) k_row
   if (MODE == INV_STORE_DOT) {
     const int kind[2] = {0, 1};
     if (reduce_partials<2>(acc, kind, partials, &S->ticket[SITE_PRECOND], gridDim.x) && tid == 0) finish_precond(S, acc.v[0], acc.v[1]);
+  }
+}
+
+// k_rows_inv's INV_BANK for small rasters: the three levels of a block's rows side by side
+// (threadIdx.y the level) instead of one after another, then their weighted sum from shared memory
+// in the same order. The weights are loaded before the transforms, so that a block waits for
+// memory once. Bound by latency: FP64 1024 x 328 took 16.6 us with the levels in sequence, and
+// 512 x 256 (whose rows had half a warp each) 42 us.
+template <class T, int LOGN>
+__global__ void __launch_bounds__(3 * (rows_per_block(LOGN, FFT_EPT_SMALL) << LOGN) / FFT_EPT_SMALL)
+    k_rows_inv_levels(int h, const cplx<T>* __restrict__ half, T* __restrict__ out, const T* __restrict__ wt,
+                      const cplx<T>* __restrict__ tw, const cplx<T>* __restrict__ post, const Scalars* S) {
+  using C = cplx<T>;
+  using P = Pad<C>;
+  if (S->stop) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int EPT = FFT_EPT_SMALL, N = 1 << LOGN, NP = P::len(N), RB = rows_per_block(LOGN, EPT), NT = RB * N / EPT;
+  constexpr int EACH = (RB * N + 3 * NT - 1) / (3 * NT);  // outputs a thread
+  C* const s0 = reinterpret_cast<C*>(smem_raw);
+  C* s = s0 + threadIdx.y * (RB * NP);
+  const int row0 = blockIdx.x * RB, tid = threadIdx.x, flat = threadIdx.y * NT + tid;
+  const size_t plane = (size_t)(2 * N) * h;
+  C xk[EPT / 2], xn[EPT / 2], ww[EACH][3];
+#pragma unroll
+  for (int u = 0; u < EPT / 2; ++u) {
+    const int idx = tid + u * NT, rb = idx >> (LOGN - 1), kk = idx & (N / 2 - 1), j = row0 + rb;
+    xk[u] = xn[u] = mk<C>((T)0, (T)0);
+    if (j < h) {
+      const C* in = half + ((size_t)threadIdx.y * h + j) * N;
+      xk[u] = in[kk];
+      xn[u] = kk > 0 ? in[N - kk] : in[N / 2];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < EACH; ++e) {
+    const int idx = flat + e * 3 * NT, j = row0 + (idx >> LOGN);
+    if (idx < RB * N && j < h) {
+      const T* at = wt + (size_t)j * (2 * N) + 2 * (idx & (N - 1));
+#pragma unroll
+      for (int l = 0; l < 3; ++l) ww[e][l] = *reinterpret_cast<const C*>(at + l * plane);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < EPT / 2; ++u) {
+    const int idx = tid + u * NT;
+    int kk = idx & (N / 2 - 1);
+    C* row = s + (idx >> (LOGN - 1)) * NP;
+    C a = xk[u];
+    const C b = xn[u];
+    if (kk == 0) {
+      row[0] = mk<C>((a.x + a.y) * (T)0.5, (a.x - a.y) * (T)0.5);  // (X[0], X[N])
+      a = b;
+      kk = N / 2;
+    }
+    const C E = mk<C>((a.x + b.x) * (T)0.5, (a.y - b.y) * (T)0.5);
+    const C D = mk<C>((a.x - b.x) * (T)0.5, (a.y + b.y) * (T)0.5);
+    const C pk = post[kk];
+    row[P::at(kk)] = cadd(E, cmuli(cmul(D, cconj(pk))));
+    if (kk != N - kk) row[P::at(N - kk)] = cadd(cconj(E), cmuli(cmul(cconj(D), pk)));
+  }
+  __syncthreads();
+  smem_fft<C, EPT, true, LOGN, NT>(s, tw);
+  const T inv_n = (T)1 / (T)N;
+#pragma unroll
+  for (int e = 0; e < EACH; ++e) {
+    const int idx = flat + e * 3 * NT, rb = idx >> LOGN, nn = idx & (N - 1), j = row0 + rb;
+    if (idx >= RB * N || j >= h) continue;
+    C acc;
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+      const C z = cscale(s0[l * (RB * NP) + rb * NP + P::at(nn)], inv_n), wl = ww[e][l];
+      acc = l == 0 ? mk<C>(z.x * wl.x, z.y * wl.y) : mk<C>(acc.x + z.x * wl.x, acc.y + z.y * wl.y);
+    }
+    *reinterpret_cast<C*>(out + (size_t)j * (2 * N) + 2 * nn) = acc;
   }
 }
 
@@ -2347,6 +2438,11 @@ const double* metric_b<double>(const dt_flex* s) { return s->met_b64; }
 template <>
 const float* metric_b<float>(const dt_flex* s) { return s->met_b32; }
 
+// The vector kernels' grid: a 16-byte word a thread, up to eight blocks an SM
+template <class T>
+static unsigned int vec_grid(const dt_flex* s) {
+  return std::max(1u, std::min<unsigned int>(ceil_div(s->n, 256 * (16 / sizeof(T))), (unsigned)s->sms * 8));
+}
 static unsigned int ew_grid(const dt_flex* s) { return std::max(1u, std::min<unsigned int>(ceil_div(s->n, 256), (unsigned)s->sms * 8)); }
 
 // ---- the TMA stencil's host side ----
@@ -2499,20 +2595,41 @@ struct FftGeo {
   unsigned int rgrid, cgrid;
   int rthreads, cthreads;
   size_t rsmem, csmem;
+  bool rsmall, csmall;
 };
+// Whether the row passes (the column pass) take the small-raster form, FFT_EPT_SMALL values a thread:
+// half the values, so twice the warps a row, and column blocks of a sector's width. Up to 2^19 cells,
+// where a pass is bound by the latency of too few warps: FP64 512 x 256 with the L2 flushed, columns
+// 18.4 -> 14.3 us, inverse rows with r.z 21.3 -> 14.9, the bank's 38.8 -> 10.2; FP64 1024 x 512 column
+// passes of three levels 29.0 -> 29.3, the bank's inverse rows 21.7 -> 20.5. Beyond it the extra stage costs
+// more: at 1024 x 1024 41.8 -> 54.1 and 26.5 -> 28.7.
+template <class T>
+static bool rows_small(const dt_flex* s) {
+  return !s->any && s->N >= 4 && ilog2(s->N) <= FFT_SMALL_LOG && s->n <= SMALL_CELLS;
+}
+template <class T>
+static bool cols_small(const dt_flex* s) {
+  const int logh = ilog2(s->h);
+  return !s->row_solve && logh >= 4 && logh <= FFT_SMALL_LOG && s->n <= SMALL_CELLS;
+}
 template <class T>
 static FftGeo fft_geometry(const dt_flex* s) {
   using C = cplx<T>;
   FftGeo g;
   int logn = ilog2(s->N), logh = ilog2(s->h);
-  int N = s->N, RB = rows_per_block(logn);
+  g.rsmall = rows_small<T>(s);
+  g.csmall = cols_small<T>(s);
+  const int rept = g.rsmall ? FFT_EPT_SMALL : FFT_EPT, cept = g.csmall ? FFT_EPT_SMALL : FFT_EPT;
+  int N = s->N, RB = rows_per_block(logn, rept);
   g.rgrid = ceil_div(s->h, RB);
-  g.rthreads = std::max(1, RB * N / FFT_EPT);
+  g.rthreads = std::max(1, RB * N / rept);
   g.rsmem = (size_t)RB * Pad<C>::len(N) * sizeof(C);
-  const bool fused = s->cols_fused && cols_fusable<T>(logh);
-  int cpb = fused ? cols_per_block_fused(logh, (int)sizeof(C)) : cols_per_block(logh, (int)sizeof(C));
+  const bool fused = !g.csmall && s->cols_fused && cols_fusable<T>(logh);
+  int cpb = g.csmall ? cols_per_block_small(logh, (int)sizeof(C))
+            : fused  ? cols_per_block_fused(logh, (int)sizeof(C))
+                     : cols_per_block(logh, (int)sizeof(C));
   g.cgrid = ceil_div(N, cpb);
-  g.cthreads = std::max(1, cpb * s->h / FFT_EPT);
+  g.cthreads = std::max(1, cpb * s->h / cept);
   g.csmem = (size_t)cpb * (fused ? col_pitch_fused(s->h, cpb) : col_pitch(s->h)) * sizeof(C);
   return g;
 }
@@ -2527,10 +2644,32 @@ using ColsFn = void (*)(int, cplx<T>*, const cplx<T>*, const cplx<T>*, const cpl
 template <class T>
 using RowsInvFn = void (*)(int, int, const cplx<T>*, T*, const T*, const T*, const cplx<T>*, const cplx<T>*, double*, Scalars*);
 
+// the small-raster instantiations, for the lengths that have them
+template <class T, bool W, int L>
+static constexpr RowsFwdFn<T, W> rows_fwd_small() {
+  if constexpr (L >= 2 && L <= FFT_SMALL_LOG)
+    return &k_rows_fwd<T, W, L, FFT_EPT_SMALL>;
+  else
+    return nullptr;
+}
+template <class T, int L>
+static constexpr ColsFn<T> cols_small_kernel() {
+  if constexpr (L >= 4 && L <= FFT_SMALL_LOG)
+    return &k_cols<T, L, FFT_EPT_SMALL>;
+  else
+    return nullptr;
+}
+template <class T, int MODE, int L>
+static constexpr RowsInvFn<T> rows_inv_small() {
+  if constexpr (L >= 2 && L <= FFT_SMALL_LOG && MODE != INV_BANK)
+    return &k_rows_inv<T, MODE, L, FFT_EPT_SMALL>;
+  else
+    return nullptr;
+}
 template <class T, bool W, int... L>
-static RowsFwdFn<T, W> rows_fwd_fn(int logn, std::integer_sequence<int, L...>) {
-  static const RowsFwdFn<T, W> table[] = {&k_rows_fwd<T, W, L>...};
-  return table[logn];
+static RowsFwdFn<T, W> rows_fwd_fn(int logn, std::integer_sequence<int, L...>, bool small = false) {
+  static const RowsFwdFn<T, W> table[2][sizeof...(L)] = {{&k_rows_fwd<T, W, L>...}, {rows_fwd_small<T, W, L>()...}};
+  return table[small ? 1 : 0][logn];
 }
 // The column kernel for length 2^L: the fused form when its last radix is below 16 (and
 // `fused`), else k_cols.
@@ -2542,14 +2681,15 @@ static constexpr ColsFn<T> cols_kernel(bool fused) {
     return &k_cols<T, L>;
 }
 template <class T, int... L>
-static ColsFn<T> cols_fn(int logh, std::integer_sequence<int, L...>, bool fused = true) {
-  static const ColsFn<T> table[2][sizeof...(L)] = {{cols_kernel<T, L>(false)...}, {cols_kernel<T, L>(true)...}};
-  return table[fused ? 1 : 0][logh];
+static ColsFn<T> cols_fn(int logh, std::integer_sequence<int, L...>, bool fused = true, bool small = false) {
+  static const ColsFn<T> table[3][sizeof...(L)] = {
+      {cols_kernel<T, L>(false)...}, {cols_kernel<T, L>(true)...}, {cols_small_kernel<T, L>()...}};
+  return table[small ? 2 : fused ? 1 : 0][logh];
 }
 template <class T, int MODE, int... L>
-static RowsInvFn<T> rows_inv_fn(int logn, std::integer_sequence<int, L...>) {
-  static const RowsInvFn<T> table[] = {&k_rows_inv<T, MODE, L>...};
-  return table[logn];
+static RowsInvFn<T> rows_inv_fn(int logn, std::integer_sequence<int, L...>, bool small) {
+  static const RowsInvFn<T> table[2][sizeof...(L)] = {{&k_rows_inv<T, MODE, L>...}, {rows_inv_small<T, MODE, L>()...}};
+  return table[small ? 1 : 0][logn];
 }
 using LogSeq = std::make_integer_sequence<int, FFT_LOGS>;
 template <class T>
@@ -2569,13 +2709,28 @@ static RowsBankFn<T> rows_bank_fn(int logn, std::integer_sequence<int, L...>) {
   return table[logn];
 }
 template <class T>
-static RowsInvFn<T> rows_inv_for(int mode, int logn) {
+static RowsInvFn<T> rows_inv_for(int mode, int logn, bool small = false) {
   switch (mode) {
-    case INV_STORE: return rows_inv_fn<T, INV_STORE>(logn, LogSeq{});
-    case INV_STORE_W: return rows_inv_fn<T, INV_STORE_W>(logn, LogSeq{});
-    case INV_BANK: return rows_inv_fn<T, INV_BANK>(logn, LogSeq{});
-    default: return rows_inv_fn<T, INV_STORE_DOT>(logn, LogSeq{});
+    case INV_STORE: return rows_inv_fn<T, INV_STORE>(logn, LogSeq{}, small);
+    case INV_STORE_W: return rows_inv_fn<T, INV_STORE_W>(logn, LogSeq{}, small);
+    case INV_BANK: return rows_inv_fn<T, INV_BANK>(logn, LogSeq{}, small);
+    default: return rows_inv_fn<T, INV_STORE_DOT>(logn, LogSeq{}, small);
   }
+}
+// the bank's inverse rows with its levels side by side, for small rasters
+template <class T>
+using RowsLevelsFn = void (*)(int, const cplx<T>*, T*, const T*, const cplx<T>*, const cplx<T>*, const Scalars*);
+template <class T, int L>
+static constexpr RowsLevelsFn<T> rows_levels_kernel() {
+  if constexpr (L >= 2 && L <= FFT_SMALL_LOG)
+    return &k_rows_inv_levels<T, L>;
+  else
+    return nullptr;
+}
+template <class T, int... L>
+static RowsLevelsFn<T> rows_levels_fn(int logn, std::integer_sequence<int, L...>) {
+  static const RowsLevelsFn<T> table[] = {rows_levels_kernel<T, L>()...};
+  return table[logn];
 }
 
 // Opt every transform instantiation in to large dynamic shared memory.
@@ -2590,6 +2745,8 @@ static void transform_smem_attributes() {
     cudaFuncSetAttribute(cols_fn<T>(l, LogSeq{}, true), cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     for (int m : {INV_STORE, INV_STORE_W, INV_STORE_DOT, INV_BANK})
       cudaFuncSetAttribute(rows_inv_for<T>(m, l), cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    if (RowsLevelsFn<T> f = rows_levels_fn<T>(l, LogSeq{}))
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (RowsBankFn<T> f = rows_bank_fn<T>(l, LogSeq{}))
       cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_bank_smem<T>(l));
   }
@@ -2694,10 +2851,10 @@ static void launch_rows_fwd(dt_flex* s, Lane<T>& L, const T* in, const T* wt, cp
   }
   int logn = ilog2(s->N);
   if (wt)
-    rows_fwd_fn<T, true>(logn, LogSeq{})<<<g.rgrid, g.rthreads, g.rsmem, st>>>(s->w, s->h, in, wt, half, L.tab.tw_row,
+    rows_fwd_fn<T, true>(logn, LogSeq{}, g.rsmall)<<<g.rgrid, g.rthreads, g.rsmem, st>>>(s->w, s->h, in, wt, half, L.tab.tw_row,
                                                                                   L.tab.post, S);
   else
-    rows_fwd_fn<T, false>(logn, LogSeq{})<<<g.rgrid, g.rthreads, g.rsmem, st>>>(s->w, s->h, in, wt, half, L.tab.tw_row,
+    rows_fwd_fn<T, false>(logn, LogSeq{}, g.rsmall)<<<g.rgrid, g.rthreads, g.rsmem, st>>>(s->w, s->h, in, wt, half, L.tab.tw_row,
                                                                                    L.tab.post, S);
   counted();
 }
@@ -2736,7 +2893,7 @@ static void launch_cols(dt_flex* s, Lane<T>& L, cplx<T>* half, const FftGeo& g, 
     }
     return;
   }
-  cols_fn<T>(ilog2(s->h), LogSeq{}, s->cols_fused)<<<dim3(g.cgrid, levels), g.cthreads, g.csmem, st>>>(
+  cols_fn<T>(ilog2(s->h), LogSeq{}, s->cols_fused, g.csmall)<<<dim3(g.cgrid, levels), g.cthreads, g.csmem, st>>>(
       s->N, half, L.tab.tw_col, L.tab.omega, L.tab.omega2, L.tab.lx, L.tab.ly, (T)(1.0 / (s->dx * s->dx)), S, level);
   counted();
 }
@@ -2748,6 +2905,12 @@ static void launch_rows_inv(dt_flex* s, Lane<T>& L, int mode, const cplx<T>* hal
     return;
   }
   const int logn = ilog2(s->N);
+  if (mode == INV_BANK && g.rsmall) {
+    rows_levels_fn<T>(logn, LogSeq{})<<<g.rgrid, dim3(g.rthreads, 3), 3 * g.rsmem, st>>>(s->h, half, out, wt, L.tab.tw_row,
+                                                                                        L.tab.post, S);
+    counted();
+    return;
+  }
   if (mode == INV_BANK && s->rows_bank) {
     if (RowsBankFn<T> f = rows_bank_fn<T>(logn, LogSeq{})) {
       // persistent: as many blocks as the SMs hold at once, at most one a row
@@ -2763,7 +2926,7 @@ static void launch_rows_inv(dt_flex* s, Lane<T>& L, int mode, const cplx<T>* hal
       return;
     }
   }
-  rows_inv_for<T>(mode, logn)<<<g.rgrid, g.rthreads, g.rsmem, st>>>(s->w, s->h, half, out, wt, r, L.tab.tw_row,
+  rows_inv_for<T>(mode, logn, g.rsmall)<<<g.rgrid, g.rthreads, g.rsmem, st>>>(s->w, s->h, half, out, wt, r, L.tab.tw_row,
                                                                     L.tab.post, s->partials, S);
   counted();
 }
@@ -2803,7 +2966,7 @@ static void launch_precondition(dt_flex* s, Lane<T>& L, const T* r, T* z, int le
   // three spectra to the weighted sum.
   if (bank_batched<T>(s)) {
     FftGeo g = fft_geometry<T>(s);
-    rows_fwd_fn<T, true>(ilog2(s->N), LogSeq{})<<<dim3(g.rgrid, 3), g.rthreads, g.rsmem, st>>>(
+    rows_fwd_fn<T, true>(ilog2(s->N), LogSeq{}, g.rsmall)<<<dim3(g.rgrid, 3), g.rthreads, g.rsmem, st>>>(
         s->w, s->h, L.left, L.wt[0], L.half, L.tab.tw_row, L.tab.post, L.S);
     counted();
     launch_cols<T>(s, L, L.half, g, 0, L.S, st, 3);
@@ -2884,7 +3047,7 @@ template <class T>
 static dt_status launch_iteration(dt_flex* s, Lane<T>& L, int levels, cudaStream_t st, bool reliable = false,
                                   cudaStream_t aside = nullptr, unsigned long long* if_handle = nullptr) {
   launch_apply<T>(s, AP_DOT, L.p, nullptr, nullptr, L.d, L.c, nullptr, L.ap, L.S, st);
-  k_update<T><<<ew_grid(s), 256, 0, st>>>(s->n, L.x, L.r, L.p, L.ap, s->partials, L.S); counted();
+  k_update<T><<<vec_grid<T>(s), 256, 0, st>>>(s->n, L.x, L.r, L.p, L.ap, s->partials, L.S); counted();
   if constexpr (sizeof(T) == 4) {
     if (reliable) {
       if (aside) {
@@ -2895,7 +3058,7 @@ static dt_status launch_iteration(dt_flex* s, Lane<T>& L, int levels, cudaStream
     }
   }
   launch_precondition<T>(s, L, L.r, L.z, levels, st);
-  k_direction<T><<<ew_grid(s), 256, 0, st>>>(s->n, L.p, L.z, L.S); counted();
+  k_direction<T><<<vec_grid<T>(s), 256, 0, st>>>(s->n, L.p, L.z, L.S); counted();
   return DT_OK;
 }
 
@@ -3882,8 +4045,8 @@ static dt_status profile_lane(dt_flex* s, Lane<T>& L, int reps, double* ms, doub
       FftGeo g = fft_geometry<T>(s);
       switch (k) {
         case 0: launch_apply<T>(s, AP_DOT, L.p, nullptr, nullptr, L.d, L.c, nullptr, L.ap, L.S, st); break;
-        case 1: k_update<T><<<ew_grid(s), 256, 0, st>>>(s->n, L.x, L.r, L.p, L.ap, s->partials, L.S); break;
-        case 2: k_direction<T><<<ew_grid(s), 256, 0, st>>>(s->n, L.p, L.z, L.S); break;
+        case 1: k_update<T><<<vec_grid<T>(s), 256, 0, st>>>(s->n, L.x, L.r, L.p, L.ap, s->partials, L.S); break;
+        case 2: k_direction<T><<<vec_grid<T>(s), 256, 0, st>>>(s->n, L.p, L.z, L.S); break;
         case 3: launch_rows_fwd<T>(s, L, L.r, nullptr, L.half, g, L.S, st); break;
         case 4:
           launch_cols<T>(s, L, L.half, g, 0, L.S, st, bank1 ? 3 : 1);
@@ -3893,7 +4056,7 @@ static dt_status profile_lane(dt_flex* s, Lane<T>& L, int reps, double* ms, doub
         case 7: launch_apply<T>(s, JAC_FINAL, nullptr, L.J, L.part, L.d, L.c, L.r, L.z, L.S, st); break;
         case 8:
           if (bank1) {
-            rows_fwd_fn<T, true>(ilog2(s->N), LogSeq{})<<<dim3(g.rgrid, 3), g.rthreads, g.rsmem, st>>>(
+            rows_fwd_fn<T, true>(ilog2(s->N), LogSeq{}, g.rsmall)<<<dim3(g.rgrid, 3), g.rthreads, g.rsmem, st>>>(
                 s->w, s->h, L.left, L.wt[0], L.half, L.tab.tw_row, L.tab.post, L.S);
             counted();
           } else {
