@@ -708,177 +708,295 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_rb(MgChain<TM> g, int nu, in
   }
 }
 
-// Two red-black Gauss-Seidel sweeps (four colour passes) of a level in one launch, over tiles of
-// TX x TY cells staged in shared memory with a halo: pass p updates its colour on the tile and
-// the rings around it that the later passes read, so the tile's cells end with the values four
-// separate passes give (temporal blocking; each update is gs_cell's, term for term).
-//   PRE   the pre-smoothing: z from 0, colours 0, 1, 0, 1; then the residual r - A z of each
-//         of the tile's cells (mg_apply_at's order) and its 2 x 2 sums, in k_mg_restrict's
-//         order, into the coarser level's r, so the restriction needs no launch of its own
-//         (halo 5: z is final one ring out);
-//   !PRE  the post-smoothing: z += P zc (the coarse correction, piecewise constant), then
-//         colours 1, 0, 1, 0 (halo 4). It reads z around its tile, which neighbouring tiles
-//         finish at the same time, so it writes its result to another buffer (zout = L.t; PRE,
-//         which reads no z, writes L.z).
-// For levels of two colours (no wrap, or an even width) at least TX + 10 cells wide, so that no
-// cell sits twice in a tile, and of fewer than 2^31 cells (32-bit offsets). Shared memory holds
-// the region in red-black order, so that a colour pass reads and writes consecutive words with
-// no idle lanes. A tile whose region lies inside the raster (most tiles) stages and updates
-// without the bounds and seam tests, whose outcome is known there: every neighbour exists and
-// none lies across the seam.
-// Tiles: 32 x 16 cells and 256 threads; FP32 levels of many tiles take 64 x 32 cells and 512
-// threads, which cuts the halo's staged cells per tile cell from 2.1 to 1.5 and its updates
-// from 3.1 to 2.5.
-constexpr int MG_TX = 32, MG_TY = 16, MG_BTX = 64, MG_BTY = 32;
-// One value from global into shared memory by an asynchronous copy (completes at the block's
-// cp.async.wait_all).
-__device__ __forceinline__ void rb2_cp_async(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void rb2_cp_async(double* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-template <class TM, bool PRE, int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT) k_mg_rb2(DLevel<TM> L, DLevel<TM> C, const TM* __restrict__ zc, TM* __restrict__ zout) {
-  constexpr int HALO = PRE ? 5 : 4;
-  constexpr int SX = TX + 2 * HALO, SY = TY + 2 * HALO;
-  constexpr int HX = SX / 2, NC = HX * SY;  // a colour's cells of a row, of the region
-  static_assert(SX % 2 == 0 && 2 * NC >= TX * TY, "rb2: even rows");
-  // red-black layout: cell (lx, ly) of colour k = (i0 + lx + j0 + ly) & 1 at a[k][ly * HX + lx / 2]
-  extern __shared__ __align__(16) unsigned char mg_smem[];
-  TM* const base = reinterpret_cast<TM*>(mg_smem);
-  // array a (0 z, 1 r, 2 diag, 3 wd, 4 east, 5 south) of colour k
-  auto A = [&](int a, int k) { return base + (2 * a + k) * NC; };
-  const int i0 = blockIdx.x * TX - HALO, j0 = blockIdx.y * TY - HALO;
-  const int off = (i0 + j0) & 1;
-  const int tid = threadIdx.x;
-  const int w = L.w, h = L.h;
-  const bool inner = i0 >= 0 && j0 >= 0 && i0 + SX <= w && j0 + SY <= h;
-  auto gcol = [&](int lx) {
-    int gi = i0 + lx;
-    if (L.wrap) gi = gi < 0 ? gi + w : (gi >= w ? gi - w : gi);
-    return gi;
+// The damped-Jacobi V-cycle's part from a level of at most MG_BLOCK_CELLS cells down, in one block:
+// the separate launches' passes in their order (first sweep, sweep, restriction; the coarsest
+// level's 16 sweeps; the corrected sweep and another), a block barrier where a launch ended. Bound by
+// the barriers' latency: some 35 phases instead of as many launches of 5 us. Seven arrays a level
+// in shared memory (z and the sweeps' other buffer t).
+template <class TM>
+__global__ void __launch_bounds__(1024) k_mg_coarse_jacobi(MgChain<TM> g, int nu, int coarse_sweeps) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  extern __shared__ __align__(16) unsigned char mg_chain_smem[];
+  TM* const sbase = reinterpret_cast<TM*>(mg_chain_smem);
+  auto sl = [&](int q) {
+    DLevel<TM> L = g.lv[q];
+    TM** const a[7] = {&L.z, &L.r, &L.diag, &L.wd, &L.east, &L.south, &L.t};
+    for (int k = 0; k < 7; ++k) *a[k] = sbase + k * g.total + g.off[q];
+    return L;
   };
-  // staging by asynchronous copies into the colour arrays, so that all of a thread's copies are
-  // in flight at once (a load into registers and a store per value would wait out each load
-  // in turn); the post-smoothing then adds the coarse correction to its own staged z values
-  auto stage = [&](int lx, int ly, int gi, int gj) {
-    const int k = (lx + ly + off) & 1, q = ly * HX + (lx >> 1);
-    const int c = gj * w + gi;
-    if (PRE)
-      A(0, k)[q] = (TM)0;
-    else
-      rb2_cp_async(A(0, k) + q, L.z + c);
-    rb2_cp_async(A(1, k) + q, L.r + c);
-    rb2_cp_async(A(2, k) + q, L.diag + c);
-    rb2_cp_async(A(3, k) + q, L.wd + c);
-    rb2_cp_async(A(4, k) + q, L.east + c);
-    rb2_cp_async(A(5, k) + q, L.south + c);
-  };
-  if (inner) {
-    for (int e = tid; e < SX * SY; e += NT) {
-      const int ly = e / SX, lx = e - ly * SX;
-      stage(lx, ly, i0 + lx, j0 + ly);
-    }
-  } else {
-    for (int e = tid; e < SX * SY; e += NT) {
-      const int ly = e / SX, lx = e - ly * SX;
-      const int gi = gcol(lx), gj = j0 + ly;
-      if (gj < 0 || gj >= h || gi < 0 || gi >= w) continue;
-      stage(lx, ly, gi, gj);
-    }
-  }
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  if (!PRE) {
-    // z = z + zc (P zc piecewise constant), each thread on the cells it staged
-#pragma unroll 4
-    for (int e = tid; e < SX * SY; e += NT) {
-      const int ly = e / SX, lx = e - ly * SX;
-      const int gi = inner ? i0 + lx : gcol(lx), gj = j0 + ly;
-      if (!inner && (gj < 0 || gj >= h || gi < 0 || gi >= w)) continue;
-      A(0, (lx + ly + off) & 1)[ly * HX + (lx >> 1)] += zc[(gj >> 1) * C.w + (gi >> 1)];
+  for (int q = 0; q < g.count; ++q) {
+    const DLevel<TM> L = sl(q);
+    const DLevel<TM>& G = g.lv[q];
+    for (int k = tid; k < G.w * G.h; k += nt) {
+      L.diag[k] = G.diag[k];
+      L.wd[k] = G.wd[k];
+      L.east[k] = G.east[k];
+      L.south[k] = G.south[k];
+      if (q == 0) L.r[k] = G.r[k];
     }
   }
   __syncthreads();
-  // pass p updates its colour at least p + 1 cells from the region's border: a row's cells of
-  // one colour are consecutive, so consecutive threads take consecutive cells
-#pragma unroll
-  for (int pass = 0; pass < 4; ++pass) {
-    const int k = PRE ? (pass & 1) : 1 - (pass & 1), o_ = 1 - k;
-    const int lo = pass + 1, RW = SX - 2 * lo, RH = SY - 2 * lo, HW = RW / 2;
-    TM* const zs = A(0, k);
-    const TM* const zo = A(0, o_);
-    const TM *const rk = A(1, k), *const dk = A(2, k), *const wk = A(3, k);
-    const TM *const ek = A(4, k), *const eo = A(4, o_), *const sk = A(5, k), *const so = A(5, o_);
-    for (int idx = tid; idx < RH * HW; idx += NT) {
-      const int ly = lo + idx / HW;
-      const int p = (k + ly + off) & 1;  // the parity of lx of colour k on this row
-      const int lx = lo + ((p - lo) & 1) + 2 * (idx - (ly - lo) * HW);
-      const int q = ly * HX + (lx >> 1);
-      const int qw = ly * HX + ((lx - 1) >> 1), qe = ly * HX + ((lx + 1) >> 1);  // the other colour's
-      const TM zk = zs[q];
-      TM o = mulr(dk[q], zk);
-      if (inner) {
-        o -= mulr(ek[q], zo[qe]);
-        o -= mulr(eo[qw], zo[qw]);
-        o -= mulr(sk[q], zo[q + HX]);
-        o -= mulr(so[q - HX], zo[q - HX]);
-      } else {
-        const int gi = gcol(lx), gj = j0 + ly;
-        if (gj < 0 || gj >= h || gi < 0 || gi >= w) continue;
-        if (gi + 1 < w) o -= mulr(ek[q], zo[qe]);
-        if (gi > 0) o -= mulr(eo[qw], zo[qw]);
-        if (L.wrap) {
-          if (gi == w - 1) o -= mulr(ek[q], zo[qe]);
-          if (gi == 0) o -= mulr(eo[qw], zo[qw]);
-        }
-        if (gj + 1 < h) o -= mulr(sk[q], zo[q + HX]);
-        if (gj > 0) o -= mulr(so[q - HX], zo[q - HX]);
-      }
-      zs[q] = zk + mulr(rk[q] - o, wk[q]);
+  // one sweep of k_mg_sweep over the level
+  auto sweep = [&](const DLevel<TM>& L, const TM* zin, TM* zo, const TM* zc, int wc) {
+    for (int k = tid; k < L.w * L.h; k += nt) {
+      const int j = k / L.w, i = k - j * L.w;
+      TM zk = zin[k];
+      if (zc) zk += zc[(j / 2) * wc + i / 2];
+      const TM az = mg_apply_at<TM>(L, zin, zc, wc, i, j);
+      zo[k] = zk + L.wd[k] * (L.r[k] - az);
     }
     __syncthreads();
-  }
-  auto at = [&](int a, int lx, int ly) -> TM { return A(a, (lx + ly + off) & 1)[ly * HX + (lx >> 1)]; };
-  if (PRE) {
-    // the residual of each of the tile's cells, in mg_apply_at's order, into the slots of 1/diag
-    // (no longer read); then each coarse cell's 2 x 2 sum in k_mg_restrict's order
-    TM* const res = A(3, 0);
-    for (int e = tid; e < TX * TY; e += NT) {
-      const int lx = HALO + e % TX, ly = HALO + e / TX;
-      const int i = i0 + lx, j = j0 + ly;
-      if (i >= w || j >= h) continue;
-      TM o = mulr(at(2, lx, ly), at(0, lx, ly));
-      if (i + 1 < w) o -= mulr(at(4, lx, ly), at(0, lx + 1, ly));
-      if (i > 0) o -= mulr(at(4, lx - 1, ly), at(0, lx - 1, ly));
-      if (L.wrap) {
-        if (i == w - 1) o -= mulr(at(4, lx, ly), at(0, lx + 1, ly));
-        if (i == 0) o -= mulr(at(4, lx - 1, ly), at(0, lx - 1, ly));
-      }
-      if (j + 1 < h) o -= mulr(at(5, lx, ly), at(0, lx, ly + 1));
-      if (j > 0) o -= mulr(at(5, lx, ly - 1), at(0, lx, ly - 1));
-      res[e] = at(1, lx, ly) - o;
-    }
+  };
+  auto first = [&](const DLevel<TM>& L) {
+    for (int k = tid; k < L.w * L.h; k += nt) L.z[k] = L.wd[k] * L.r[k];
     __syncthreads();
-    constexpr int CX = TX / 2, CY = TY / 2;
-    for (int t = tid; t < CX * CY; t += NT) {
-      const int ic = blockIdx.x * CX + t % CX, jc = blockIdx.y * CY + t / CX;
-      if (ic >= C.w || jc >= C.h) continue;
-      TM acc = 0;
-      for (int j = 2 * jc; j < min(2 * jc + 2, h); ++j)
-        for (int i = 2 * ic; i < min(2 * ic + 2, w); ++i) acc += res[(j - j0 - HALO) * TX + (i - i0 - HALO)];
-      C.r[jc * C.w + ic] = acc;
+  };
+  // after the sweeps down a level's z is in t when nu is even, else in z
+  for (int q = 0; q + 1 < g.count; ++q) {
+    const DLevel<TM> L = sl(q), C = sl(q + 1);
+    first(L);
+    TM *cur = L.z, *nxt = L.t;
+    for (int k = 1; k < nu; ++k) {
+      sweep(L, cur, nxt, nullptr, 0);
+      TM* u = cur;
+      cur = nxt;
+      nxt = u;
     }
+    for (int k = tid; k < C.w * C.h; k += nt) restrict_cell<TM>(L, cur, C, k);
+    __syncthreads();
   }
-  for (int e = tid; e < TX * TY; e += NT) {
-    const int ly = HALO + e / TX, lx = HALO + e % TX;
-    const int gi = i0 + lx, gj = j0 + ly;
-    if (gi < w && gj < h) zout[gj * w + gi] = at(0, lx, ly);
+  const TM* zc;
+  {
+    const DLevel<TM> L = sl(g.count - 1);
+    first(L);
+    TM *cur = L.z, *nxt = L.t;
+    for (int k = 1; k < coarse_sweeps; ++k) {
+      sweep(L, cur, nxt, nullptr, 0);
+      TM* u = cur;
+      cur = nxt;
+      nxt = u;
+    }
+    zc = cur;
   }
+  for (int q = g.count - 2; q >= 0; --q) {
+    const DLevel<TM> L = sl(q);
+    const int wc = g.lv[q + 1].w;
+    TM *cur = nu & 1 ? L.z : L.t, *nxt = nu & 1 ? L.t : L.z;
+    for (int k = 0; k < nu; ++k) {
+      sweep(L, cur, nxt, k == 0 ? zc : nullptr, wc);
+      TM* u = cur;
+      cur = nxt;
+      nxt = u;
+    }
+    zc = cur;
+  }
+  for (int k = tid; k < g.lv[0].w * g.lv[0].h; k += nt) g.lv[0].z[k] = zc[k];
 }
-template <class TM, bool PRE, int TX = MG_TX, int TY = MG_TY>
-constexpr size_t mg_rb2_smem() {
-  return (size_t)6 * (TX + 2 * (PRE ? 5 : 4)) * (TY + 2 * (PRE ? 5 : 4)) * sizeof(TM);
+
+// A level's smoothing in one launch: both sweeps of the pre-smoothing from z = 0 with the residual
+// and its restriction, or the coarse correction and both sweeps of the post-smoothing. Over tiles
+// held in registers: a block takes a region of 64 columns by R = MG_WARPS RPW rows, a lane two
+// neighbouring columns of its warp's RPW rows (z, r, diag, 1/diag or omega/diag, east, south of
+// each cell). A pass's horizontal neighbours come from the next lane by a shuffle, its vertical ones
+// from the lane's own rows, or for a warp's first and last row from the neighbouring warp's through
+// shared memory (one barrier a pass). The region's rim computes without its outer neighbours; what
+// that spoils moves in one ring a pass (the first pass from z = 0 spoils none), so the tile is the
+// region less H rings: 4 for the Gauss-Seidel sweeps (4 colour passes, or 3 and the residual), 2
+// for the Jacobi ones. Each cell's terms are mg_apply_at's in its order (which takes the west term
+// before the east one in the last column of a wrapping level), so the values are the separate
+// launches'. Cells outside the raster hold zeros, couplings included; x wraps in the loads.
+//   RB, PRE    colours 0, 1, 0, 1;  !PRE  colours 1, 0, 1, 0 (colour: (i + j) % 2, so a level of two
+//              colours: no wrap, or an even width)
+//   Jacobi     z = wd r and one sweep; !PRE two sweeps
+// !PRE reads z around its tile, which neighbouring tiles finish at the same time: it writes another
+// buffer (zout = L.t). Levels of fewer than 2^31 cells (32-bit offsets). VEC: an even width, so
+// that a lane's two columns are one aligned word.
+// Bound by HBM on the largest levels: 25 (PRE) and 29 bytes a cell in FP32. The earlier form kept
+// the six arrays in shared memory in red-black order (12 reads an update, 360 thread instructions
+// a cell): FP32 8192 x 4096 PRE 505 us, !PRE 482 with the L2 flushed; this 164 (0.78 of the measured
+// copy rate) and 222; 2048 x 1024 45 and 44 to 20 and 26. For the Jacobi cycle it takes the place of
+// three launches each way: a 2048 x 656 cycle of 49 launches becomes 11.
+// Regions: 64 rows in FP32 on levels of many tiles (the rim is 1.3 times the tile), else 32.
+constexpr int MG_WARPS = 16;
+template <class TM>
+struct Pair2 {
+  TM v[2];
+};
+template <class TM, bool VEC>
+__device__ __forceinline__ Pair2<TM> mg_load2(const TM* __restrict__ a, int row, int c0, int c1, bool ok0, bool ok1) {
+  Pair2<TM> p;
+  if constexpr (VEC) {
+    using V = typename std::conditional<sizeof(TM) == 4, float2, double2>::type;
+    V t;
+    t.x = t.y = (TM)0;
+    if (ok0) t = *reinterpret_cast<const V*>(a + (row + c0));
+    p.v[0] = t.x;
+    p.v[1] = t.y;
+  } else {
+    p.v[0] = ok0 ? a[row + c0] : (TM)0;
+    p.v[1] = ok1 ? a[row + c1] : (TM)0;
+  }
+  return p;
+}
+
+template <class TM, bool RB, bool PRE, int RPW, bool VEC>
+__global__ void __launch_bounds__(32 * MG_WARPS, sizeof(TM) == 4 ? 2 : 1)
+    k_mg_tile(DLevel<TM> L, DLevel<TM> C, const TM* __restrict__ zc, TM* __restrict__ zout) {
+  constexpr int H = RB ? 4 : 2, R = MG_WARPS * RPW, TX = 64 - 2 * H, TY = R - 2 * H;
+  static_assert(RPW % 2 == 0 && TX % 2 == 0 && TY % 2 == 0, "even rows: a cell's colour and its coarse cell are known per row");
+  // the warps' first and last rows, two buffers by pass
+  __shared__ Pair2<TM> edge[2][2][MG_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int w = L.w, h = L.h;
+  const int raw = (int)blockIdx.x * TX - H + 2 * lane, j0 = (int)blockIdx.y * TY - H + warp * RPW;
+  int c0 = raw, c1 = raw + 1;
+  bool ok0 = c0 >= 0 && c0 < w, ok1 = c1 >= 0 && c1 < w;
+  if (L.wrap) {
+    c0 %= w;
+    c0 += c0 < 0 ? w : 0;
+    c1 = c0 + 1 == w ? 0 : c0 + 1;
+    ok0 = ok1 = true;
+  }
+  const bool seam0 = L.wrap && c0 == w - 1, seam1 = L.wrap && c1 == w - 1;
+  Pair2<TM> z[RPW], r[RPW], dg[RPW], wd[RPW], es[RPW], so[RPW], so_up;
+#pragma unroll
+  for (int q = 0; q < RPW; ++q) {
+    const int j = j0 + q;
+    const bool in = j >= 0 && j < h;
+    const int row = j * w;
+    r[q] = mg_load2<TM, VEC>(L.r, row, c0, c1, in && ok0, in && ok1);
+    wd[q] = mg_load2<TM, VEC>(L.wd, row, c0, c1, in && ok0, in && ok1);
+    if (!PRE) z[q] = mg_load2<TM, VEC>(L.z, row, c0, c1, in && ok0, in && ok1);
+    dg[q] = mg_load2<TM, VEC>(L.diag, row, c0, c1, in && ok0, in && ok1);
+    es[q] = mg_load2<TM, VEC>(L.east, row, c0, c1, in && ok0, in && ok1);
+    so[q] = mg_load2<TM, VEC>(L.south, row, c0, c1, in && ok0, in && ok1);
+  }
+  {
+    const bool in = j0 > 0 && j0 <= h;
+    so_up = mg_load2<TM, VEC>(L.south, (j0 - 1) * w, c0, c1, in && ok0, in && ok1);
+  }
+  if constexpr (PRE) {
+#pragma unroll
+    for (int q = 0; q < RPW; ++q)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) z[q].v[c] = !RB || ((q + c) & 1) == 0 ? (RB ? mulr(r[q].v[c], wd[q].v[c]) : wd[q].v[c] * r[q].v[c]) : (TM)0;
+  } else {
+#pragma unroll
+    for (int q = 0; q < RPW; q += 2) {
+      const int j = j0 + q;
+      const bool in = j >= 0 && j < h;
+      const int cr = (j >> 1) * C.w;
+      const TM a = in && ok0 ? zc[cr + (c0 >> 1)] : (TM)0;
+      const TM b = VEC ? a : (in && ok1 ? zc[cr + (c1 >> 1)] : (TM)0);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (in && (u == 0 || j + 1 < h)) {
+          z[q + u].v[0] += a;
+          z[q + u].v[1] += b;
+        }
+      }
+    }
+  }
+  TM ew[RPW];  // the west neighbour's east coupling of the even columns
+#pragma unroll
+  for (int q = 0; q < RPW; ++q) ew[q] = __shfl_up_sync(0xffffffffu, es[q].v[1], 1);
+  int buf = 0;
+  auto publish = [&](int b) {
+    edge[b][0][warp][lane] = z[0];
+    edge[b][1][warp][lane] = z[RPW - 1];
+  };
+  // A z at the lane's cell (q, c) from its row's and neighbours' values
+  auto apply = [&](int q, int c, TM zk, TM ze, TM zw, TM zn, TM zs) {
+    TM o = mulr(dg[q].v[c], zk);
+    const TM a = mulr(es[q].v[c], ze), b = mulr(c ? es[q].v[0] : ew[q], zw);
+    const bool seam = c ? seam1 : (!VEC && seam0);
+    o -= seam ? b : a;
+    o -= seam ? a : b;
+    o -= mulr(so[q].v[c], zs);
+    o -= mulr(q ? so[q ? q - 1 : 0].v[c] : so_up.v[c], zn);
+    return o;
+  };
+  auto neighbours = [&](Pair2<TM>& up, Pair2<TM>& down) {
+    up.v[0] = up.v[1] = down.v[0] = down.v[1] = (TM)0;
+    if (warp > 0) up = edge[buf][1][warp - 1][lane];
+    if (warp < MG_WARPS - 1) down = edge[buf][0][warp + 1][lane];
+  };
+  constexpr int PASSES = RB ? (PRE ? 3 : 4) : (PRE ? 1 : 2);
+  publish(0);
+  __syncthreads();
+#pragma unroll
+  for (int pass = 0; pass < PASSES; ++pass) {
+    Pair2<TM> up, down;
+    neighbours(up, down);
+    if constexpr (RB) {
+      const int k = 1 - (pass & 1);  // PRE: the first pass (colour 0) is done; both go 1, 0, 1(, 0)
+#pragma unroll
+      for (int q = 0; q < RPW; ++q) {
+        const int c = (k + q) & 1;  // the row's column of colour k
+        const TM zk = z[q].v[c], in = z[q].v[1 - c];
+        const TM out = c ? __shfl_down_sync(0xffffffffu, in, 1) : __shfl_up_sync(0xffffffffu, in, 1);
+        const TM zn = q ? z[q ? q - 1 : 0].v[c] : up.v[c], zs = q + 1 < RPW ? z[q + 1 < RPW ? q + 1 : q].v[c] : down.v[c];
+        const TM o = apply(q, c, zk, c ? out : in, c ? in : out, zn, zs);
+        z[q].v[c] = zk + mulr(r[q].v[c] - o, wd[q].v[c]);
+      }
+    } else {
+      Pair2<TM> prev = up;  // the row above before this sweep
+#pragma unroll
+      for (int q = 0; q < RPW; ++q) {
+        const Pair2<TM> old = z[q], next = q + 1 < RPW ? z[q + 1 < RPW ? q + 1 : q] : down;
+        const TM zr = __shfl_down_sync(0xffffffffu, old.v[0], 1), zl = __shfl_up_sync(0xffffffffu, old.v[1], 1);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const TM az = apply(q, c, old.v[c], c ? zr : old.v[1], c ? old.v[0] : zl, prev.v[c], next.v[c]);
+          z[q].v[c] = old.v[c] + wd[q].v[c] * (r[q].v[c] - az);
+        }
+        prev = old;
+      }
+    }
+    if (PRE || pass + 1 < PASSES) {
+      publish(buf ^ 1);
+      __syncthreads();
+      buf ^= 1;
+    }
+  }
+  const bool lanes_in = lane >= H / 2 && lane < 32 - H / 2;
+  if constexpr (PRE) {
+    Pair2<TM> up, down;
+    neighbours(up, down);
+    TM acc = 0;
+#pragma unroll
+    for (int q = 0; q < RPW; ++q) {
+      const Pair2<TM> next = q + 1 < RPW ? z[q + 1 < RPW ? q + 1 : q] : down, prev = q ? z[q ? q - 1 : 0] : up;
+      const TM zr = __shfl_down_sync(0xffffffffu, z[q].v[0], 1), zl = __shfl_up_sync(0xffffffffu, z[q].v[1], 1);
+      if ((q & 1) == 0) acc = (TM)0;
+      const TM a0 = r[q].v[0] - apply(q, 0, z[q].v[0], z[q].v[1], zl, prev.v[0], next.v[0]);
+      const TM a1 = r[q].v[1] - apply(q, 1, z[q].v[1], zr, z[q].v[0], prev.v[1], next.v[1]);
+      if (j0 + q < h) {
+        acc += a0;
+        if (VEC || raw + 1 < w) acc += a1;
+      }
+      if (q & 1) {
+        const int j = j0 + q - 1, rr = warp * RPW + q - 1;
+        if (lanes_in && raw < w && rr >= H && rr < R - H && j < h) C.r[(j >> 1) * C.w + (raw >> 1)] = acc;
+      }
+    }
+  }
+  if (!lanes_in || raw >= w) return;
+#pragma unroll
+  for (int q = 0; q < RPW; ++q) {
+    const int j = j0 + q, rr = warp * RPW + q;
+    if (rr < H || rr >= R - H || j >= h) continue;
+    if constexpr (VEC) {
+      using V = typename std::conditional<sizeof(TM) == 4, float2, double2>::type;
+      V t;
+      t.x = z[q].v[0];
+      t.y = z[q].v[1];
+      *reinterpret_cast<V*>(zout + (j * w + raw)) = t;
+    } else {
+      zout[j * w + raw] = z[q].v[0];
+      if (raw + 1 < w) zout[j * w + raw + 1] = z[q].v[1];
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1340,28 +1458,15 @@ struct dt_diff {
   dt::Hier<float> hf[2];
   dt::Hier<double> hd[2];
   dt::DGraph graph[4][2];  // [lane: 0 split, 1 FP64, 2 FP32 inner, 3 FP32 reliable][cycle]
-  // the Gauss-Seidel cycle's fused kernels (k_mg_rb2, k_mg_coarse_rb); DT_MG_FUSED=0 at create
-  // keeps one launch per colour pass (the same values)
+  // the cycles' fused kernels (k_mg_tile, k_mg_coarse_rb, k_mg_coarse_jacobi); DT_MG_FUSED=0 at
+  // create keeps one launch per sweep or colour pass (the same values)
   bool mg_fused = true;
-  // k_mg_rb2's 64 x 32 tiles on FP32 levels of many tiles; DT_MG_BIG_TILES=0 at create keeps
-  // 32 x 16 tiles everywhere (the same values)
+  // k_mg_tile's 64-row regions on FP32 levels of many tiles; DT_MG_BIG_TILES=0 at create keeps
+  // 32-row ones everywhere (the same values)
   bool mg_big_tiles = true;
 };
 
 namespace dt {
-
-// Opt k_mg_rb2's instantiations in to their dynamic shared memory.
-template <class TM>
-static void rb2_attributes() {
-  cudaFuncSetAttribute(k_mg_rb2<TM, true, MG_TX, MG_TY, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)mg_rb2_smem<TM, true>());
-  cudaFuncSetAttribute(k_mg_rb2<TM, false, MG_TX, MG_TY, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)mg_rb2_smem<TM, false>());
-  cudaFuncSetAttribute(k_mg_rb2<TM, true, MG_BTX, MG_BTY, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)mg_rb2_smem<TM, true, MG_BTX, MG_BTY>());
-  cudaFuncSetAttribute(k_mg_rb2<TM, false, MG_BTX, MG_BTY, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)mg_rb2_smem<TM, false, MG_BTX, MG_BTY>());
-}
 
 template <class T>
 static dt_status ddalloc(dt_diff* s, T** p, size_t count) {
@@ -1426,26 +1531,36 @@ static void fill_levels(dt_diff* s, Hier<TM>& H, int kind, cudaStream_t st) {
   }
 }
 
-// Whether k_mg_rb2 takes a level: at least MG_TX + 10 cells wide (no cell twice in a tile's
-// region) and fewer than 2^31 cells (its 32-bit offsets).
-template <class TM>
-static bool rb2_fits(const DLevel<TM>& L) {
-  return L.w >= MG_TX + 10 && (size_t)L.w * L.h < ((size_t)1 << 31);
+// A level's smoothing by k_mg_tile (PRE: from z = 0, the restriction into C.r; else with the coarse
+// correction zc).
+template <class TM, bool RB, bool PRE, int RPW>
+static void launch_tile_rows(const DLevel<TM>& L, const DLevel<TM>& C, const TM* zc, TM* zout, cudaStream_t st) {
+  constexpr int H = RB ? 4 : 2;
+  const dim3 tg(ceil_div(L.w, 64 - 2 * H), ceil_div(L.h, MG_WARPS * RPW - 2 * H));
+  if (L.w % 2 == 0)
+    k_mg_tile<TM, RB, PRE, RPW, true><<<tg, 32 * MG_WARPS, 0, st>>>(L, C, zc, zout);
+  else
+    k_mg_tile<TM, RB, PRE, RPW, false><<<tg, 32 * MG_WARPS, 0, st>>>(L, C, zc, zout);
 }
-// The two tiled sweeps of a level (PRE: from z = 0 with the restriction into C.r; else with the
-// coarse correction zc): 64 x 32 tiles for FP32 levels of at least four tiles an SM, else 32 x 16.
-template <class TM, bool PRE>
-static void launch_rb2(dt_diff* s, const DLevel<TM>& L, const DLevel<TM>& C, const TM* zc, TM* zout, cudaStream_t st) {
-  const bool big = std::is_same<TM, float>::value && s->mg_big_tiles && L.w >= MG_BTX + 10 &&
-                   (size_t)ceil_div(L.w, MG_BTX) * ceil_div(L.h, MG_BTY) >= (size_t)4 * s->sms;
-  if (big) {
-    const dim3 tg(ceil_div(L.w, MG_BTX), ceil_div(L.h, MG_BTY));
-    k_mg_rb2<TM, PRE, MG_BTX, MG_BTY, 512><<<tg, 512, mg_rb2_smem<TM, PRE, MG_BTX, MG_BTY>(), st>>>(L, C, zc, zout);
-  } else {
-    const dim3 tg(ceil_div(L.w, MG_TX), ceil_div(L.h, MG_TY));
-    k_mg_rb2<TM, PRE, MG_TX, MG_TY, 256><<<tg, 256, mg_rb2_smem<TM, PRE>(), st>>>(L, C, zc, zout);
+template <class TM, bool RB, bool PRE>
+static void launch_tile(dt_diff* s, const DLevel<TM>& L, const DLevel<TM>& C, const TM* zc, TM* zout, cudaStream_t st) {
+  // 64-row regions on FP32 levels where those alone make at least four tiles an SM (FP64 rows of
+  // four would not fit the registers)
+  if constexpr (sizeof(TM) == 4) {
+    constexpr int H = RB ? 4 : 2;
+    if (s->mg_big_tiles && (size_t)ceil_div(L.w, 64 - 2 * H) * ceil_div(L.h, 64 - 2 * H) >= (size_t)4 * s->sms) {
+      launch_tile_rows<TM, RB, PRE, 4>(L, C, zc, zout, st);
+      count_launch();
+      return;
+    }
   }
+  launch_tile_rows<TM, RB, PRE, 2>(L, C, zc, zout, st);
   count_launch();
+}
+// k_mg_tile's 32-bit offsets
+template <class TM>
+static bool tile_fits(const DLevel<TM>& L) {
+  return (size_t)L.w * L.h < ((size_t)1 << 31);
 }
 
 // One V-cycle from z = 0 on level l with r set; returns the buffer holding the level's z.
@@ -1464,6 +1579,44 @@ static TM* vcycle(dt_diff* s, Hier<TM>& H, size_t l, int kind, cudaStream_t st) 
     return L.z;
   }
   DLevel<TM>& C = H.lv[l + 1];
+  if (s->mg_fused) {
+    // this level and every coarser one in one block, when it is small enough
+    if (n <= (size_t)MG_BLOCK_CELLS && H.lv.size() - l <= (size_t)MG_BLOCK_LEVELS) {
+      MgChain<TM> m{};
+      m.count = (int)(H.lv.size() - l);
+      m.total = 0;
+      for (int q = 0; q < m.count; ++q) {
+        m.lv[q] = H.lv[l + q];
+        m.off[q] = m.total;
+        m.total += H.lv[l + q].w * H.lv[l + q].h;
+      }
+      const size_t smem = (size_t)(kind == DT_CYCLE_JACOBI ? 7 : 6) * m.total * sizeof(TM);
+      const DLevel<TM>& last = H.lv.back();
+      if (smem <= 200 * 1024 && last.w * last.h <= 128) {  // the coarsest takes one thread a cell of 128
+        if (kind == DT_CYCLE_JACOBI)
+          k_mg_coarse_jacobi<TM><<<1, 1024, smem, st>>>(m, NU, COARSE_SWEEPS);
+        else
+          k_mg_coarse_rb<TM><<<1, 1024, smem, st>>>(m, NU, COARSE_SWEEPS_GS);
+        count_launch();
+        return L.z;
+      }
+    }
+    // both sweeps of the smoothing in one launch over tiles, the restriction fused into the
+    // pre-smoothing (the Gauss-Seidel cycle on two-colour levels)
+    const bool jacobi = kind == DT_CYCLE_JACOBI;
+    if (NU == 2 && tile_fits(L) && (jacobi || gs_colours(L.w, L.wrap) == 2)) {
+      if (jacobi)
+        launch_tile<TM, false, true>(s, L, C, nullptr, L.z, st);
+      else
+        launch_tile<TM, true, true>(s, L, C, nullptr, L.z, st);
+      TM* zc = vcycle<TM>(s, H, l + 1, kind, st);
+      if (jacobi)
+        launch_tile<TM, false, false>(s, L, C, zc, L.t, st);
+      else
+        launch_tile<TM, true, false>(s, L, C, zc, L.t, st);
+      return L.t;  // the level's z, in its spare buffer
+    }
+  }
   if (kind == DT_CYCLE_JACOBI) {
     // multigrid.rs:514-522
     TM *cur = L.z, *nxt = L.t;
@@ -1489,34 +1642,6 @@ static TM* vcycle(dt_diff* s, Hier<TM>& H, size_t l, int kind, cudaStream_t st) 
   }
   // multi-colour Gauss-Seidel V(NU, NU): colours forward, coarse correction, colours backward
   int ncol = gs_colours(L.w, L.wrap);
-  if (s->mg_fused) {
-    // this level and every coarser one in one block, when it is small enough
-    if (n <= (size_t)MG_BLOCK_CELLS && H.lv.size() - l <= (size_t)MG_BLOCK_LEVELS) {
-      MgChain<TM> m{};
-      m.count = (int)(H.lv.size() - l);
-      m.total = 0;
-      for (int q = 0; q < m.count; ++q) {
-        m.lv[q] = H.lv[l + q];
-        m.off[q] = m.total;
-        m.total += H.lv[l + q].w * H.lv[l + q].h;
-      }
-      const size_t smem = (size_t)6 * m.total * sizeof(TM);
-      const DLevel<TM>& last = H.lv.back();
-      if (smem <= 200 * 1024 && last.w * last.h <= 128) {  // the coarsest takes one thread a cell of 128
-        k_mg_coarse_rb<TM><<<1, 1024, smem, st>>>(m, NU, COARSE_SWEEPS_GS);
-        count_launch();
-        return L.z;
-      }
-    }
-    // both sweeps of the smoothing in one launch over tiles, the restriction fused into the
-    // pre-smoothing (two-colour levels wide enough)
-    if (ncol == 2 && NU == 2 && rb2_fits(L)) {
-      launch_rb2<TM, true>(s, L, C, nullptr, L.z, st);
-      TM* zc = vcycle<TM>(s, H, l + 1, kind, st);
-      launch_rb2<TM, false>(s, L, C, zc, L.t, st);
-      return L.t;  // the level's z, in its spare buffer
-    }
-  }
   for (int sweep = 0; sweep < NU; ++sweep)
     for (int c = 0; c < ncol; ++c) {
       if (sweep == 0)
@@ -1954,9 +2079,9 @@ dt_status dt_diff_create(int w, int h, double dx, int wrap_x, dt_diff** out) {
   // rounding up) in six arrays
   cudaFuncSetAttribute(k_mg_coarse_rb<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaFuncSetAttribute(k_mg_coarse_rb<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_mg_coarse_jacobi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_mg_coarse_jacobi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (const char* e = getenv("DT_MG_BIG_TILES")) s->mg_big_tiles = e[0] != '0';
-  rb2_attributes<float>();
-  rb2_attributes<double>();
   s->n = (size_t)w * h;
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, 0) == cudaSuccess) s->sms = prop.multiProcessorCount;
@@ -2197,7 +2322,7 @@ dt_status dt_diff_profile_kernels(dt_diff* s, const double* kd, double dt, int r
   Hier<double>& HD = s->hd[DT_CYCLE_RBGS];
   DT_TRY(build_levels<float>(s, HF, COARSEST_GS));
   DT_TRY(build_levels<double>(s, HD, COARSEST_GS));
-  if (HF.lv.size() < 2 || gs_colours(HF.lv[0].w, HF.lv[0].wrap) != 2 || !rb2_fits(HF.lv[0])) {
+  if (HF.lv.size() < 2 || gs_colours(HF.lv[0].w, HF.lv[0].wrap) != 2 || HF.lv[0].w < 42 || !tile_fits(HF.lv[0])) {
     set_error("dt_diff_profile_kernels: the finest level of a %d x %d raster does not take the tiled sweeps", s->w, s->h);
     return DT_UNSUPPORTED;
   }
@@ -2223,10 +2348,10 @@ dt_status dt_diff_profile_kernels(dt_diff* s, const double* kd, double dt, int r
         k_d_apply<float, float, DA_PAP><<<g, 256, 0, st>>>(s->w, s->h, wrap, s->east32, s->south32, s->diag32, s->p32, nullptr,
                                                            s->ap32, nullptr, s->partials, s->S32);
         break;
-      case 2: launch_rb2<float, true>(s, F0, F1, nullptr, F0.z, st); break;
-      case 3: launch_rb2<float, false>(s, F0, F1, F1.z, F0.t, st); break;
-      case 4: launch_rb2<double, true>(s, D0, D1, nullptr, D0.z, st); break;
-      default: launch_rb2<double, false>(s, D0, D1, D1.z, D0.t, st); break;
+      case 2: launch_tile<float, true, true>(s, F0, F1, nullptr, F0.z, st); break;
+      case 3: launch_tile<float, true, false>(s, F0, F1, F1.z, F0.t, st); break;
+      case 4: launch_tile<double, true, true>(s, D0, D1, nullptr, D0.z, st); break;
+      default: launch_tile<double, true, false>(s, D0, D1, D1.z, D0.t, st); break;
     }
   };
   // algorithmic bytes: the operator x, east, south, diag in and y out; the pre-smoothing r, diag,
