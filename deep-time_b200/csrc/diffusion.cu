@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(256) k_d_apply(int w, int h, int wrap, const T
         } else if (MODE == DA_RESID) {
           const T r = bv.a[e] - a;
           out.a[e] = r;
-          ym[c + e] = (TM)r;
+          if (ym) ym[c + e] = (TM)r;
           acc.v[0] += (double)r * (double)r;
         } else if (MODE == DA_RESID_GATED) {
           const T r = bv.a[e] - a;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) k_d_apply(int w, int h, int wrap, const T
       } else if (MODE == DA_RESID) {
         T r = b[k] - ax;
         y[k] = r;
-        ym[k] = (TM)r;
+        if (ym) ym[k] = (TM)r;
         acc.v[0] += (double)r * (double)r;
       } else if (MODE == DA_RESID_GATED) {
         T r = b[k] - ax;
@@ -273,22 +273,44 @@ __global__ void __launch_bounds__(256) k_d_apply(int w, int h, int wrap, const T
   }
 }
 
-// x += alpha p; r -= alpha Ap; rm = (TM) r; reduce r.r and test the stopping rule.
+// x += alpha p; r -= alpha Ap; rm = (TM) r (unless null: the cycle reads r itself); reduce r.r and
+// test the stopping rule. In 16-byte words of T (the handle's buffers are aligned), up to eight blocks
+// an SM. Bound by HBM.
 template <class T, class TM>
-__global__ void __launch_bounds__(256) k_d_update(size_t n, T* __restrict__ x, T* __restrict__ r, TM* __restrict__ rm,
+__global__ void __launch_bounds__(256, 8) k_d_update(size_t n, T* __restrict__ x, T* __restrict__ r, TM* __restrict__ rm,
                                                   const T* __restrict__ p, const T* __restrict__ ap, double* partials, DScalars* S) {
   if (S->stop) {
     if (blockIdx.x == 0 && threadIdx.x == 0) dset_cond(S, 0);
     return;
   }
+  constexpr int V = 16 / sizeof(T);
+  using W = DV16<T>;
   T alpha = (T)S->alpha;
   Acc<1> acc;
   acc.v[0] = 0.0;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
+  const size_t nv = n / V, t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+#pragma unroll 1
+  for (size_t kv = t0; kv < nv; kv += stride) {
+    W xx = reinterpret_cast<W*>(x)[kv], rr = reinterpret_cast<W*>(r)[kv];
+    const W pp = reinterpret_cast<const W*>(p)[kv], aa = reinterpret_cast<const W*>(ap)[kv];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      xx.a[e] += alpha * pp.a[e];
+      rr.a[e] = rr.a[e] - alpha * aa.a[e];
+      acc.v[0] += (double)rr.a[e] * (double)rr.a[e];
+    }
+    reinterpret_cast<W*>(x)[kv] = xx;
+    reinterpret_cast<W*>(r)[kv] = rr;
+    if (rm) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) rm[kv * V + e] = (TM)rr.a[e];
+    }
+  }
+  for (size_t k = nv * V + t0; k < n; k += stride) {
     x[k] += alpha * p[k];
     T rv = r[k] - alpha * ap[k];
     r[k] = rv;
-    rm[k] = (TM)rv;
+    if (rm) rm[k] = (TM)rv;
     acc.v[0] += (double)rv * (double)rv;
   }
   const int kind[1] = {0};
@@ -321,37 +343,46 @@ __global__ void __launch_bounds__(256) k_d_update(size_t n, T* __restrict__ x, T
   }
 }
 
-// rz = r . z after the cycle; beta = rz / rz_old (multigrid.rs:721-727).
+// After the cycle, with rz = r . z: beta = rz / rz_old (multigrid.rs:721-727).
+__device__ __forceinline__ void d_finish_rz(DScalars* S, double rz) {
+  if (!S->started) {
+    S->started = 1;
+    S->rz = rz;
+    if (!isfinite(rz)) S->stop = DSTOP_NONFINITE;
+    return;
+  }
+  if (!(isfinite(rz) && S->rz > 0.0)) {
+    S->stop = isfinite(rz) ? DSTOP_BREAKDOWN : DSTOP_NONFINITE;
+    dset_cond(S, 0);
+    return;
+  }
+  S->beta = rz / S->rz;
+  S->rz = rz;
+}
+// rz = r . z, where the finest level's post-smoothing does not form it (k_mg_tile).
 template <class T, class TM>
-__global__ void __launch_bounds__(256) k_d_rz(size_t n, const T* __restrict__ r, const TM* __restrict__ z, double* partials,
+__global__ void __launch_bounds__(256, 8) k_d_rz(size_t n, const T* __restrict__ r, const TM* __restrict__ z, double* partials,
                                               DScalars* S) {
   if (S->stop) return;
   Acc<1> acc;
   acc.v[0] = 0.0;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-    acc.v[0] += (double)r[k] * (double)z[k];
+  constexpr int V = 16 / sizeof(T);
+  const size_t nv = n / V, t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t kv = t0; kv < nv; kv += stride) {
+    const DV16<T> rr = reinterpret_cast<const DV16<T>*>(r)[kv];
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc.v[0] += (double)rr.a[e] * (double)z[kv * V + e];
+  }
+  for (size_t k = nv * V + t0; k < n; k += stride) acc.v[0] += (double)r[k] * (double)z[k];
   const int kind[1] = {0};
   if (reduce_partials<1>(acc, kind, partials, &S->ticket[DSITE_RZ], gridDim.x) && threadIdx.x == 0) {
-    double rz = acc.v[0];
-    if (!S->started) {
-      S->started = 1;
-      S->rz = rz;
-      if (!isfinite(rz)) S->stop = DSTOP_NONFINITE;
-      return;
-    }
-    if (!(isfinite(rz) && S->rz > 0.0)) {
-      S->stop = isfinite(rz) ? DSTOP_BREAKDOWN : DSTOP_NONFINITE;
-      dset_cond(S, 0);
-      return;
-    }
-    S->beta = rz / S->rz;
-    S->rz = rz;
+    d_finish_rz(S, acc.v[0]);
   }
 }
 
 // p = z + beta p (p = z on the first direction), and the loop guard.
 template <class T, class TM>
-__global__ void __launch_bounds__(256) k_d_direction(size_t n, T* __restrict__ p, const TM* __restrict__ z, DScalars* S, int first) {
+__global__ void __launch_bounds__(256, 8) k_d_direction(size_t n, T* __restrict__ p, const TM* __restrict__ z, DScalars* S, int first) {
   if (!first && blockIdx.x == 0 && threadIdx.x == 0) {
     int runs = ++S->body_runs;
     bool again = S->stop == 0 && runs < S->max_it + 2;
@@ -360,8 +391,21 @@ __global__ void __launch_bounds__(256) k_d_direction(size_t n, T* __restrict__ p
   }
   if (S->stop) return;
   T beta = first ? (T)0 : (T)S->beta;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-    p[k] = first ? (T)z[k] : (T)z[k] + beta * p[k];
+  constexpr int V = 16 / sizeof(T);
+  using W = DV16<T>;
+  const size_t nv = n / V, t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+#pragma unroll 1
+  for (size_t kv = t0; kv < nv; kv += stride) {
+    W pp;
+    if (!first) pp = reinterpret_cast<const W*>(p)[kv];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const T zz = (T)z[kv * V + e];
+      pp.a[e] = first ? zz : zz + beta * pp.a[e];
+    }
+    reinterpret_cast<W*>(p)[kv] = pp;
+  }
+  for (size_t k = nv * V + t0; k < n; k += stride) p[k] = first ? (T)z[k] : (T)z[k] + beta * p[k];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -373,18 +417,10 @@ struct DLevel {
   TM *east, *south, *diag, *wd, *mass, *r, *z, *t;
 };
 
+// The finest level's wd = omega / diag; its other coefficients are the operator's own arrays.
 template <class TM>
-__global__ void k_mg_finest(size_t n, const double* __restrict__ e, const double* __restrict__ s, const double* __restrict__ g,
-                            TM omega, TM* __restrict__ east, TM* __restrict__ south, TM* __restrict__ diag, TM* __restrict__ wd,
-                            TM* __restrict__ mass) {
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-    east[k] = (TM)e[k];
-    south[k] = (TM)s[k];
-    TM gg = (TM)g[k];
-    diag[k] = gg;
-    wd[k] = omega / gg;
-    mass[k] = (TM)1;
-  }
+__global__ void k_mg_finest(size_t n, const TM* __restrict__ diag, TM omega, TM* __restrict__ wd) {
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) wd[k] = omega / diag[k];
 }
 
 // Coarse mass and faces: mass = sum of the 2 x 2 block's; east = SCALE * the fine east faces
@@ -398,7 +434,7 @@ __global__ void k_mg_coarsen(DLevel<TM> f, DLevel<TM> c, TM scale) {
     int last_row = r1 - 1, last_col = c1 - 1;
     TM m = 0;
     for (int j = r0; j < r1; ++j)
-      for (int i = c0; i < c1; ++i) m += f.mass[(size_t)j * f.w + i];
+      for (int i = c0; i < c1; ++i) m += f.mass ? f.mass[(size_t)j * f.w + i] : (TM)1;
     c.mass[k] = m;
     TM e = 0;
     if (ic + 1 < c.w || c.wrap) {
@@ -598,199 +634,197 @@ __global__ void k_mg_coarsest(DLevel<TM> L, TM* __restrict__ z, int sweeps) {
   coarsest_solve<TM, KIND>(L, z, sweeps);
 }
 
-// The Gauss-Seidel V-cycle's part from a level of at most MG_BLOCK_CELLS cells down, in one
-// block of 1024 threads (the coarsest level on the first 128): the same passes in the same order as the separate launches (pre-sweeps,
-// restriction, the coarser levels, prolongation, post-sweeps), a block barrier where a launch
-// ended, so the same values. The levels' arrays are staged in shared memory first (off[q]: the
-// level's first cell there, six arrays of `total` cells); the top level's z goes back at the end.
+// The V-cycle's part from a level of at most MG_BLOCK_CELLS cells down, in one block: the separate
+// launches' passes in their order (pre-sweeps, restriction, the coarser levels, coarse correction,
+// post-sweeps; the coarsest level's sweeps), so the same values. The levels' arrays are staged in
+// shared memory (off[q]: the level's first cell there, seven arrays of `total` cells). Bound by the
+// latency of some 35 to 60 dependent passes, so a thread keeps its cells' couplings and neighbours'
+// places in registers through a level's passes, and a level's barriers take only the warps that hold
+// its cells (barrier q + 1; the others wait where they meet the level again on the way up). With the
+// indexes worked out in every pass and all 1024 threads in every barrier a Gauss-Seidel chain from
+// 64 x 32 cells took 29 us and a Jacobi one from 64 x 21 21.6 us; this RBCH and JACCH.
 constexpr int MG_BLOCK_LEVELS = 8;
+constexpr int MG_BLOCK_CELLS = 2048;  // two cells a thread
 template <class TM>
 struct MgChain {
   DLevel<TM> lv[MG_BLOCK_LEVELS];
   int off[MG_BLOCK_LEVELS];
   int count, total;
 };
+// One cell of a staged level: couplings (0 where there is no neighbour, whose place is then the
+// cell's own), in mg_apply_at's order of terms (`seam`: the west term before the east one).
 template <class TM>
-__global__ void __launch_bounds__(1024) k_mg_coarse_rb(MgChain<TM> g, int nu, int coarse_sweeps) {
+struct MgCell {
+  TM d, wd, r, e, w, s, n;
+  int k, ke, kw, ks, kn, colour;
+  bool seam;
+  __device__ __forceinline__ TM apply(const TM* z) const {
+    TM o = mulr(d, z[k]);
+    const TM a = mulr(e, z[ke]), b = mulr(w, z[kw]);
+    o -= seam ? b : a;
+    o -= seam ? a : b;
+    o -= mulr(s, z[ks]);
+    o -= mulr(n, z[kn]);
+    return o;
+  }
+};
+template <class TM, bool JAC>
+__global__ void __launch_bounds__(1024) k_mg_coarse(MgChain<TM> g, int nu, int coarse_sweeps) {
   const int tid = threadIdx.x, nt = blockDim.x;
   extern __shared__ __align__(16) unsigned char mg_chain_smem[];
   TM* const sbase = reinterpret_cast<TM*>(mg_chain_smem);
-  // level q as staged in shared memory (built in registers where it is used)
-  auto sl = [&](int q) {
-    DLevel<TM> L = g.lv[q];
-    L.z = sbase + 0 * g.total + g.off[q];
-    L.r = sbase + 1 * g.total + g.off[q];
-    L.diag = sbase + 2 * g.total + g.off[q];
-    L.wd = sbase + 3 * g.total + g.off[q];
-    L.east = sbase + 4 * g.total + g.off[q];
-    L.south = sbase + 5 * g.total + g.off[q];
-    return L;
-  };
+  // arrays of a level: 0 z, 1 t (Jacobi's other buffer; the residuals), 2 r, 3 diag, 4 wd, 5 east, 6 south
+  auto arr = [&](int a, int q) { return sbase + a * g.total + g.off[q]; };
   for (int q = 0; q < g.count; ++q) {
-    const DLevel<TM> L = sl(q);
-    const DLevel<TM>& G = g.lv[q];
-    const int n = G.w * G.h;
-    for (int k = tid; k < n; k += nt) {
-      L.z[k] = (TM)0;
-      L.r[k] = q == 0 ? G.r[k] : (TM)0;
-      L.diag[k] = G.diag[k];
-      L.wd[k] = G.wd[k];
-      L.east[k] = G.east[k];
-      L.south[k] = G.south[k];
-    }
-  }
-  __syncthreads();
-  for (int q = 0; q + 1 < g.count; ++q) {
-    const DLevel<TM> L = sl(q);
-    const int n = L.w * L.h;
-    const int ncol = (L.wrap && (L.w & 1)) ? 4 : 2;
-    for (int sweep = 0; sweep < nu; ++sweep)
-      for (int c = 0; c < ncol; ++c) {
-        for (int k = tid; k < n; k += nt) {
-          const int j = k / L.w, i = k - j * L.w;
-          if (gs_colour(L.w, L.wrap, i, j) != c) continue;
-          if (sweep == 0)
-            gs_cell_at<TM, true>(L, L.z, c, k, i, j);
-          else
-            gs_cell_at<TM, false>(L, L.z, c, k, i, j);
-        }
-        __syncthreads();
-      }
-    const DLevel<TM> C = sl(q + 1);
-    for (int k = tid; k < C.w * C.h; k += nt) restrict_cell<TM>(L, L.z, C, k);
-    __syncthreads();
-  }
-  {
-    // the coarsest level (at most 128 cells, one a thread) on the block's first 128 threads:
-    // coarsest_solve's Gauss-Seidel passes in place on the staged z, with a barrier of those
-    // threads between passes
-    const DLevel<TM> L = sl(g.count - 1);
-    if (tid < 128) {
-      const int n = L.w * L.h;
-      const int ncol = (L.wrap && (L.w & 1)) ? 4 : 2;
-      const int j = tid / L.w, i = tid - j * L.w;
-      for (int pass = 0; pass < 2 * coarse_sweeps; ++pass) {
-        const bool forward = pass < coarse_sweeps;
-        for (int q = 0; q < ncol; ++q) {
-          const int colour = forward ? q : ncol - 1 - q;
-          if (tid < n && gs_colour(L.w, L.wrap, i, j) == colour) {
-            TM az = mg_apply_at<TM>(L, L.z, nullptr, 0, i, j);
-            L.z[tid] = L.z[tid] + mulr(L.r[tid] - az, L.wd[tid]);
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (int q = g.count - 2; q >= 0; --q) {
-    const DLevel<TM> L = sl(q), C = sl(q + 1);
-    const int n = L.w * L.h;
-    const int ncol = (L.wrap && (L.w & 1)) ? 4 : 2;
-    for (int k = tid; k < n; k += nt) {
-      const int j = k / L.w, i = k - j * L.w;
-      L.z[k] += C.z[(j / 2) * C.w + i / 2];
-    }
-    __syncthreads();
-    for (int sweep = 0; sweep < nu; ++sweep)
-      for (int c = ncol - 1; c >= 0; --c) {
-        for (int k = tid; k < n; k += nt) {
-          const int j = k / L.w, i = k - j * L.w;
-          if (gs_colour(L.w, L.wrap, i, j) != c) continue;
-          gs_cell_at<TM, false>(L, L.z, c, k, i, j);
-        }
-        __syncthreads();
-      }
-  }
-  {
-    const DLevel<TM> L = sl(0);
-    for (int k = tid; k < L.w * L.h; k += nt) g.lv[0].z[k] = L.z[k];
-  }
-}
-
-// The damped-Jacobi V-cycle's part from a level of at most MG_BLOCK_CELLS cells down, in one block:
-// the separate launches' passes in their order (first sweep, sweep, restriction; the coarsest
-// level's 16 sweeps; the corrected sweep and another), a block barrier where a launch ended. Bound by
-// the barriers' latency: some 35 phases instead of as many launches of 5 us. Seven arrays a level
-// in shared memory (z and the sweeps' other buffer t).
-template <class TM>
-__global__ void __launch_bounds__(1024) k_mg_coarse_jacobi(MgChain<TM> g, int nu, int coarse_sweeps) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  extern __shared__ __align__(16) unsigned char mg_chain_smem[];
-  TM* const sbase = reinterpret_cast<TM*>(mg_chain_smem);
-  auto sl = [&](int q) {
-    DLevel<TM> L = g.lv[q];
-    TM** const a[7] = {&L.z, &L.r, &L.diag, &L.wd, &L.east, &L.south, &L.t};
-    for (int k = 0; k < 7; ++k) *a[k] = sbase + k * g.total + g.off[q];
-    return L;
-  };
-  for (int q = 0; q < g.count; ++q) {
-    const DLevel<TM> L = sl(q);
     const DLevel<TM>& G = g.lv[q];
     for (int k = tid; k < G.w * G.h; k += nt) {
-      L.diag[k] = G.diag[k];
-      L.wd[k] = G.wd[k];
-      L.east[k] = G.east[k];
-      L.south[k] = G.south[k];
-      if (q == 0) L.r[k] = G.r[k];
+      arr(0, q)[k] = (TM)0;
+      if (q == 0) arr(2, q)[k] = G.r[k];
+      arr(3, q)[k] = G.diag[k];
+      arr(4, q)[k] = G.wd[k];
+      arr(5, q)[k] = G.east[k];
+      arr(6, q)[k] = G.south[k];
     }
   }
   __syncthreads();
-  // one sweep of k_mg_sweep over the level
-  auto sweep = [&](const DLevel<TM>& L, const TM* zin, TM* zo, const TM* zc, int wc) {
-    for (int k = tid; k < L.w * L.h; k += nt) {
-      const int j = k / L.w, i = k - j * L.w;
-      TM zk = zin[k];
-      if (zc) zk += zc[(j / 2) * wc + i / 2];
-      const TM az = mg_apply_at<TM>(L, zin, zc, wc, i, j);
-      zo[k] = zk + L.wd[k] * (L.r[k] - az);
+  auto cells = [&](int q) { return g.lv[q].w * g.lv[q].h; };
+  auto threads = [&](int q) { return min(nt, (cells(q) + 31) & ~31); };
+  auto bar = [&](int q) { asm volatile("bar.sync %0, %1;" ::"r"(q + 1), "r"(threads(q)) : "memory"); };
+  MgCell<TM> cell[2];
+  bool has[2];
+  auto load = [&](int q) {
+    const int w = g.lv[q].w, h = g.lv[q].h, wrap = g.lv[q].wrap;
+    const TM *east = arr(5, q), *south = arr(6, q);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int k = tid + u * nt;
+      has[u] = k < w * h;
+      if (!has[u]) continue;
+      const int j = k / w, i = k - j * w;
+      MgCell<TM>& c = cell[u];
+      c.k = k;
+      c.d = arr(3, q)[k];
+      c.wd = arr(4, q)[k];
+      c.r = arr(2, q)[k];
+      const bool he = i + 1 < w || wrap, hw = i > 0 || wrap;
+      c.ke = i + 1 < w ? k + 1 : wrap ? j * w : k;
+      c.kw = i > 0 ? k - 1 : wrap ? k + w - 1 : k;
+      c.ks = j + 1 < h ? k + w : k;
+      c.kn = j > 0 ? k - w : k;
+      c.e = he ? east[k] : (TM)0;
+      c.w = hw ? east[c.kw] : (TM)0;
+      c.s = j + 1 < h ? south[k] : (TM)0;
+      c.n = j > 0 ? south[k - w] : (TM)0;
+      c.seam = wrap && i == w - 1;
+      c.colour = gs_colour(w, wrap, i, j);
     }
-    __syncthreads();
   };
-  auto first = [&](const DLevel<TM>& L) {
-    for (int k = tid; k < L.w * L.h; k += nt) L.z[k] = L.wd[k] * L.r[k];
-    __syncthreads();
+  // `count` sweeps of level q on its current z (in buffer `cur`, 0 z or 1 t; Gauss-Seidel: z in place,
+  // colours up when `forward`); the buffer that holds the result
+  auto sweeps = [&](int q, int cur, int count, bool forward) {
+    if constexpr (JAC) {
+      for (int sw = 0; sw < count; ++sw, cur ^= 1) {
+        const TM* zi = arr(cur, q);
+        TM* zo = arr(cur ^ 1, q);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (has[u]) {
+            const TM zk = zi[cell[u].k];
+            zo[cell[u].k] = zk + cell[u].wd * (cell[u].r - cell[u].apply(zi));
+          }
+        bar(q);
+      }
+    } else {
+      const int ncol = (g.lv[q].wrap && (g.lv[q].w & 1)) ? 4 : 2;
+      TM* z = arr(0, q);
+      for (int sw = 0; sw < count; ++sw)
+        for (int p = 0; p < ncol; ++p) {
+          const int colour = forward ? p : ncol - 1 - p;
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            if (has[u] && cell[u].colour == colour) z[cell[u].k] += mulr(cell[u].r - cell[u].apply(z), cell[u].wd);
+          bar(q);
+        }
+    }
+    return cur;
   };
-  // after the sweeps down a level's z is in t when nu is even, else in z
-  for (int q = 0; q + 1 < g.count; ++q) {
-    const DLevel<TM> L = sl(q), C = sl(q + 1);
-    first(L);
-    TM *cur = L.z, *nxt = L.t;
-    for (int k = 1; k < nu; ++k) {
-      sweep(L, cur, nxt, nullptr, 0);
-      TM* u = cur;
-      cur = nxt;
-      nxt = u;
+  // z = wd r, Jacobi's first sweep
+  auto first = [&](int q) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (has[u]) arr(0, q)[cell[u].k] = cell[u].wd * cell[u].r;
+    bar(q);
+  };
+  // a Jacobi level's z is in buffer `down` after its nu sweeps down (the first in z)
+  const int last = g.count - 1, down = JAC ? (nu - 1) & 1 : 0;
+  int q = 0;
+  for (; tid < threads(q); ++q) {
+    load(q);
+    if (q > 0) {
+      // r: the sum over the block of 2 x 2 finer cells of their residuals
+      const int w = g.lv[q].w, wf = g.lv[q - 1].w, hf = g.lv[q - 1].h;
+      const TM* res = arr(down ^ 1, q - 1);
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (has[u]) {
+          const int jc = cell[u].k / w, ic = cell[u].k - jc * w;
+          TM acc = 0;
+          for (int j = 2 * jc; j < min(2 * jc + 2, hf); ++j)
+            for (int i = 2 * ic; i < min(2 * ic + 2, wf); ++i) acc += res[j * wf + i];
+          cell[u].r = acc;
+          arr(2, q)[cell[u].k] = acc;
+        }
     }
-    for (int k = tid; k < C.w * C.h; k += nt) restrict_cell<TM>(L, cur, C, k);
-    __syncthreads();
+    if (JAC) first(q);
+    if (q == last) break;
+    if (JAC)
+      sweeps(q, 0, nu - 1, true);
+    else
+      sweeps(q, 0, nu, true);
+    // the residuals into the buffer that does not hold z
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (has[u]) arr(down ^ 1, q)[cell[u].k] = cell[u].r - cell[u].apply(arr(down, q));
+    bar(q);
   }
-  const TM* zc;
-  {
-    const DLevel<TM> L = sl(g.count - 1);
-    first(L);
-    TM *cur = L.z, *nxt = L.t;
-    for (int k = 1; k < coarse_sweeps; ++k) {
-      sweep(L, cur, nxt, nullptr, 0);
-      TM* u = cur;
-      cur = nxt;
-      nxt = u;
+  int top = down;  // the buffer of the finest level's result
+  if (q == last && tid < threads(last)) {
+    int cur;
+    if (JAC) {
+      cur = sweeps(last, 0, coarse_sweeps - 1, true);
+    } else {
+      sweeps(last, 0, coarse_sweeps, true);
+      cur = sweeps(last, 0, coarse_sweeps, false);
     }
-    zc = cur;
-  }
-  for (int q = g.count - 2; q >= 0; --q) {
-    const DLevel<TM> L = sl(q);
-    const int wc = g.lv[q + 1].w;
-    TM *cur = nu & 1 ? L.z : L.t, *nxt = nu & 1 ? L.t : L.z;
-    for (int k = 0; k < nu; ++k) {
-      sweep(L, cur, nxt, k == 0 ? zc : nullptr, wc);
-      TM* u = cur;
-      cur = nxt;
-      nxt = u;
+    if (last == 0) top = cur;
+    // the level above reads the result from z
+    if (last > 0 && cur == 1) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (has[u]) arr(0, last)[cell[u].k] = arr(1, last)[cell[u].k];
     }
-    zc = cur;
   }
-  for (int k = tid; k < g.lv[0].w * g.lv[0].h; k += nt) g.lv[0].z[k] = zc[k];
+  // where a level's result lies on the way up: nu sweeps from `down`
+  const int up = JAC ? (down + nu) & 1 : 0;
+  for (q = min(q, g.count) - 1; q >= 0; --q) {
+    bar(q);  // the coarser level's result is there
+    load(q);
+    const int wc = g.lv[q + 1].w, w = g.lv[q].w;
+    const TM* zc = arr(q + 1 == last ? 0 : up, q + 1);
+    TM* z = arr(down, q);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (has[u]) {
+        const int j = cell[u].k / w, i = cell[u].k - j * w;
+        z[cell[u].k] += zc[(j / 2) * wc + i / 2];
+      }
+    bar(q);
+    top = sweeps(q, down, nu, false);
+  }
+  if (tid < threads(0)) {
+    // every thread of the finest level wrote its own cells
+    for (int k = tid; k < cells(0); k += nt) g.lv[0].z[k] = arr(top, 0)[k];
+  }
 }
 
 // A level's smoothing in one launch: both sweeps of the pre-smoothing from z = 0 with the residual
@@ -839,9 +873,13 @@ __device__ __forceinline__ Pair2<TM> mg_load2(const TM* __restrict__ a, int row,
   return p;
 }
 
-template <class TM, bool RB, bool PRE, int RPW, bool VEC>
+//
+// DOT (the finest level's post-smoothing in an FP32 CG): r . z too, so that the two are not read again
+// for it (62 us at 8192 x 4096).
+template <class TM, bool RB, bool PRE, int RPW, bool VEC, bool DOT>
 __global__ void __launch_bounds__(32 * MG_WARPS, sizeof(TM) == 4 ? 2 : 1)
-    k_mg_tile(DLevel<TM> L, DLevel<TM> C, const TM* __restrict__ zc, TM* __restrict__ zout) {
+    k_mg_tile(DLevel<TM> L, DLevel<TM> C, const TM* __restrict__ zc, TM* __restrict__ zout, double* partials, DScalars* S) {
+  static_assert(!(PRE && DOT), "r . z of the cycle's result");
   constexpr int H = RB ? 4 : 2, R = MG_WARPS * RPW, TX = 64 - 2 * H, TY = R - 2 * H;
   static_assert(RPW % 2 == 0 && TX % 2 == 0 && TY % 2 == 0, "even rows: a cell's colour and its coarse cell are known per row");
   // the warps' first and last rows, two buffers by pass
@@ -981,21 +1019,32 @@ __global__ void __launch_bounds__(32 * MG_WARPS, sizeof(TM) == 4 ? 2 : 1)
       }
     }
   }
-  if (!lanes_in || raw >= w) return;
+  Acc<1> acc;
+  acc.v[0] = 0.0;
 #pragma unroll
   for (int q = 0; q < RPW; ++q) {
-    const int j = j0 + q, rr = warp * RPW + q;
-    if (rr < H || rr >= R - H || j >= h) continue;
+    const int j = j0 + q, rr = warp * RPW + q, at = j * w + raw;
+    if (!lanes_in || raw >= w || rr < H || rr >= R - H || j >= h) continue;
     if constexpr (VEC) {
       using V = typename std::conditional<sizeof(TM) == 4, float2, double2>::type;
       V t;
       t.x = z[q].v[0];
       t.y = z[q].v[1];
-      *reinterpret_cast<V*>(zout + (j * w + raw)) = t;
+      *reinterpret_cast<V*>(zout + at) = t;
     } else {
-      zout[j * w + raw] = z[q].v[0];
-      if (raw + 1 < w) zout[j * w + raw + 1] = z[q].v[1];
+      zout[at] = z[q].v[0];
+      if (raw + 1 < w) zout[at + 1] = z[q].v[1];
     }
+    if constexpr (DOT) {
+      acc.v[0] += (double)r[q].v[0] * (double)z[q].v[0];
+      if (VEC || raw + 1 < w) acc.v[0] += (double)r[q].v[1] * (double)z[q].v[1];
+    }
+  }
+  if constexpr (DOT) {
+    if (S->stop) return;
+    const int kind[1] = {0};
+    if (reduce_partials<1>(acc, kind, partials, &S->ticket[DSITE_RZ], gridDim.x * gridDim.y) && threadIdx.x == 0)
+      d_finish_rz(S, acc.v[0]);
   }
 }
 
@@ -1355,7 +1404,7 @@ __global__ void k_d_rr_is_bb(DScalars* S) { S->rr = S->bb; }
 // first residual's RMS). In an iteration that replaces the residual (gate_it == it):
 //   k_d_rel_accumulate                x64 += x32 / s; x32 = 0
 //   k_d_apply<.., DA_RESID_GATED>     r64 = b - A x64, ||r64||^2 -> rr_true
-//   k_d_rel_reset                     r32 = s r64 (and the cycle's copy); rr, maxrr from rr_true;
+//   k_d_rel_reset                     r32 = s r64; rr, maxrr from rr_true;
 //                                     stop when rr_true meets the tolerance
 __global__ void k_d_rel_accumulate(size_t n, double* __restrict__ x, float* __restrict__ x32, const double* scale,
                                    const DScalars* S) {
@@ -1366,14 +1415,11 @@ __global__ void k_d_rel_accumulate(size_t n, double* __restrict__ x, float* __re
     x32[k] = 0.0f;
   }
 }
-__global__ void k_d_rel_reset(size_t n, const double* __restrict__ r, float* __restrict__ r32, float* __restrict__ rm,
-                              const double* scale, DScalars* S) {
+__global__ void k_d_rel_reset(size_t n, const double* __restrict__ r, float* __restrict__ r32, const double* scale, DScalars* S) {
   if (S->stop || S->gate_it != S->it) return;
   double sc = *scale;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-    float v = (float)(r[k] * sc);
-    r32[k] = v;
-    rm[k] = v;
+    r32[k] = (float)(r[k] * sc);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     double rr = S->rr_true * sc * sc;
@@ -1420,7 +1466,6 @@ static const int COARSEST = 64;     // multigrid.rs:54
 static const int COARSE_SWEEPS = 16;  // multigrid.rs:56
 static const int COARSEST_GS = 128;   // the Gauss-Seidel cycle's coarsest level: 16 x 8 cells
 static const int COARSE_SWEEPS_GS = 8;
-static const int MG_BLOCK_CELLS = 2048;  // Gauss-Seidel levels this small run their part of the cycle in one block
 
 template <class TM>
 struct Hier {
@@ -1458,7 +1503,7 @@ struct dt_diff {
   dt::Hier<float> hf[2];
   dt::Hier<double> hd[2];
   dt::DGraph graph[4][2];  // [lane: 0 split, 1 FP64, 2 FP32 inner, 3 FP32 reliable][cycle]
-  // the cycles' fused kernels (k_mg_tile, k_mg_coarse_rb, k_mg_coarse_jacobi); DT_MG_FUSED=0 at
+  // the cycles' fused kernels (k_mg_tile, k_mg_coarse); DT_MG_FUSED=0 at
   // create keeps one launch per sweep or colour pass (the same values)
   bool mg_fused = true;
   // k_mg_tile's 64-row regions on FP32 levels of many tiles; DT_MG_BIG_TILES=0 at create keeps
@@ -1489,6 +1534,21 @@ static unsigned int dgrid(const dt_diff* s, size_t n) {
   return std::max(1u, std::min<unsigned int>(ceil_div(n, 256), (unsigned)s->sms * 8));
 }
 
+static void finest_arrays(dt_diff* s, DLevel<float>& L) {
+  L.east = s->east32;
+  L.south = s->south32;
+  L.diag = s->diag32;
+  L.r = s->r32;
+  L.mass = nullptr;
+}
+static void finest_arrays(dt_diff* s, DLevel<double>& L) {
+  L.east = s->east;
+  L.south = s->south;
+  L.diag = s->diag;
+  L.r = s->r;
+  L.mass = nullptr;
+}
+
 // The level shapes of the hierarchy (multigrid.rs:117-123): halve (rounding up) until the level
 // has at most `coarsest` cells or stops shrinking; x wraps on a level while it is wider than 1.
 template <class TM>
@@ -1501,7 +1561,14 @@ static dt_status build_levels(dt_diff* s, Hier<TM>& H, int coarsest) {
     L.h = h;
     L.wrap = wrap;
     size_t n = (size_t)w * h;
-    for (TM** q : {&L.east, &L.south, &L.diag, &L.wd, &L.mass, &L.r, &L.z, &L.t}) DT_TRY(ddalloc(s, q, n));
+    for (TM** q : {&L.wd, &L.z, &L.t}) DT_TRY(ddalloc(s, q, n));
+    if (H.lv.empty()) {
+      // the finest level: the operator's coefficients and the CG's residual (FP64 CG around an FP32
+      // cycle leaves that residual's FP32 copy there), every mass 1
+      finest_arrays(s, L);
+    } else {
+      for (TM** q : {&L.east, &L.south, &L.diag, &L.mass, &L.r}) DT_TRY(ddalloc(s, q, n));
+    }
     H.lv.push_back(L);
     int wc = (w + 1) / 2, hc = (h + 1) / 2;
     if ((long)w * h <= coarsest || (wc == w && hc == h)) break;
@@ -1513,14 +1580,14 @@ static dt_status build_levels(dt_diff* s, Hier<TM>& H, int coarsest) {
   return DT_OK;
 }
 
-// Level coefficients for the current operator: the finest from the FP64 couplings, the rest by
+// Level coefficients for the current operator: the finest are the operator's, the rest by
 // aggregation.
 // wd: omega / diag for the damped-Jacobi cycle, 1 / diag for the Gauss-Seidel one.
 template <class TM>
 static void fill_levels(dt_diff* s, Hier<TM>& H, int kind, cudaStream_t st) {
   DLevel<TM>& f = H.lv[0];
   const TM omega = kind == DT_CYCLE_JACOBI ? (TM)OMEGA : (TM)1;
-  k_mg_finest<TM><<<dgrid(s, s->n), 256, 0, st>>>(s->n, s->east, s->south, s->diag, omega, f.east, f.south, f.diag, f.wd, f.mass);
+  k_mg_finest<TM><<<dgrid(s, s->n), 256, 0, st>>>(s->n, f.diag, omega, f.wd);
   count_launch();
   for (size_t l = 1; l < H.lv.size(); ++l) {
     size_t nc = (size_t)H.lv[l].w * H.lv[l].h;
@@ -1531,31 +1598,49 @@ static void fill_levels(dt_diff* s, Hier<TM>& H, int kind, cudaStream_t st) {
   }
 }
 
+// An FP32 CG's r . z asked of its cycle: `done` once the finest level's post-smoothing forms it.
+struct RzArg {
+  DScalars* S;
+  bool done;
+};
 // A level's smoothing by k_mg_tile (PRE: from z = 0, the restriction into C.r; else with the coarse
 // correction zc).
-template <class TM, bool RB, bool PRE, int RPW>
-static void launch_tile_rows(const DLevel<TM>& L, const DLevel<TM>& C, const TM* zc, TM* zout, cudaStream_t st) {
+template <class TM, bool RB, bool PRE, int RPW, bool DOT>
+static void launch_tile_rows(dt_diff* s, const DLevel<TM>& L, const DLevel<TM>& C, const TM* zc, TM* zout, DScalars* S,
+                             cudaStream_t st) {
   constexpr int H = RB ? 4 : 2;
   const dim3 tg(ceil_div(L.w, 64 - 2 * H), ceil_div(L.h, MG_WARPS * RPW - 2 * H));
   if (L.w % 2 == 0)
-    k_mg_tile<TM, RB, PRE, RPW, true><<<tg, 32 * MG_WARPS, 0, st>>>(L, C, zc, zout);
+    k_mg_tile<TM, RB, PRE, RPW, true, DOT><<<tg, 32 * MG_WARPS, 0, st>>>(L, C, zc, zout, s->partials, S);
   else
-    k_mg_tile<TM, RB, PRE, RPW, false><<<tg, 32 * MG_WARPS, 0, st>>>(L, C, zc, zout);
+    k_mg_tile<TM, RB, PRE, RPW, false, DOT><<<tg, 32 * MG_WARPS, 0, st>>>(L, C, zc, zout, s->partials, S);
 }
-template <class TM, bool RB, bool PRE>
-static void launch_tile(dt_diff* s, const DLevel<TM>& L, const DLevel<TM>& C, const TM* zc, TM* zout, cudaStream_t st) {
+template <class TM, bool RB, bool PRE, bool DOT>
+static void launch_tile_dot(dt_diff* s, const DLevel<TM>& L, const DLevel<TM>& C, const TM* zc, TM* zout, DScalars* S,
+                            cudaStream_t st) {
   // 64-row regions on FP32 levels where those alone make at least four tiles an SM (FP64 rows of
   // four would not fit the registers)
   if constexpr (sizeof(TM) == 4) {
     constexpr int H = RB ? 4 : 2;
     if (s->mg_big_tiles && (size_t)ceil_div(L.w, 64 - 2 * H) * ceil_div(L.h, 64 - 2 * H) >= (size_t)4 * s->sms) {
-      launch_tile_rows<TM, RB, PRE, 4>(L, C, zc, zout, st);
-      count_launch();
+      launch_tile_rows<TM, RB, PRE, 4, DOT>(s, L, C, zc, zout, S, st);
       return;
     }
   }
-  launch_tile_rows<TM, RB, PRE, 2>(L, C, zc, zout, st);
+  launch_tile_rows<TM, RB, PRE, 2, DOT>(s, L, C, zc, zout, S, st);
+}
+template <class TM, bool RB, bool PRE>
+static void launch_tile(dt_diff* s, const DLevel<TM>& L, const DLevel<TM>& C, const TM* zc, TM* zout, cudaStream_t st,
+                        RzArg* rz = nullptr) {
   count_launch();
+  if constexpr (!PRE && sizeof(TM) == 4) {
+    if (rz) {
+      launch_tile_dot<TM, RB, PRE, true>(s, L, C, zc, zout, rz->S, st);
+      rz->done = true;
+      return;
+    }
+  }
+  launch_tile_dot<TM, RB, PRE, false>(s, L, C, zc, zout, nullptr, st);
 }
 // k_mg_tile's 32-bit offsets
 template <class TM>
@@ -1563,9 +1648,10 @@ static bool tile_fits(const DLevel<TM>& L) {
   return (size_t)L.w * L.h < ((size_t)1 << 31);
 }
 
-// One V-cycle from z = 0 on level l with r set; returns the buffer holding the level's z.
+// One V-cycle from z = 0 on level l with r set; returns the buffer holding the level's z. With `rz` on
+// the finest level, r . z as well where its post-smoothing forms it (rz->done).
 template <class TM>
-static TM* vcycle(dt_diff* s, Hier<TM>& H, size_t l, int kind, cudaStream_t st) {
+static TM* vcycle(dt_diff* s, Hier<TM>& H, size_t l, int kind, cudaStream_t st, RzArg* rz = nullptr) {
   DLevel<TM>& L = H.lv[l];
   size_t n = (size_t)L.w * L.h;
   unsigned int g = dgrid(s, n);
@@ -1590,13 +1676,13 @@ static TM* vcycle(dt_diff* s, Hier<TM>& H, size_t l, int kind, cudaStream_t st) 
         m.off[q] = m.total;
         m.total += H.lv[l + q].w * H.lv[l + q].h;
       }
-      const size_t smem = (size_t)(kind == DT_CYCLE_JACOBI ? 7 : 6) * m.total * sizeof(TM);
+      const size_t smem = (size_t)7 * m.total * sizeof(TM);
       const DLevel<TM>& last = H.lv.back();
-      if (smem <= 200 * 1024 && last.w * last.h <= 128) {  // the coarsest takes one thread a cell of 128
+      if (smem <= 200 * 1024 && last.w * last.h <= 128) {
         if (kind == DT_CYCLE_JACOBI)
-          k_mg_coarse_jacobi<TM><<<1, 1024, smem, st>>>(m, NU, COARSE_SWEEPS);
+          k_mg_coarse<TM, true><<<1, 1024, smem, st>>>(m, NU, COARSE_SWEEPS);
         else
-          k_mg_coarse_rb<TM><<<1, 1024, smem, st>>>(m, NU, COARSE_SWEEPS_GS);
+          k_mg_coarse<TM, false><<<1, 1024, smem, st>>>(m, NU, COARSE_SWEEPS_GS);
         count_launch();
         return L.z;
       }
@@ -1611,9 +1697,9 @@ static TM* vcycle(dt_diff* s, Hier<TM>& H, size_t l, int kind, cudaStream_t st) 
         launch_tile<TM, true, true>(s, L, C, nullptr, L.z, st);
       TM* zc = vcycle<TM>(s, H, l + 1, kind, st);
       if (jacobi)
-        launch_tile<TM, false, false>(s, L, C, zc, L.t, st);
+        launch_tile<TM, false, false>(s, L, C, zc, L.t, st, rz);
       else
-        launch_tile<TM, true, false>(s, L, C, zc, L.t, st);
+        launch_tile<TM, true, false>(s, L, C, zc, L.t, st, rz);
       return L.t;  // the level's z, in its spare buffer
     }
   }
@@ -1673,6 +1759,18 @@ struct CgLane {
   TM* z;  // where the cycle leaves its result (set when the launch sequence is built)
 };
 
+// z = M^-1 r by one cycle, and r . z
+template <class TC, class TM>
+static TM* cycle_rz(dt_diff* s, CgLane<TC, TM>& C, int kind, cudaStream_t st) {
+  RzArg rz{C.S, false};
+  TM* z = vcycle<TM>(s, *C.H, 0, kind, st, std::is_same<TC, float>::value ? &rz : nullptr);
+  if (!rz.done) {
+    k_d_rz<TC, TM><<<dgrid(s, s->n), 256, 0, st>>>(s->n, C.r, z, s->partials, C.S);
+    count_launch();
+  }
+  return z;
+}
+
 // The residual replacement of a reliable-update iteration (the FP32 lane): gated kernels that do
 // nothing unless the iteration's update asked for it. `count`: count their launches (not inside
 // the loop body's IF node, whose runs are counted from the replacements).
@@ -1681,7 +1779,7 @@ static void launch_reliable_d(dt_diff* s, Hier<float>& H, cudaStream_t st, bool 
   k_d_rel_accumulate<<<g, 256, 0, st>>>(s->n, s->x, s->x32, s->scale, s->S32);
   k_d_apply<double, float, DA_RESID_GATED><<<g, 256, 0, st>>>(s->w, s->h, s->wrap && s->w > 1, s->east, s->south, s->diag, s->x,
                                                               s->b, s->r, nullptr, s->partials, s->S32);
-  k_d_rel_reset<<<g, 256, 0, st>>>(s->n, s->r, s->r32, H.lv[0].r, s->scale, s->S32);
+  k_d_rel_reset<<<g, 256, 0, st>>>(s->n, s->r, s->r32, s->scale, s->S32);
   if (count)
     for (int k = 0; k < 3; ++k) count_launch();
 }
@@ -1729,7 +1827,8 @@ static dt_status cg_iteration(dt_diff* s, CgLane<TC, TM>& C, int kind, cudaStrea
   k_d_apply<TC, TM, DA_PAP><<<g, 256, 0, st>>>(s->w, s->h, s->wrap && s->w > 1, C.east, C.south, C.diag, C.p, nullptr, C.ap,
                                                 nullptr, s->partials, C.S);
   count_launch();
-  k_d_update<TC, TM><<<g, 256, 0, st>>>(s->n, C.x, C.r, C.H->lv[0].r, C.p, C.ap, s->partials, C.S);
+  k_d_update<TC, TM><<<g, 256, 0, st>>>(s->n, C.x, C.r, std::is_same<TC, TM>::value ? nullptr : C.H->lv[0].r, C.p, C.ap,
+                                        s->partials, C.S);
   count_launch();
   if constexpr (std::is_same<TM, float>::value) {
     if (reliable) {
@@ -1739,10 +1838,8 @@ static dt_status cg_iteration(dt_diff* s, CgLane<TC, TM>& C, int kind, cudaStrea
         launch_reliable_d(s, *C.H, st, true);
     }
   }
-  TM* z = vcycle<TM>(s, *C.H, 0, kind, st);
+  TM* z = cycle_rz<TC, TM>(s, C, kind, st);
   C.z = z;
-  k_d_rz<TC, TM><<<g, 256, 0, st>>>(s->n, C.r, z, s->partials, C.S);
-  count_launch();
   k_d_direction<TC, TM><<<g, 256, 0, st>>>(s->n, C.p, z, C.S, 0);
   count_launch();
   return DT_OK;
@@ -1813,10 +1910,8 @@ static dt_status run_cg(dt_diff* s, CgLane<TC, TM>& C, int lane, int kind, const
   k_d_begin<<<1, 1, 0, st>>>(C.S, prob, 0);
   count_launch();
   // the first direction: z = M^-1 r, rz, p = z
-  TM* z = vcycle<TM>(s, *C.H, 0, kind, st);
-  k_d_rz<TC, TM><<<g, 256, 0, st>>>(s->n, C.r, z, s->partials, C.S);
+  TM* z = cycle_rz<TC, TM>(s, C, kind, st);
   k_d_direction<TC, TM><<<g, 256, 0, st>>>(s->n, C.p, z, C.S, 1);
-  count_launch();
   count_launch();
   if (!host_loop) {
     DGraph* G;
@@ -1905,7 +2000,8 @@ static dt_status solve_fp64_cg(dt_diff* s, const dt_diff_params* p, int lane, dt
   // bb, then r = b - A x, rm, rr
   k_d_dot<double><<<g, 256, 0, st>>>(s->n, s->b, s->b, s->partials, s->S64);
   k_d_begin<<<1, 1, 0, st>>>(s->S64, DProblem{p->tol, p->max_iterations, p->stop, (int)s->n}, 1);
-  k_d_apply<double, TM, DA_RESID><<<g, 256, 0, st>>>(s->w, s->h, wrap, s->east, s->south, s->diag, s->x, s->b, s->r, H.lv[0].r,
+  k_d_apply<double, TM, DA_RESID><<<g, 256, 0, st>>>(s->w, s->h, wrap, s->east, s->south, s->diag, s->x, s->b, s->r,
+                                                     std::is_same<TM, double>::value ? nullptr : H.lv[0].r,
                                                      s->partials, s->S64);
   count_launch();
   count_launch();
@@ -1951,8 +2047,6 @@ static dt_status solve_mixed_cg(dt_diff* s, const dt_diff_params* p, dt_report* 
     k_d_dot<float><<<g, 256, 0, st>>>(s->n, s->r32, s->r32, s->partials, s->S32);
     k_d_begin<<<1, 1, 0, st>>>(s->S32, DProblem{itol, p->max_iterations - iterations, DT_STOP_REL_RESIDUAL, (int)s->n}, 1);
     k_d_rr_is_bb<<<1, 1, 0, st>>>(s->S32);
-    // the cycle's finest rhs is the inner CG's r in FP32
-    cudaMemcpyAsync(H.lv[0].r, s->r32, s->n * sizeof(float), cudaMemcpyDeviceToDevice, st);
     count_launch();
     count_launch();
     count_launch();
@@ -2001,7 +2095,6 @@ static dt_status solve_mixed_reliable(dt_diff* s, const dt_diff_params* p, dt_re
   // replace when the FP32 residual has fallen a hundredfold: the V-cycle cuts it more than
   // tenfold an iteration, so a tenfold trigger would replace it every iteration
   k_d_rel_init<<<1, 1, 0, st>>>(s->S32, s->S64, s->scale, 0.01, p->stop == DT_STOP_RMS_RESIDUAL);
-  DT_CUDA(cudaMemcpyAsync(H.lv[0].r, s->r32, s->n * sizeof(float), cudaMemcpyDeviceToDevice, st));  // the cycle's rhs
   for (int k = 0; k < 6; ++k) count_launch();
   CgLane<float, float> C{s->x32, s->r32, s->p32, s->ap32, s->east32, s->south32, s->diag32, &H, s->S32, nullptr};
   DScalars h32;
@@ -2076,11 +2169,11 @@ dt_status dt_diff_create(int w, int h, double dx, int wrap_x, dt_diff** out) {
   s->wrap = wrap_x ? 1 : 0;
   if (const char* e = getenv("DT_MG_FUSED")) s->mg_fused = e[0] != '0';
   // the one-block coarse cycle stages at most about 4/3 MG_BLOCK_CELLS cells (plus the levels'
-  // rounding up) in six arrays
-  cudaFuncSetAttribute(k_mg_coarse_rb<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_mg_coarse_rb<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_mg_coarse_jacobi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_mg_coarse_jacobi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  // rounding up) in seven arrays
+  cudaFuncSetAttribute(k_mg_coarse<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_mg_coarse<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_mg_coarse<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_mg_coarse<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (const char* e = getenv("DT_MG_BIG_TILES")) s->mg_big_tiles = e[0] != '0';
   s->n = (size_t)w * h;
   cudaDeviceProp prop;
@@ -2104,7 +2197,10 @@ dt_status dt_diff_create(int w, int h, double dx, int wrap_x, dt_diff** out) {
     const size_t chunks = (size_t)ceil_div(s->w, LOD_CHUNK) * s->h + (size_t)ceil_div(s->h, LOD_CHUNK) * s->w;
     if ((st = ddalloc(s, &s->lod[6], 12 * chunks + s->h + s->w)) != DT_OK) return fail(st);
   }
-  if ((st = ddalloc(s, &s->partials, (size_t)s->sms * 8 * 2)) != DT_OK) return fail(st);
+  // a reducing kernel's blocks: two values each of at most eight an SM, or one of each of
+  // k_mg_tile's tiles (56 x 24 cells at the least)
+  const size_t tiles = (size_t)ceil_div(s->w, 56) * ceil_div(s->h, 24);
+  if ((st = ddalloc(s, &s->partials, std::max((size_t)s->sms * 8 * 2, tiles))) != DT_OK) return fail(st);
   if ((st = ddalloc(s, &s->scale, 1)) != DT_OK) return fail(st);
   if ((st = ddalloc(s, &s->S64, 1)) != DT_OK) return fail(st);
   if ((st = ddalloc(s, &s->S32, 1)) != DT_OK) return fail(st);
