@@ -86,6 +86,19 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return __ffma2_rn(make_float2(-a.y, a.y), make_float2(b.y, b.x), __fmul2_rn(make_float2(a.x, a.x), b));
 }
 
+// Reciprocals of normal numbers with no slow-path call: float, the correctly rounded intrinsic;
+// double, of m 2^e, the hardware's float estimate of 1 / m, m in [1, 2), scaled by 2^-e in the exponent bits and refined by two Newton-Raphson steps r <- r + r (1 - x r)
+// (each squares the relative error: 2^-22 -> 2^-44 -> 2^-88, so the last rounding is what is left).
+__device__ __forceinline__ double recip(double x) {
+  const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
+  const double m = __hiloint2double(hi - (e << 20), __double2loint(x));
+  double r = (double)__fdividef(1.0f, (float)m);
+  r = __hiloint2double(__double2hiint(r) - (e << 20), __double2loint(r));
+  r = fma(r, fma(-x, r, 1.0), r);
+  return fma(r, fma(-x, r, 1.0), r);
+}
+__device__ __forceinline__ float recip(float x) { return __frcp_rn(x); }
+
 // ---- deterministic reductions -------------------------------------------------------------
 // A reducing kernel writes one partial per block (fixed grid, fixed in-block order); the last
 // block to finish (an atomic ticket) sums the partials in index order. The result therefore does

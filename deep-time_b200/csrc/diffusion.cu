@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include <cuda_pipeline.h>
 
 namespace dt {
 
@@ -642,7 +643,8 @@ __global__ void k_mg_coarsest(DLevel<TM> L, TM* __restrict__ z, int sweeps) {
 // places in registers through a level's passes, and a level's barriers take only the warps that hold
 // its cells (barrier q + 1; the others wait where they meet the level again on the way up). With the
 // indexes worked out in every pass and all 1024 threads in every barrier a Gauss-Seidel chain from
-// 64 x 32 cells took 29 us and a Jacobi one from 64 x 21 21.6 us; this RBCH and JACCH.
+// 64 x 32 cells took 29 us and a Jacobi one from 64 x 21 21.6 us; this 18.7 and
+// 14.4 (cold caches).
 constexpr int MG_BLOCK_LEVELS = 8;
 constexpr int MG_BLOCK_CELLS = 2048;  // two cells a thread
 template <class TM>
@@ -679,13 +681,15 @@ __global__ void __launch_bounds__(1024) k_mg_coarse(MgChain<TM> g, int nu, int c
     const DLevel<TM>& G = g.lv[q];
     for (int k = tid; k < G.w * G.h; k += nt) {
       arr(0, q)[k] = (TM)0;
-      if (q == 0) arr(2, q)[k] = G.r[k];
-      arr(3, q)[k] = G.diag[k];
-      arr(4, q)[k] = G.wd[k];
-      arr(5, q)[k] = G.east[k];
-      arr(6, q)[k] = G.south[k];
+      if (q == 0) __pipeline_memcpy_async(arr(2, q) + k, G.r + k, sizeof(TM));
+      __pipeline_memcpy_async(arr(3, q) + k, G.diag + k, sizeof(TM));
+      __pipeline_memcpy_async(arr(4, q) + k, G.wd + k, sizeof(TM));
+      __pipeline_memcpy_async(arr(5, q) + k, G.east + k, sizeof(TM));
+      __pipeline_memcpy_async(arr(6, q) + k, G.south + k, sizeof(TM));
     }
   }
+  __pipeline_commit();
+  __pipeline_wait_prior(0);
   __syncthreads();
   auto cells = [&](int q) { return g.lv[q].w * g.lv[q].h; };
   auto threads = [&](int q) { return min(nt, (cells(q) + 31) & ~31); };
@@ -1123,137 +1127,278 @@ __global__ void k_lod_rows(int w, int h, int wrap, double* __restrict__ hf, cons
   }
 }
 
-// 32 x 32 tiles through shared memory: out (cols x rows) = the transpose of in (rows x cols)
-__global__ void k_transpose(int rows, int cols, const double* __restrict__ in, double* __restrict__ out) {
-  __shared__ double tile[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int r = r0 + k, c = c0 + threadIdx.x;
-    if (r < rows && c < cols) tile[k][threadIdx.x] = in[(size_t)r * cols + c];
-  }
-  __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int c = c0 + k, r = r0 + threadIdx.x;
-    if (r < rows && c < cols) out[(size_t)c * rows + r] = tile[threadIdx.x][k];
-  }
-}
-
-// The LOD passes as partitioned tridiagonal solves: L independent lines of n unknowns, stored
-// line-fastest (element (l, i) at i L + l: the rows on transposed copies, the columns as they lie),
-// each split into chunks of LOD_CHUNK unknowns solved in parallel (L x chunks threads instead of
-// L): a thread eliminates its chunk (Thomas, diffusion.rs:1029-1046) for the right-hand sides
-// and for the two unit couplings to the unknowns just outside the chunk, y = p + q y_(s-1) +
-// r y_e; one thread a line then solves the chunks' end values from those relations (a two-term
-// recurrence, forward and back), and every cell forms its y. The coefficients are the LOD's
-// (diffusion.rs:370-489), formed on the fly from kd: faces 0.5 (k_i + k_(i+1)) dt / dx^2 and
-// diagonal (1 + west) + east. ROWS: the periodic rows through Sherman-Morrison (diffusion.rs:
-// 1048-1071): the system with the corners folded into the first and last diagonal, solved for b
-// and for u = (gamma, 0, .., 0, alpha), then x - fact z. Columns: rows closed, one right-hand side.
-constexpr int LOD_CHUNK = 64;
+// The LOD passes as partitioned tridiagonal solves: L independent lines of n unknowns, rows as they
+// lie (ROWS: the periodic rows, element (l, i) at l n + i) or columns (element (l, i) at i L + l).
+// A block takes G lines (columns: neighbouring ones, a row's segment of G words) over a segment of
+// 16 Pb unknowns, a thread 16 of them in registers:
+//   1. Thomas's elimination of the thread's chunk (diffusion.rs:1029-1046), with the chunk's first and
+//      last values as A = pA + qA y_left + rA y_right, B = pB + qB y_left + rB y_right, y_left and
+//      y_right the unknowns just outside it;
+//   2. neighbouring chunks merged pairwise up a tree in shared memory to the segment's own relation,
+//      and the outside values handed down it again;
+//   3. the chunk's solution from its outside values.
+// So kd and the right-hand side are read once and the solution written once (24 bytes a cell). Bound
+// by latency (16 dependent reciprocals, two passes over log2(Pb) tree levels) below about a wave of
+// blocks, then by HBM. As separate passes over scratch arrays, with the rows on transposed copies, the
+// two directions took 2.6 ms at 8192 x 4096 and 330 us at 2048 x 1024; this 1.1 ms and 65 us.
+// The coefficients are the LOD's (diffusion.rs:370-489), formed from kd: faces 0.5 (k_i + k_(i+1))
+// dt / dx^2 and diagonal (1 + west) + east. ROWS: Sherman-Morrison (diffusion.rs:1048-1071): the
+// corners folded into the first and last diagonal, solved for b and u = (gamma, 0, .., 0, alpha), then
+// x - fact z; u's response rides along as a second p, and the last step solves for b - fact u.
+// Lines of more than a segment: STEP 1 writes each segment's relation, k_lod_reduce solves those a
+// line, STEP 2 solves the segments between their outside values (kd and b read twice). STEP 0: one
+// segment a line.
+constexpr int LOD_CH = 16, LOD_THREADS = 512;
 template <bool ROWS>
 struct LodLine {
   const double* kd;
   int L, n, l;
   double dtdx2;
-  __device__ double K(int i) const { return kd[(size_t)i * L + l]; }
+  __device__ double K(int i) const { return ROWS ? kd[(size_t)l * n + i] : kd[(size_t)i * L + l]; }
   // the face between positions i and i + 1 (across the seam for the rows' last one)
   __device__ double face(int i) const {
     if (i + 1 < n) return 0.5 * (K(i) + K(i + 1)) * dtdx2;
     return ROWS ? 0.5 * (K(n - 1) + K(0)) * dtdx2 : 0.0;
   }
 };
-
-template <bool ROWS>
-__global__ void __launch_bounds__(128) k_lod_chunks(int L, int n, int P, double dtdx2, const double* __restrict__ kd,
-                                                    double* __restrict__ p0, double* __restrict__ p1, double* __restrict__ q,
-                                                    double* __restrict__ r, double* __restrict__ c, double* __restrict__ edge) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= L * P) return;
-  const int l = t % L, k = t / L;
-  const int s = k * LOD_CHUNK, e = min(s + LOD_CHUNK, n);
+// shared memory: 8 values a chunk's relation, 4 its outside values, and for the rows their kd and
+// right-hand side, spaced by one word after every 16 so that the threads' chunks fall in distinct banks
+__host__ __device__ constexpr size_t lod_smem(bool rows) {
+  return (size_t)LOD_THREADS * (12 + (rows ? 2 * (LOD_CH + 1) : 0)) * sizeof(double);
+}
+template <bool ROWS, int STEP>
+__global__ void __launch_bounds__(LOD_THREADS, 1) k_lod_lines(int L, int n, int Pb, int G, double dtdx2, const double* kd,
+                                                              const double* b, double* x, double* edge, const double* fact) {
+  extern __shared__ __align__(16) unsigned char lod_raw[];
+  double* const rel = reinterpret_cast<double*>(lod_raw);  // [8][threads]: pA0, pA1, qA, rA, pB0, pB1, qB, rB
+  double* const out = rel + 8 * LOD_THREADS;               // [4][threads]: y_left for b, for u; y_right for b, for u
+  double* const sk = out + 4 * LOD_THREADS;                // ROWS: kd, then b, of the block's lines
+  double* const sb = sk + LOD_THREADS * (LOD_CH + 1);
+  __shared__ double s_fact[LOD_THREADS];
+  const int tid = threadIdx.x, nt = Pb * G;
+  const int c = ROWS ? tid % Pb : tid / G, g = ROWS ? tid / Pb : tid % G;
+  const int l = blockIdx.x * G + g, s0 = blockIdx.y * Pb * LOD_CH, s = s0 + c * LOD_CH;
+  const bool on = tid < nt && l < L;
+  const int len = on ? min(max(n - s, 0), LOD_CH) : 0;
+  const int chunks = (min(n - s0, Pb * LOD_CH) + LOD_CH - 1) / LOD_CH;  // of this segment
   const LodLine<ROWS> ln{kd, L, n, l, dtdx2};
-  auto at = [&](int i) { return (size_t)i * L + l; };
+  double kv[LOD_CH + 2], p[LOD_CH], m[LOD_CH], cc[LOD_CH];  // kv: columns only, kd of s - 1 .. s + LOD_CH
+  double k_before = 0.0, k_after = 0.0, k_first = 0.0, k_last = 0.0;
+  if constexpr (ROWS) {
+    const int width = min(n - s0, Pb * LOD_CH), lines = min(G, L - (int)blockIdx.x * G);
+    for (int e = tid; e < lines * width; e += blockDim.x) {
+      const int ge = e / width, i = e - ge * width;
+      const size_t src = (size_t)(blockIdx.x * G + ge) * n + s0 + i;
+      const int dst = ge * Pb * (LOD_CH + 1) + i + i / LOD_CH;
+      __pipeline_memcpy_async(sk + dst, kd + src, 8);
+      __pipeline_memcpy_async(sb + dst, b + src, 8);
+    }
+    __pipeline_commit();
+    if (len > 0) {
+      if (s > 0) k_before = ln.K(s - 1);
+      if (s + len < n) k_after = ln.K(s + len);
+      k_first = ln.K(0);
+      k_last = ln.K(n - 1);
+    }
+    __pipeline_wait_prior(0);
+    __syncthreads();
+  } else {
+#pragma unroll
+    for (int t = 0; t < LOD_CH + 2; ++t) {
+      const int i = s + t - 1;
+      kv[t] = len > 0 && i >= 0 && i < n ? ln.K(i) : 0.0;
+    }
+#pragma unroll
+    for (int t = 0; t < LOD_CH; ++t) p[t] = t < len ? b[(size_t)(s + t) * L + l] : 0.0;
+  }
+  double* const mk = sk + (g * Pb + c) * (LOD_CH + 1);
+  double* const mb = sb + (g * Pb + c) * (LOD_CH + 1);
+
   // rows: the folded corners (k_lod_rows' alpha = up[n-1], beta = lo[0], gamma = -di[0])
-  double fw = 0.0, alpha = 0.0, beta = 0.0, gamma = -1.0;
-  if (ROWS) {
-    fw = ln.face(n - 1);
-    const double di0 = 1.0 + fw + ln.face(0);
+  double fw = 0.0, alpha = 0.0, gamma = -1.0;
+  if (ROWS && len > 0) {
+    fw = 0.5 * (k_last + k_first) * dtdx2;
     alpha = -fw;
-    beta = -fw;
-    gamma = -di0;
+    if (s == 0) gamma = -(1.0 + fw + 0.5 * (k_first + (len > 1 ? mk[1] : k_after)) * dtdx2);
+    else if (s + len == n) gamma = -(1.0 + fw + ln.face(0));
   }
-  double west = s == 0 ? (ROWS ? fw : 0.0) : ln.face(s - 1);
-  double bt = 1.0, cprev = 0.0, pv0 = 0.0, pv1 = 0.0, qv = 0.0, rv = 0.0;
-  // the walk's inputs one position ahead (K(i + 1) and the right-hand side), so that their loads
-  // overlap the recurrence; each K read once (face(i) = 0.5 (K(i) + K(i + 1)) dt / dx^2)
-  double kn = ln.K(s), bn = p0[at(s)];
-  for (int i = s; i < e; ++i) {
-    const double ki = kn, b0 = bn;
-    double east;
-    if (i + 1 < n) {
-      kn = ln.K(i + 1);
-      east = 0.5 * (ki + kn) * dtdx2;
-    } else {
-      east = ROWS ? 0.5 * (ki + ln.K(0)) * dtdx2 : 0.0;
+  double lo0 = 0.0, ib0 = 0.0, ibl = 0.0;
+  // kd of the chunk's unknowns t = -1 .. len
+  auto K = [&](int t) {
+    if constexpr (ROWS)
+      return t < 0 ? k_before : t < len ? mk[t] : k_after;
+    else
+      return kv[t + 1];
+  };
+  {
+    double west = s == 0 ? (ROWS ? fw : 0.0) : 0.5 * (K(-1) + K(0)) * dtdx2, last_c = 0.0;
+    double pv = 0.0, ev = 0.0, pA0 = 0.0, pA1 = 0.0, eA = 0.0, rA = 1.0;
+#pragma unroll
+    for (int t = 0; t < LOD_CH; ++t) {
+      m[t] = cc[t] = 0.0;
+      if (t < len) {
+        const int i = s + t;
+        const bool end = i == n - 1;
+        const double east = end ? (ROWS ? fw : 0.0) : 0.5 * (K(t) + K(t + 1)) * dtdx2;
+        double di = 1.0 + west + east;
+        if (ROWS && i == 0) di = di - gamma;
+        if (ROWS && end) di = di - alpha * alpha / gamma;  // beta = alpha
+        const double lo = i == 0 ? 0.0 : -west, up = end ? 0.0 : -east;
+        const double ib = recip(t == 0 ? di : di - lo * cc[t > 0 ? t - 1 : 0]);
+        m[t] = lo * ib;
+        cc[t] = up * ib;
+        const double b0 = (ROWS ? mb[t] : p[t]) * ib;
+        if (t == 0) {
+          lo0 = lo;
+          ib0 = ib;
+          pv = b0;
+          ev = ib;  // the response to a unit right-hand side at the chunk's first unknown
+        } else {
+          pv = b0 - m[t] * pv;
+          ev = -m[t] * ev;
+        }
+        p[t] = pv;
+        // y_first = pA + eA u + rA y_next, one unknown further each step
+        pA0 += rA * pv;
+        eA += rA * ev;
+        if (ROWS && end) {
+          pA1 = rA * (alpha * ib);
+          ibl = ib;
+        }
+        rA *= -cc[t];
+        last_c = cc[t];
+        west = east;
+      }
     }
-    if (i + 1 < e) bn = p0[at(i + 1)];
-    double di = 1.0 + west + east;
-    if (ROWS && i == 0) di = di - gamma;
-    if (ROWS && i == n - 1) di = di - alpha * beta / gamma;
-    const double lo = i == 0 ? 0.0 : -west;
-    const double up = (ROWS && i == n - 1) ? 0.0 : -east;
-    const double b1 = ROWS ? (i == 0 ? gamma : (i == n - 1 ? alpha : 0.0)) : 0.0;
-    const double rr = i == e - 1 ? -up : 0.0;
-    // one reciprocal a position for the five quotients
-    bt = i == s ? di : di - lo * cprev;
-    const double ib = 1.0 / bt;
-    if (i == s) {
-      pv0 = b0 * ib;
-      pv1 = b1 * ib;
-      qv = -lo * ib;
-      rv = rr * ib;
-    } else {
-      pv0 = (b0 - lo * pv0) * ib;
-      pv1 = (b1 - lo * pv1) * ib;
-      qv = (0.0 - lo * qv) * ib;
-      rv = (rr - lo * rv) * ib;
+    if (on) {
+      const double u0 = ROWS && s == 0 ? gamma : 0.0;
+      rel[0 * LOD_THREADS + tid] = pA0;
+      rel[1 * LOD_THREADS + tid] = u0 * eA + pA1;
+      rel[2 * LOD_THREADS + tid] = -lo0 * eA;
+      rel[3 * LOD_THREADS + tid] = rA;
+      rel[4 * LOD_THREADS + tid] = pv;
+      rel[5 * LOD_THREADS + tid] = u0 * ev + (ROWS && len > 0 && s + len == n ? alpha * ibl : 0.0);
+      rel[6 * LOD_THREADS + tid] = -lo0 * ev;
+      rel[7 * LOD_THREADS + tid] = -last_c;
     }
-    cprev = up * ib;
-    c[at(i)] = cprev;
-    p0[at(i)] = pv0;
-    if (ROWS) p1[at(i)] = pv1;
-    q[at(i)] = qv;
-    r[at(i)] = rv;
-    west = east;
   }
-  // back substitution inside the chunk: y_i -= c_i y_(i+1)
-  const double e0 = pv0, e1 = pv1, eq = qv, er = rv;  // the last position's values are final
-#pragma unroll 4
-  for (int i = e - 2; i >= s; --i) {
-    const double ci = c[at(i)];
-    pv0 = p0[at(i)] - ci * pv0;
-    p0[at(i)] = pv0;
-    if (ROWS) {
-      pv1 = p1[at(i)] - ci * pv1;
-      p1[at(i)] = pv1;
+  __syncthreads();
+  // up the tree: the relations of chunks [c, c + 2^k) and [c + 2^k, c + 2^(k+1)) merge into c's slot; the
+  // values they meet at, first of the right and last of the left part, as relations to the merged
+  // chunk's outside, take the right part's slot
+  const int step = ROWS ? 1 : G;  // a chunk's neighbour's slot
+  auto R = [&](int k, int t) -> double& { return rel[k * LOD_THREADS + t]; };
+  int levels = 0;
+  for (; (1 << levels) < chunks; ++levels) {
+    const int d = 1 << levels, t2 = tid + d * step;
+    if (on && (c & (2 * d - 1)) == 0 && c + d < chunks) {
+      const double qA2 = R(2, t2), rB1 = R(7, tid), qB1 = R(6, tid), rA1 = R(3, tid), qB2 = R(6, t2);
+      const double D = recip(1.0 - qA2 * rB1);
+      const double a0 = D * (R(0, t2) + qA2 * R(4, tid)), aq = D * (qA2 * qB1), ar = D * R(3, t2);
+      const double b0 = R(4, tid) + rB1 * a0, bq = qB1 + rB1 * aq, br = rB1 * ar;
+      R(0, tid) += rA1 * a0;
+      R(2, tid) += rA1 * aq;
+      R(3, tid) = rA1 * ar;
+      const double pB = R(4, t2) + qB2 * b0, rB = R(7, t2) + qB2 * br;
+      if (ROWS) {
+        const double a1 = D * (R(1, t2) + qA2 * R(5, tid)), b1 = R(5, tid) + rB1 * a1;
+        R(1, tid) += rA1 * a1;
+        R(5, tid) = R(5, t2) + qB2 * b1;
+        R(1, t2) = a1;
+        R(5, t2) = b1;
+      }
+      R(4, tid) = pB;
+      R(6, tid) = qB2 * bq;
+      R(7, tid) = rB;
+      R(0, t2) = a0;
+      R(2, t2) = aq;
+      R(3, t2) = ar;
+      R(4, t2) = b0;
+      R(6, t2) = bq;
+      R(7, t2) = br;
     }
-    qv = q[at(i)] - ci * qv;
-    q[at(i)] = qv;
-    rv = r[at(i)] - ci * rv;
-    r[at(i)] = rv;
+    __syncthreads();
   }
-  double* ed = edge + (size_t)t * 8;  // (k L + l) * 8: first position, then last
-  ed[0] = pv0;
-  ed[1] = pv1;
-  ed[2] = qv;
-  ed[3] = rv;
-  ed[4] = e0;
-  ed[5] = e1;
-  ed[6] = eq;
-  ed[7] = er;
+  const size_t seg = (size_t)blockIdx.y * L + l;
+  if constexpr (STEP == 1) {
+    if (on && c == 0)
+      for (int k = 0; k < 8; ++k) edge[seg * 8 + k] = R(k, tid);
+    return;
+  }
+  if (on && c == 0) {
+    double y[4] = {0.0, 0.0, 0.0, 0.0}, f = 0.0;
+    if constexpr (STEP == 2) {
+      if (blockIdx.y > 0) {
+        const double* em = edge + (seg - L) * 8;
+        y[0] = em[4];
+        if (ROWS) y[1] = em[5];
+      }
+      if (blockIdx.y + 1 < gridDim.y) {
+        const double* ep = edge + (seg + L) * 8;
+        y[2] = ep[0];
+        if (ROWS) y[3] = ep[1];
+      }
+      if (ROWS) f = fact[l];
+    } else if (ROWS) {
+      // the line's own first and last values: the root's, with nothing outside
+      f = (R(0, tid) + alpha * R(4, tid) / gamma) / (1.0 + R(1, tid) + alpha * R(5, tid) / gamma);
+    }
+    for (int k = 0; k < 4; ++k) out[k * LOD_THREADS + tid] = y[k];
+    if (ROWS) s_fact[g] = f;
+  }
+  // down the tree: the outside values of each half from the whole's
+  for (int k = levels - 1; k >= 0; --k) {
+    __syncthreads();
+    const int d = 1 << k, t2 = tid + d * step;
+    if (on && (c & (2 * d - 1)) == 0 && c + d < chunks) {
+      const double L0 = out[tid], R0 = out[2 * LOD_THREADS + tid];
+      out[t2] = R(4, t2) + R(6, t2) * L0 + R(7, t2) * R0;
+      out[2 * LOD_THREADS + t2] = R0;
+      out[2 * LOD_THREADS + tid] = R(0, t2) + R(2, t2) * L0 + R(3, t2) * R0;
+      if (ROWS) {
+        const double L1 = out[LOD_THREADS + tid], R1 = out[3 * LOD_THREADS + tid];
+        out[LOD_THREADS + t2] = R(5, t2) + R(6, t2) * L1 + R(7, t2) * R1;
+        out[3 * LOD_THREADS + t2] = R1;
+        out[3 * LOD_THREADS + tid] = R(1, t2) + R(2, t2) * L1 + R(3, t2) * R1;
+      }
+    }
+  }
+  __syncthreads();
+  if (len > 0) {
+    const double f = ROWS ? s_fact[g] : 0.0;
+    const double left = out[tid] - (ROWS ? f * out[LOD_THREADS + tid] : 0.0);
+    const double right = out[2 * LOD_THREADS + tid] - (ROWS ? f * out[3 * LOD_THREADS + tid] : 0.0);
+    // b - fact u, with the outside values on the right-hand side
+    double ev = (-lo0 * left - (ROWS && s == 0 ? f * gamma : 0.0)) * ib0;
+#pragma unroll
+    for (int t = 0; t < LOD_CH; ++t) {
+      if (t > 0) ev = -m[t] * ev;
+      p[t] += ev;
+      if (ROWS && t < len && s + t == n - 1) p[t] -= f * (alpha * ibl);
+    }
+    double y = right;
+#pragma unroll
+    for (int t = LOD_CH - 1; t >= 0; --t) {
+      if (t < len) {
+        y = p[t] - cc[t] * y;
+        if (ROWS)
+          mb[t] = y;
+        else
+          x[(size_t)(s + t) * L + l] = y;
+      }
+    }
+  }
+  if constexpr (ROWS) {
+    __syncthreads();
+    const int width = min(n - s0, Pb * LOD_CH), lines = min(G, L - (int)blockIdx.x * G);
+    for (int e = tid; e < lines * width; e += blockDim.x) {
+      const int ge = e / width, i = e - ge * width;
+      x[(size_t)(blockIdx.x * G + ge) * n + s0 + i] = sb[ge * Pb * (LOD_CH + 1) + i + i / LOD_CH];
+    }
+  }
 }
 
-// One thread a line: the chunks' first (A_k) and last (B_k) values from A_k = pA + qA B_(k-1) +
+// One thread a line: the segments' first (A_k) and last (B_k) values from A_k = pA + qA B_(k-1) +
 // rA A_(k+1), B_k = pB + qB B_(k-1) + rB A_(k+1): forward, B_(k-1) = g + h A_k; back from A_P = 0.
 // Written over the edge record's p entries (A_k into [0], [1], B_k into [4], [5]); ROWS: fact of
 // the line into fact[l].
@@ -1298,28 +1443,6 @@ __global__ void __launch_bounds__(128) k_lod_reduce(int L, int n, int P, double 
     const double fw = ln.face(n - 1);
     const double beta = -fw, gamma = -(1.0 + fw + ln.face(0));
     fact[l] = (A0[0] + beta * Bl[0] / gamma) / (1.0 + A0[1] + beta * Bl[1] / gamma);
-  }
-}
-
-// Every cell: y = p + q B_(k-1) + r A_(k+1) per right-hand side; ROWS: out = y_b - fact y_u.
-// The result over p0.
-template <bool ROWS>
-__global__ void __launch_bounds__(256) k_lod_finish(int L, int n, int P, double* __restrict__ p0, const double* __restrict__ p1,
-                                                    const double* __restrict__ q, const double* __restrict__ r,
-                                                    const double* __restrict__ edge, const double* __restrict__ fact) {
-  const size_t total = (size_t)L * n;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int l = (int)(t % L), i = (int)(t / L), k = i / LOD_CHUNK;
-    const double* em = k > 0 ? edge + ((size_t)(k - 1) * L + l) * 8 : nullptr;
-    const double* ep = k + 1 < P ? edge + ((size_t)(k + 1) * L + l) * 8 : nullptr;
-    const double qv = q[t], rv = r[t];
-    const double y0 = p0[t] + qv * (em ? em[4] : 0.0) + rv * (ep ? ep[0] : 0.0);
-    if (ROWS) {
-      const double y1 = p1[t] + qv * (em ? em[5] : 0.0) + rv * (ep ? ep[1] : 0.0);
-      p0[t] = y0 - fact[l] * y1;
-    } else {
-      p0[t] = y0;
-    }
   }
 }
 
@@ -1496,7 +1619,7 @@ struct dt_diff {
   double *east = nullptr, *south = nullptr, *diag = nullptr;
   float *east32 = nullptr, *south32 = nullptr, *diag32 = nullptr;
   float *x32 = nullptr, *r32 = nullptr, *p32 = nullptr, *ap32 = nullptr;
-  double* lod[7] = {};  // the LOD first guess's scratch (lod[6]: its chunks' end values)
+  double* lod[7] = {};  // the LOD first guess's scratch (lod[6]: its segments' relations)
   double* partials = nullptr;
   double* scale = nullptr;
   dt::DScalars *S64 = nullptr, *S32 = nullptr;
@@ -1933,47 +2056,61 @@ static dt_status run_cg(dt_diff* s, CgLane<TC, TM>& C, int lane, int kind, const
   return DT_OK;
 }
 
+// Chunks of a segment of a line, and lines a block: columns in segments of 64 chunks (8 columns a
+// block, or more of fewer chunks), rows of up to 512.
+static void lod_shape(bool rows, int n, int* Pb, int* G, int* segments) {
+  const int P = (int)ceil_div(n, LOD_CH), most = rows ? LOD_THREADS : LOD_THREADS / 8;
+  *Pb = std::min(P, most);
+  *G = std::max(1, std::min(LOD_THREADS / *Pb, rows ? LOD_THREADS : 32));
+  *segments = (int)ceil_div(P, *Pb);
+}
+// L lines of n unknowns: b (the raster, or x itself) into s->x.
+template <bool ROWS>
+static void lod_lines(dt_diff* s, int L, int n, double dtdx2, const double* b) {
+  cudaStream_t st = s->stream;
+  int Pb, G, segments;
+  lod_shape(ROWS, n, &Pb, &G, &segments);
+  const dim3 grid(ceil_div(L, G), segments);
+  const int threads = (int)ceil_div(Pb * G, 32) * 32;
+  const size_t smem = lod_smem(ROWS);
+  if (segments == 1) {
+    k_lod_lines<ROWS, 0><<<grid, threads, smem, st>>>(L, n, Pb, G, dtdx2, s->kd, b, s->x, nullptr, nullptr);
+    count_launch();
+    return;
+  }
+  double* edge = s->lod[6];
+  double* al = edge + (size_t)8 * segments * L;
+  double* fact = al + (size_t)4 * segments * L;
+  k_lod_lines<ROWS, 1><<<grid, threads, smem, st>>>(L, n, Pb, G, dtdx2, s->kd, b, s->x, edge, nullptr);
+  k_lod_reduce<ROWS><<<ceil_div(L, 128), 128, 0, st>>>(L, n, segments, dtdx2, s->kd, edge, al, fact);
+  k_lod_lines<ROWS, 2><<<grid, threads, smem, st>>>(L, n, Pb, G, dtdx2, s->kd, b, s->x, edge, fact);
+  for (int k = 0; k < 3; ++k) count_launch();
+}
+static void lod_attributes() {
+  cudaFuncSetAttribute(k_lod_lines<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lod_smem(true));
+  cudaFuncSetAttribute(k_lod_lines<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lod_smem(true));
+  cudaFuncSetAttribute(k_lod_lines<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lod_smem(true));
+  cudaFuncSetAttribute(k_lod_lines<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lod_smem(false));
+  cudaFuncSetAttribute(k_lod_lines<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lod_smem(false));
+  cudaFuncSetAttribute(k_lod_lines<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lod_smem(false));
+}
+
 static dt_status diff_first_guess(dt_diff* s, const dt_diff_params* p, double dt) {
   cudaStream_t st = s->stream;
-  DT_CUDA(cudaMemcpyAsync(s->x, s->b, s->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  if (p->first_guess) {
-    double dtdx2 = dt / (s->dx * s->dx);
-    if (s->wrap && s->w > 2) {
-      // rows through transposed copies, so each thread's walk reads contiguous words
-      const dim3 tb(32, 8), tg_in(ceil_div(s->w, 32), ceil_div(s->h, 32)), tg_out(ceil_div(s->h, 32), ceil_div(s->w, 32));
-      k_transpose<<<tg_in, tb, 0, st>>>(s->h, s->w, s->kd, s->lod[0]);
-      k_transpose<<<tg_in, tb, 0, st>>>(s->h, s->w, s->x, s->lod[1]);
-      // the rows (lines of w unknowns, h of them) in chunks: lod[1] b -> x, lod[2] z, lod[3] q, lod[4] r,
-      // lod[5] c, lod[6] the chunks' end values and the recurrence's scratch (8 + 4 values a chunk)
-      // and the rows' Sherman-Morrison factors
-      const int P = (int)ceil_div(s->w, LOD_CHUNK);
-      double* edge = s->lod[6];
-      double* al = edge + (size_t)8 * P * s->h;
-      double* fact = al + (size_t)4 * P * s->h;
-      k_lod_chunks<true><<<ceil_div((size_t)s->h * P, 128), 128, 0, st>>>(s->h, s->w, P, dtdx2, s->lod[0], s->lod[1], s->lod[2],
-                                                                        s->lod[3], s->lod[4], s->lod[5], edge);
-      k_lod_reduce<true><<<ceil_div(s->h, 128), 128, 0, st>>>(s->h, s->w, P, dtdx2, s->lod[0], edge, al, fact);
-      k_lod_finish<true><<<dgrid(s, s->n), 256, 0, st>>>(s->h, s->w, P, s->lod[1], s->lod[2], s->lod[3], s->lod[4], edge, fact);
-      k_transpose<<<tg_out, tb, 0, st>>>(s->w, s->h, s->lod[1], s->x);
-      for (int k = 0; k < 6; ++k) count_launch();
-    } else {
-      k_lod_rows<<<ceil_div(s->h, 64), 64, 0, st>>>(s->w, s->h, s->wrap, s->x, s->kd, dtdx2, s->lod[0], s->lod[1], s->lod[2],
-                                                    s->lod[3], s->lod[4], s->lod[5]);
-      count_launch();
-    }
-    {
-      // the columns (lines of h unknowns, w of them, as they lie) in chunks: x in place, lod[2] q,
-      // lod[3] r, lod[4] c, lod[6] the chunks' end values
-      const int P = (int)ceil_div(s->h, LOD_CHUNK);
-      double* edge = s->lod[6];
-      double* al = edge + (size_t)8 * P * s->w;
-      k_lod_chunks<false><<<ceil_div((size_t)s->w * P, 128), 128, 0, st>>>(s->w, s->h, P, dtdx2, s->kd, s->x, nullptr,
-                                                                         s->lod[2], s->lod[3], s->lod[4], edge);
-      k_lod_reduce<false><<<ceil_div(s->w, 128), 128, 0, st>>>(s->w, s->h, P, dtdx2, s->kd, edge, al, nullptr);
-      k_lod_finish<false><<<dgrid(s, s->n), 256, 0, st>>>(s->w, s->h, P, s->x, nullptr, s->lod[2], s->lod[3], edge, nullptr);
-      for (int k = 0; k < 3; ++k) count_launch();
-    }
+  if (!p->first_guess) {
+    DT_CUDA(cudaMemcpyAsync(s->x, s->b, s->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    return DT_OK;
   }
+  const double dtdx2 = dt / (s->dx * s->dx);
+  if (s->wrap && s->w > 2) {
+    lod_lines<true>(s, s->h, s->w, dtdx2, s->b);
+  } else {
+    DT_CUDA(cudaMemcpyAsync(s->x, s->b, s->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    k_lod_rows<<<ceil_div(s->h, 64), 64, 0, st>>>(s->w, s->h, s->wrap, s->x, s->kd, dtdx2, s->lod[0], s->lod[1], s->lod[2],
+                                                  s->lod[3], s->lod[4], s->lod[5]);
+    count_launch();
+  }
+  lod_lines<false>(s, s->w, s->h, dtdx2, s->x);
   return DT_OK;
 }
 
@@ -2189,14 +2326,19 @@ dt_status dt_diff_create(int w, int h, double dx, int wrap_x, dt_diff** out) {
     if ((st = ddalloc(s, q, s->n)) != DT_OK) return fail(st);
   for (float** q : {&s->east32, &s->south32, &s->diag32, &s->x32, &s->r32, &s->p32, &s->ap32})
     if ((st = ddalloc(s, q, s->n)) != DT_OK) return fail(st);
-  for (int k = 0; k < 6; ++k)
-    if ((st = ddalloc(s, &s->lod[k], s->n)) != DT_OK) return fail(st);
+  // the LOD's scratch: the serial rows' arrays where the rows do not wrap, and the segments' relations
+  // (8 values, 4 of their recurrence's) and Sherman-Morrison factors of lines of several segments
+  if (!(s->wrap && s->w > 2))
+    for (int k = 0; k < 6; ++k)
+      if ((st = ddalloc(s, &s->lod[k], s->n)) != DT_OK) return fail(st);
   {
-    // the LOD chunks' end values, their recurrence's scratch (12 values a chunk of a line) and
-    // the rows' Sherman-Morrison factors
-    const size_t chunks = (size_t)ceil_div(s->w, LOD_CHUNK) * s->h + (size_t)ceil_div(s->h, LOD_CHUNK) * s->w;
-    if ((st = ddalloc(s, &s->lod[6], 12 * chunks + s->h + s->w)) != DT_OK) return fail(st);
+    int Pb, G, rows, cols;
+    lod_shape(true, s->w, &Pb, &G, &rows);
+    lod_shape(false, s->h, &Pb, &G, &cols);
+    const size_t need = std::max(rows > 1 ? ((size_t)12 * rows + 1) * s->h : 0, cols > 1 ? (size_t)12 * cols * s->w : 0);
+    if (need && (st = ddalloc(s, &s->lod[6], need)) != DT_OK) return fail(st);
   }
+  lod_attributes();
   // a reducing kernel's blocks: two values each of at most eight an SM, or one of each of
   // k_mg_tile's tiles (56 x 24 cells at the least)
   const size_t tiles = (size_t)ceil_div(s->w, 56) * ceil_div(s->h, 24);

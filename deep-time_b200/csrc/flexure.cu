@@ -707,19 +707,6 @@ __global__ void __launch_bounds__(256) k_bank_weights(int w, int h, const T* __r
 // INV_BANK: the bank's three levels in one pass, out = sum_k wt_k x_k, the levels' spectra and
 // weights consecutive (half + k h N, wt + k w h)
 enum { INV_STORE = 0, INV_STORE_DOT = 2, INV_STORE_W = 3, INV_BANK = 4 };
-// Reciprocals of the spectral divisors d lambda^2 + c_ref, with no slow-path call: float, the
-// correctly rounded intrinsic; double, of a normal number m 2^e, the hardware's float estimate of 1 / m, m in [1, 2),
-// scaled by 2^-e in the exponent bits and refined by two Newton-Raphson steps r <- r + r (1 - x r)
-// (each squares the relative error: 2^-22 -> 2^-44 -> 2^-88, so the last rounding is what is left).
-__device__ __forceinline__ double recip(double x) {
-  const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
-  const double m = __hiloint2double(hi - (e << 20), __double2loint(x));
-  double r = (double)__fdividef(1.0f, (float)m);
-  r = __hiloint2double(__double2hiint(r) - (e << 20), __double2loint(r));
-  r = fma(r, fma(-x, r, 1.0), r);
-  return fma(r, fma(-x, r, 1.0), r);
-}
-__device__ __forceinline__ float recip(float x) { return __frcp_rn(x); }
 // float, the hardware's approximate reciprocal (__fdividef, at most 2 ulp for |x| in
 // [2^-126, 2^126]), for the divisors of the fused column pass, which lie in (c_ref, 1e36)
 __device__ __forceinline__ float recip_fast(float x) { return __fdividef(1.0f, x); }
