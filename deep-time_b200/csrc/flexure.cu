@@ -295,8 +295,7 @@ __device__ __forceinline__ T lap5(T we, T ea, T no, T so, T x, const RowCoef<T, 
 // MET: on the sphere's row metric (ma: h values a_j, mb: h + 1 values b_j); the block metric
 // otherwise.
 template <class T, int MODE, bool MET = false>
-__global__ void __launch_bounds__(TBX* TTY) k_apply(int w, int h, T inv_dx2, const T* __restrict__ v, const T* __restrict__ J,
-                                                    const T* __restrict__ part, const T* __restrict__ d,
+__global__ void __launch_bounds__(TBX* TTY) k_apply(int w, int h, T inv_dx2, const T* __restrict__ v, const T* __restrict__ d,
                                                     const T* __restrict__ c, const T* __restrict__ rb, T* __restrict__ y,
                                                     double* partials, Scalars* S, const T* __restrict__ ma = nullptr,
                                                     const T* __restrict__ mb = nullptr) {
@@ -307,26 +306,19 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply(int w, int h, T inv_dx2, con
     }
   }
   if (MODE == RESID_GATED && S->gate_it != S->it) return;
-  constexpr bool JAC = MODE == JAC_LEFT || MODE == JAC_FINAL;
   constexpr bool HAS_B = MODE == RESID || MODE == RESID_GATED;
   constexpr int TBY = tile_rows<T>(), SEG = TBY / TTY;
   constexpr int P = Tile<T>::PITCH, OFF = Tile<T>::OFF;
   constexpr int UR = TBY + 4, MR = TBY + 2;  // vector rows -2 .. TBY + 1; d / m rows -1 .. TBY
-  __shared__ __align__(16) T sv[UR * P];                    // the vector (JAC: r)
-  __shared__ __align__(16) T sJ[JAC ? UR * P : 1];          // JAC: J
-  __shared__ __align__(16) T sP[JAC ? UR * P : 1];          // JAC_FINAL: part; then (JAC) u
-  __shared__ __align__(16) T sd[MR * P];                    // d; then m = d L u in place
+  __shared__ __align__(16) T sv[UR * P];  // the vector
+  __shared__ __align__(16) T sd[MR * P];  // d; then m = d L u in place
   const int i0 = blockIdx.x * TBX, j0 = blockIdx.y * TBY;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int tid = tx + ty * TBX;
-  const T* src = JAC ? rb : v;
-  const bool vec = i0 + TBX <= w && (w * (int)sizeof(T)) % 16 == 0 && aligned16(src) && aligned16(d) &&
-                   (!JAC || aligned16(J)) && (MODE != JAC_FINAL || aligned16(part));
+  const bool vec = i0 + TBX <= w && (w * (int)sizeof(T)) % 16 == 0 && aligned16(v) && aligned16(d);
   // Stage the tiles with asynchronous copies (every load in flight at once): rows clamp, columns
   // wrap.
-  stage_tile<T, UR, 2, -2>(sv, src, w, h, i0, j0, vec, tid);
-  if (JAC) stage_tile<T, UR, 2, -2>(sJ, J, w, h, i0, j0, vec, tid);
-  if (MODE == JAC_FINAL) stage_tile<T, UR, 2, -2>(sP, part, w, h, i0, j0, vec, tid);
+  stage_tile<T, UR, 2, -2>(sv, v, w, h, i0, j0, vec, tid);
   stage_tile<T, MR, 1, -1>(sd, d, w, h, i0, j0, vec, tid);
   __pipeline_commit();
   // c (and b) for the thread's own output cells, in flight with the tiles
@@ -342,21 +334,11 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply(int w, int h, T inv_dx2, con
   }
   __pipeline_wait_prior(0);
   __syncthreads();
-  if (JAC) {
-    // the vector the mode forms: u = J r (+ part); r and J stay readable for the outputs
-    for (int e = tid; e < UR * P; e += TBX * TTY) {
-      T u = sJ[e] * sv[e];
-      if (MODE == JAC_FINAL) u += sP[e];
-      sP[e] = u;
-    }
-    __syncthreads();
-  }
-  const T* su = JAC ? sP : sv;
   // m = d . L u at local rows -1 .. TBY, columns -1 .. TBX. Column tx over the thread's strip
   // (the first strip also takes row -1, the last row TBY) with a sliding window down the column.
   {
     const int a = r0 - (ty == 0 ? 1 : 0);
-    const T* ucol = su + OFF + tx;  // row lr at (lr + 2) * P
+    const T* ucol = sv + OFF + tx;  // row lr at (lr + 2) * P
     T* mcol = sd + OFF + tx;        // row lr at (lr + 1) * P
     T un = ucol[(a + 1) * P], uc = ucol[(a + 2) * P];
 #pragma unroll
@@ -374,7 +356,7 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply(int w, int h, T inv_dx2, con
   // columns -1 and TBX over all rows
   for (int e = tid; e < 2 * MR; e += TBX * TTY) {
     int lr = (e >> 1) - 1, lc = (e & 1) ? TBX : -1;
-    const T* uc = su + (lr + 2) * P + OFF + lc;
+    const T* uc = sv + (lr + 2) * P + OFF + lc;
     T lap = lap5<T, MET>(uc[-1], uc[1], uc[-P], uc[P], uc[0], row_coef<T, MET>(ma, mb, j0 + lr, h), inv_dx2);
     T* m = sd + (lr + 1) * P + OFF + lc;
     *m = lap * *m;
@@ -392,9 +374,8 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply(int w, int h, T inv_dx2, con
       __syncthreads();
     }
   }
-  Acc<2> acc;
+  Acc<1> acc;
   acc.v[0] = 0.0;
-  acc.v[1] = 0.0;
   {
     const T* mcol = sd + OFF + tx;  // m row lr at (lr + 1) * P
     T mn = mcol[r0 * P], mc = mcol[(r0 + 1) * P];
@@ -409,7 +390,7 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply(int w, int h, T inv_dx2, con
       int j = j0 + lr;
       if (i < w && j < h) {
         size_t k = (size_t)j * w + i;
-        T u = su[(lr + 2) * P + OFF + tx];
+        T u = sv[(lr + 2) * P + OFF + tx];
         if (MODE == BEND) {
           y[k] = lm;
         } else {
@@ -419,39 +400,28 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply(int w, int h, T inv_dx2, con
             acc.v[0] += (double)u * (double)au;
           } else if (MODE == PLAIN) {
             y[k] = au;
-          } else if (HAS_B) {
+          } else {
             T rr = br[q] - au;
             y[k] = rr;
             acc.v[0] += (double)rr * (double)rr;
-          } else if (MODE == JAC_LEFT) {
-            y[k] = sv[(lr + 2) * P + OFF + tx] - au;
-          } else {  // JAC_FINAL
-            T r = sv[(lr + 2) * P + OFF + tx];
-            T z = u + sJ[(lr + 2) * P + OFF + tx] * (r - au);
-            y[k] = z;
-            acc.v[0] += (double)r * (double)z;
-            acc.v[1] = fmax(acc.v[1], fabs((double)z));
           }
         }
       }
     }
   }
-  if (MODE == AP_DOT || MODE == RESID || MODE == RESID_GATED || MODE == JAC_FINAL) {
-    const int kind[2] = {0, 1};
-    unsigned int nb = gridDim.x * gridDim.y;
-    int site = MODE == AP_DOT ? SITE_PAP : (MODE == RESID || MODE == RESID_GATED) ? SITE_RESID : SITE_PRECOND;
-    bool last = MODE == JAC_FINAL ? reduce_partials<2>(acc, kind, partials, &S->ticket[site], nb)
-                                  : reduce_partials<1>(*reinterpret_cast<Acc<1>*>(&acc), kind, partials, &S->ticket[site], nb);
-    if (last && tid == 0) {
+  if (MODE == AP_DOT || MODE == RESID || MODE == RESID_GATED) {
+    const int kind[1] = {0};
+    const int site = MODE == AP_DOT ? SITE_PAP : SITE_RESID;
+    if (reduce_partials<1>(acc, kind, partials, &S->ticket[site], gridDim.x * gridDim.y) && tid == 0) {
       if (MODE == AP_DOT) finish_pap(S, acc.v[0]);
       if (MODE == RESID) S->rr = acc.v[0];
       if (MODE == RESID_GATED) S->rr_true = acc.v[0];
-      if (MODE == JAC_FINAL) finish_precond(S, acc.v[0], acc.v[1]);
     }
   }
 }
 
 }  // namespace dt
+#include "stencil_tile.cuh"
 #include "stencil_tma.cuh"
 #include <cudaTypedefs.h>
 namespace dt {
@@ -2481,10 +2451,7 @@ static void tma_setup() {
 }
 template <class T>
 static void tma_setup_all() {
-  tma_setup<T, AP_DOT>();
   tma_setup<T, RESID>();
-  tma_setup<T, JAC_LEFT>();
-  tma_setup<T, JAC_FINAL>();
   tma_setup<T, PLAIN>();
   tma_setup<T, BEND>();
   tma_setup<T, RESID_GATED>();
@@ -2492,22 +2459,19 @@ static void tma_setup_all() {
 
 // The persistent TMA stencil; false (nothing launched) when a buffer cannot be mapped.
 template <class T, int MODE>
-static bool launch_apply_tma(dt_flex* s, const T* vsrc, const T* J, const T* part, const T* d, const T* c, const T* rb, T* y,
-                             Scalars* S, cudaStream_t st) {
+static bool launch_apply_tma(dt_flex* s, const T* v, const T* d, const T* c, const T* rb, T* y, Scalars* S, cudaStream_t st) {
   using ST = TmaStage<T, MODE>;
-  CUtensorMap mv, mJ, mP, md, mc, mb;
-  if (!tensor_map(s, vsrc, sizeof(T), ST::P, ST::UR, &mv)) return false;
-  mJ = mP = mc = mb = mv;
-  if (ST::JAC && !tensor_map(s, J, sizeof(T), ST::P, ST::UR, &mJ)) return false;
-  if (MODE == JAC_FINAL && !tensor_map(s, part, sizeof(T), ST::P, ST::UR, &mP)) return false;
+  CUtensorMap mv, md, mc, mb;
+  if (!tensor_map(s, v, sizeof(T), ST::P, ST::UR, &mv)) return false;
+  mc = mb = mv;
   if (!tensor_map(s, d, sizeof(T), ST::P, ST::MR, &md)) return false;
   if (ST::HAS_C && !tensor_map(s, c, sizeof(T), TBX, ST::TBY, &mc)) return false;
   if (ST::HAS_B && !tensor_map(s, rb, sizeof(T), TBX, ST::TBY, &mb)) return false;
   const int tiles_x = s->w / TBX, ntiles = tiles_x * (int)ceil_div(s->h, ST::TBY);
   const int grid = std::max(1, std::min(ntiles, g_tma_per_sm[sizeof(T) == 8][MODE] * s->sms));
   T inv = (T)(1.0 / (s->dx * s->dx));
-  k_apply_tma<T, MODE><<<grid, dim3(TBX, TTY), ST::SMEM, st>>>(mv, mJ, mP, md, mc, mb, s->w, s->h, inv, vsrc, J, part, d, y,
-                                                              s->partials, S, tiles_x, ntiles);
+  k_apply_tma<T, MODE><<<grid, dim3(TBX, TTY), ST::SMEM, st>>>(mv, md, mc, mb, s->w, s->h, inv, v, d, y, s->partials, S, tiles_x,
+                                                              ntiles);
   counted();
   return true;
 }
@@ -2515,17 +2479,14 @@ static bool launch_apply_tma(dt_flex* s, const T* vsrc, const T* J, const T* par
 // The operator on the sphere's row metric: the per-block kernel (the TMA stencil has the block
 // metric only), the handle's couplings in the lane's precision.
 template <class T>
-static void launch_apply_metric(dt_flex* s, int mode, dim3 grid, dim3 block, T inv, const T* v, const T* J, const T* part,
-                                const T* d, const T* c, const T* rb, T* y, Scalars* S, cudaStream_t st) {
+static void launch_apply_metric(dt_flex* s, int mode, dim3 grid, dim3 block, T inv, const T* v, const T* d, const T* c, const T* rb,
+                                T* y, Scalars* S, cudaStream_t st) {
   const T* ma = metric_a<T>(s);
   const T* mb = metric_b<T>(s);
 #define DT_MET_CASE(M) \
-  case M: k_apply<T, M, true><<<grid, block, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, rb, y, s->partials, S, ma, mb); break;
+  case M: k_apply<T, M, true><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S, ma, mb); break;
   switch (mode) {
-    DT_MET_CASE(AP_DOT)
     DT_MET_CASE(RESID)
-    DT_MET_CASE(JAC_LEFT)
-    DT_MET_CASE(JAC_FINAL)
     DT_MET_CASE(PLAIN)
     DT_MET_CASE(BEND)
     DT_MET_CASE(RESID_GATED)
@@ -2534,37 +2495,73 @@ static void launch_apply_metric(dt_flex* s, int mode, dim3 grid, dim3 block, T i
   counted();
 }
 
+// The loop's stencils (AP_DOT, JAC_LEFT, JAC_FINAL) over register tiles.
+template <class T, int MODE, bool MET, int WARPS, int RPW>
+static void launch_tile_rows(dt_flex* s, const T* v, const T* J, const T* part, const T* d, const T* c, T* y, Scalars* S,
+                             cudaStream_t st) {
+  const int tiles_x = (int)ceil_div(s->w, FT_TX), ntiles = tiles_x * (int)ceil_div(s->h, WARPS * RPW - 2 * FT_H);
+  const int grid = std::min(ntiles, 2 * s->sms);
+  const T inv = (T)(1.0 / (s->dx * s->dx));
+  const T *ma = MET ? metric_a<T>(s) : nullptr, *mb = MET ? metric_b<T>(s) : nullptr;
+  if (s->w % 2 == 0)
+    k_flex_tile<T, MODE, MET, WARPS, RPW, true><<<grid, 32 * WARPS, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, y, s->partials, S, tiles_x, ntiles, ma, mb);
+  else
+    k_flex_tile<T, MODE, MET, WARPS, RPW, false><<<grid, 32 * WARPS, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, y, s->partials, S, tiles_x, ntiles, ma, mb);
+  counted();
+}
+template <class T, int MODE>
+static void launch_tile(dt_flex* s, const T* v, const T* J, const T* part, const T* d, const T* c, T* y, Scalars* S,
+                        cudaStream_t st) {
+  // Regions of 64 rows (16 warps of 4) in FP32 on rasters of many tiles, else of 32: 16 warps of 2, or
+  // for FP64 JAC_FINAL, whose five arrays do not fit 64 registers a thread, 8 warps of 4 (4096 x 2048
+  // 93.7 -> 81.9 us; the other two are faster with 16: 59.1 against 65.9 and 63.8 against 66.5).
+  constexpr bool wide = sizeof(T) == 8 && MODE == JAC_FINAL;
+  constexpr int W2 = wide ? 8 : 16, R2 = wide ? 4 : 2;
+  if constexpr (sizeof(T) == 4) {
+    if ((size_t)ceil_div(s->w, FT_TX) * ceil_div(s->h, 64 - 2 * FT_H) >= (size_t)4 * s->sms) {
+      if (s->metric)
+        launch_tile_rows<T, MODE, true, 16, 4>(s, v, J, part, d, c, y, S, st);
+      else
+        launch_tile_rows<T, MODE, false, 16, 4>(s, v, J, part, d, c, y, S, st);
+      return;
+    }
+  }
+  if (s->metric)
+    launch_tile_rows<T, MODE, true, W2, R2>(s, v, J, part, d, c, y, S, st);
+  else
+    launch_tile_rows<T, MODE, false, W2, R2>(s, v, J, part, d, c, y, S, st);
+}
+
 template <class T>
 static void launch_apply(dt_flex* s, int mode, const T* v, const T* J, const T* part, const T* d, const T* c, const T* rb, T* y,
                          Scalars* S, cudaStream_t st) {
+  switch (mode) {
+    case AP_DOT: launch_tile<T, AP_DOT>(s, v, nullptr, nullptr, d, c, y, S, st); return;
+    case JAC_LEFT: launch_tile<T, JAC_LEFT>(s, rb, J, nullptr, d, c, y, S, st); return;
+    case JAC_FINAL: launch_tile<T, JAC_FINAL>(s, rb, J, part, d, c, y, S, st); return;
+    default: break;
+  }
   if (s->tma && !s->metric) {
-    const T* vsrc = (mode == JAC_LEFT || mode == JAC_FINAL) ? rb : v;
     bool done = false;
     switch (mode) {
-      case AP_DOT: done = launch_apply_tma<T, AP_DOT>(s, vsrc, J, part, d, c, rb, y, S, st); break;
-      case RESID: done = launch_apply_tma<T, RESID>(s, vsrc, J, part, d, c, rb, y, S, st); break;
-      case JAC_LEFT: done = launch_apply_tma<T, JAC_LEFT>(s, vsrc, J, part, d, c, rb, y, S, st); break;
-      case JAC_FINAL: done = launch_apply_tma<T, JAC_FINAL>(s, vsrc, J, part, d, c, rb, y, S, st); break;
-      case PLAIN: done = launch_apply_tma<T, PLAIN>(s, vsrc, J, part, d, c, rb, y, S, st); break;
-      case BEND: done = launch_apply_tma<T, BEND>(s, vsrc, J, part, d, c, rb, y, S, st); break;
-      case RESID_GATED: done = launch_apply_tma<T, RESID_GATED>(s, vsrc, J, part, d, c, rb, y, S, st); break;
+      case RESID: done = launch_apply_tma<T, RESID>(s, v, d, c, rb, y, S, st); break;
+      case PLAIN: done = launch_apply_tma<T, PLAIN>(s, v, d, c, rb, y, S, st); break;
+      case BEND: done = launch_apply_tma<T, BEND>(s, v, d, c, rb, y, S, st); break;
+      case RESID_GATED: done = launch_apply_tma<T, RESID_GATED>(s, v, d, c, rb, y, S, st); break;
     }
     if (done) return;
   }
   dim3 grid(ceil_div(s->w, TBX), ceil_div(s->h, tile_rows<T>())), block(TBX, TTY);
   T inv = (T)(1.0 / (s->dx * s->dx));
   if (s->metric) {
-    launch_apply_metric<T>(s, mode, grid, block, inv, v, J, part, d, c, rb, y, S, st);
+    launch_apply_metric<T>(s, mode, grid, block, inv, v, d, c, rb, y, S, st);
     return;
   }
   switch (mode) {
-    case AP_DOT: k_apply<T, AP_DOT><<<grid, block, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, rb, y, s->partials, S); counted(); break;
-    case RESID: k_apply<T, RESID><<<grid, block, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, rb, y, s->partials, S); counted(); break;
-    case JAC_LEFT: k_apply<T, JAC_LEFT><<<grid, block, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, rb, y, s->partials, S); counted(); break;
-    case JAC_FINAL: k_apply<T, JAC_FINAL><<<grid, block, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, rb, y, s->partials, S); counted(); break;
-    case PLAIN: k_apply<T, PLAIN><<<grid, block, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, rb, y, s->partials, S); counted(); break;
-    case BEND: k_apply<T, BEND><<<grid, block, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, rb, y, s->partials, S); counted(); break;
-    case RESID_GATED: k_apply<T, RESID_GATED><<<grid, block, 0, st>>>(s->w, s->h, inv, v, J, part, d, c, rb, y, s->partials, S); counted(); break;
+    case RESID: k_apply<T, RESID><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); counted(); break;
+    case PLAIN: k_apply<T, PLAIN><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); counted(); break;
+    case BEND: k_apply<T, BEND><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); counted(); break;
+    case RESID_GATED: k_apply<T, RESID_GATED><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); counted(); break;
   }
 }
 
@@ -4171,7 +4168,7 @@ extern "C" dt_status dt_flex_operator_dot_noalloc(int w, int h, double dx, const
   // every tile writes its own before the last tile reads them.
   DT_CUDA(cudaMemsetAsync(S, 0, sizeof(Scalars), st));
   dim3 grid(ceil_div((size_t)w, TBX), ceil_div((size_t)h, tile_rows<double>())), block(TBX, TTY);
-  k_apply<double, AP_DOT><<<grid, block, 0, st>>>(w, h, 1.0 / (dx * dx), v, nullptr, nullptr, d, c, nullptr, y, partials, S);
+  k_apply<double, AP_DOT><<<grid, block, 0, st>>>(w, h, 1.0 / (dx * dx), v, d, c, nullptr, y, partials, S);
   counted();
   DT_CUDA(cudaGetLastError());
   DT_CUDA(cudaMemcpyAsync(vav, &S->pap, sizeof(double), cudaMemcpyDeviceToDevice, st));

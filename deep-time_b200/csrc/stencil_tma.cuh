@@ -1,9 +1,10 @@
-// The 13-point operator as a persistent kernel fed by the Tensor Memory Accelerator.
+// The 13-point operator as a persistent kernel fed by the Tensor Memory Accelerator: y = A v, L (d L v)
+// and the residual b - A v with its norm (the loop's stencils are stencil_tile.cuh's).
 //
 // Each block loops over tiles (tile t, t + gridDim.x, ...). Two shared-memory stages alternate:
 // while a tile is computed, the bulk tensor copies of the block's next tile land in the other
 // stage, signalled by that stage's mbarrier (complete_tx). One thread issues the copies. The
-// boxes are those of k_apply's tiles: the vector (and J, part) with two halo rows and columns,
+// boxes are those of k_apply's tiles: the vector with two halo rows and columns,
 // d with one, c and b without; each box starts on the tile's 16-byte-aligned column i0 - OFF.
 // The copies zero-fill outside the raster. After they land, the block writes the wrapped halo
 // columns of the first and last tile columns from global memory, and repeats the raster's edge
@@ -71,7 +72,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 // copies of one tile write.
 template <class T, int MODE>
 struct TmaStage {
-  static constexpr bool JAC = MODE == JAC_LEFT || MODE == JAC_FINAL;
   static constexpr bool HAS_C = MODE != BEND;
   static constexpr bool HAS_B = MODE == RESID || MODE == RESID_GATED;
   static constexpr int TBY = tile_rows<T>(), P = Tile<T>::PITCH;
@@ -79,28 +79,21 @@ struct TmaStage {
   static constexpr int BV = UR * P * (int)sizeof(T), BD = MR * P * (int)sizeof(T), BI = TBY * TBX * (int)sizeof(T);
   static constexpr int r128(int b) { return (b + 127) / 128 * 128; }
   static constexpr int OV = 0;
-  static constexpr int OJ = OV + r128(BV);
-  static constexpr int OP = OJ + (JAC ? r128(BV) : 0);
-  static constexpr int OD = OP + (JAC ? r128(BV) : 0);
+  static constexpr int OD = OV + r128(BV);
   static constexpr int OC = OD + r128(BD);
   static constexpr int OB = OC + (HAS_C ? r128(BI) : 0);
   static constexpr int BYTES = OB + (HAS_B ? r128(BI) : 0);
-  // part is copied only for JAC_FINAL (JAC_LEFT uses its slot as scratch for u)
-  static constexpr int TX = BV + (JAC ? BV : 0) + (MODE == JAC_FINAL ? BV : 0) + BD + (HAS_C ? BI : 0) + (HAS_B ? BI : 0);
+  static constexpr int TX = BV + BD + (HAS_C ? BI : 0) + (HAS_B ? BI : 0);
   static constexpr int SMEM = 2 * BYTES + 16;  // two stages and their mbarriers
 };
 
 template <class T, int MODE>
-__global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mJ,
-                                                        const __grid_constant__ CUtensorMap mpart,
-                                                        const __grid_constant__ CUtensorMap md, const __grid_constant__ CUtensorMap mc,
-                                                        const __grid_constant__ CUtensorMap mb, int w, int h, T inv_dx2,
-                                                        const T* __restrict__ vsrc, const T* __restrict__ J,
-                                                        const T* __restrict__ part, const T* __restrict__ d,
-                                                        T* __restrict__ y, double* partials, Scalars* S, int tiles_x,
-                                                        int ntiles) {
+__global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap md,
+                                                        const __grid_constant__ CUtensorMap mc, const __grid_constant__ CUtensorMap mb,
+                                                        int w, int h, T inv_dx2, const T* __restrict__ vsrc, const T* __restrict__ d,
+                                                        T* __restrict__ y, double* partials, Scalars* S, int tiles_x, int ntiles) {
   using ST = TmaStage<T, MODE>;
-  constexpr bool JAC = ST::JAC, HAS_B = ST::HAS_B;
+  constexpr bool HAS_B = ST::HAS_B;
   constexpr int TBY = ST::TBY, SEG = TBY / TTY, P = ST::P, OFF = Tile<T>::OFF, UR = ST::UR, MR = ST::MR;
   constexpr int NTH = TBX * TTY;
   if (MODE != PLAIN && MODE != BEND && MODE != RESID) {
@@ -128,8 +121,6 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
     const uint32_t bar = smem_u32(&mbar[b]);
     mbar_expect_tx(bar, ST::TX);
     tma_load_2d(smem_u32(base + ST::OV), &mv, i0 - OFF, j0 - 2, bar);
-    if (JAC) tma_load_2d(smem_u32(base + ST::OJ), &mJ, i0 - OFF, j0 - 2, bar);
-    if (MODE == JAC_FINAL) tma_load_2d(smem_u32(base + ST::OP), &mpart, i0 - OFF, j0 - 2, bar);
     tma_load_2d(smem_u32(base + ST::OD), &md, i0 - OFF, j0 - 1, bar);
     if (ST::HAS_C) tma_load_2d(smem_u32(base + ST::OC), &mc, i0, j0, bar);
     if (HAS_B) tma_load_2d(smem_u32(base + ST::OB), &mb, i0, j0, bar);
@@ -146,9 +137,8 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
     }
   }
   uint32_t phase[2] = {0u, 0u};
-  Acc<2> acc;
+  Acc<1> acc;
   acc.v[0] = 0.0;
-  acc.v[1] = 0.0;
   const int r0 = ty * SEG;
   auto wrapc = [&](int g) { return g < 0 ? g + w : (g >= w ? g - w : g); };
   auto clampr = [&](int g) { return min(max(g, 0), h - 1); };
@@ -175,8 +165,6 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
     }
     unsigned char* base = smem + b * ST::BYTES;
     T* sv = reinterpret_cast<T*>(base + ST::OV);
-    T* sJ = reinterpret_cast<T*>(base + ST::OJ);
-    T* sP = reinterpret_cast<T*>(base + ST::OP);
     T* sd = reinterpret_cast<T*>(base + ST::OD);
     const T* sc = reinterpret_cast<const T*>(base + ST::OC);
     const T* sB = reinterpret_cast<const T*>(base + ST::OB);
@@ -191,8 +179,6 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
         size_t gi = (size_t)clampr(j0 - 2 + rr) * w + wrapc(i0 + lc);
         int si = rr * P + OFF + lc;
         sv[si] = vsrc[gi];
-        if (JAC) sJ[si] = J[gi];
-        if (MODE == JAC_FINAL) sP[si] = part[gi];
       }
       for (int e = tid; e < MR * 2; e += NTH) {
         int rr = e >> 1, q = e & 1;
@@ -211,8 +197,6 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
         if (g >= 0 && g < h) continue;
         int si = rr * P + col, so = (clampr(g) - j0 + 2) * P + col;
         sv[si] = sv[so];
-        if (JAC) sJ[si] = sJ[so];
-        if (MODE == JAC_FINAL) sP[si] = sP[so];
       }
       for (int e = tid; e < MR * P; e += NTH) {
         int rr = e / P, col = e - rr * P;
@@ -222,19 +206,9 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
       }
       __syncthreads();
     }
-    if (JAC) {
-      // u = J r (+ part); r and J stay readable for the outputs
-      for (int e = tid; e < UR * P; e += NTH) {
-        T u = sJ[e] * sv[e];
-        if (MODE == JAC_FINAL) u += sP[e];
-        sP[e] = u;
-      }
-      __syncthreads();
-    }
-    const T* su = JAC ? sP : sv;
     // m = d . L u at local rows -1 .. TBY, columns -1 .. TBX (as k_apply)
     {
-      const T* ucol = su + OFF + tx;
+      const T* ucol = sv + OFF + tx;
       T* mcol = sd + OFF + tx;
       T un = ucol[(r0 + 1) * P], uc = ucol[(r0 + 2) * P];
 #pragma unroll
@@ -256,7 +230,7 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
         lr = (e - 2 * (TBX + 2)) >> 1;
         lc = (e & 1) ? TBX : -1;
       }
-      const T* uc = su + (lr + 2) * P + OFF + lc;
+      const T* uc = sv + (lr + 2) * P + OFF + lc;
       T lap = (uc[-1] + uc[1] + uc[-P] + uc[P] - (T)4 * uc[0]) * inv_dx2;
       T* m = sd + (lr + 1) * P + OFF + lc;
       *m = lap * *m;
@@ -287,28 +261,17 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
         const int j = j0 + lr;
         if (j < h) {
           size_t kk = (size_t)j * w + i;
-          T u = su[(lr + 2) * P + OFF + tx];
+          T u = sv[(lr + 2) * P + OFF + tx];
           if (MODE == BEND) {
             y[kk] = lm;
           } else {
             T au = lm + sc[lr * TBX + tx] * u;
-            if (MODE == AP_DOT) {
+            if (MODE == PLAIN) {
               y[kk] = au;
-              acc.v[0] += (double)u * (double)au;
-            } else if (MODE == PLAIN) {
-              y[kk] = au;
-            } else if (HAS_B) {
+            } else {
               T rr = sB[lr * TBX + tx] - au;
               y[kk] = rr;
               acc.v[0] += (double)rr * (double)rr;
-            } else if (MODE == JAC_LEFT) {
-              y[kk] = sv[(lr + 2) * P + OFF + tx] - au;
-            } else {  // JAC_FINAL
-              T r = sv[(lr + 2) * P + OFF + tx];
-              T z = u + sJ[(lr + 2) * P + OFF + tx] * (r - au);
-              y[kk] = z;
-              acc.v[0] += (double)r * (double)z;
-              acc.v[1] = fmax(acc.v[1], fabs((double)z));
             }
           }
         }
@@ -322,17 +285,11 @@ __global__ void __launch_bounds__(TBX* TTY) k_apply_tma(const __grid_constant__ 
       pending[b] = true;
     }
   }
-  if (MODE == AP_DOT || MODE == RESID || MODE == RESID_GATED || MODE == JAC_FINAL) {
-    const int kind[2] = {0, 1};
-    unsigned int nb = gridDim.x;
-    int site = MODE == AP_DOT ? SITE_PAP : (MODE == RESID || MODE == RESID_GATED) ? SITE_RESID : SITE_PRECOND;
-    bool last = MODE == JAC_FINAL ? reduce_partials<2>(acc, kind, partials, &S->ticket[site], nb)
-                                  : reduce_partials<1>(*reinterpret_cast<Acc<1>*>(&acc), kind, partials, &S->ticket[site], nb);
-    if (last && tid == 0) {
-      if (MODE == AP_DOT) finish_pap(S, acc.v[0]);
+  if (HAS_B) {
+    const int kind[1] = {0};
+    if (reduce_partials<1>(acc, kind, partials, &S->ticket[SITE_RESID], gridDim.x) && tid == 0) {
       if (MODE == RESID) S->rr = acc.v[0];
       if (MODE == RESID_GATED) S->rr_true = acc.v[0];
-      if (MODE == JAC_FINAL) finish_precond(S, acc.v[0], acc.v[1]);
     }
   }
 }
