@@ -41,6 +41,7 @@
 
 #include "common.cuh"
 #include "fft.cuh"
+#include <cooperative_groups.h>
 #include <cuda_pipeline.h>
 
 namespace dt {
@@ -2240,14 +2241,14 @@ static dt_status make_tables(dt_flex* s, Tables<T>& tb) {
 // The plan of the transform along x for a width whose half is not a power of two: mixed-radix
 // stages when every prime factor of w is at most ANY_MAX_PRIME, else Bluestein through the power
 // of two M >= 2 w - 1.
-static AnyPlan make_any_plan(int w, int h) {
+static AnyPlan make_any_plan(int w, int h, int most = 16) {
   AnyPlan p;
   p.w = w;
   p.pairs = (h + 1) / 2;
   std::vector<int> f;
   int n = w;
   for (int r : {16, 8, 4, 2})
-    while (n % r == 0) {
+    while (r <= most && n % r == 0) {
       f.push_back(r);
       n /= r;
     }
@@ -2262,11 +2263,14 @@ static AnyPlan make_any_plan(int w, int h) {
     while (m < 2 * w - 1) m *= 2;
     f.clear();
     for (int r : {16, 8, 4, 2})
-      while (m % r == 0) {
+      while (r <= most && m % r == 0) {
         f.push_back(r);
         m /= r;
       }
   }
+  // odd radices first: the first stage's outputs lie a radix apart, which in shared memory keeps the
+  // powers of two's from falling in the same banks
+  std::stable_partition(f.begin(), f.end(), [](int r) { return r % 2 != 0; });
   p.L = 1;
   for (int x : f) p.L *= x;
   p.nst = (int)f.size();
@@ -2276,6 +2280,8 @@ static AnyPlan make_any_plan(int w, int h) {
     p.span[k] = span;
     span *= f[k];
   }
+  // a row pair in one FP64 block: radix 8 at most
+  if (most > 8 && any_block_smem<double>(p) <= ANY_BLOCK_SMEM) return make_any_plan(w, h, 8);
   return p;
 }
 
@@ -2721,6 +2727,12 @@ static RowsLevelsFn<T> rows_levels_fn(int logn, std::integer_sequence<int, L...>
 template <class T>
 static void transform_smem_attributes() {
   int big = 200 * 1024;
+  cudaFuncSetAttribute(k_any_block_fwd<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
+  cudaFuncSetAttribute(k_any_block_fwd<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
+  cudaFuncSetAttribute(k_any_block_inv<T, INV_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
+  cudaFuncSetAttribute(k_any_block_inv<T, INV_STORE_W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
+  cudaFuncSetAttribute(k_any_block_bank<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
+  cudaFuncSetAttribute(k_any_block_inv<T, INV_STORE_DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
   cudaFuncSetAttribute(k_row_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   for (int l = 0; l < FFT_LOGS; ++l) {
     cudaFuncSetAttribute(rows_fwd_fn<T, true>(l, LogSeq{}), cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -2784,10 +2796,28 @@ static cplx<T>* any_slot(dt_flex* s, Lane<T>& L, int level) {
   return L.any_buf + (size_t)level * 2 * s->plan.pairs * s->plan.L;
 }
 
+// Whether a row pair of the plan is transformed in one block's shared memory, both ways.
+template <class T>
+static bool any_in_block(const AnyPlan& p) {
+  return any_block_smem<T>(p) <= ANY_BLOCK_SMEM;
+}
+
 template <class T>
 static void any_rows_fwd(dt_flex* s, Lane<T>& L, const T* in, const T* wt, cplx<T>* half, int level, Scalars* S,
-                         cudaStream_t st) {
+                         cudaStream_t st, int levels = 1) {
   const AnyPlan& p = s->plan;
+  if (any_in_block<T>(p)) {
+    const dim3 grid(p.pairs, levels);
+    const int nt = any_block_threads(p);
+    if (wt)
+      k_any_block_fwd<T, true><<<grid, nt, any_block_smem<T>(p), st>>>(p, s->h, s->N, in, wt, half, L.any_tw, L.any_chirp,
+                                                                              L.any_bhat, S);
+    else
+      k_any_block_fwd<T, false><<<grid, nt, any_block_smem<T>(p), st>>>(p, s->h, s->N, in, wt, half, L.any_tw, L.any_chirp,
+                                                                               L.any_bhat, S);
+    counted();
+    return;
+  }
   cplx<T>* a = any_slot<T>(s, L, level);
   cplx<T>* b = a + (size_t)p.pairs * p.L;
   const unsigned g = any_grid((size_t)p.pairs * p.L);
@@ -2805,6 +2835,23 @@ template <class T>
 static void any_rows_inv(dt_flex* s, Lane<T>& L, int mode, const cplx<T>* half, T* out, const T* wt, const T* r,
                          Scalars* S, cudaStream_t st) {
   const AnyPlan& p = s->plan;
+  if (any_in_block<T>(p)) {
+    const size_t smem = any_block_smem<T>(p);
+    const int nt = any_block_threads(p);
+    auto go = [&](auto kernel) {
+      kernel<<<p.pairs, nt, smem, st>>>(p, s->h, s->N, half, out, wt, r, L.any_tw, L.any_chirp, L.any_bhat, s->partials, S);
+    };
+    switch (mode) {
+      case INV_STORE: go(k_any_block_inv<T, INV_STORE>); break;
+      case INV_STORE_W: go(k_any_block_inv<T, INV_STORE_W>); break;
+      case INV_BANK:
+        k_any_block_bank<T><<<dim3(p.pairs, 3), nt, smem, st>>>(p, s->h, s->N, half, out, wt, L.any_tw, L.any_chirp, L.any_bhat, S);
+        break;
+      default: go(k_any_block_inv<T, INV_STORE_DOT>); break;
+    }
+    counted();
+    return;
+  }
   const int levels = mode == INV_BANK ? 3 : 1;
   const size_t pl = (size_t)p.pairs * p.L;
   cplx<T>* f0 = nullptr;
@@ -2931,7 +2978,7 @@ static void launch_spectral(dt_flex* s, Lane<T>& L, const T* in, const T* wt, T*
 // transforms, and along y the cosine transform or k_row_solve).
 template <class T>
 static bool bank_batched(const dt_flex* s) {
-  return s->bank_one_launch && !s->any && !(s->row_solve && row_groups<T>(s->h) < 0);
+  return s->bank_one_launch && !(s->any && !any_in_block<T>(s->plan)) && !(s->row_solve && row_groups<T>(s->h) < 0);
 }
 
 // z = M^-1 r with r.z and max|z| reduced into S (finish_precond). levels 1: one spectral solve at
@@ -2950,9 +2997,13 @@ static void launch_precondition(dt_flex* s, Lane<T>& L, const T* r, T* z, int le
   // three spectra to the weighted sum.
   if (bank_batched<T>(s)) {
     FftGeo g = fft_geometry<T>(s);
-    rows_fwd_fn<T, true>(ilog2(s->N), LogSeq{}, g.rsmall)<<<dim3(g.rgrid, 3), g.rthreads, g.rsmem, st>>>(
-        s->w, s->h, L.left, L.wt[0], L.half, L.tab.tw_row, L.tab.post, L.S);
-    counted();
+    if (s->any) {
+      any_rows_fwd<T>(s, L, L.left, L.wt[0], L.half, 0, L.S, st, 3);
+    } else {
+      rows_fwd_fn<T, true>(ilog2(s->N), LogSeq{}, g.rsmall)<<<dim3(g.rgrid, 3), g.rthreads, g.rsmem, st>>>(
+          s->w, s->h, L.left, L.wt[0], L.half, L.tab.tw_row, L.tab.post, L.S);
+      counted();
+    }
     launch_cols<T>(s, L, L.half, g, 0, L.S, st, 3);
     launch_rows_inv<T>(s, L, INV_BANK, L.half, L.part, L.wt[0], nullptr, g, L.S, st);
     launch_apply<T>(s, JAC_FINAL, nullptr, L.J, L.part, L.d, L.c, r, z, L.S, st);  // z = u + J(r - A u)
@@ -4039,7 +4090,9 @@ static dt_status profile_lane(dt_flex* s, Lane<T>& L, int reps, double* ms, doub
         case 6: launch_apply<T>(s, JAC_LEFT, nullptr, L.J, nullptr, L.d, L.c, L.r, L.left, L.S, st); break;
         case 7: launch_apply<T>(s, JAC_FINAL, nullptr, L.J, L.part, L.d, L.c, L.r, L.z, L.S, st); break;
         case 8:
-          if (bank1) {
+          if (bank1 && s->any) {
+            any_rows_fwd<T>(s, L, L.left, L.wt[0], L.half, 0, L.S, st, 3);
+          } else if (bank1) {
             rows_fwd_fn<T, true>(ilog2(s->N), LogSeq{}, g.rsmall)<<<dim3(g.rgrid, 3), g.rthreads, g.rsmem, st>>>(
                 s->w, s->h, L.left, L.wt[0], L.half, L.tab.tw_row, L.tab.post, L.S);
             counted();

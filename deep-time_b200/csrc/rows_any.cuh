@@ -296,3 +296,290 @@ __global__ void __launch_bounds__(256) k_any_emit(AnyPlan p, int h, const cplx<T
       finish_precond(S, acc.v[0], acc.v[1]);
   }
 }
+// ---- the same transform with a row pair in one block's shared memory ----
+// Where two buffers of L values (and for the bank's inverse a row pair of sums) fit one block, each pass
+// takes a row pair from the raster to the spectrum or back: the stages alternate between the buffers, a
+// barrier each, and nothing of them goes through global memory. The values of the passes above, stage for
+// stage. Bound by the stages' latency: the block's threads are chosen so that the stages' butterflies
+// fill whole rounds of them (any_block_threads; 256 threads on 300 butterflies of radix 5 leave two
+// thirds of the second round idle), the FP64 plans take radix 8 at most to keep four blocks an SM, and the
+// bank's three levels run side by side as a cluster of blocks. FP64 1500 x 750 (radices 4, 3, 5, 5, 5), a
+// bank pass of three levels: forward 44 us and inverse 65 (cold caches), against 21 launches of 6 us each
+// way and a summing one on three streams; the step's solve there 2.43 to 2.10 ms.
+constexpr size_t ANY_BLOCK_SMEM = 200 * 1024;
+template <class T>
+static size_t any_block_smem(const AnyPlan& p) {
+  return (size_t)2 * p.L * sizeof(cplx<T>);
+}
+// The threads of a row pair's block: of 96 to 256, the fewest idle lanes over the plan's stages.
+static int any_block_threads(const AnyPlan& p) {
+  int best = 128;
+  long least = -1;
+  for (int nt = 96; nt <= 256; nt += 32) {
+    long cost = 0;
+    for (int s = 0; s < p.nst; ++s) cost += (long)ceil_div(p.L / p.radix[s], nt) * nt * p.radix[s];
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = nt;
+    }
+  }
+  return best;
+}
+
+template <class T, int R>
+__device__ __forceinline__ void any_block_stage(const AnyPlan& p, int stage, const cplx<T>* in, cplx<T>* out,
+                                                const cplx<T>* __restrict__ tw) {
+  using C = cplx<T>;
+  const int L = p.L, Ns = p.span[stage], LR = L / R, step = L / (Ns * R);
+  C wr[R];  // w_R^q of a small odd radix
+  if constexpr (R == 3 || R == 5 || R == 7) {
+#pragma unroll
+    for (int q = 0; q < R; ++q) wr[q] = tw[q * LR];
+  }
+  for (int j = threadIdx.x; j < LR; j += blockDim.x) {
+    const int hi = j / Ns, k = j - hi * Ns;
+    C v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = in[j + r * LR];
+    if (k) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], any_tw(tw, r * k * step));
+    }
+    C* o = out + hi * Ns * R + k;
+    if constexpr (R == 3 || R == 5 || R == 7) {
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        C acc = v[0];
+#pragma unroll
+        for (int r = 1; r < R; ++r) acc = cadd(acc, cmul(v[r], wr[(r * m) % R]));
+        o[m * Ns] = acc;
+      }
+    } else {
+      dft_r<C, R, false>(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) o[r * Ns] = v[r];
+    }
+  }
+}
+// any prime radix up to ANY_MAX_PRIME, an output a thread
+template <class T>
+__device__ __forceinline__ void any_block_prime(const AnyPlan& p, int stage, const cplx<T>* in, cplx<T>* out,
+                                                const cplx<T>* __restrict__ tw) {
+  using C = cplx<T>;
+  const int L = p.L, Ns = p.span[stage], R = p.radix[stage], LR = L / R, step = L / (Ns * R);
+  for (int q = threadIdx.x; q < L; q += blockDim.x) {
+    const int j = q / R, m = q - j * R, hi = j / Ns, k = j - hi * Ns;
+    C acc = in[j];
+    for (int r = 1; r < R; ++r) {
+      C x = in[j + r * LR];
+      if (k) x = cmul(x, any_tw(tw, r * k * step));
+      acc = cadd(acc, cmul(x, any_tw(tw, ((r * m) % R) * LR)));
+    }
+    out[hi * Ns * R + k + m * Ns] = acc;
+  }
+}
+// One FFT of length L between the buffers a and b; returns the one that holds the result.
+template <class T>
+__device__ __forceinline__ cplx<T>* any_block_fft(const AnyPlan& p, cplx<T>* a, cplx<T>* b, const cplx<T>* __restrict__ tw) {
+  for (int s = 0; s < p.nst; ++s) {
+    switch (p.radix[s]) {
+      case 2: any_block_stage<T, 2>(p, s, a, b, tw); break;
+      case 3: any_block_stage<T, 3>(p, s, a, b, tw); break;
+      case 4: any_block_stage<T, 4>(p, s, a, b, tw); break;
+      case 5: any_block_stage<T, 5>(p, s, a, b, tw); break;
+      case 7: any_block_stage<T, 7>(p, s, a, b, tw); break;
+      case 8: any_block_stage<T, 8>(p, s, a, b, tw); break;
+      case 16:
+        if constexpr (sizeof(T) == 4) any_block_stage<T, 16>(p, s, a, b, tw);  // FP64 plans: radix 8 at most
+        break;
+      default: any_block_prime<T>(p, s, a, b, tw); break;
+    }
+    __syncthreads();
+    cplx<T>* t = a;
+    a = b;
+    b = t;
+  }
+  return a;
+}
+// DFT_w of the row pair in a (Bluestein: up to any_fetch's last product)
+template <class T>
+__device__ __forceinline__ cplx<T>* any_block_dft(const AnyPlan& p, cplx<T>* a, cplx<T>* b, const cplx<T>* __restrict__ tw,
+                                  const cplx<T>* __restrict__ bhat) {
+  cplx<T>* f = any_block_fft<T>(p, a, b, tw);
+  if (p.bluestein) {
+    for (int q = threadIdx.x; q < p.L; q += blockDim.x) f[q] = cconj(cmul(f[q], bhat[q]));
+    __syncthreads();
+    f = any_block_fft<T>(p, f, f == a ? b : a, tw);
+  }
+  return f;
+}
+
+// Forward: the row pair blockIdx.x (times the weights of the bank's level blockIdx.y) into the level's half
+// spectrum; the levels' weights and spectra consecutive.
+template <class T, bool WEIGHT>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_any_block_fwd(AnyPlan p, int h, int N, const T* __restrict__ v, const T* __restrict__ wt,
+                                                       cplx<T>* __restrict__ half, const cplx<T>* __restrict__ tw,
+                                                       const cplx<T>* __restrict__ chirp, const cplx<T>* __restrict__ bhat,
+                                                       const Scalars* S) {
+  using C = cplx<T>;
+  if (S->stop) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* const a = reinterpret_cast<C*>(smem_raw);
+  const int w = p.w, pr = blockIdx.x;
+  const bool has_b = 2 * pr + 1 < h;
+  if (WEIGHT) wt += (size_t)blockIdx.y * w * h;
+  half += (size_t)blockIdx.y * h * N;
+  const T *ra = v + (size_t)(2 * pr) * w, *rb = ra + w, *wa = wt + (size_t)(2 * pr) * w, *wb = wa + w;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < p.L; i += blockDim.x) {
+    C z = mk<C>((T)0, (T)0);
+    if (i < w) {
+      T x = ra[i], y = has_b ? rb[i] : (T)0;
+      if (WEIGHT) {
+        x *= wa[i];
+        y = has_b ? y * wb[i] : (T)0;
+      }
+      z = mk<C>(x, y);
+      if (p.bluestein) z = cmul(z, cconj(chirp[i]));
+    }
+    a[i] = z;
+  }
+  __syncthreads();
+  const C* row = any_block_dft<T>(p, a, a + p.L, tw, bhat);
+  C *ha = half + (size_t)(2 * pr) * N, *hb = ha + N;
+  const T half_ = (T)0.5;
+  auto parts = [&](int kk, C& A, C& B) {
+    C z = any_fetch(p, row, kk, chirp), zc = cconj(any_fetch(p, row, kk == 0 ? 0 : w - kk, chirp));
+    A = cscale(cadd(z, zc), half_);
+    C d = csub(z, zc);
+    B = mk<C>(d.y * half_, -d.x * half_);  // (z - conj z') / 2i
+  };
+  for (int k = threadIdx.x; k < N; k += blockDim.x) {
+    C A, B;
+    parts(k, A, B);
+    if (k == 0) {
+      T an = (T)0, bn = (T)0;
+      if ((w & 1) == 0) {
+        C A2, B2;
+        parts(w / 2, A2, B2);
+        an = A2.x;
+        bn = B2.x;
+      }
+      A = mk<C>(A.x, an);
+      B = mk<C>(B.x, bn);
+    }
+    ha[k] = A;
+    if (has_b) hb[k] = B;
+  }
+}
+
+// The row pair's spectrum (half: its first row) into a, conjugated, for the forward transform.
+template <class T>
+__device__ __forceinline__ void any_block_load_half(const AnyPlan& p, bool has_b, int N, const cplx<T>* __restrict__ ra,
+                                                    cplx<T>* a, const cplx<T>* __restrict__ chirp) {
+  using C = cplx<T>;
+  const int w = p.w, nk = w / 2 + 1;
+  const C* rb = ra + N;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < p.L; i += blockDim.x) {
+    C z = mk<C>((T)0, (T)0);
+    if (i < w) {
+      const bool up = i < nk;  // else i = w - k with 1 <= k < nk: conj A[k] + i conj B[k]
+      const int k = up ? i : w - i;
+      C A = any_unpack(ra, k, w), B = has_b ? any_unpack(rb, k, w) : mk<C>((T)0, (T)0);
+      if (!up) {
+        A = cconj(A);
+        B = cconj(B);
+      }
+      z = cconj(cadd(A, cmuli(B)));
+      if (p.bluestein) z = cmul(z, cconj(chirp[i]));
+    }
+    a[i] = z;
+  }
+}
+
+// Inverse of one level, in k_any_emit's modes other than INV_BANK.
+template <class T, int MODE>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4)
+    k_any_block_inv(AnyPlan p, int h, int N, const cplx<T>* __restrict__ half, T* __restrict__ out, const T* __restrict__ wt,
+                    const T* __restrict__ r, const cplx<T>* __restrict__ tw, const cplx<T>* __restrict__ chirp,
+                    const cplx<T>* __restrict__ bhat, double* partials, Scalars* S) {
+  using C = cplx<T>;
+  if (S->stop) {
+    if (MODE == INV_STORE_DOT && blockIdx.x == 0 && threadIdx.x == 0) set_cond(S, 0);
+    return;
+  }
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* const a = reinterpret_cast<C*>(smem_raw);
+  const int w = p.w, pr = blockIdx.x;
+  const bool has_b = 2 * pr + 1 < h;
+  const size_t ka = (size_t)(2 * pr) * w, kb = ka + w;
+  const T inv_w = (T)1 / (T)w;
+  Acc<2> acc;
+  acc.v[0] = acc.v[1] = 0.0;
+  any_block_load_half<T>(p, has_b, N, half + (size_t)(2 * pr) * N, a, chirp);
+  __syncthreads();
+  const C* row = any_block_dft<T>(p, a, a + p.L, tw, bhat);
+#pragma unroll 2
+  for (int i = threadIdx.x; i < w; i += blockDim.x) {
+    const C z = cconj(any_fetch(p, row, i, chirp));
+    T x = z.x * inv_w, y = z.y * inv_w;
+    if (MODE == INV_STORE_W) {
+      x *= wt[ka + i];
+      y = has_b ? y * wt[kb + i] : (T)0;
+    }
+    out[ka + i] = x;
+    if (has_b) out[kb + i] = y;
+    if (MODE == INV_STORE_DOT) {
+      acc.v[0] += (double)r[ka + i] * (double)x;
+      acc.v[1] = fmax(acc.v[1], fabs((double)x));
+      if (has_b) {
+        acc.v[0] += (double)r[kb + i] * (double)y;
+        acc.v[1] = fmax(acc.v[1], fabs((double)y));
+      }
+    }
+  }
+  if (MODE == INV_STORE_DOT) {
+    const int kind[2] = {0, 1};
+    if (reduce_partials<2>(acc, kind, partials, &S->ticket[SITE_PRECOND], gridDim.x) && threadIdx.x == 0)
+      finish_precond(S, acc.v[0], acc.v[1]);
+  }
+}
+
+// The bank's inverse: a cluster of three blocks a row pair, a level each; then each block sums a third of
+// the pair's columns over the three blocks' shared memory, in the levels' order.
+template <class T>
+__global__ void __cluster_dims__(1, 3, 1) __launch_bounds__(256, sizeof(T) == 8 ? 2 : 4)
+    k_any_block_bank(AnyPlan p, int h, int N, const cplx<T>* __restrict__ half, T* __restrict__ out, const T* __restrict__ wt,
+                     const cplx<T>* __restrict__ tw, const cplx<T>* __restrict__ chirp, const cplx<T>* __restrict__ bhat,
+                     const Scalars* S) {
+  using C = cplx<T>;
+  if (S->stop) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* const a = reinterpret_cast<C*>(smem_raw);
+  const int w = p.w, pr = blockIdx.x, lv = blockIdx.y;
+  const bool has_b = 2 * pr + 1 < h;
+  const size_t ka = (size_t)(2 * pr) * w, kb = ka + w;
+  const T inv_w = (T)1 / (T)w;
+  wt += (size_t)lv * w * h;
+  any_block_load_half<T>(p, has_b, N, half + ((size_t)lv * h + 2 * pr) * N, a, chirp);
+  __syncthreads();
+  // the level's weighted rows over its transform (every level's ends in the same buffer)
+  C* row = any_block_dft<T>(p, a, a + p.L, tw, bhat);
+#pragma unroll 2
+  for (int i = threadIdx.x; i < w; i += blockDim.x) {
+    const C z = cconj(any_fetch(p, row, i, chirp));
+    row[i] = mk<C>(z.x * inv_w * wt[ka + i], has_b ? z.y * inv_w * wt[kb + i] : (T)0);
+  }
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  const C *r0 = cluster.map_shared_rank(row, 0), *r1 = cluster.map_shared_rank(row, 1), *r2 = cluster.map_shared_rank(row, 2);
+  const int third = (w + 2) / 3, end = min(w, (lv + 1) * third);
+#pragma unroll 2
+  for (int i = lv * third + threadIdx.x; i < end; i += blockDim.x) {
+    const C x0 = r0[i], x1 = r1[i], x2 = r2[i];
+    out[ka + i] = x0.x + x1.x + x2.x;
+    if (has_b) out[kb + i] = x0.y + x1.y + x2.y;
+  }
+  cluster.sync();  // no block leaves while another reads its rows
+}
