@@ -8,11 +8,9 @@
 // with the taps mirrored and the weight matrix transposed.
 //
 // Forward / input-gradient: out[p][co] = sum_{tap, ci} in[p + off(tap)][ci] W[tap][ci][co], a GEMM
-// with M = pixels, N = output channels, K = 9 x input channels. A block computes 64 consecutive
-// pixels of one image row by BN output channels; K advances one tap and 32 input channels at a
-// time. Tiles are staged by cp.async in two stages, fragments are loaded with ldmatrix (x4 for A,
-// x4.trans for B, both from XOR-swizzled shared memory) and multiplied with
-// mma.sync.m16n8k16.row.col.f32.bf16.bf16.f32; 4 warps as 2 x 2, each 32 x (BN / 2).
+// with M = pixels, N = output channels, K = 9 x input channels (k_conv3x3_res). Fragments are loaded with
+// ldmatrix (x4 for A, x4.trans for B from XOR-swizzled shared memory) and multiplied with
+// mma.sync.m16n8k16.row.col.f32.bf16.bf16.f32.
 //
 // Weight gradient: dW[tap][ci][co] = sum_p in[p + off(tap)][ci] g[p][co], a GEMM with M = input
 // channels, N = output channels, K = pixels; each block reduces a chunk of pixel tiles and writes
@@ -75,28 +73,90 @@ __device__ __forceinline__ int swz_b(int row, int chunk) {
 
 enum { EPI_BIAS_RELU = 0, EPI_BIAS = 1, EPI_STORE = 2, EPI_ACCUM = 3, EPI_MASK = 4 };
 
-// One 3 x 3 convolution (or its input gradient with mirrored, transposed weights): W is
-// [9][Cin][Cout] bf16, tap = ky * 3 + kx reading in[y + ky - 1][x + kx - 1]. Image rows of width
-// `w` (a multiple of 64), `h` rows, `nimg` images.
-template <int BN, int EPI>
-__global__ void __launch_bounds__(128) k_conv3x3(int nimg, int h, int w, Tensor4 in, const bf16* __restrict__ W,
-                                                 const float* __restrict__ bias, Tensor4 out, Tensor4 mask) {
-  constexpr int BM = 64, BK = 32;
-  __shared__ __align__(128) bf16 sA[2][BM * BK];
-  __shared__ __align__(128) bf16 sB[2][BK * BN];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;  // warp tile: rows wm*32.., cols wn*(BN/2)..
-  const int tiles_x = w / BM;
+// Two neighbouring channels of a pixel's output: the bias and ReLU, or the producing ReLU's mask.
+template <int EPI>
+__device__ __forceinline__ void conv_store(bf16* dst, int col, float v0, float v1, const float* __restrict__ bias, int co0,
+                                           const Tensor4& mask, size_t pix) {
+  if (EPI == EPI_BIAS_RELU || EPI == EPI_BIAS) {
+    v0 += bias[co0 + col];
+    v1 += bias[co0 + col + 1];
+  }
+  if (EPI == EPI_BIAS_RELU) {
+    v0 = fmaxf(v0, 0.f);
+    v1 = fmaxf(v1, 0.f);
+  }
+  __nv_bfloat162* d2 = reinterpret_cast<__nv_bfloat162*>(dst + col);
+  if (EPI == EPI_MASK) {
+    // the gradient through the producing ReLU: zero where its output was zero
+    __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(mask.p + pix * mask.stride + mask.off + co0 + col);
+    if (!(__bfloat162float(m.x) > 0.f)) v0 = 0.f;
+    if (!(__bfloat162float(m.y) > 0.f)) v1 = 0.f;
+  }
+  if (EPI == EPI_ACCUM) {
+    __nv_bfloat162 prev = *d2;
+    v0 += __bfloat162float(prev.x);
+    v1 += __bfloat162float(prev.y);
+  }
+  *d2 = __floats2bfloat162_rn(v0, v1);
+}
+
+// One 3 x 3 convolution (or its input gradient with mirrored, transposed weights): W is [9][Cin][Cout]
+// bf16, tap = ky * 3 + kx reading in[y + ky - 1][x + kx - 1]; image rows of width `w` (a multiple of 64),
+// `h` rows, `nimg` images. A block takes RY rows by 64 pixels of one image and BN output channels, its
+// warps 32 pixels each of one row by all BN channels. The region's (RY + 2) x 66 pixels of every input
+// channel are copied once into shared memory (padding and wrap in the copies) and the nine taps read them
+// at shifted addresses; the weights come a tap and 32 channels at a time through a ring of STAGES.
+// Products are summed by tap, then channel, 16 at a time. A pixel's channels are spaced by 16 bytes
+// more than their own, which puts the eight rows of an ldmatrix in distinct banks.
+// 2 RY x COW warps of 32 pixels by NC channels each, BN = NC COW.
+// Bound by the legacy tensor path's issue (mma.sync) and its ldmatrix loads. Staging every tap's 128
+// pixels anew through shared memory (nine times the input traffic) took, at 16 x 512 x 256 cells,
+// 357 us for 32 -> 32 channels (now 253, 153 TFLOP/s), 716 for the gradient 32 -> 96 (522), 265
+// for a masked gradient 32 -> 32 (184), 492 for 64 -> 192 at half the size (430) and 875 for 384 -> 128
+// at a quarter (552).
+__host__ __device__ constexpr size_t conv_res_smem(int cin, int ry, int bn, int stages) {
+  return (size_t)(ry + 2) * 66 * (cin * 2 + 16) + (size_t)stages * 32 * bn * 2;
+}
+template <int NC, int COW, int RY, int STAGES, int EPI>
+__global__ void __launch_bounds__(64 * RY * COW) k_conv3x3_res(int nimg, int h, int w, Tensor4 in, const bf16* __restrict__ W,
+                                                         const float* __restrict__ bias, Tensor4 out, Tensor4 mask) {
+  constexpr int BN = NC * COW, NTH = 64 * RY * COW, BK = 32, NT = NC / 8;
+  extern __shared__ __align__(128) unsigned char conv_smem[];
+  const int cin = in.c, pitch = cin * 2 + 16;  // bytes a pixel
+  bf16* const sB = reinterpret_cast<bf16*>(conv_smem);
+  unsigned char* const sA = conv_smem + (size_t)STAGES * BK * BN * 2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = (warp >> 1) % RY, px0 = (warp & 1) * 32,
+            nc0 = warp / (2 * RY) * NC;
+  const int tiles_x = w / 64, tiles_y = (h + RY - 1) / RY;
   int bid = blockIdx.x;
-  const int xt = bid % tiles_x;
+  const int x0 = (bid % tiles_x) * 64;
   bid /= tiles_x;
-  const int y = bid % h;
-  const int n = bid / h;
-  const int x0 = xt * BM;
-  const int co0 = blockIdx.y * BN;
-  const int cin = in.c;
-  const int kchunks = 9 * (cin / BK);
-  constexpr int NT = BN / 16;  // n8 tiles per warp
+  const int y0 = (bid % tiles_y) * RY, n = bid / tiles_y;
+  const int co0 = blockIdx.y * BN, cchunks = cin / BK, steps = 9 * cchunks;
+  auto load_b = [&](int s) {
+    if (s < steps) {
+      const int tap = s / cchunks, ci0 = (s - tap * cchunks) * BK;
+      bf16* dst = sB + (s % STAGES) * BK * BN;
+      for (int c = tid; c < BK * BN / 8; c += NTH) {
+        const int r = c / (BN / 8), ch = c % (BN / 8);
+        cp_async16(dst + swz_b<BN>(r, ch), W + ((size_t)tap * cin + ci0 + r) * out.c + co0 + ch * 8, true);
+      }
+    }
+    cp_async_commit();
+  };
+  {
+    const int per = cin / 8, total = (RY + 2) * 66 * per;
+    for (int c = tid; c < total; c += NTH) {
+      const int px = c / per, ch = c - px * per, ry = px / 66, rx = px - ry * 66;
+      const int yy = y0 + ry - 1;
+      int xx = x0 + rx - 1;
+      xx = xx < 0 ? xx + w : (xx >= w ? xx - w : xx);
+      const bool ok = yy >= 0 && yy < h;
+      cp_async16(sA + px * pitch + ch * 16, in.p + ((size_t)((size_t)n * h + (ok ? yy : 0)) * w + xx) * in.stride + in.off + ch * 8, ok);
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) load_b(s);  // the region's copies are in the first group
   float acc[2][NT][4];
 #pragma unroll
   for (int a = 0; a < 2; ++a)
@@ -104,63 +164,23 @@ __global__ void __launch_bounds__(128) k_conv3x3(int nimg, int h, int w, Tensor4
     for (int b = 0; b < NT; ++b)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[a][b][c] = 0.f;
-
-  auto load = [&](int kc, int stage) {
-    int tap = kc / (cin / BK);
-    int ci0 = (kc % (cin / BK)) * BK;
-    int ky = tap / 3, kx = tap % 3;
-    int yy = y + ky - 1;
-    bool yok = yy >= 0 && yy < h;
-    // A: 64 pixels x 32 channels = 256 chunks of 16 B; 2 a thread
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      int cidx = tid + q * 128;
-      int row = cidx >> 2, ch = cidx & 3;
-      int xx = x0 + row + kx - 1;
-      xx = xx < 0 ? xx + w : (xx >= w ? xx - w : xx);
-      const bf16* src = in.p + ((size_t)((size_t)n * h + (yok ? yy : 0)) * w + xx) * in.stride + in.off + ci0 + ch * 8;
-      cp_async16(&sA[stage][swz_a(row, ch)], src, yok);
-    }
-    // B: 32 k-rows x BN channels
-    constexpr int BCH = BK * BN / 8;
-#pragma unroll
-    for (int q = 0; q < (BCH + 127) / 128; ++q) {
-      int cidx = tid + q * 128;
-      if (cidx < BCH) {
-        int row = cidx / (BN / 8), ch = cidx % (BN / 8);
-        const bf16* src = W + ((size_t)tap * cin + ci0 + row) * out.c + co0 + ch * 8;
-        cp_async16(&sB[stage][swz_b<BN>(row, ch)], src, true);
-      }
-    }
-    cp_async_commit();
-  };
-
-  load(0, 0);
-  for (int kc = 0; kc < kchunks; ++kc) {
-    int stage = kc & 1;
-    if (kc + 1 < kchunks) {
-      load(kc + 1, stage ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+  int tap = 0, ci0 = 0;
+  for (int s = 0; s < steps; ++s) {
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();  // step s's weights are there, and step s - 1's stage is read
+    load_b(s + STAGES - 1);
+    const bf16* b = sB + (s % STAGES) * BK * BN;
+    const int ky = tap / 3, kx = tap - 3 * ky;
+    const unsigned char* a = sA + ((row + ky) * 66 + px0 + kx + (lane & 15)) * pitch + (ci0 + (lane >> 4) * 8) * 2;
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 16) {
-      unsigned af[2][4];
+      unsigned af[2][4], bfr[NT][2];
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
-        int row = wm * 32 + mt * 16 + (lane & 15);
-        int chunk = (kk >> 3) + (lane >> 4);
-        ldmatrix_x4(af[mt][0], af[mt][1], af[mt][2], af[mt][3], &sA[stage][swz_a(row, chunk)]);
-      }
-      unsigned bfr[NT][2];
+      for (int mt = 0; mt < 2; ++mt) ldmatrix_x4(af[mt][0], af[mt][1], af[mt][2], af[mt][3], a + mt * 16 * pitch + kk * 2);
 #pragma unroll
       for (int nt = 0; nt < NT; nt += 2) {
-        int krow = kk + (lane & 15);
-        int chunk = (wn * (BN / 2) + nt * 8) / 8 + (lane >> 4);
         unsigned r0, r1, r2, r3;
-        ldmatrix_x4_trans(r0, r1, r2, r3, &sB[stage][swz_b<BN>(krow, chunk)]);
+        ldmatrix_x4_trans(r0, r1, r2, r3, b + swz_b<BN>(kk + (lane & 15), nc0 / 8 + nt + (lane >> 4)));
         bfr[nt][0] = r0;
         bfr[nt][1] = r1;
         bfr[nt + 1][0] = r2;
@@ -171,42 +191,25 @@ __global__ void __launch_bounds__(128) k_conv3x3(int nimg, int h, int w, Tensor4
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) mma_bf16(acc[mt][nt], af[mt], bfr[nt]);
     }
-    __syncthreads();
+    ci0 += BK;
+    if (ci0 == cin) {
+      ci0 = 0;
+      ++tap;
+    }
   }
-  // epilogue: rows = pixels, cols = output channels
+  cp_async_wait<0>();
+  if (y0 + row >= h) return;
   const int g = lane >> 2, t4 = lane & 3;
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      int row = wm * 32 + mt * 16 + g + half * 8;
-      size_t pix = ((size_t)n * h + y) * w + x0 + row;
+      const size_t pix = ((size_t)n * h + y0 + row) * w + x0 + px0 + mt * 16 + g + half * 8;
       bf16* dst = out.p + pix * out.stride + out.off + co0;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
-        int col = wn * (BN / 2) + nt * 8 + t4 * 2;
-        float v0 = acc[mt][nt][half * 2], v1 = acc[mt][nt][half * 2 + 1];
-        if (EPI == EPI_BIAS_RELU || EPI == EPI_BIAS) {
-          v0 += bias[co0 + col];
-          v1 += bias[co0 + col + 1];
-        }
-        if (EPI == EPI_BIAS_RELU) {
-          v0 = fmaxf(v0, 0.f);
-          v1 = fmaxf(v1, 0.f);
-        }
-        __nv_bfloat162* d2 = reinterpret_cast<__nv_bfloat162*>(dst + col);
-        if (EPI == EPI_MASK) {
-          // the gradient through the producing ReLU: zero where its output was zero
-          __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(mask.p + pix * mask.stride + mask.off + co0 + col);
-          if (!(__bfloat162float(m.x) > 0.f)) v0 = 0.f;
-          if (!(__bfloat162float(m.y) > 0.f)) v1 = 0.f;
-        }
-        if (EPI == EPI_ACCUM) {
-          __nv_bfloat162 prev = *d2;
-          v0 += __bfloat162float(prev.x);
-          v1 += __bfloat162float(prev.y);
-        }
-        *d2 = __floats2bfloat162_rn(v0, v1);
+        const int col = nc0 + nt * 8 + t4 * 2;
+        conv_store<EPI>(dst, col, acc[mt][nt][half * 2], acc[mt][nt][half * 2 + 1], bias, co0, mask, pix);
       }
     }
 }

@@ -11,7 +11,7 @@
 //
 // One thread issues the MMAs (K = 16 each, two per step) and commits them to the step's mbarrier;
 // the stage is restaged only after that barrier completes. The accumulator is read back with
-// tcgen05.ld (each warp its 32 TMEM lanes = 32 pixels) for the same epilogues as k_conv3x3.
+// tcgen05.ld (each warp its 32 TMEM lanes = 32 pixels) for the same epilogues as k_conv3x3_res.
 // Every wait is bounded; TMEM is always released before the block leaves.
 #pragma once
 #include "conv.cuh"

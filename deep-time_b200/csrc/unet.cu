@@ -479,60 +479,78 @@ static bool conv_tc(dt_unet* u, int B, int h, int w, Tensor4 in, const bf16* Bk,
   return true;
 }
 
-static void conv_fwd(dt_unet* u, const ConvLayer& L, int B, int h, int w, Tensor4 in, Tensor4 out, bool relu, cudaStream_t st) {
-  {
-    // B[tap][co][ci] = W[tap][ci][co] = WT[8 - tap][co][ci]
-    const float* bias = u->prm + L.b_off;
-    Tensor4 none = T4(nullptr, 0, 0, 0);
-    bool done = relu ? conv_tc<EPI_BIAS_RELU>(u, B, h, w, in, L.WT, L.cout, bias, out, none, st)
-                     : conv_tc<EPI_BIAS>(u, B, h, w, in, L.WT, L.cout, bias, out, none, st);
-    if (done) return;
-  }
-  bool wide = L.cout % 64 == 0;
-  dim3 grid((unsigned)((size_t)B * h * (w / 64)), L.cout / (wide ? 64 : 32));
-  const float* bias = u->prm + L.b_off;
-  Tensor4 none = T4(nullptr, 0, 0, 0);
-  if (wide) {
-    if (relu)
-      k_conv3x3<64, EPI_BIAS_RELU><<<grid, 128, 0, st>>>(B, h, w, in, L.W, bias, out, none);
+// One convolution on the mma.sync path.
+template <int NC, int COW, int RY, int STAGES, int EPI>
+static void conv_res_go(int B, int h, int w, Tensor4 in, const bf16* W, const float* bias, Tensor4 out, Tensor4 mask,
+                        cudaStream_t st) {
+  const dim3 grid((unsigned)((size_t)B * ceil_div(h, RY) * (w / 64)), out.c / (NC * COW));
+  k_conv3x3_res<NC, COW, RY, STAGES, EPI>
+      <<<grid, 64 * RY * COW, conv_res_smem(in.c, RY, NC * COW, STAGES), st>>>(B, h, w, in, W, bias, out, mask);
+}
+// The tile by the input channels, whose region has to stay in shared memory beside the weights' ring:
+// up to 96, 8 warps of 32 pixels and two or more blocks an SM; beyond, one block of 16 warps that
+// share the region over twice the output channels (8 warps and two rows a block took 288 us where
+// this takes 171, 128 -> 128 channels at 16 x 128 x 64 pixels); 384 channels leave room for two rows only.
+template <int EPI>
+static void conv_res(int B, int h, int w, Tensor4 in, const bf16* W, const float* bias, Tensor4 out, Tensor4 mask,
+                     cudaStream_t st) {
+  if (in.c <= 96) {
+    if (out.c % 64 == 0)
+      conv_res_go<64, 1, 4, 4, EPI>(B, h, w, in, W, bias, out, mask, st);
     else
-      k_conv3x3<64, EPI_BIAS><<<grid, 128, 0, st>>>(B, h, w, in, L.W, bias, out, none);
+      conv_res_go<32, 1, 4, 4, EPI>(B, h, w, in, W, bias, out, mask, st);
+  } else if (in.c <= 192) {
+    if (out.c % 128 == 0)
+      conv_res_go<64, 2, 4, 4, EPI>(B, h, w, in, W, bias, out, mask, st);
+    else
+      conv_res_go<32, 2, 4, 4, EPI>(B, h, w, in, W, bias, out, mask, st);
+  } else if (in.c <= 256) {
+    conv_res_go<64, 2, 4, 2, EPI>(B, h, w, in, W, bias, out, mask, st);
   } else {
-    if (relu)
-      k_conv3x3<32, EPI_BIAS_RELU><<<grid, 128, 0, st>>>(B, h, w, in, L.W, bias, out, none);
-    else
-      k_conv3x3<32, EPI_BIAS><<<grid, 128, 0, st>>>(B, h, w, in, L.W, bias, out, none);
+    conv_res_go<32, 4, 2, 2, EPI>(B, h, w, in, W, bias, out, mask, st);
   }
   count_launch();
+}
+template <int EPI>
+static dt_status conv_res_attributes() {
+  const int big = 227 * 1024;
+  DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<64, 1, 4, 4, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<32, 1, 4, 4, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<64, 2, 4, 4, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<32, 2, 4, 4, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<64, 2, 4, 2, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<32, 4, 2, 2, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  return DT_OK;
+}
+
+static void conv_fwd(dt_unet* u, const ConvLayer& L, int B, int h, int w, Tensor4 in, Tensor4 out, bool relu, cudaStream_t st) {
+  // B[tap][co][ci] = W[tap][ci][co] = WT[8 - tap][co][ci]
+  const float* bias = u->prm + L.b_off;
+  Tensor4 none = T4(nullptr, 0, 0, 0);
+  bool done = relu ? conv_tc<EPI_BIAS_RELU>(u, B, h, w, in, L.WT, L.cout, bias, out, none, st)
+                   : conv_tc<EPI_BIAS>(u, B, h, w, in, L.WT, L.cout, bias, out, none, st);
+  if (done) return;
+  if (relu)
+    conv_res<EPI_BIAS_RELU>(B, h, w, in, L.W, bias, out, none, st);
+  else
+    conv_res<EPI_BIAS>(B, h, w, in, L.W, bias, out, none, st);
 }
 
 // input gradient gin = conv(g, WT) (times the ReLU mask of `mask` when given)
 static void conv_dgrad(dt_unet* u, const ConvLayer& L, int B, int h, int w, Tensor4 g, Tensor4 gin, const Tensor4* mask,
                        cudaStream_t st) {
   int cout = L.cin;  // the transposed problem's output channels (96, 192, 384 at the concatenations)
-  bool wide = cout % 64 == 0;
-  dim3 grid((unsigned)((size_t)B * h * (w / 64)), cout / (wide ? 64 : 32));
   Tensor4 none = T4(nullptr, 0, 0, 0);
   Tensor4 gout = T4(gin.p, gin.stride, gin.off, cout);
   Tensor4 gg = T4(g.p, g.stride, g.off, L.cout);
-  {
-    // the transposed problem's B[tap][n = ci][k = co] = W[8 - tap][ci][co]
-    bool done = mask ? conv_tc<EPI_MASK>(u, B, h, w, gg, L.W, cout, nullptr, gout, *mask, st)
-                     : conv_tc<EPI_STORE>(u, B, h, w, gg, L.W, cout, nullptr, gout, none, st);
-    if (done) return;
-  }
-  if (wide) {
-    if (mask)
-      k_conv3x3<64, EPI_MASK><<<grid, 128, 0, st>>>(B, h, w, gg, L.WT, nullptr, gout, *mask);
-    else
-      k_conv3x3<64, EPI_STORE><<<grid, 128, 0, st>>>(B, h, w, gg, L.WT, nullptr, gout, none);
-  } else {
-    if (mask)
-      k_conv3x3<32, EPI_MASK><<<grid, 128, 0, st>>>(B, h, w, gg, L.WT, nullptr, gout, *mask);
-    else
-      k_conv3x3<32, EPI_STORE><<<grid, 128, 0, st>>>(B, h, w, gg, L.WT, nullptr, gout, none);
-  }
-  count_launch();
+  // the transposed problem's B[tap][n = ci][k = co] = W[8 - tap][ci][co]
+  bool done = mask ? conv_tc<EPI_MASK>(u, B, h, w, gg, L.W, cout, nullptr, gout, *mask, st)
+                   : conv_tc<EPI_STORE>(u, B, h, w, gg, L.W, cout, nullptr, gout, none, st);
+  if (done) return;
+  if (mask)
+    conv_res<EPI_MASK>(B, h, w, gg, L.WT, nullptr, gout, *mask, st);
+  else
+    conv_res<EPI_STORE>(B, h, w, gg, L.WT, nullptr, gout, none, st);
 }
 
 // weight and bias gradients of a layer into u->grad
@@ -799,6 +817,11 @@ dt_status dt_unet_create(int base_channels, unsigned long long seed, dt_unet** o
       dt_unet_destroy(u);
       return st;
     }
+  }
+  if ((st = conv_res_attributes<EPI_BIAS_RELU>()) != DT_OK || (st = conv_res_attributes<EPI_BIAS>()) != DT_OK ||
+      (st = conv_res_attributes<EPI_MASK>()) != DT_OK || (st = conv_res_attributes<EPI_STORE>()) != DT_OK) {
+    dt_unet_destroy(u);
+    return st;
   }
   *out = u;
   return DT_OK;
