@@ -13,8 +13,8 @@
 // mma.sync.m16n8k16.row.col.f32.bf16.bf16.f32.
 //
 // Weight gradient: dW[tap][ci][co] = sum_p in[p + off(tap)][ci] g[p][co], a GEMM with M = input
-// channels, N = output channels, K = pixels; each block reduces a chunk of pixel tiles and writes
-// a partial tile, and a second pass sums the partials in a fixed order (deterministic).
+// channels, N = output channels, K = pixels; each block reduces a chunk of the pixels for all nine
+// taps and writes a partial tile, and a second pass sums the partials in a fixed order (deterministic).
 #pragma once
 #include <cuda_bf16.h>
 
@@ -214,127 +214,102 @@ __global__ void __launch_bounds__(64 * RY * COW) k_conv3x3_res(int nimg, int h, 
     }
 }
 
-// Weight gradient partials: block (tap, ci tile of 64, co tile of BN) x chunk of pixel tiles.
-// part[chunk][tap][ci][co] (FP32).
-template <int BN>
-__global__ void __launch_bounds__(128) k_conv3x3_wgrad(int nimg, int h, int w, Tensor4 in, Tensor4 g, int tiles_per_chunk,
-                                                       float* __restrict__ part) {
-  constexpr int BM = 64;  // input channels per block (GEMM M)
-  constexpr int BK = 32;  // pixels per k step
-  __shared__ __align__(128) bf16 sA[2][BK * BM];  // [pixel][ci] : 32 rows of 64 channels
-  __shared__ __align__(128) bf16 sB[2][BK * BN];  // [pixel][co]
+// Weight gradient partials: a block takes all nine taps of 16 CIG input by 32 COG output channels
+// over a chunk of the pixels, in order, 32 a tile; part[chunk][tap][ci][co] (FP32). A step's 64 pixels of
+// the output gradient and the three rows of 66 they multiply are copied once into shared memory for all
+// taps (WG_STAGES in flight), and a warp keeps TAPS taps (a row of three, or one) of 16 x 32 channels
+// in registers, so an output-gradient fragment serves TAPS products. Pixels are spaced as in
+// k_conv3x3_res. Each sum takes its chunk's pixels 16 at a time in raster order, whatever the tile
+// of channels: spreading a step's rows over warps or finer chunks moves the FP32 sums of 32768
+// pixels by 3e-5 of the gradient.
+// Bound by its chain of 16-pixel products a warp (64 chunks leave one or two blocks an SM) and the
+// ldmatrix loads. A block a tap, each staging the pixels anew, took 705 us for 32 -> 32 channels at
+// 16 x 512 x 256 pixels (its 64-channel tile half empty), now 360; 96 -> 32 1325, now 701; 64 -> 64 at half
+// the size 218, now 172; 384 -> 128 at a quarter 587, now 409.
+constexpr int WG_STAGES = 4;
+__host__ __device__ constexpr int wg_stage(int cig, int cog) { return 3 * 66 * (cig * 32 + 16) + 64 * (cog * 64 + 16); }
+__host__ __device__ constexpr int wg_threads(int cig, int cog, int taps) { return 32 * 9 / taps * cig * cog; }
+template <int CIG, int COG, int TAPS>
+__global__ void __launch_bounds__(wg_threads(CIG, COG, TAPS), 2)
+    k_conv3x3_wgrad(int nimg, int h, int w, Tensor4 in, Tensor4 g, int tiles_per_chunk, float* __restrict__ part) {
+  constexpr int NTH = wg_threads(CIG, COG, TAPS), PA = CIG * 32 + 16, PB = COG * 64 + 16;
+  constexpr int REGION = 3 * 66 * PA, STAGE = wg_stage(CIG, COG), TG = 9 / TAPS;
+  extern __shared__ __align__(128) unsigned char conv_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  const int cin = in.c, cout = g.c;
-  const int ci_tiles = (cin + BM - 1) / BM;
-  int bx = blockIdx.x;
-  const int co0 = (bx % (cout / BN)) * BN;
-  bx /= cout / BN;
-  const int ci0 = (bx % ci_tiles) * BM;
-  const int tap = bx / ci_tiles;
-  const int ky = tap / 3, kx = tap % 3;
-  const int chunk = blockIdx.y;
-  const int tiles_x = w / BK;
-  const int total_tiles = nimg * h * tiles_x;
-  constexpr int NT = BN / 16;
-  float acc[2][NT][4];
+  const int tap0 = warp % TG * TAPS, ky = tap0 / 3, kx0 = tap0 % 3, cig = warp / TG % CIG, cog = warp / (TG * CIG);
+  const int cin = in.c, cout = g.c, co_tiles = cout / (32 * COG);
+  const int co0 = blockIdx.x % co_tiles * (32 * COG), ci0 = blockIdx.x / co_tiles * (16 * CIG);
+  const int tiles_x = w / 64, total = nimg * h * (w / 32);
+  const int t_begin = blockIdx.y * tiles_per_chunk, t_end = min(total, t_begin + tiles_per_chunk);
+  const int s_begin = t_begin / 2, s_end = (t_end + 1) / 2;  // steps of two tiles, the first and last perhaps half
+  float acc[TAPS][4][4];
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+  for (int a = 0; a < TAPS; ++a)
 #pragma unroll
-    for (int b = 0; b < NT; ++b)
+    for (int b = 0; b < 4; ++b)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[a][b][c] = 0.f;
-  const int t_begin = chunk * tiles_per_chunk;
-  const int t_end = min(total_tiles, t_begin + tiles_per_chunk);
-
-  auto load = [&](int t, int stage) {
-    int xt = t % tiles_x;
-    int rest = t / tiles_x;
-    int y = rest % h, n = rest / h;
-    int x0 = xt * BK;
-    int yy = y + ky - 1;
-    bool yok = yy >= 0 && yy < h;
-    // A: 32 pixels x 64 channels (shifted by the tap) = 256 chunks
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      int cidx = tid + q * 128;
-      int row = cidx >> 3, ch = cidx & 7;
-      int xx = x0 + row + kx - 1;
-      xx = xx < 0 ? xx + w : (xx >= w ? xx - w : xx);
-      bool ok = yok && (ci0 + ch * 8 < cin);
-      const bf16* src = in.p + ((size_t)((size_t)n * h + (yok ? yy : 0)) * w + xx) * in.stride + in.off + (ok ? ci0 + ch * 8 : 0);
-      cp_async16(&sA[stage][swz_b<BM>(row, ch)], src, ok);
-    }
-    // B: 32 pixels x BN output-channel gradients
-    constexpr int BCH = BK * BN / 8;
-#pragma unroll
-    for (int q = 0; q < (BCH + 127) / 128; ++q) {
-      int cidx = tid + q * 128;
-      if (cidx < BCH) {
-        int row = cidx / (BN / 8), ch = cidx % (BN / 8);
-        const bf16* src = g.p + ((size_t)((size_t)n * h + y) * w + x0 + row) * g.stride + g.off + co0 + ch * 8;
-        cp_async16(&sB[stage][swz_b<BN>(row, ch)], src, true);
+  auto load = [&](int s) {
+    if (s < s_end) {
+      unsigned char* const sA = conv_smem + (s - s_begin) % WG_STAGES * STAGE;
+      const int x0 = s % tiles_x * 64, line = s / tiles_x, y = line % h;  // line = image * h + y
+      for (int c = tid; c < 3 * 66 * CIG * 2; c += NTH) {
+        const int px = c / (CIG * 2), ch = c % (CIG * 2), r = px / 66, yy = y + r - 1;
+        int xx = x0 + px - r * 66 - 1;
+        xx = xx < 0 ? xx + w : (xx >= w ? xx - w : xx);
+        const bool ok = yy >= 0 && yy < h;
+        cp_async16(sA + px * PA + ch * 16, in.p + ((size_t)(ok ? line + r - 1 : line) * w + xx) * in.stride + in.off + ci0 + ch * 8, ok);
+      }
+      for (int c = tid; c < 64 * COG * 4; c += NTH) {
+        const int px = c / (COG * 4), ch = c % (COG * 4);
+        cp_async16(sA + REGION + px * PB + ch * 16, g.p + ((size_t)line * w + x0 + px) * g.stride + g.off + co0 + ch * 8, true);
       }
     }
     cp_async_commit();
   };
-
-  if (t_begin < t_end) {
-    load(t_begin, 0);
-    for (int t = t_begin; t < t_end; ++t) {
-      int stage = (t - t_begin) & 1;
-      if (t + 1 < t_end) {
-        load(t + 1, stage ^ 1);
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
+#pragma unroll
+  for (int q = 0; q < WG_STAGES - 1; ++q) load(s_begin + q);
+  for (int s = s_begin; s < s_end; ++s) {
+    cp_async_wait<WG_STAGES - 2>();
+    __syncthreads();  // step s is there, and step s - 1's stage is read
+    load(s + WG_STAGES - 1);
+    const unsigned char* const sA = conv_smem + (s - s_begin) % WG_STAGES * STAGE;
+    // A = in^T (rows input channels, columns pixels) from [pixel][ci], so loaded transposed
+    const unsigned char* a = sA + (ky * 66 + kx0 + (lane & 7) + ((lane >> 4) << 3)) * PA + cig * 32 + ((lane >> 3) & 1) * 16;
+    const unsigned char* b = sA + REGION + (lane & 15) * PB + cog * 64 + (lane >> 4) * 16;
+    auto tile = [&](int x) {  // 32 pixels
+#pragma unroll
+      for (int px = 0; px < 32; px += 16) {
+        unsigned bf[4][2], af[TAPS][4];
+        ldmatrix_x4_trans(bf[0][0], bf[0][1], bf[1][0], bf[1][1], b + (x + px) * PB);
+        ldmatrix_x4_trans(bf[2][0], bf[2][1], bf[3][0], bf[3][1], b + (x + px) * PB + 32);
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k)
+          ldmatrix_x4_trans(af[k][0], af[k][1], af[k][2], af[k][3], a + (x + px + k) * PA);
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k)
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) mma_bf16(acc[k][nt], af[k], bf[nt]);
       }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < BK; kk += 16) {
-        // A = in^T: rows ci, cols pixels; the tile is [pixel][ci], so load transposed
-        unsigned af[2][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-          // matrices: (ci 0-7, px 0-7), (ci 8-15, px 0-7), (ci 0-7, px 8-15), (ci 8-15, px 8-15)
-          int prow = kk + (lane & 7) + ((lane >> 4) << 3);
-          int chunk = (wm * 32 + mt * 16) / 8 + ((lane >> 3) & 1);
-          ldmatrix_x4_trans(af[mt][0], af[mt][1], af[mt][2], af[mt][3], &sA[stage][swz_b<BM>(prow, chunk)]);
-        }
-        unsigned bfr[NT][2];
-#pragma unroll
-        for (int nt = 0; nt < NT; nt += 2) {
-          int krow = kk + (lane & 15);
-          int chunk = (wn * (BN / 2) + nt * 8) / 8 + (lane >> 4);
-          unsigned r0, r1, r2, r3;
-          ldmatrix_x4_trans(r0, r1, r2, r3, &sB[stage][swz_b<BN>(krow, chunk)]);
-          bfr[nt][0] = r0;
-          bfr[nt][1] = r1;
-          bfr[nt + 1][0] = r2;
-          bfr[nt + 1][1] = r3;
-        }
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) mma_bf16(acc[mt][nt], af[mt], bfr[nt]);
-      }
-      __syncthreads();
+    };
+    if (2 * s >= t_begin && 2 * s + 1 < t_end) {
+      tile(0);
+      tile(32);
+    } else {
+      tile(2 * s >= t_begin ? 0 : 32);
     }
   }
+  cp_async_wait<0>();
   const int gq = lane >> 2, t4 = lane & 3;
-  float* dst = part + ((size_t)chunk * 9 + tap) * cin * cout;
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+  for (int k = 0; k < TAPS; ++k)
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      int ci = ci0 + wm * 32 + mt * 16 + gq + half * 8;
-      if (ci >= cin) continue;
+      const int ci = ci0 + cig * 16 + gq + half * 8;
+      float* dst = part + (((size_t)blockIdx.y * 9 + tap0 + k) * cin + ci) * cout + co0 + cog * 32 + t4 * 2;
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        int co = co0 + wn * (BN / 2) + nt * 8 + t4 * 2;
-        dst[(size_t)ci * cout + co] = acc[mt][nt][half * 2];
-        dst[(size_t)ci * cout + co + 1] = acc[mt][nt][half * 2 + 1];
-      }
+      for (int nt = 0; nt < 4; ++nt)
+        *reinterpret_cast<float2*>(dst + nt * 8) = make_float2(acc[k][nt][half * 2], acc[k][nt][half * 2 + 1]);
     }
 }
 

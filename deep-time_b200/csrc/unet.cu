@@ -511,6 +511,16 @@ static void conv_res(int B, int h, int w, Tensor4 in, const bf16* W, const float
   }
   count_launch();
 }
+static dt_status wgrad_attributes() {
+  const auto set = [](const void* f, int cig, int cog) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_STAGES * wg_stage(cig, cog));
+  };
+  DT_CUDA(set((const void*)k_conv3x3_wgrad<2, 2, 3>, 2, 2));
+  DT_CUDA(set((const void*)k_conv3x3_wgrad<1, 2, 3>, 1, 2));
+  DT_CUDA(set((const void*)k_conv3x3_wgrad<2, 1, 3>, 2, 1));
+  DT_CUDA(set((const void*)k_conv3x3_wgrad<1, 1, 1>, 1, 1));
+  return DT_OK;
+}
 template <int EPI>
 static dt_status conv_res_attributes() {
   const int big = 227 * 1024;
@@ -559,14 +569,21 @@ static void conv_wgrad(dt_unet* u, const ConvLayer& L, int B, int h, int w, Tens
   int chunks = std::min(64, tiles);
   int per = (tiles + chunks - 1) / chunks;
   chunks = (tiles + per - 1) / per;
-  int ci_tiles = (L.cin + 63) / 64;
-  int bn = L.cout % 64 == 0 ? 64 : 32;
-  dim3 grid(9 * ci_tiles * (L.cout / bn), chunks);
   Tensor4 gi = T4(in.p, in.stride, in.off, L.cin);
-  if (bn == 64)
-    k_conv3x3_wgrad<64><<<grid, 128, 0, st>>>(B, h, w, gi, g, per, u->part);
+  g.c = L.cout;
+  auto go = [&](auto kernel, int cig, int cog, int taps) {
+    const dim3 grid((L.cin / (16 * cig)) * (L.cout / (32 * cog)), chunks);
+    kernel<<<grid, wg_threads(cig, cog, taps), WG_STAGES * wg_stage(cig, cog), st>>>(B, h, w, gi, g, per, u->part);
+  };
+  // blocks of 32 x 64 channels, smaller where 64 chunks of them would leave SMs without one
+  if (L.cout % 64 == 0 && L.cin > 32)
+    go(k_conv3x3_wgrad<2, 2, 3>, 2, 2, 3);
+  else if (L.cout % 64 == 0)
+    go(k_conv3x3_wgrad<1, 2, 3>, 1, 2, 3);
+  else if (L.cin > 32)
+    go(k_conv3x3_wgrad<2, 1, 3>, 2, 1, 3);
   else
-    k_conv3x3_wgrad<32><<<grid, 128, 0, st>>>(B, h, w, gi, g, per, u->part);
+    go(k_conv3x3_wgrad<1, 1, 1>, 1, 1, 1);
   size_t nw = (size_t)9 * L.cin * L.cout;
   k_sum_parts<<<ugrid(u, nw), 256, 0, st>>>(nw, chunks, u->part, u->grad + L.w_off);
   // bias: per-block partials over pixels, then their sum
@@ -819,7 +836,8 @@ dt_status dt_unet_create(int base_channels, unsigned long long seed, dt_unet** o
     }
   }
   if ((st = conv_res_attributes<EPI_BIAS_RELU>()) != DT_OK || (st = conv_res_attributes<EPI_BIAS>()) != DT_OK ||
-      (st = conv_res_attributes<EPI_MASK>()) != DT_OK || (st = conv_res_attributes<EPI_STORE>()) != DT_OK) {
+      (st = conv_res_attributes<EPI_MASK>()) != DT_OK || (st = conv_res_attributes<EPI_STORE>()) != DT_OK ||
+      (st = wgrad_attributes()) != DT_OK) {
     dt_unet_destroy(u);
     return st;
   }
