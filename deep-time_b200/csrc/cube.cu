@@ -48,6 +48,7 @@ constexpr int CUBE_CG_MAX_ITER = 400;  // surface/diffusion.rs:497
 constexpr int CUBE_RED_BLOCKS = 592;   // partial sums per reduction (4 per SM)
 constexpr size_t CUBE_FUSE_CELLS = 1536;  // levels this small run their part of the cycle in one block
 constexpr int CUBE_MAX_FUSED = 24;        // levels one fused launch carries
+constexpr size_t CUBE_COARSE_SMEM = 220 * 1024;  // and the shared memory it may take
 
 // ---- the operator ----
 __global__ void k_cube_couplings(size_t cells, const uint32_t* __restrict__ slots, const double* __restrict__ lap,
@@ -113,11 +114,19 @@ __device__ __forceinline__ double block_sum(double v) {
   return v;  // thread 0 holds the block's sum
 }
 
-__global__ void k_cube_finish(int nparts, const double* __restrict__ partials, double* __restrict__ out) {
+// then(sum) runs on thread 0: the CG scalar that the sum gives, without a launch of its own
+template <class F>
+__device__ __forceinline__ void finish_sum(int nparts, const double* __restrict__ partials, double* __restrict__ out, F then) {
   double v = 0.0;
   for (int q = threadIdx.x; q < nparts; q += blockDim.x) v += partials[q];
   v = block_sum(v);
-  if (threadIdx.x == 0) *out = v;
+  if (threadIdx.x == 0) {
+    *out = v;
+    then(v);
+  }
+}
+__global__ void k_cube_finish(int nparts, const double* __restrict__ partials, double* __restrict__ out) {
+  finish_sum(nparts, partials, out, [](double) {});
 }
 
 // r = rhs - A x; partial r.r
@@ -171,13 +180,16 @@ __global__ void k_cube_direction(size_t cells, const uint32_t* __restrict__ slot
 // x += alpha p; r -= alpha A p; partial r.r (diffusion.rs:448-475)
 __global__ void k_cube_update(size_t cells, const double* __restrict__ alpha_p, const double* __restrict__ broke,
                               const double* __restrict__ p, const double* __restrict__ ap, double* __restrict__ x,
-                              double* __restrict__ r, double* __restrict__ partials, const double* __restrict__ loop) {
+                              double* __restrict__ r, double* __restrict__ po, double* __restrict__ partials,
+                              const double* __restrict__ loop) {
   if (*broke != 0.0) return;  // the loop stops before the update
   if (loop && loop[13] != 0.0) return;
   const double alpha = *alpha_p;
   double acc = 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
-    x[i] = __dadd_rn(x[i], __dmul_rn(alpha, p[i]));
+    const double pi = p[i];
+    if (po) po[i] = pi;  // the next direction's p, where the caller does not swap the two
+    x[i] = __dadd_rn(x[i], __dmul_rn(alpha, pi));
     const double rv = __dsub_rn(r[i], __dmul_rn(alpha, ap[i]));
     r[i] = rv;
     acc += rv * rv;
@@ -439,138 +451,310 @@ __global__ void k_mg_mass(size_t cells, const uint32_t* __restrict__ kid_ptr, co
 __device__ __forceinline__ float mg_az(size_t i, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
                                        const float* __restrict__ val, const float* __restrict__ diag,
                                        const float* __restrict__ z) {
+  const uint32_t end = ptr[i + 1];
   float az = __fmul_rn(diag[i], z[i]);
-  for (uint32_t e = ptr[i]; e < ptr[i + 1]; ++e) az = __fsub_rn(az, __fmul_rn(val[e], z[col[e]]));
+  for (uint32_t e = ptr[i]; e < end; e += 8) {
+    // eight entries' reads in flight (the last repeated past the row's end), then their serial sum
+    float v[8], x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t k = min(e + u, end - 1);
+      v[u] = val[k];
+      x[u] = z[col[k]];
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float next = __fsub_rn(az, __fmul_rn(v[u], x[u]));
+      az = e + u < end ? next : az;
+    }
+  }
   return az;
 }
 
-__global__ void k_mg_sweep_first(size_t cells, const float* __restrict__ r, const float* __restrict__ diag, float* __restrict__ z) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x)
-    z[i] = __fdiv_rn(__fmul_rn(CUBE_OMEGA, r[i]), diag[i]);
+// zf += v over coarse cell q's block, its reads before its writes
+__device__ __forceinline__ void mg_hand_down(size_t q, const uint32_t* __restrict__ kid_ptr, const uint32_t* __restrict__ kids,
+                                             float v, float* zf) {
+  const uint32_t end = kid_ptr[q + 1];
+  for (uint32_t e = kid_ptr[q]; e < end; e += 4) {
+    uint32_t k[4];
+    float f[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      k[u] = kids[min(e + u, end - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) f[u] = zf[k[u]];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (e + u < end) zf[k[u]] = __fadd_rn(f[u], v);
+  }
 }
 
+// The cycle's start on the finest level: the residual in FP32 and the first sweep from z = 0
+__global__ void k_mg_start(size_t cells, const double* __restrict__ r64, const float* __restrict__ diag, float* __restrict__ r,
+                           float* __restrict__ z) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
+    const float v = (float)r64[i];
+    r[i] = v;
+    z[i] = __fdiv_rn(__fmul_rn(CUBE_OMEGA, v), diag[i]);
+  }
+}
+
+__device__ __forceinline__ float mg_swept(size_t i, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
+                                          const float* __restrict__ val, const float* __restrict__ diag,
+                                          const float* __restrict__ r, const float* __restrict__ z) {
+  const float az = mg_az(i, ptr, col, val, diag, z);
+  return __fadd_rn(z[i], __fdiv_rn(__fmul_rn(CUBE_OMEGA, __fsub_rn(r[i], az)), diag[i]));
+}
+
+// A sweep. zf (the level's last): the correction is also added to its cells of the next finer level.
 __global__ void k_mg_sweep(size_t cells, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
                            const float* __restrict__ val, const float* __restrict__ diag, const float* __restrict__ r,
-                           const float* __restrict__ z, float* __restrict__ t) {
+                           const float* __restrict__ z, float* __restrict__ t, const uint32_t* __restrict__ kid_ptr,
+                           const uint32_t* __restrict__ kids, float* __restrict__ zf) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
-    const float az = mg_az(i, ptr, col, val, diag, z);
-    t[i] = __fadd_rn(z[i], __fdiv_rn(__fmul_rn(CUBE_OMEGA, __fsub_rn(r[i], az)), diag[i]));
+    const float v = mg_swept(i, ptr, col, val, diag, r, z);
+    t[i] = v;
+    if (zf) mg_hand_down(i, kid_ptr, kids, v, zf);
   }
 }
 
-__global__ void k_mg_resid(size_t cells, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                           const float* __restrict__ val, const float* __restrict__ diag, const float* __restrict__ r,
-                           const float* __restrict__ z, float* __restrict__ t) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x)
-    t[i] = __fsub_rn(r[i], mg_az(i, ptr, col, val, diag, z));
+// The finest level's last sweep: the cycle's result in FP64 and the partials of r.z (as k_cube_dot's)
+__global__ void k_mg_sweep_out(size_t cells, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
+                               const float* __restrict__ val, const float* __restrict__ diag, const float* __restrict__ r,
+                               const float* __restrict__ z, const double* __restrict__ r64, double* __restrict__ z64,
+                               double* __restrict__ partials) {
+  double acc = 0.0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
+    const double v = (double)mg_swept(i, ptr, col, val, diag, r, z);
+    z64[i] = v;
+    acc += r64[i] * v;
+  }
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) partials[blockIdx.x] = acc;
+}
+// The same from a finished z (a cycle whose finest level ran in one block)
+__global__ void k_mg_out(size_t cells, const float* __restrict__ z, const double* __restrict__ r64, double* __restrict__ z64,
+                         double* __restrict__ partials) {
+  double acc = 0.0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
+    const double v = (double)z[i];
+    z64[i] = v;
+    acc += r64[i] * v;
+  }
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) partials[blockIdx.x] = acc;
 }
 
+// The finer level's residual summed over each coarse cell's block (in the order of its cells), and the
+// coarse level's first sweep from z = 0. A launch of the small levels costs 3-5 us whatever it does, so
+// the cycle's passes are joined where a cell's values allow: residual, restriction and first sweep; the
+// last sweep and the prolongation. At 6 x 256^2 cells a solve's
+// launches went from 385 to 242.
 __global__ void k_mg_restrict(size_t cells, const uint32_t* __restrict__ kid_ptr, const uint32_t* __restrict__ kids,
-                              const float* __restrict__ t, float* __restrict__ rc) {
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < cells; q += (size_t)gridDim.x * blockDim.x) {
+                              const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const float* __restrict__ val,
+                              const float* __restrict__ diag, const float* __restrict__ r, const float* __restrict__ z,
+                              const float* __restrict__ cdiag, float* __restrict__ cr, float* __restrict__ cz) {
+  const size_t step = gridDim.x * (size_t)blockDim.x / 4;
+  for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; (g & ~(size_t)31) / 4 < cells; g += 4 * step) {
+    const size_t q = min(g / 4, cells - 1);  // the last warp's idle lanes repeat the last cell
+    // four lanes a coarse cell, one residual each; lane 0 adds them in order (a block has 1, 2 or 4 cells)
+    const uint32_t e = kid_ptr[q] + (threadIdx.x & 3);
+    float t = 0.f;
+    const unsigned n = kid_ptr[q + 1] - kid_ptr[q];
+    if ((threadIdx.x & 3) < n) {
+      const size_t i = kids[e];
+      t = __fsub_rn(r[i], mg_az(i, ptr, col, val, diag, z));
+    }
     float s = 0.f;
-    for (uint32_t e = kid_ptr[q]; e < kid_ptr[q + 1]; ++e) s = __fadd_rn(s, t[kids[e]]);
-    rc[q] = s;
+    for (unsigned u = 0; u < 4; ++u) {
+      const float w = __shfl_sync(0xffffffffu, t, u, 4);
+      if (u < n) s = __fadd_rn(s, w);
+    }
+    if ((threadIdx.x & 3) == 0 && g / 4 < cells) {
+      cr[q] = s;
+      cz[q] = __fdiv_rn(__fmul_rn(CUBE_OMEGA, s), cdiag[q]);
+    }
   }
 }
 
-__global__ void k_mg_prolong(size_t cells, const uint32_t* __restrict__ parent, const float* __restrict__ zc, float* __restrict__ z) {
-  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < cells; c += (size_t)gridDim.x * blockDim.x)
-    z[c] = __fadd_rn(z[c], zc[parent[c]]);
-}
-
-__global__ void k_to_f32(size_t n, const double* __restrict__ a, float* __restrict__ b) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) b[i] = (float)a[i];
-}
-__global__ void k_to_f64(size_t n, const float* __restrict__ a, double* __restrict__ b) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) b[i] = (double)a[i];
-}
-
-// The coarse levels' part of the V-cycle in one block of 1024 threads: the launches of those
-// levels (sweeps, residual, restriction, the coarsest level's sweeps, prolongation) in the same
-// order and with the same arithmetic per cell, a block barrier where a launch ended. The vectors
-// written here are read through plain pointers (not the read-only path), so that every phase sees
-// the last one's writes.
+// The coarse levels' part of the V-cycle in one block of 1024 threads: the passes of those levels
+// (sweeps, residual, restriction, the coarsest level's sweeps, prolongation) in the same order and
+// with the same arithmetic per cell, a block barrier where a launch ends (the coarsest level, at
+// most 64 cells, in one warp). A chain of some 40 short passes, each bound by the latency of its
+// gathers, so the levels' rows and vectors are brought into shared memory first, by asynchronous
+// copies: the rows entry by entry (a level's e-th entries contiguous, for reads free of bank
+// conflicts). From global memory the 1536-cell level and those below took 56 us a
+// cycle, now 35.
 struct MgLevelDev {
   unsigned cells;
-  const uint32_t *ptr, *col, *kid_ptr, *kids, *parent;
+  const uint32_t *ptr, *col, *kid_ptr, *kids;
   const float *val, *diag;
-  float *r, *z, *t;
+  // places in the block's shared memory, of 32-bit words: val and col [width][cells]; diag, r, z, t, cnt;
+  // kid_ptr [cells + 1] and kids [cells of the finer level], where there is one
+  unsigned o_val, o_col, o_diag, o_r, o_z, o_t, o_cnt, o_kid_ptr, o_kids;
 };
 struct MgCoarse {
-  int count;  // levels carried; the last is the coarsest
+  int count;         // levels carried; the last is the coarsest
+  unsigned cells;    // of all of them
+  unsigned above;    // cells of the next finer level, 0 where there is none
+  const float* r;    // the first level's right-hand side
+  float* z;          // its correction, or (zf not null) added to the next finer level's zf by block
+  float* zf;
   MgLevelDev lv[CUBE_MAX_FUSED];
 };
 
-__device__ __forceinline__ float mg_az_plain(unsigned i, const MgLevelDev& L, const float* z) {
-  float az = __fmul_rn(L.diag[i], z[i]);
-  for (uint32_t e = L.ptr[i]; e < L.ptr[i + 1]; ++e) az = __fsub_rn(az, __fmul_rn(L.val[e], z[L.col[e]]));
-  return az;
+__device__ __forceinline__ void cp_async4(unsigned char* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-__global__ void __launch_bounds__(1024) k_mg_coarse_cycle(MgCoarse m) {
+__global__ void __launch_bounds__(1024) k_mg_coarse_cycle(const __grid_constant__ MgCoarse m) {
+  extern __shared__ __align__(16) unsigned char mg_smem[];
   const unsigned tid = threadIdx.x, nt = blockDim.x;
-  float* z[CUBE_MAX_FUSED];
-  float* t[CUBE_MAX_FUSED];
-  for (int l = 0; l < m.count; ++l) {
-    z[l] = m.lv[l].z;
-    t[l] = m.lv[l].t;
-  }
-  auto sweep = [&](int l, bool first) {
-    const MgLevelDev& L = m.lv[l];
-    if (first) {
-      for (unsigned i = tid; i < L.cells; i += nt) z[l][i] = __fdiv_rn(__fmul_rn(CUBE_OMEGA, L.r[i]), L.diag[i]);
-    } else {
-      for (unsigned i = tid; i < L.cells; i += nt) {
-        const float az = mg_az_plain(i, L, z[l]);
-        t[l][i] = __fadd_rn(z[l][i], __fdiv_rn(__fmul_rn(CUBE_OMEGA, __fsub_rn(L.r[i], az)), L.diag[i]));
-      }
-      float* q = z[l];
-      z[l] = t[l];
-      t[l] = q;
-    }
-    __syncthreads();
-  };
+  const auto F = [&](unsigned o) { return reinterpret_cast<float*>(mg_smem + o); };
+  const auto H = [&](unsigned o) { return reinterpret_cast<uint32_t*>(mg_smem + o); };
   const int last = m.count - 1;
-  for (int l = 0; l < last; ++l) {
-    for (int k = 0; k < CUBE_NU; ++k) sweep(l, k == 0);
+  for (int l = 0; l <= last; ++l) {
     const MgLevelDev& L = m.lv[l];
-    for (unsigned i = tid; i < L.cells; i += nt) t[l][i] = __fsub_rn(L.r[i], mg_az_plain(i, L, z[l]));
+    const unsigned fine = l ? m.lv[l - 1].cells : m.above;
+    if (fine) {
+      for (unsigned i = tid; i <= L.cells; i += nt) cp_async4(mg_smem + L.o_kid_ptr + 4 * i, L.kid_ptr + i);
+      for (unsigned i = tid; i < fine; i += nt) cp_async4(mg_smem + L.o_kids + 4 * i, L.kids + i);
+    }
+  }
+  for (unsigned g0 = tid; g0 < m.cells; g0 += 2 * nt) {  // the levels' cells one after another, two a thread in flight
+    unsigned lev[2], at[2];
+    uint32_t a[2], b[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      unsigned l = 0, i = min(g0 + u * nt, m.cells - 1);  // past the end: the last cell again
+      while (i >= m.lv[l].cells) i -= m.lv[l++].cells;
+      lev[u] = l;
+      at[u] = i;
+      a[u] = m.lv[l].ptr[i];
+      b[u] = m.lv[l].ptr[i + 1];
+      cp_async4(mg_smem + m.lv[l].o_diag + 4 * i, m.lv[l].diag + i);
+      if (l == 0) cp_async4(mg_smem + m.lv[0].o_r + 4 * i, m.r + i);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const MgLevelDev& L = m.lv[lev[u]];
+      H(L.o_cnt)[at[u]] = b[u] - a[u];
+      for (uint32_t e = a[u]; e < b[u]; ++e) {
+        const unsigned o = 4 * ((e - a[u]) * L.cells + at[u]);
+        cp_async4(mg_smem + L.o_val + o, L.val + e);
+        cp_async4(mg_smem + L.o_col + o, L.col + e);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  for (unsigned i = tid; i < m.lv[0].cells; i += nt)
+    F(m.lv[0].o_z)[i] = __fdiv_rn(__fmul_rn(CUBE_OMEGA, F(m.lv[0].o_r)[i]), F(m.lv[0].o_diag)[i]);
+  __syncthreads();
+  const auto az = [&](const MgLevelDev& L, unsigned i, const float* z) {
+    const float* val = F(L.o_val) + i;
+    const uint32_t* col = H(L.o_col) + i;
+    const unsigned cnt = H(L.o_cnt)[i];
+    float a = __fmul_rn(F(L.o_diag)[i], z[i]);
+    for (unsigned e = 0; e < cnt; e += 8) {
+      float v[8], x[8];  // the reads first, then the serial sum
+#pragma unroll
+      for (unsigned u = 0; u < 8; ++u) {
+        const unsigned k = min(e + u, cnt - 1) * L.cells;
+        v[u] = val[k];
+        x[u] = z[col[k]];
+      }
+#pragma unroll
+      for (unsigned u = 0; u < 8; ++u) {
+        const float next = __fsub_rn(a, __fmul_rn(v[u], x[u]));
+        a = e + u < cnt ? next : a;
+      }
+    }
+    return a;
+  };
+  const auto sweep = [&](const MgLevelDev& L, const float* z, float* t, unsigned i) {
+    t[i] = __fadd_rn(z[i], __fdiv_rn(__fmul_rn(CUBE_OMEGA, __fsub_rn(F(L.o_r)[i], az(L, i, z))), F(L.o_diag)[i]));
+  };
+  // the buffer that holds a level's z after `swaps` sweeps of its two
+  const auto buf = [&](const MgLevelDev& L, int swaps) { return F(swaps & 1 ? L.o_t : L.o_z); };
+  for (int l = 0; l < last; ++l) {
+    const MgLevelDev &L = m.lv[l], &C = m.lv[l + 1];
+    for (int k = 0; k < CUBE_NU - 1; ++k) {
+      for (unsigned i = tid; i < L.cells; i += nt) sweep(L, buf(L, k), buf(L, k + 1), i);
+      __syncthreads();
+    }
+    const float* z = buf(L, CUBE_NU - 1);
+    float* t = buf(L, CUBE_NU);
+    for (unsigned i = tid; i < L.cells; i += nt) t[i] = __fsub_rn(F(L.o_r)[i], az(L, i, z));
     __syncthreads();
-    const MgLevelDev& C = m.lv[l + 1];
     for (unsigned q = tid; q < C.cells; q += nt) {
       float sum = 0.f;
-      for (uint32_t e = C.kid_ptr[q]; e < C.kid_ptr[q + 1]; ++e) sum = __fadd_rn(sum, t[l][C.kids[e]]);
-      C.r[q] = sum;
+      const unsigned end = H(C.o_kid_ptr)[q + 1];
+      for (unsigned e = H(C.o_kid_ptr)[q]; e < end; ++e) sum = __fadd_rn(sum, t[H(C.o_kids)[e]]);
+      F(C.o_r)[q] = sum;
+      F(C.o_z)[q] = __fdiv_rn(__fmul_rn(CUBE_OMEGA, sum), F(C.o_diag)[q]);
     }
     __syncthreads();
   }
-  for (int k = 0; k < CUBE_COARSE_SWEEPS; ++k) sweep(last, k == 0);
-  for (int l = last - 1; l >= 0; --l) {
-    const MgLevelDev& L = m.lv[l];
-    const MgLevelDev& C = m.lv[l + 1];
-    for (unsigned c = tid; c < L.cells; c += nt) z[l][c] = __fadd_rn(z[l][c], z[l + 1][C.parent[c]]);
+  {
+    const MgLevelDev& L = m.lv[last];
+    const bool one = L.cells <= 64;
+    if (!one || tid < 32)
+      for (int k = 0; k < CUBE_COARSE_SWEEPS - 1; ++k) {
+        for (unsigned i = tid; i < L.cells; i += one ? 32 : nt) sweep(L, buf(L, k), buf(L, k + 1), i);
+        if (one)
+          __syncwarp();
+        else
+          __syncthreads();
+      }
     __syncthreads();
-    for (int k = 0; k < CUBE_NU; ++k) sweep(l, false);
+  }
+  for (int l = last; l >= 0; --l) {
+    const MgLevelDev& L = m.lv[l];
+    const int from = CUBE_NU - 1, to = l == last ? CUBE_COARSE_SWEEPS - 1 : 2 * CUBE_NU - 1;
+    if (l < last)
+      for (int k = from; k < to; ++k) {
+        for (unsigned i = tid; i < L.cells; i += nt) sweep(L, buf(L, k), buf(L, k + 1), i);
+        __syncthreads();
+      }
+    const float* z = buf(L, to);
+    if (l > 0) {
+      float* f = buf(m.lv[l - 1], from);
+      for (unsigned q = tid; q < L.cells; q += nt) {
+        const unsigned end = H(L.o_kid_ptr)[q + 1];
+        for (unsigned e = H(L.o_kid_ptr)[q]; e < end; ++e) f[H(L.o_kids)[e]] = __fadd_rn(f[H(L.o_kids)[e]], z[q]);
+      }
+      __syncthreads();
+    } else {
+      for (unsigned q = tid; q < L.cells; q += nt) {
+        m.z[q] = z[q];
+        if (m.zf) mg_hand_down(q, H(L.o_kid_ptr), H(L.o_kids), z[q], m.zf);
+      }
+    }
   }
 }
 
-// alpha = rz / pap; beta = rz_new / rz, rz = rz_new (the CG scalars, on the device)
-// alpha = rz / pap, or the breakdown flag (pap not positive, or NaN: diffusion.rs:444-446)
-__global__ void k_cube_alpha(const double* __restrict__ rz, const double* __restrict__ pap, double* __restrict__ alpha,
-                             double* __restrict__ broke, const double* __restrict__ loop) {
-  if (loop && loop[13] != 0.0) return;
-  const double p = *pap;
-  if (isnan(p) || p <= 0.0) {
-    *broke = 1.0;
-  } else {
-    *broke = 0.0;
-    *alpha = *rz / p;
-  }
+// p.Ap's sum, and alpha = rz / pap or the breakdown flag (pap not positive, or NaN: diffusion.rs:444-446)
+__global__ void k_cube_alpha(int nparts, const double* __restrict__ partials, const double* __restrict__ rz,
+                             double* __restrict__ pap, double* __restrict__ alpha, double* __restrict__ broke,
+                             const double* __restrict__ loop) {
+  finish_sum(nparts, partials, pap, [&](double p) {
+    if (loop && loop[13] != 0.0) return;
+    if (isnan(p) || p <= 0.0) {
+      *broke = 1.0;
+    } else {
+      *broke = 0.0;
+      *alpha = *rz / p;
+    }
+  });
 }
-__global__ void k_cube_beta(const double* __restrict__ rz_new, double* __restrict__ rz, double* __restrict__ beta) {
-  *beta = *rz_new / *rz;
-  *rz = *rz_new;
+// The new r.z, and beta = rz_new / rz, rz = rz_new
+__global__ void k_cube_beta(int nparts, const double* __restrict__ partials, double* __restrict__ rz_new,
+                            double* __restrict__ rz, double* __restrict__ beta) {
+  finish_sum(nparts, partials, rz_new, [&](double v) {
+    *beta = v / *rz;
+    *rz = v;
+  });
 }
 
 // The device loop's control: sc[12] iterations, sc[13] the stop flag, sc[14] tol^2 n, sc[15] the
@@ -580,23 +764,23 @@ __global__ void k_cube_beta(const double* __restrict__ rz_new, double* __restric
 __global__ void k_cube_arm(const double* __restrict__ sc, unsigned long long while_h) {
   cudaGraphSetConditional((cudaGraphConditionalHandle)while_h, sc[13] == 0.0 ? 1u : 0u);
 }
-__global__ void k_cube_check(double* __restrict__ sc, unsigned long long while_h, unsigned long long if_h) {
-  bool stop = sc[13] != 0.0;
-  if (!stop) {
-    if (sc[10] != 0.0) {  // p.Ap not positive or NaN: no update (diffusion.rs:444-446)
-      stop = true;
-    } else {
-      sc[0] = sc[11];
-      sc[12] += 1.0;
-      stop = sc[11] <= sc[14] || sc[12] >= sc[15];
+__global__ void k_cube_check(int nparts, const double* __restrict__ partials, double* __restrict__ sc,
+                             unsigned long long while_h, unsigned long long if_h) {
+  finish_sum(nparts, partials, sc + 11, [&](double rr) {  // the update's r.r
+    bool stop = sc[13] != 0.0;
+    if (!stop) {
+      if (sc[10] != 0.0) {  // p.Ap not positive or NaN: no update (diffusion.rs:444-446)
+        stop = true;
+      } else {
+        sc[0] = rr;
+        sc[12] += 1.0;
+        stop = rr <= sc[14] || sc[12] >= sc[15];
+      }
     }
-  }
-  if (stop) sc[13] = 1.0;
-  cudaGraphSetConditional((cudaGraphConditionalHandle)while_h, stop ? 0u : 1u);
-  cudaGraphSetConditional((cudaGraphConditionalHandle)if_h, stop ? 0u : 1u);
-}
-__global__ void k_cube_copy(size_t cells, const double* __restrict__ a, double* __restrict__ b) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) b[i] = a[i];
+    if (stop) sc[13] = 1.0;
+    cudaGraphSetConditional((cudaGraphConditionalHandle)while_h, stop ? 0u : 1u);
+    cudaGraphSetConditional((cudaGraphConditionalHandle)if_h, stop ? 0u : 1u);
+  });
 }
 
 // partials of (rhs - ap) and of s, for the put-back
@@ -624,9 +808,10 @@ namespace {
 // One level of the hierarchy: its sparsity (device), its values and vectors.
 struct CubeLevel {
   size_t cells = 0, nnz = 0, side = 0;
+  size_t width = 0;                                              // entries of the longest row
   uint32_t *ptr = nullptr, *col = nullptr;                      // CSR neighbours
   uint32_t *src_ptr = nullptr, *src = nullptr;                  // level >= 1: the finer entries summed
-  uint32_t *kid_ptr = nullptr, *kids = nullptr, *parent = nullptr;  // level >= 1: blocks
+  uint32_t *kid_ptr = nullptr, *kids = nullptr;              // level >= 1: blocks
   float *val = nullptr, *mass = nullptr, *diag = nullptr, *r = nullptr, *z = nullptr, *t = nullptr;
 };
 
@@ -719,11 +904,7 @@ struct dt_cube {
   double* sc = nullptr;  // scalars: 0 rr, 1 pap, 2 rz, 3 rz_new, 4 alpha, 5 beta, 6 lost, 7 weight, 8 kk, 9 rhs.rhs,
                         // 10 breakdown flag, 11 the update's r.r
   std::vector<CubeLevel> levels;
-  // The V-cycle's launches as CUDA graphs. Every level swaps its sweep buffers an odd number of
-  // times a cycle, so the buffers alternate between two layouts: one graph for each, captured on
-  // first use.
-  cudaGraphExec_t vcycle_exec[2] = {nullptr, nullptr};
-  int vcycle_layout = 0;
+  cudaGraphExec_t vcycle_exec = nullptr;  // the V-cycle's launches, captured on first use
   // the CG loop as a graph (a WHILE node over one iteration, the tail under an IF node), made on
   // the first solve; DT_CUBE_HOST_LOOP=1 at create drives the loop from the host instead (the
   // same kernels, three scalars read back an iteration)
@@ -785,84 +966,114 @@ void cube_prepare(dt_cube* s) {
   }
 }
 
-void cube_sweep(dt_cube* s, CubeLevel& lv, bool first) {
-  if (first) {
-    k_mg_sweep_first<<<cube_grid(lv.cells), 256, 0, s->stream>>>(lv.cells, lv.r, lv.diag, lv.z);
-    return;
-  }
-  k_mg_sweep<<<cube_grid(lv.cells), 256, 0, s->stream>>>(lv.cells, lv.ptr, lv.col, lv.val, lv.diag, lv.r, lv.z, lv.t);
+// One sweep of level l; `down` (the level's last): its correction also to the next finer level
+void cube_sweep(dt_cube* s, size_t l, bool down) {
+  CubeLevel& lv = s->levels[l];
+  k_mg_sweep<<<cube_grid(lv.cells), 256, 0, s->stream>>>(lv.cells, lv.ptr, lv.col, lv.val, lv.diag, lv.r, lv.z, lv.t, lv.kid_ptr,
+                                                         lv.kids, down && l > 0 ? s->levels[l - 1].z : nullptr);
   std::swap(lv.z, lv.t);
 }
 
-// The cycle from level l0 down in one block (k_mg_coarse_cycle). The host's view of each level's
-// z and t then takes the swaps the replaced launches make: NU - 1 + NU on a level with a coarser
-// one below, COARSE_SWEEPS - 1 on the coarsest.
-void cube_coarse_cycle(dt_cube* s, size_t l0) {
-  MgCoarse m{};
-  m.count = (int)(s->levels.size() - l0);
-  for (int i = 0; i < m.count; ++i) {
+// The levels from l0 down laid out in one block's shared memory; its size, or 0 where they do not fit.
+size_t coarse_layout(const dt_cube* s, size_t l0, MgCoarse* m) {
+  size_t at = 0;
+  const auto take = [&](size_t bytes) {
+    const size_t o = at;
+    at += bytes;
+    return (unsigned)o;
+  };
+  m->count = (int)(s->levels.size() - l0);
+  if (m->count > CUBE_MAX_FUSED) return 0;
+  m->cells = 0;
+  m->above = l0 > 0 ? (unsigned)s->levels[l0 - 1].cells : 0;
+  for (int i = 0; i < m->count; ++i) {
     const CubeLevel& lv = s->levels[l0 + i];
-    m.lv[i] = MgLevelDev{(unsigned)lv.cells, lv.ptr, lv.col, lv.kid_ptr, lv.kids, lv.parent, lv.val, lv.diag, lv.r, lv.z, lv.t};
+    const size_t c = lv.cells;
+    if (c > CUBE_COARSE_SMEM) return 0;
+    m->cells += (unsigned)c;
+    MgLevelDev& d = m->lv[i];
+    d = MgLevelDev{(unsigned)c, lv.ptr, lv.col, lv.kid_ptr, lv.kids, lv.val, lv.diag};
+    d.o_val = take(4 * lv.width * c);
+    d.o_col = take(4 * lv.width * c);
+    d.o_diag = take(4 * c);
+    d.o_r = take(4 * c);
+    d.o_z = take(4 * c);
+    d.o_t = take(4 * c);
+    d.o_cnt = take(4 * c);
+    if (l0 + i > 0) {
+      d.o_kid_ptr = take(4 * (c + 1));
+      d.o_kids = take(4 * s->levels[l0 + i - 1].cells);
+    }
   }
-  k_mg_coarse_cycle<<<1, 1024, 0, s->stream>>>(m);
-  for (size_t l = l0; l < s->levels.size(); ++l) {
-    const int swaps = l + 1 == s->levels.size() ? CUBE_COARSE_SWEEPS - 1 : 2 * CUBE_NU - 1;
-    if (swaps & 1) std::swap(s->levels[l].z, s->levels[l].t);
-  }
+  return at <= CUBE_COARSE_SMEM ? at : 0;
 }
 
-// multigrid.rs:312-363
-void cube_vcycle(dt_cube* s, size_t l) {
+// The cycle from level l on in one block?
+bool cube_fused(const dt_cube* s, size_t l) {
+  MgCoarse m;
+  return s->levels[l].cells <= s->fuse_cells && coarse_layout(s, l, &m) > 0;
+}
+
+// The cycle from level l down, lv.r and (but where one block takes it) its first sweep from zero
+// in lv.z given; the result in lv.z and, but on the finest, added to the next finer level's
+// (multigrid.rs:312-363)
+void cube_vcycle(dt_cube* s, size_t l, const double* r, double* z) {
   CubeLevel& lv = s->levels[l];
-  if (lv.cells <= s->fuse_cells && s->levels.size() - l <= (size_t)CUBE_MAX_FUSED) {
-    cube_coarse_cycle(s, l);
-    return;
+  if (cube_fused(s, l)) {
+    MgCoarse m;
+    const size_t smem = coarse_layout(s, l, &m);
+    m.r = lv.r;
+    m.z = lv.z;
+    m.zf = l > 0 ? s->levels[l - 1].z : nullptr;
+    k_mg_coarse_cycle<<<1, 1024, smem, s->stream>>>(m);
+  } else if (l + 1 == s->levels.size()) {
+    for (int k = 1; k < CUBE_COARSE_SWEEPS; ++k) cube_sweep(s, l, k + 1 == CUBE_COARSE_SWEEPS);
+  } else {
+    for (int k = 1; k < CUBE_NU; ++k) cube_sweep(s, l, false);
+    CubeLevel& cl = s->levels[l + 1];
+    k_mg_restrict<<<cube_grid(4 * cl.cells), 256, 0, s->stream>>>(cl.cells, cl.kid_ptr, cl.kids, lv.ptr, lv.col, lv.val, lv.diag,
+                                                              lv.r, lv.z, cl.diag, cl.r, cl.z);
+    cube_vcycle(s, l + 1, nullptr, nullptr);
+    for (int k = 0; k < CUBE_NU - (l == 0); ++k) cube_sweep(s, l, k + 1 == CUBE_NU);
+    if (l == 0) {
+      k_mg_sweep_out<<<CUBE_RED_BLOCKS, 256, 0, s->stream>>>(lv.cells, lv.ptr, lv.col, lv.val, lv.diag, lv.r, lv.z, r, z,
+                                                             s->partials);
+      return;
+    }
   }
-  if (l + 1 == s->levels.size()) {
-    for (int k = 0; k < CUBE_COARSE_SWEEPS; ++k) cube_sweep(s, lv, k == 0);
-    return;
-  }
-  for (int k = 0; k < CUBE_NU; ++k) cube_sweep(s, lv, k == 0);
-  k_mg_resid<<<cube_grid(lv.cells), 256, 0, s->stream>>>(lv.cells, lv.ptr, lv.col, lv.val, lv.diag, lv.r, lv.z, lv.t);
-  CubeLevel& cl = s->levels[l + 1];
-  k_mg_restrict<<<cube_grid(cl.cells), 256, 0, s->stream>>>(cl.cells, cl.kid_ptr, cl.kids, lv.t, cl.r);
-  cube_vcycle(s, l + 1);
-  k_mg_prolong<<<cube_grid(lv.cells), 256, 0, s->stream>>>(lv.cells, cl.parent, cl.z, lv.z);
-  for (int k = 0; k < CUBE_NU; ++k) cube_sweep(s, lv, false);
+  if (l == 0) k_mg_out<<<CUBE_RED_BLOCKS, 256, 0, s->stream>>>(lv.cells, lv.z, r, z, s->partials);
 }
 
-// z = V-cycle(r) (multigrid.rs:271-282)
+// z = V-cycle(r) and the partials of r.z (multigrid.rs:271-282)
 void cube_precondition_launches(dt_cube* s, const double* r, double* z) {
   CubeLevel& l0 = s->levels[0];
-  k_to_f32<<<cube_grid(s->cells), 256, 0, s->stream>>>(s->cells, r, l0.r);
-  cube_vcycle(s, 0);
-  k_to_f64<<<cube_grid(s->cells), 256, 0, s->stream>>>(s->cells, l0.z, z);
+  std::vector<std::pair<float*, float*>> keep;  // the sweeps swap a level's buffers; nothing is kept in them
+  for (const CubeLevel& lv : s->levels) keep.emplace_back(lv.z, lv.t);
+  k_mg_start<<<cube_grid(s->cells), 256, 0, s->stream>>>(s->cells, r, l0.diag, l0.r, l0.z);
+  cube_vcycle(s, 0, r, z);
+  for (size_t l = 0; l < keep.size(); ++l) {
+    s->levels[l].z = keep[l].first;
+    s->levels[l].t = keep[l].second;
+  }
 }
 
-// z = V-cycle(r) for the handle's r and z, through the graph of the current buffer layout
-// (captured the first time; capturing runs the host side of the cycle, which leaves the layout
-// flipped as the graph's run does)
+// z = V-cycle(r) for the handle's r and z, with r.z's partials, through a graph (captured the first time)
 dt_status cube_precondition(dt_cube* s) {
-  const int lay = s->vcycle_layout;
-  if (!s->vcycle_exec[lay]) {
+  if (!s->vcycle_exec) {
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       // a stream that cannot be captured (the legacy default stream): the launches themselves
       cudaGetLastError();
       cube_precondition_launches(s, s->r, s->z);
-      s->vcycle_layout ^= 1;
       return DT_OK;
     }
     cube_precondition_launches(s, s->r, s->z);
     DT_CUDA(cudaStreamEndCapture(s->stream, &g));
-    cudaError_t e = cudaGraphInstantiate(&s->vcycle_exec[lay], g, 0);
+    cudaError_t e = cudaGraphInstantiate(&s->vcycle_exec, g, 0);
     cudaGraphDestroy(g);
     DT_CUDA(e);
-  } else {
-    for (CubeLevel& lv : s->levels) std::swap(lv.z, lv.t);  // the layout the run leaves
   }
-  DT_CUDA(cudaGraphLaunch(s->vcycle_exec[lay], s->stream));
-  s->vcycle_layout ^= 1;
+  DT_CUDA(cudaGraphLaunch(s->vcycle_exec, s->stream));
   return DT_OK;
 }
 
@@ -941,11 +1152,10 @@ dt_status cube_cg_graph(dt_cube* s) {
   }
   k_cube_direction<<<G, 256, 0, s->stream>>>(l, s->slots, s->k, s->diag, s->z, s->po, s->sc + 5, 0, s->pn, s->ap, s->partials,
                                              s->sc);
-  cube_finish(s, s->partials, s->sc + 1);
-  k_cube_alpha<<<1, 1, 0, s->stream>>>(s->sc + 2, s->sc + 1, s->sc + 4, s->sc + 10, s->sc);
-  k_cube_update<<<G, 256, 0, s->stream>>>(l, s->sc + 4, s->sc + 10, s->pn, s->ap, s->x, s->r, s->partials, s->sc);
-  cube_finish(s, s->partials, s->sc + 11);
-  k_cube_check<<<1, 1, 0, s->stream>>>(s->sc, hwv, hifv);
+  k_cube_alpha<<<1, 1024, 0, s->stream>>>(CUBE_RED_BLOCKS, s->partials, s->sc + 2, s->sc + 1, s->sc + 4, s->sc + 10, s->sc);
+  k_cube_update<<<G, 256, 0, s->stream>>>(l, s->sc + 4, s->sc + 10, s->pn, s->ap, s->x, s->r, s->po, s->partials,
+                                          s->sc);
+  k_cube_check<<<1, 1024, 0, s->stream>>>(CUBE_RED_BLOCKS, s->partials, s->sc, hwv, hifv);
   // the IF node after the head, its body captured on the side stream (the launch helpers use
   // s->stream, so it stands in for the side stream meanwhile; the capture's host-side swaps of
   // the levels' sweep buffers are undone after it)
@@ -969,20 +1179,11 @@ dt_status cube_cg_graph(dt_cube* s) {
       err = cudaStreamBeginCaptureToGraph(s->aside, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                           cudaStreamCaptureModeThreadLocal);
     if (err == cudaSuccess) {
-      std::vector<std::pair<float*, float*>> keep;
-      for (const CubeLevel& lv : s->levels) keep.emplace_back(lv.z, lv.t);
       cudaStream_t main = s->stream;
       s->stream = s->aside;
-      k_cube_copy<<<cube_grid(l), 256, 0, s->stream>>>(l, s->pn, s->po);
       cube_precondition_launches(s, s->r, s->z);
-      k_cube_dot<<<G, 256, 0, s->stream>>>(l, s->r, s->z, s->partials);
-      cube_finish(s, s->partials, s->sc + 3);
-      k_cube_beta<<<1, 1, 0, s->stream>>>(s->sc + 3, s->sc + 2, s->sc + 5);
+      k_cube_beta<<<1, 1024, 0, s->stream>>>(CUBE_RED_BLOCKS, s->partials, s->sc + 3, s->sc + 2, s->sc + 5);
       s->stream = main;
-      for (size_t q = 0; q < s->levels.size(); ++q) {
-        s->levels[q].z = keep[q].first;
-        s->levels[q].t = keep[q].second;
-      }
       cudaGraph_t ifbody = nullptr;
       err = cudaStreamEndCapture(s->aside, &ifbody);
     }
@@ -1035,7 +1236,6 @@ dt_status cube_solve(dt_cube* s, double* h, const double* kd, double dt, double 
   int iterations = 0;
   if (!(rr <= tol2)) {
     DT_TRY(cube_precondition(s));
-    k_cube_dot<<<G, 256, 0, s->stream>>>(l, s->r, s->z, s->partials);
     cube_finish(s, s->partials, s->sc + 2);
     // the loop on the device, one read back at its end; on a stream that cannot be captured (the
     // legacy default stream), driven from the host
@@ -1060,10 +1260,9 @@ dt_status cube_solve(dt_cube* s, double* h, const double* kd, double dt, double 
     for (int it = 0; host && it < CUBE_CG_MAX_ITER; ++it) {
       k_cube_direction<<<G, 256, 0, s->stream>>>(l, s->slots, s->k, s->diag, s->z, s->po, s->sc + 5, it == 0, s->pn, s->ap,
                                                  s->partials, nullptr);
-      cube_finish(s, s->partials, s->sc + 1);
       std::swap(s->po, s->pn);
-      k_cube_alpha<<<1, 1, 0, s->stream>>>(s->sc + 2, s->sc + 1, s->sc + 4, s->sc + 10, nullptr);
-      k_cube_update<<<G, 256, 0, s->stream>>>(l, s->sc + 4, s->sc + 10, s->po, s->ap, s->x, s->r, s->partials, nullptr);
+      k_cube_alpha<<<1, 1024, 0, s->stream>>>(CUBE_RED_BLOCKS, s->partials, s->sc + 2, s->sc + 1, s->sc + 4, s->sc + 10, nullptr);
+      k_cube_update<<<G, 256, 0, s->stream>>>(l, s->sc + 4, s->sc + 10, s->po, s->ap, s->x, s->r, nullptr, s->partials, nullptr);
       cube_finish(s, s->partials, s->sc + 11);
       // one read back an iteration: the new r.r and the breakdown flag
       double back[2] = {std::nan(""), 1.0};
@@ -1079,9 +1278,7 @@ dt_status cube_solve(dt_cube* s, double* h, const double* kd, double dt, double 
       ++iterations;
       if (rr <= tol2) break;
       DT_TRY(cube_precondition(s));
-      k_cube_dot<<<G, 256, 0, s->stream>>>(l, s->r, s->z, s->partials);
-      cube_finish(s, s->partials, s->sc + 3);
-      k_cube_beta<<<1, 1, 0, s->stream>>>(s->sc + 3, s->sc + 2, s->sc + 5);
+      k_cube_beta<<<1, 1024, 0, s->stream>>>(CUBE_RED_BLOCKS, s->partials, s->sc + 3, s->sc + 2, s->sc + 5);
     }
   }
   // the residual's sum back to the cells, in proportion to their coupling
@@ -1122,8 +1319,7 @@ extern "C" {
 dt_status dt_cube_destroy(dt_cube* s) {
   if (!s) return DT_OK;
   if (s->stream) cudaStreamSynchronize(s->stream);
-  for (cudaGraphExec_t& e : s->vcycle_exec)
-    if (e) cudaGraphExecDestroy(e);
+  if (s->vcycle_exec) cudaGraphExecDestroy(s->vcycle_exec);
   if (s->cg_exec) cudaGraphExecDestroy(s->cg_exec);
   if (s->aside) cudaStreamDestroy(s->aside);
   for (void* p : s->allocs) cudaFree(p);
@@ -1207,6 +1403,10 @@ dt_status dt_cube_create(int n, const uint32_t* slots, const double* lap, const 
     if ((st = cube_alloc(s, &s->ledge, chunks * 6)) != DT_OK) return fail(st);
     if ((st = cube_alloc(s, &s->lal, chunks * 4)) != DT_OK) return fail(st);
   }
+  if (cudaFuncSetAttribute(k_mg_coarse_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CUBE_COARSE_SMEM) != cudaSuccess) {
+    set_error("dt_cube_create: %s", cudaGetErrorString(cudaGetLastError()));
+    return fail(DT_DEVICE_ERROR);
+  }
   if (const char* e = std::getenv("DT_CUBE_LOD_CHUNKED")) s->lod_chunked = e[0] != '0';
   if ((st = cube_alloc(s, &s->partials, 2 * CUBE_RED_BLOCKS)) != DT_OK) return fail(st);
   if ((st = cube_alloc(s, &s->sc, 16)) != DT_OK) return fail(st);
@@ -1222,10 +1422,10 @@ dt_status dt_cube_create(int n, const uint32_t* slots, const double* lap, const 
     lv.cells = p.cells;
     lv.nnz = p.col.size();
     lv.side = p.side;
+    for (size_t c = 0; c < p.cells; ++c) lv.width = std::max<size_t>(lv.width, p.ptr[c + 1] - p.ptr[c]);
     if ((st = cube_upload(s, &lv.ptr, p.ptr)) != DT_OK || (st = cube_upload(s, &lv.col, p.col)) != DT_OK) return fail(st);
     if (l > 0 && ((st = cube_upload(s, &lv.src_ptr, p.src_ptr)) != DT_OK || (st = cube_upload(s, &lv.src, p.src)) != DT_OK ||
-                  (st = cube_upload(s, &lv.kid_ptr, p.kid_ptr)) != DT_OK || (st = cube_upload(s, &lv.kids, p.kids)) != DT_OK ||
-                  (st = cube_upload(s, &lv.parent, p.parent)) != DT_OK))
+                  (st = cube_upload(s, &lv.kid_ptr, p.kid_ptr)) != DT_OK || (st = cube_upload(s, &lv.kids, p.kids)) != DT_OK))
       return fail(st);
     if ((st = cube_alloc(s, &lv.val, lv.nnz)) != DT_OK) return fail(st);
     for (float** q : {&lv.mass, &lv.diag, &lv.r, &lv.z, &lv.t})
