@@ -416,11 +416,17 @@ __global__ void k_cube_untranspose(int n, const double* __restrict__ t, double* 
 // ---- the V-cycle's levels (multigrid.rs:199-363), FP32 without fused multiply-adds ----
 __global__ void k_mg_val0(size_t cells, const uint32_t* __restrict__ slots, const double* __restrict__ k,
                           const double* __restrict__ mu, const double* __restrict__ diag64, const uint32_t* __restrict__ ptr,
-                          float* __restrict__ val, float* __restrict__ mass, float* __restrict__ diag) {
+                          float* __restrict__ val, float* __restrict__ ell, float* __restrict__ mass, float* __restrict__ diag) {
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < cells; c += (size_t)gridDim.x * blockDim.x) {
     uint32_t at = ptr[c];
+    size_t o = c;
     for (int s = 0; s < 8; ++s)
-      if (slots[c * 8 + s] != CUBE_NO_CELL) val[at++] = (float)k[c * 8 + s];
+      if (slots[c * 8 + s] != CUBE_NO_CELL) {
+        const float v = (float)k[c * 8 + s];
+        val[at++] = v;
+        ell[o] = v;
+        o += cells;
+      }
     mass[c] = (float)mu[c];
     diag[c] = (float)diag64[c];
   }
@@ -437,35 +443,42 @@ __global__ void k_mg_valc(size_t nnz, const uint32_t* __restrict__ src_ptr, cons
 
 __global__ void k_mg_mass(size_t cells, const uint32_t* __restrict__ kid_ptr, const uint32_t* __restrict__ kids,
                           const float* __restrict__ fmass, const uint32_t* __restrict__ ptr, const float* __restrict__ val,
-                          float* __restrict__ mass, float* __restrict__ diag) {
+                          float* __restrict__ ell, float* __restrict__ mass, float* __restrict__ diag) {
   for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < cells; r += (size_t)gridDim.x * blockDim.x) {
     float s = 0.f;
     for (uint32_t q = kid_ptr[r]; q < kid_ptr[r + 1]; ++q) s = __fadd_rn(s, fmass[kids[q]]);
     float kk = 0.f;
-    for (uint32_t e = ptr[r]; e < ptr[r + 1]; ++e) kk = __fadd_rn(kk, val[e]);
+    size_t o = r;
+    for (uint32_t e = ptr[r]; e < ptr[r + 1]; ++e, o += cells) {
+      kk = __fadd_rn(kk, val[e]);
+      ell[o] = val[e];
+    }
     mass[r] = s;
     diag[r] = __fadd_rn(s, kk);
   }
 }
 
-__device__ __forceinline__ float mg_az(size_t i, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                                       const float* __restrict__ val, const float* __restrict__ diag,
-                                       const float* __restrict__ z) {
-  const uint32_t end = ptr[i + 1];
+// The level's row i on z. The rows are stored entry by entry (col and val [width][cells]: a warp's
+// reads of its rows' e-th entries are contiguous; row after row a sweep of 6 x 256^2 cells took 13.1 us,
+// now 10.6).
+__device__ __forceinline__ float mg_az(size_t i, size_t cells, const uint32_t* __restrict__ ptr,
+                                       const uint32_t* __restrict__ col, const float* __restrict__ val,
+                                       const float* __restrict__ diag, const float* __restrict__ z) {
+  const uint32_t cnt = ptr[i + 1] - ptr[i];
   float az = __fmul_rn(diag[i], z[i]);
-  for (uint32_t e = ptr[i]; e < end; e += 8) {
+  for (uint32_t e = 0; e < cnt; e += 8) {
     // eight entries' reads in flight (the last repeated past the row's end), then their serial sum
     float v[8], x[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const uint32_t k = min(e + u, end - 1);
+      const size_t k = min(e + u, cnt - 1) * cells + i;
       v[u] = val[k];
       x[u] = z[col[k]];
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const float next = __fsub_rn(az, __fmul_rn(v[u], x[u]));
-      az = e + u < end ? next : az;
+      az = e + u < cnt ? next : az;
     }
   }
   return az;
@@ -499,10 +512,10 @@ __global__ void k_mg_start(size_t cells, const double* __restrict__ r64, const f
   }
 }
 
-__device__ __forceinline__ float mg_swept(size_t i, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
+__device__ __forceinline__ float mg_swept(size_t i, size_t cells, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
                                           const float* __restrict__ val, const float* __restrict__ diag,
                                           const float* __restrict__ r, const float* __restrict__ z) {
-  const float az = mg_az(i, ptr, col, val, diag, z);
+  const float az = mg_az(i, cells, ptr, col, val, diag, z);
   return __fadd_rn(z[i], __fdiv_rn(__fmul_rn(CUBE_OMEGA, __fsub_rn(r[i], az)), diag[i]));
 }
 
@@ -512,7 +525,7 @@ __global__ void k_mg_sweep(size_t cells, const uint32_t* __restrict__ ptr, const
                            const float* __restrict__ z, float* __restrict__ t, const uint32_t* __restrict__ kid_ptr,
                            const uint32_t* __restrict__ kids, float* __restrict__ zf) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
-    const float v = mg_swept(i, ptr, col, val, diag, r, z);
+    const float v = mg_swept(i, cells, ptr, col, val, diag, r, z);
     t[i] = v;
     if (zf) mg_hand_down(i, kid_ptr, kids, v, zf);
   }
@@ -525,7 +538,7 @@ __global__ void k_mg_sweep_out(size_t cells, const uint32_t* __restrict__ ptr, c
                                double* __restrict__ partials) {
   double acc = 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
-    const double v = (double)mg_swept(i, ptr, col, val, diag, r, z);
+    const double v = (double)mg_swept(i, cells, ptr, col, val, diag, r, z);
     z64[i] = v;
     acc += r64[i] * v;
   }
@@ -550,7 +563,7 @@ __global__ void k_mg_out(size_t cells, const float* __restrict__ z, const double
 // the cycle's passes are joined where a cell's values allow: residual, restriction and first sweep; the
 // last sweep and the prolongation. At 6 x 256^2 cells a solve's
 // launches went from 385 to 242.
-__global__ void k_mg_restrict(size_t cells, const uint32_t* __restrict__ kid_ptr, const uint32_t* __restrict__ kids,
+__global__ void k_mg_restrict(size_t cells, size_t fine, const uint32_t* __restrict__ kid_ptr, const uint32_t* __restrict__ kids,
                               const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const float* __restrict__ val,
                               const float* __restrict__ diag, const float* __restrict__ r, const float* __restrict__ z,
                               const float* __restrict__ cdiag, float* __restrict__ cr, float* __restrict__ cz) {
@@ -563,7 +576,7 @@ __global__ void k_mg_restrict(size_t cells, const uint32_t* __restrict__ kid_ptr
     const unsigned n = kid_ptr[q + 1] - kid_ptr[q];
     if ((threadIdx.x & 3) < n) {
       const size_t i = kids[e];
-      t = __fsub_rn(r[i], mg_az(i, ptr, col, val, diag, z));
+      t = __fsub_rn(r[i], mg_az(i, fine, ptr, col, val, diag, z));
     }
     float s = 0.f;
     for (unsigned u = 0; u < 4; ++u) {
@@ -582,20 +595,18 @@ __global__ void k_mg_restrict(size_t cells, const uint32_t* __restrict__ kid_ptr
 // with the same arithmetic per cell, a block barrier where a launch ends (the coarsest level, at
 // most 64 cells, in one warp). A chain of some 40 short passes, each bound by the latency of its
 // gathers, so the levels' rows and vectors are brought into shared memory first, by asynchronous
-// copies: the rows entry by entry (a level's e-th entries contiguous, for reads free of bank
-// conflicts). From global memory the 1536-cell level and those below took 56 us a
-// cycle, now 35.
+// copies (rows stored entry by entry read free of bank conflicts). From global memory the 1536-cell level and those below took 56 us a
+// cycle, now 29.
 struct MgLevelDev {
-  unsigned cells;
+  unsigned cells, entries;  // entries = width cells
   const uint32_t *ptr, *col, *kid_ptr, *kids;
   const float *val, *diag;
-  // places in the block's shared memory, of 32-bit words: val and col [width][cells]; diag, r, z, t, cnt;
-  // kid_ptr [cells + 1] and kids [cells of the finer level], where there is one
-  unsigned o_val, o_col, o_diag, o_r, o_z, o_t, o_cnt, o_kid_ptr, o_kids;
+  // places in the block's shared memory, of 32-bit words: val and col [width][cells]; diag, r, z, t; ptr
+  // and kid_ptr [cells + 1] and kids [cells of the finer level], where there is one
+  unsigned o_val, o_col, o_diag, o_r, o_z, o_t, o_ptr, o_kid_ptr, o_kids;
 };
 struct MgCoarse {
   int count;         // levels carried; the last is the coarsest
-  unsigned cells;    // of all of them
   unsigned above;    // cells of the next finer level, 0 where there is none
   const float* r;    // the first level's right-hand side
   float* z;          // its correction, or (zf not null) added to the next finer level's zf by block
@@ -613,37 +624,20 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_cycle(const __grid_constant_
   const auto F = [&](unsigned o) { return reinterpret_cast<float*>(mg_smem + o); };
   const auto H = [&](unsigned o) { return reinterpret_cast<uint32_t*>(mg_smem + o); };
   const int last = m.count - 1;
+  const auto copy = [&](unsigned o, const void* src, unsigned n) {
+    for (unsigned i = tid; i < n; i += nt) cp_async4(mg_smem + o + 4 * i, reinterpret_cast<const uint32_t*>(src) + i);
+  };
   for (int l = 0; l <= last; ++l) {
     const MgLevelDev& L = m.lv[l];
     const unsigned fine = l ? m.lv[l - 1].cells : m.above;
+    copy(L.o_val, L.val, L.entries);
+    copy(L.o_col, L.col, L.entries);
+    copy(L.o_diag, L.diag, L.cells);
+    copy(L.o_ptr, L.ptr, L.cells + 1);
+    if (l == 0) copy(L.o_r, m.r, L.cells);
     if (fine) {
-      for (unsigned i = tid; i <= L.cells; i += nt) cp_async4(mg_smem + L.o_kid_ptr + 4 * i, L.kid_ptr + i);
-      for (unsigned i = tid; i < fine; i += nt) cp_async4(mg_smem + L.o_kids + 4 * i, L.kids + i);
-    }
-  }
-  for (unsigned g0 = tid; g0 < m.cells; g0 += 2 * nt) {  // the levels' cells one after another, two a thread in flight
-    unsigned lev[2], at[2];
-    uint32_t a[2], b[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      unsigned l = 0, i = min(g0 + u * nt, m.cells - 1);  // past the end: the last cell again
-      while (i >= m.lv[l].cells) i -= m.lv[l++].cells;
-      lev[u] = l;
-      at[u] = i;
-      a[u] = m.lv[l].ptr[i];
-      b[u] = m.lv[l].ptr[i + 1];
-      cp_async4(mg_smem + m.lv[l].o_diag + 4 * i, m.lv[l].diag + i);
-      if (l == 0) cp_async4(mg_smem + m.lv[0].o_r + 4 * i, m.r + i);
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const MgLevelDev& L = m.lv[lev[u]];
-      H(L.o_cnt)[at[u]] = b[u] - a[u];
-      for (uint32_t e = a[u]; e < b[u]; ++e) {
-        const unsigned o = 4 * ((e - a[u]) * L.cells + at[u]);
-        cp_async4(mg_smem + L.o_val + o, L.val + e);
-        cp_async4(mg_smem + L.o_col + o, L.col + e);
-      }
+      copy(L.o_kid_ptr, L.kid_ptr, L.cells + 1);
+      copy(L.o_kids, L.kids, fine);
     }
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -654,7 +648,7 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_cycle(const __grid_constant_
   const auto az = [&](const MgLevelDev& L, unsigned i, const float* z) {
     const float* val = F(L.o_val) + i;
     const uint32_t* col = H(L.o_col) + i;
-    const unsigned cnt = H(L.o_cnt)[i];
+    const unsigned cnt = H(L.o_ptr)[i + 1] - H(L.o_ptr)[i];
     float a = __fmul_rn(F(L.o_diag)[i], z[i]);
     for (unsigned e = 0; e < cnt; e += 8) {
       float v[8], x[8];  // the reads first, then the serial sum
@@ -809,9 +803,10 @@ namespace {
 struct CubeLevel {
   size_t cells = 0, nnz = 0, side = 0;
   size_t width = 0;                                              // entries of the longest row
-  uint32_t *ptr = nullptr, *col = nullptr;                      // CSR neighbours
+  uint32_t *ptr = nullptr, *col = nullptr;                      // rows, neighbours by entry
   uint32_t *src_ptr = nullptr, *src = nullptr;                  // level >= 1: the finer entries summed
   uint32_t *kid_ptr = nullptr, *kids = nullptr;              // level >= 1: blocks
+  float* ell = nullptr;  // val by entry, [width][cells], as col; val itself is by row (CSR, ptr)
   float *val = nullptr, *mass = nullptr, *diag = nullptr, *r = nullptr, *z = nullptr, *t = nullptr;
 };
 
@@ -957,19 +952,20 @@ void cube_build(dt_cube* s, const double* kd, double dt) {
 // the hierarchy's values for the built operator (multigrid.rs:199-269)
 void cube_prepare(dt_cube* s) {
   CubeLevel& l0 = s->levels[0];
-  k_mg_val0<<<cube_grid(s->cells), 256, 0, s->stream>>>(s->cells, s->slots, s->k, s->mu, s->diag, l0.ptr, l0.val, l0.mass,
+  k_mg_val0<<<cube_grid(s->cells), 256, 0, s->stream>>>(s->cells, s->slots, s->k, s->mu, s->diag, l0.ptr, l0.val, l0.ell, l0.mass,
                                                         l0.diag);
   for (size_t l = 1; l < s->levels.size(); ++l) {
     CubeLevel &f = s->levels[l - 1], &c = s->levels[l];
     k_mg_valc<<<cube_grid(c.nnz), 256, 0, s->stream>>>(c.nnz, c.src_ptr, c.src, f.val, c.val);
-    k_mg_mass<<<cube_grid(c.cells), 256, 0, s->stream>>>(c.cells, c.kid_ptr, c.kids, f.mass, c.ptr, c.val, c.mass, c.diag);
+    k_mg_mass<<<cube_grid(c.cells), 256, 0, s->stream>>>(c.cells, c.kid_ptr, c.kids, f.mass, c.ptr, c.val, c.ell, c.mass,
+                                                            c.diag);
   }
 }
 
 // One sweep of level l; `down` (the level's last): its correction also to the next finer level
 void cube_sweep(dt_cube* s, size_t l, bool down) {
   CubeLevel& lv = s->levels[l];
-  k_mg_sweep<<<cube_grid(lv.cells), 256, 0, s->stream>>>(lv.cells, lv.ptr, lv.col, lv.val, lv.diag, lv.r, lv.z, lv.t, lv.kid_ptr,
+  k_mg_sweep<<<cube_grid(lv.cells), 256, 0, s->stream>>>(lv.cells, lv.ptr, lv.col, lv.ell, lv.diag, lv.r, lv.z, lv.t, lv.kid_ptr,
                                                          lv.kids, down && l > 0 ? s->levels[l - 1].z : nullptr);
   std::swap(lv.z, lv.t);
 }
@@ -984,22 +980,20 @@ size_t coarse_layout(const dt_cube* s, size_t l0, MgCoarse* m) {
   };
   m->count = (int)(s->levels.size() - l0);
   if (m->count > CUBE_MAX_FUSED) return 0;
-  m->cells = 0;
   m->above = l0 > 0 ? (unsigned)s->levels[l0 - 1].cells : 0;
   for (int i = 0; i < m->count; ++i) {
     const CubeLevel& lv = s->levels[l0 + i];
     const size_t c = lv.cells;
     if (c > CUBE_COARSE_SMEM) return 0;
-    m->cells += (unsigned)c;
     MgLevelDev& d = m->lv[i];
-    d = MgLevelDev{(unsigned)c, lv.ptr, lv.col, lv.kid_ptr, lv.kids, lv.val, lv.diag};
+    d = MgLevelDev{(unsigned)c, (unsigned)(lv.width * c), lv.ptr, lv.col, lv.kid_ptr, lv.kids, lv.ell, lv.diag};
     d.o_val = take(4 * lv.width * c);
     d.o_col = take(4 * lv.width * c);
     d.o_diag = take(4 * c);
     d.o_r = take(4 * c);
     d.o_z = take(4 * c);
     d.o_t = take(4 * c);
-    d.o_cnt = take(4 * c);
+    d.o_ptr = take(4 * (c + 1));
     if (l0 + i > 0) {
       d.o_kid_ptr = take(4 * (c + 1));
       d.o_kids = take(4 * s->levels[l0 + i - 1].cells);
@@ -1031,12 +1025,12 @@ void cube_vcycle(dt_cube* s, size_t l, const double* r, double* z) {
   } else {
     for (int k = 1; k < CUBE_NU; ++k) cube_sweep(s, l, false);
     CubeLevel& cl = s->levels[l + 1];
-    k_mg_restrict<<<cube_grid(4 * cl.cells), 256, 0, s->stream>>>(cl.cells, cl.kid_ptr, cl.kids, lv.ptr, lv.col, lv.val, lv.diag,
+    k_mg_restrict<<<cube_grid(4 * cl.cells), 256, 0, s->stream>>>(cl.cells, lv.cells, cl.kid_ptr, cl.kids, lv.ptr, lv.col, lv.ell, lv.diag,
                                                               lv.r, lv.z, cl.diag, cl.r, cl.z);
     cube_vcycle(s, l + 1, nullptr, nullptr);
     for (int k = 0; k < CUBE_NU - (l == 0); ++k) cube_sweep(s, l, k + 1 == CUBE_NU);
     if (l == 0) {
-      k_mg_sweep_out<<<CUBE_RED_BLOCKS, 256, 0, s->stream>>>(lv.cells, lv.ptr, lv.col, lv.val, lv.diag, lv.r, lv.z, r, z,
+      k_mg_sweep_out<<<CUBE_RED_BLOCKS, 256, 0, s->stream>>>(lv.cells, lv.ptr, lv.col, lv.ell, lv.diag, lv.r, lv.z, r, z,
                                                              s->partials);
       return;
     }
@@ -1423,11 +1417,14 @@ dt_status dt_cube_create(int n, const uint32_t* slots, const double* lap, const 
     lv.nnz = p.col.size();
     lv.side = p.side;
     for (size_t c = 0; c < p.cells; ++c) lv.width = std::max<size_t>(lv.width, p.ptr[c + 1] - p.ptr[c]);
-    if ((st = cube_upload(s, &lv.ptr, p.ptr)) != DT_OK || (st = cube_upload(s, &lv.col, p.col)) != DT_OK) return fail(st);
+    std::vector<uint32_t> col(lv.width * p.cells, 0);
+    for (size_t c = 0; c < p.cells; ++c)
+      for (uint32_t e = p.ptr[c]; e < p.ptr[c + 1]; ++e) col[(e - p.ptr[c]) * p.cells + c] = p.col[e];
+    if ((st = cube_upload(s, &lv.ptr, p.ptr)) != DT_OK || (st = cube_upload(s, &lv.col, col)) != DT_OK) return fail(st);
     if (l > 0 && ((st = cube_upload(s, &lv.src_ptr, p.src_ptr)) != DT_OK || (st = cube_upload(s, &lv.src, p.src)) != DT_OK ||
                   (st = cube_upload(s, &lv.kid_ptr, p.kid_ptr)) != DT_OK || (st = cube_upload(s, &lv.kids, p.kids)) != DT_OK))
       return fail(st);
-    if ((st = cube_alloc(s, &lv.val, lv.nnz)) != DT_OK) return fail(st);
+    if ((st = cube_alloc(s, &lv.val, lv.nnz)) != DT_OK || (st = cube_alloc(s, &lv.ell, lv.width * lv.cells)) != DT_OK) return fail(st);
     for (float** q : {&lv.mass, &lv.diag, &lv.r, &lv.z, &lv.t})
       if ((st = cube_alloc(s, q, lv.cells)) != DT_OK) return fail(st);
   }
