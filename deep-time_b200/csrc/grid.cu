@@ -13,9 +13,9 @@
 // Every result is bit-for-bit the reference's: the same operations in the same order, and the
 // products and sums that the compiler could fuse into one multiply-add written with the
 // round-to-nearest intrinsics, which it never fuses. The box blur keeps the reference's running
-// sums, so one thread walks each row and each column (k_blur_lines: a block takes 32 lines and
-// streams them through a ring of 32 x 32 shared-memory tiles filled by cp.async, so that both
-// directions read, and write, whole 256-byte row segments; the differences, the running sums
+// sums, so one thread walks each row and each column (k_blur_lines: a block takes 8 to 32 lines and
+// streams them through a ring of 32-position shared-memory tiles filled by cp.async, so that both
+// directions read, and write, row segments of 64 to 256 bytes; the differences, the running sums
 // and the stores run on separate warps). The element-wise helpers run on 2-D
 // grids (a block's threads on consecutive columns, rows strided over the grid's y) with 32-bit
 // index arithmetic; all of them are HBM-bound.
@@ -193,8 +193,8 @@ __global__ void k_blur_cols(int w, int h, int r, double norm, const double* __re
   }
 }
 
-// The box blur's running sums with the lines streamed through shared memory. A block takes 32
-// lines (rows with ROWS, else columns); line line0 + l is lane l's: out(k) = acc (1 / (2r + 1)),
+// The box blur's running sums with the lines streamed through shared memory. A block takes LINES
+// (8, 16 or 32) lines (rows with ROWS, else columns); line line0 + l is lane l's (and l + LINES's, ...): out(k) = acc (1 / (2r + 1)),
 // acc += v(k + r + 1) - v(k - r), with acc started as the sum of v(-r .. r) in order, the
 // reference's loop bit for bit. Only the running sum is serial, so six warps split the work, one
 // tile of 32 positions a step, skewed by a step and separated by one block barrier a step:
@@ -202,25 +202,25 @@ __global__ void k_blur_cols(int w, int h, int r, double norm, const double* __re
 //           copies of one 256-byte row segment per line (ROWS) or per position (columns), into a
 //           ring of RING positions per line;
 //   warps 2-5  the differences d(k) = v(k + r + 1) - v(k - r) of step s's tile (8 positions
-//           each) from the ring, or from global memory past the line's ends (wrap, clamp or
+//           each, shared by the lanes of a line) from the ring, or from global memory past the line's ends (wrap, clamp or
 //           reflection); and the stores of step s - 2's sums times 1 / (2r + 1), whole row
 //           segments in both directions;
 //   warp 0  the running sum over step s - 1's differences.
 // The ring is line-major with ROWS (a line's RING positions contiguous, pitch RING + 1) and
-// position-major for columns (pitch 33), both free of bank conflicts for the accesses they get,
+// position-major for columns (pitch LINES + 1), both free of bank conflicts for the accesses they get,
 // and a position's place in it is k & (RING - 1). B = ceil((r + 1) / 32) (1 or 2, so r <= 63):
-// the ring holds tiles s - B .. s + B while step s's differences are taken. The row pass has one
-// block per 32 rows, fewer than the SMs on the rasters it is meant for, so its ring is deep (512
-// positions, one block an SM); the column pass has twice the blocks and keeps two an SM (256).
-constexpr int BL_PITCH = 33;
-constexpr int BL_TILE = 32 * BL_PITCH;
+// the ring holds tiles s - B .. s + B while step s's differences are taken. A step is a
+// round of shared-memory accesses and the 32 dependent sums (9 cycles each) of one warp; fewer lines a
+// block make the round shorter (a double a lane is two wavefronts for 32 lines) and put more SMs to
+// work. The row pass's ring is deep (512 positions).
+constexpr int BL_PITCH = 33;  // a line's 32 differences or sums
 constexpr int BL_THREADS = 192;
 constexpr int BL_RING_ROWS = 512;
 constexpr int BL_RING_COLS = 256;
 
-template <bool ROWS>
+template <bool ROWS, int LINES>
 constexpr size_t blur_lines_smem() {
-  return sizeof(double) * ((ROWS ? 32 * (BL_RING_ROWS + 1) : BL_RING_COLS * BL_PITCH) + 4 * BL_TILE);
+  return sizeof(double) * ((ROWS ? LINES * (BL_RING_ROWS + 1) : BL_RING_COLS * (LINES + 1)) + 4 * LINES * BL_PITCH);
 }
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
@@ -233,26 +233,29 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-template <bool ROWS, int B>
+template <bool ROWS, int B, int LINES>
 __global__ void __launch_bounds__(BL_THREADS) k_blur_lines(int w, int h, int r, bool wrap, double norm,
                                                            const double* __restrict__ v, double* __restrict__ out) {
+  constexpr int PARTS = 32 / LINES, PER = 8 / PARTS;  // parts of a warp's positions, positions a lane
+  constexpr int BL_TILE = LINES * BL_PITCH;
   constexpr int RING = ROWS ? BL_RING_ROWS : BL_RING_COLS;
   constexpr int MASK = RING - 1;
-  constexpr int RP = ROWS ? RING + 1 : BL_PITCH;  // ring pitch: per line (ROWS) or per position
+  constexpr int RP = ROWS ? RING + 1 : LINES + 1;  // ring pitch: per line (ROWS) or per position
   constexpr int AHEAD = RING / 32 - B - 1;        // tiles in flight beyond the one differenced
   constexpr int PENDING = AHEAD - B - 1;          // copy groups left pending once tiles <= s + B + 1 landed
   static_assert(PENDING >= 0, "the ring must hold the window's tiles and one step ahead");
   extern __shared__ double bl_smem[];
   double* const ring = bl_smem;
-  double* const dif = bl_smem + (ROWS ? 32 * RP : RING * RP);  // two tiles of differences
+  double* const dif = bl_smem + (ROWS ? LINES * RP : RING * RP);  // two tiles of differences
   double* const sum = dif + 2 * BL_TILE;                       // two tiles of running sums
   const int lines = ROWS ? h : w, len = ROWS ? w : h;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int line0 = blockIdx.x * 32, line = line0 + lane;
-  const bool mine = line < lines, full_block = line0 + 32 <= lines;
+  const int ln = lane % LINES, sub = lane / LINES;  // a lane's line, and which part of a warp's positions
+  const int line0 = blockIdx.x * LINES, line = line0 + ln;
+  const bool mine = line < lines, full_block = line0 + LINES <= lines;
   const int tiles = (len + 31) >> 5;
   // this lane's line in the ring: position k at mine_ring[(k & MASK) * step]
-  const double* const my_ring = ROWS ? ring + lane * RP : ring + lane;
+  const double* const my_ring = ROWS ? ring + ln * RP : ring + ln;
   constexpr int KSTEP = ROWS ? 1 : RP;
 
   auto issue = [&](int t) {
@@ -263,21 +266,21 @@ __global__ void __launch_bounds__(BL_THREADS) k_blur_lines(int w, int h, int r, 
           const double* src = v + (size_t)line0 * len + k0 + lane;
           double* dst = ring + ((k0 + lane) & MASK);
 #pragma unroll 8
-          for (int rr = 0; rr < 32; ++rr, src += len, dst += RP) cp_async8(dst, src);
+          for (int rr = 0; rr < LINES; ++rr, src += len, dst += RP) cp_async8(dst, src);
         } else {
-          const double* src = v + (size_t)k0 * w + line;
-          double* dst = ring + (k0 & MASK) * RP + lane;
+          const double* src = v + (size_t)(k0 + sub) * w + line;
+          double* dst = ring + ((k0 & MASK) + sub) * RP + ln;
 #pragma unroll 8
-          for (int rr = 0; rr < 32; ++rr, src += w, dst += RP) cp_async8(dst, src);
+          for (int rr = 0; rr < LINES; ++rr, src += PARTS * (size_t)w, dst += PARTS * RP) cp_async8(dst, src);
         }
       } else {
-        for (int rr = 0; rr < 32; ++rr) {
+        for (int rr = 0; rr < LINES; ++rr) {
           if (ROWS) {
-            const int ln = line0 + rr, pos = k0 + lane;
-            if (ln < lines && pos < len) cp_async8(ring + rr * RP + (pos & MASK), v + (size_t)ln * len + pos);
+            const int pos = k0 + lane;
+            if (line0 + rr < lines && pos < len) cp_async8(ring + rr * RP + (pos & MASK), v + (size_t)(line0 + rr) * len + pos);
           } else {
-            const int pos = k0 + rr;
-            if (mine && pos < len) cp_async8(ring + (pos & MASK) * RP + lane, v + (size_t)pos * w + line);
+            const int pos = k0 + PARTS * rr + sub;
+            if (mine && pos < len) cp_async8(ring + (pos & MASK) * RP + ln, v + (size_t)pos * w + line);
           }
         }
       }
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(BL_THREADS) k_blur_lines(int w, int h, int r, 
   }
   __syncthreads();
   double acc = 0.0;
-  if (warp == 0 && mine)
+  if (warp == 0 && sub == 0 && mine)
     for (int k = -r; k <= r; ++k) acc = __dadd_rn(acc, at(k));
   for (int s = 0; s < tiles + 2; ++s) {
     if (warp == 1) {
@@ -318,24 +321,24 @@ __global__ void __launch_bounds__(BL_THREADS) k_blur_lines(int w, int h, int r, 
       issue(s + AHEAD);
       cp_async_wait<PENDING>();  // tiles <= s + B + 1 landed, for the next step's differences
     } else if (warp >= 2) {
-      const int part = (warp - 2) * 8;
+      const int part = (warp - 2) * 8 + sub * PER;
       if (s < tiles && mine) {
         const int k0 = 32 * s;
-        double* d = dif + (s & 1) * BL_TILE + lane * BL_PITCH + part;
+        double* d = dif + (s & 1) * BL_TILE + ln * BL_PITCH + part;
         const int kh = k0 + part + r + 1, kl = k0 + part - r;
         if (k0 + 32 <= len && k0 - r >= 0 && k0 + 32 + r < len) {
           // every read before the first store: the tiles share one shared-memory array, so the
           // compiler would not move a read above a store
-          double hi[8], lo[8];
+          double hi[PER], lo[PER];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
+          for (int u = 0; u < PER; ++u) {
             hi[u] = ring_at(kh + u);
             lo[u] = ring_at(kl + u);
           }
 #pragma unroll
-          for (int u = 0; u < 8; ++u) d[u] = __dsub_rn(hi[u], lo[u]);
+          for (int u = 0; u < PER; ++u) d[u] = __dsub_rn(hi[u], lo[u]);
         } else {
-          const int n = min(8, len - k0 - part);
+          const int n = min(PER, len - k0 - part);
           for (int u = 0; u < n; ++u) d[u] = __dsub_rn(at(kh + u), at(kl + u));
         }
       }
@@ -345,32 +348,33 @@ __global__ void __launch_bounds__(BL_THREADS) k_blur_lines(int w, int h, int r, 
         if (ROWS) {
           const int pos = 32 * q + lane;
           if (pos < len) {
-            const double* ar = a + part * BL_PITCH + lane;
-            double* o = out + (size_t)(line0 + part) * len + pos;
+            const int l0 = (warp - 2) * (LINES / 4);  // this warp's lines
+            const double* ar = a + l0 * BL_PITCH + lane;
+            double* o = out + (size_t)(line0 + l0) * len + pos;
             if (full_block) {
 #pragma unroll
-              for (int u = 0; u < 8; ++u) o[(size_t)u * len] = __dmul_rn(ar[u * BL_PITCH], norm);
+              for (int u = 0; u < LINES / 4; ++u) o[(size_t)u * len] = __dmul_rn(ar[u * BL_PITCH], norm);
             } else {
-              for (int u = 0; u < 8 && line0 + part + u < lines; ++u) o[(size_t)u * len] = __dmul_rn(ar[u * BL_PITCH], norm);
+              for (int u = 0; u < LINES / 4 && line0 + l0 + u < lines; ++u) o[(size_t)u * len] = __dmul_rn(ar[u * BL_PITCH], norm);
             }
           }
         } else if (mine) {
           const int p0 = 32 * q + part;
-          const double* ar = a + lane * BL_PITCH + part;
+          const double* ar = a + ln * BL_PITCH + part;
           double* o = out + (size_t)p0 * w + line;
-          if (p0 + 8 <= len) {
+          if (p0 + PER <= len) {
 #pragma unroll
-            for (int u = 0; u < 8; ++u) o[(size_t)u * w] = __dmul_rn(ar[u], norm);
+            for (int u = 0; u < PER; ++u) o[(size_t)u * w] = __dmul_rn(ar[u], norm);
           } else {
-            for (int u = 0; p0 + u < len; ++u) o[(size_t)u * w] = __dmul_rn(ar[u], norm);
+            for (int u = 0; u < PER && p0 + u < len; ++u) o[(size_t)u * w] = __dmul_rn(ar[u], norm);
           }
         }
       }
-    } else if (s >= 1 && s <= tiles && mine) {
+    } else if (s >= 1 && s <= tiles && sub == 0 && mine) {
       // warp 0: the running sum over the previous step's differences
       const int q = s - 1;
-      const double* d = dif + (q & 1) * BL_TILE + lane * BL_PITCH;
-      double* a = sum + (q & 1) * BL_TILE + lane * BL_PITCH;
+      const double* d = dif + (q & 1) * BL_TILE + ln * BL_PITCH;
+      double* a = sum + (q & 1) * BL_TILE + ln * BL_PITCH;
       const int kend = min(32, len - 32 * q);
       if (kend == 32) {
         double x[32];  // the reads first, then the serial sum (see the differences above)
@@ -406,22 +410,34 @@ static dim3 grid2d(int w, int h) {
 static bool prolong_pairs(int w, const double* out) { return (w % 2) == 0 && ((uintptr_t)out % 16) == 0; }
 
 // The box blur's line kernel for one direction: false when r is too wide for its ring.
-template <bool ROWS>
+template <bool ROWS, int LINES>
 static bool launch_blur_lines(int w, int h, int r, bool wrap, double norm, const double* v, double* out, cudaStream_t st) {
   const int lines = ROWS ? h : w;
-  constexpr size_t smem = blur_lines_smem<ROWS>();
-  const unsigned blocks = (unsigned)ceil_div((size_t)lines, 32);
+  constexpr size_t smem = blur_lines_smem<ROWS, LINES>();
+  const unsigned blocks = (unsigned)ceil_div((size_t)lines, LINES);
   if (r + 1 <= 32) {
-    cudaFuncSetAttribute(k_blur_lines<ROWS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_blur_lines<ROWS, 1><<<blocks, BL_THREADS, smem, st>>>(w, h, r, wrap, norm, v, out);
+    cudaFuncSetAttribute(k_blur_lines<ROWS, 1, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_blur_lines<ROWS, 1, LINES><<<blocks, BL_THREADS, smem, st>>>(w, h, r, wrap, norm, v, out);
     return true;
   }
   if (r + 1 <= 64) {
-    cudaFuncSetAttribute(k_blur_lines<ROWS, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_blur_lines<ROWS, 2><<<blocks, BL_THREADS, smem, st>>>(w, h, r, wrap, norm, v, out);
+    cudaFuncSetAttribute(k_blur_lines<ROWS, 2, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_blur_lines<ROWS, 2, LINES><<<blocks, BL_THREADS, smem, st>>>(w, h, r, wrap, norm, v, out);
     return true;
   }
   return false;
+}
+// Lines a block, two passes (a row and a column sweep each) with 32 / 16 / 8 in both directions:
+// 2048 x 656 110 / 89 / 87 us (83 with 8 for rows and 16 for columns), 1000 x 400 81 / 63 / 52,
+// 4096 x 2048 208 / 183 / 224, 8192 x 4096 509 / 518 / 716 (503 with 16 for rows and 32 for columns). So 8
+// while each block has an SM of its own, then 16; and 32 columns, whose segments are whole 256
+// bytes, once blocks of 16 are more than three an SM.
+template <bool ROWS>
+static bool launch_blur(int w, int h, int r, bool wrap, double norm, const double* v, double* out, cudaStream_t st) {
+  const int lines = ROWS ? h : w;
+  if (ceil_div((size_t)lines, 8) <= 148) return launch_blur_lines<ROWS, 8>(w, h, r, wrap, norm, v, out, st);
+  if (ROWS || ceil_div((size_t)lines, 16) <= 3 * 148) return launch_blur_lines<ROWS, 16>(w, h, r, wrap, norm, v, out, st);
+  return launch_blur_lines<ROWS, 32>(w, h, r, wrap, norm, v, out, st);
 }
 
 }  // namespace dt
@@ -498,9 +514,9 @@ dt_status dt_grid_box_blur_dev(int w, int h, int wrap_x, int r, int passes, doub
   cudaStream_t st = (cudaStream_t)stream;
   for (int p = 0; p < passes; ++p) {
     // radii past the ring's reach (r > 63) take the plain one-thread-per-line kernels
-    if (!launch_blur_lines<true>(w, h, r, wrap_x != 0, norm, v, scratch, st))
+    if (!launch_blur<true>(w, h, r, wrap_x != 0, norm, v, scratch, st))
       k_blur_rows<<<ceil_div(h, 128), 128, 0, st>>>(w, h, r, wrap_x != 0, norm, v, scratch);
-    if (!launch_blur_lines<false>(w, h, r, false, norm, scratch, v, st))
+    if (!launch_blur<false>(w, h, r, false, norm, scratch, v, st))
       k_blur_cols<<<ceil_div(w, 128), 128, 0, st>>>(w, h, r, norm, scratch, v);
   }
   DT_CUDA(cudaGetLastError());
