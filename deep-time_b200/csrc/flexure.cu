@@ -1228,29 +1228,33 @@ __global__ void __launch_bounds__(FFT_MAX_THREADS / 2, 3) k_cols_fused(int N, cp
 // e(j) and n1 = m1 - m2 l1(j-1) the row's chain is l1 = n1 rd, dd = m0 - l1 n1 - l2 m2 and one
 // reciprocal (the reference's carried value l2 dd(j-2) l1 is m2 l1). With two divisions a row and a
 // launch a level it took 90 us a level at 513 wavenumbers x 328 rows (FP64), three in sequence.
+// The chain runs in FP64 for FP32 factors too: it amplifies rounding on tall rasters, and the factors
+// rounded once save iterations (8192 x 2944, FP32 with reliable updates to 1e-8, two inputs: 131 and 158 with an
+// FP32 chain, 103 and 118 with this one, 180 and 217 ms to 143 and 163).
 template <class T>
 __global__ void __launch_bounds__(64) k_row_factor(int N, int h, const T* __restrict__ lx, const T* __restrict__ ma,
                                                    const T* __restrict__ mb, T inv_dx2, const Scalars* S, T* __restrict__ fac) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q > N) return;
-  const T d = (T)S->node_d[blockIdx.y], c = (T)S->c_ref;
-  const T lxk = lx[q];
+  using A = double;
+  const A d = (T)S->node_d[blockIdx.y], c = (T)S->c_ref, s2 = inv_dx2;
+  const A lxk = lx[q];
   const size_t stride = (size_t)N + 1, plane = (size_t)h * stride;
   fac += (size_t)blockIdx.y * 3 * plane + q;
-  T r1 = 0, r2 = 0, l1p = 0;  // 1 / dd[j-1], 1 / dd[j-2], l1[j-1]
-  T t1 = 0, e1 = 0, e2 = 0;   // t(j-1), e(j-1), e(j-2)
+  A r1 = 0, r2 = 0, l1p = 0;  // 1 / dd[j-1], 1 / dd[j-2], l1[j-1]
+  A t1 = 0, e1 = 0, e2 = 0;   // t(j-1), e(j-1), e(j-2)
 #pragma unroll 4
   for (int j = 0; j < h; ++j) {
-    const T tj = (ma[j] * lxk - mb[j] - mb[j + 1]) * inv_dx2;
-    const T ej = j + 1 < h ? mb[j + 1] * inv_dx2 : (T)0;
-    const T m2 = d * e2 * e1;                    // 0 for j < 2
-    const T n1 = d * e1 * (t1 + tj) - m2 * l1p;  // 0 for j < 1
-    const T p1 = n1 * r1, p2 = m2 * r2;
-    const T dj = (d * (tj * tj + e1 * e1 + ej * ej) + c - p2 * m2) - p1 * n1;
-    const T rj = recip(dj);
-    fac[(size_t)j * stride] = rj;
-    fac[plane + (size_t)j * stride] = p1;
-    fac[2 * plane + (size_t)j * stride] = p2;
+    const A tj = (ma[j] * lxk - mb[j] - mb[j + 1]) * s2;
+    const A ej = j + 1 < h ? mb[j + 1] * s2 : (A)0;
+    const A m2 = d * e2 * e1;                    // 0 for j < 2
+    const A n1 = d * e1 * (t1 + tj) - m2 * l1p;  // 0 for j < 1
+    const A p1 = n1 * r1, p2 = m2 * r2;
+    const A dj = (d * (tj * tj + e1 * e1 + ej * ej) + c - p2 * m2) - p1 * n1;
+    const A rj = recip(dj);
+    fac[(size_t)j * stride] = (T)rj;
+    fac[plane + (size_t)j * stride] = (T)p1;
+    fac[2 * plane + (size_t)j * stride] = (T)p2;
     r2 = r1;
     r1 = rj;
     l1p = p1;
