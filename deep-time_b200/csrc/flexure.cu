@@ -2107,9 +2107,10 @@ struct Lane {
   T* row_factors = nullptr;
   T* row_transfer = nullptr;
   cplx<T>* row_state = nullptr;
-  // widths whose half is not a power of two (rows_any.cuh): per bank level two buffers of
-  // pairs x L complex values, the passes' twiddles (L), and for Bluestein the chirp (w) and the
-  // chirp's transform (L)
+  // widths whose half is not a power of two (rows_any.cuh): whether a row pair's transform takes one block
+  // (any_block_pays), one level's and the bank's; per bank level two buffers of pairs x L complex
+  // values, the passes' twiddles (L), and for Bluestein the chirp (w) and the chirp's transform (L)
+  bool block_one = false, block_bank = false;
   cplx<T>* any_buf = nullptr;
   cplx<T>* any_tw = nullptr;
   cplx<T>* any_chirp = nullptr;
@@ -2128,7 +2129,7 @@ static const long double PI_L = 3.14159265358979323846264338327950288L;
 struct dt_flex {
   int w = 0, h = 0, N = 0;  // N = ceil(w / 2): complex values a row of the packed half spectrum
   bool any = false;         // the transform along x by rows_any.cuh (w / 2 not a power of two)
-  dt::AnyPlan plan;
+  dt::AnyPlan plan, block_plan;  // its passes through global memory and its row pair in one block
   double dx = 0;
   size_t n = 0;
   cudaStream_t stream = nullptr;
@@ -2244,37 +2245,38 @@ static dt_status make_tables(dt_flex* s, Tables<T>& tb) {
 
 // The plan of the transform along x for a width whose half is not a power of two: mixed-radix
 // stages when every prime factor of w is at most ANY_MAX_PRIME, else Bluestein through the power
-// of two M >= 2 w - 1.
-static AnyPlan make_any_plan(int w, int h, int most = 16) {
+// of two M >= 2 w - 1. For the passes through global memory the largest powers of two come first. For a
+// row pair in one block (`block`) radix 8 at most, which keeps four FP64 blocks an SM, and the odd
+// radices first: the first stage's outputs lie a radix apart, which in shared memory keeps the powers of
+// two's from falling in the same banks.
+static AnyPlan make_any_plan(int w, int h, bool block) {
   AnyPlan p;
   p.w = w;
   p.pairs = (h + 1) / 2;
   std::vector<int> f;
-  int n = w;
-  for (int r : {16, 8, 4, 2})
-    while (r <= most && n % r == 0) {
-      f.push_back(r);
-      n /= r;
-    }
-  for (int q = 3; q <= ANY_MAX_PRIME && n > 1; q += 2)
-    while (n % q == 0) {
-      f.push_back(q);
-      n /= q;
-    }
+  int n;
+  auto factor = [&](int length) {
+    f.clear();
+    n = length;
+    for (int r : {16, 8, 4, 2})
+      while ((r <= 8 || !block) && n % r == 0) {
+        f.push_back(r);
+        n /= r;
+      }
+    for (int q = 3; q <= ANY_MAX_PRIME && n > 1; q += 2)
+      while (n % q == 0) {
+        f.push_back(q);
+        n /= q;
+      }
+  };
+  factor(w);
   if (n > 1) {  // a prime factor beyond ANY_MAX_PRIME
     p.bluestein = 1;
     int m = 1;
     while (m < 2 * w - 1) m *= 2;
-    f.clear();
-    for (int r : {16, 8, 4, 2})
-      while (r <= most && m % r == 0) {
-        f.push_back(r);
-        m /= r;
-      }
+    factor(m);
   }
-  // odd radices first: the first stage's outputs lie a radix apart, which in shared memory keeps the
-  // powers of two's from falling in the same banks
-  std::stable_partition(f.begin(), f.end(), [](int r) { return r % 2 != 0; });
+  if (block) std::stable_partition(f.begin(), f.end(), [](int r) { return r % 2 != 0; });
   p.L = 1;
   for (int x : f) p.L *= x;
   p.nst = (int)f.size();
@@ -2284,9 +2286,48 @@ static AnyPlan make_any_plan(int w, int h, int most = 16) {
     p.span[k] = span;
     span *= f[k];
   }
-  // a row pair in one FP64 block: radix 8 at most
-  if (most > 8 && any_block_smem<double>(p) <= ANY_BLOCK_SMEM) return make_any_plan(w, h, 8);
   return p;
+}
+
+// Whether row pairs are transformed in one block each (rows_any.cuh, plan p) for `levels` bank levels a
+// pass, rather than by the passes through global memory (plan q). Measured, an iteration of the solve in
+// blocks against one with the passes:
+// - One level turns with the times of the two forms of a transform. The block: a thread's values through
+//   the stages, 0.13 us each and 0.08 for a term of a prime radix's sum (R terms a value). The passes: a
+//   launch each of 2.2 us (4 in Bluestein's two transforms) and their bytes, and a prime radix's terms at 0.3 us. FP64 1500 x 256 67 us
+//   against 86, 1830 x 256 (radix 61) 263 against 177, 3000 x 16 84 against 73, 3000 x 256 100 against 109.
+// - The bank's three levels side by side hide more of the chain, half of the primes' table reads:
+//   FP64 740 x 256 (radix 37) 137 us against 183, 1859 x 16 (11, 13, 13) 181 against 125.
+// - Rows that fill the SMs more than once (the bank with a short chain: twice; FP64 1301 x 100 by Bluestein,
+//   4096 values, 187 us against 229) want 384 threads an SM at work, 448 where the passes have less
+//   to move (FP32) or the chain is a prime's. The bank: FP64 2000 x 1024, 288 threads, 421 us against
+//   380; 1800 x 1024, 384, 355 against 373; 6000 x 1000, 96, 2480 against 1360; FP32 4375 x 1024, 384,
+//   568 against 539; 4800 x 1024, 480, 562 against 595.
+template <class T>
+static bool any_block_pays(const AnyPlan& p, const AnyPlan& q, int levels, int sms) {
+  const size_t smem = any_block_smem<T>(p);
+  if (smem > ANY_BLOCK_SMEM) return false;
+  const int nt = any_block_threads(p), ffts = p.bluestein ? 2 : 1;
+  int small = 0, prime = 0;
+  for (int k = 0; k < p.nst; ++k) {
+    const int R = p.radix[k];
+    if (R <= 8)
+      small += (int)ceil_div(p.L / R, nt) * R;
+    else
+      prime += (int)ceil_div(p.L, nt) * R;
+  }
+  if (levels == 1) {
+    const double pass = (p.bluestein ? 4.0 : 2.2) + (double)q.pairs * q.L * 2 * sizeof(cplx<T>) / 12e6;
+    double passes = (ffts * q.nst + ffts + 1) * pass;
+    for (int k = 0; k < q.nst; ++k) passes += q.radix[k] > 16 || q.radix[k] % 2 && q.radix[k] > 8 ? 0.3 * q.radix[k] : 0.0;
+    if (1.1 * (3.0 + ffts * (0.13 * small + 0.08 * prime)) > passes) return false;
+  } else if (small + prime / 2 > 255) {
+    return false;
+  }
+  const int blocks = std::min((int)(228 * 1024 / (smem + 1024)), 2048 / nt);
+  const long fill = (long)sms * blocks;
+  if (p.pairs * levels <= (levels == 3 && small + prime / 2 <= 160 ? 2 * fill : fill)) return true;
+  return blocks * nt >= (p.bluestein || (sizeof(T) == 8 && prime == 0) ? 384 : 448);
 }
 
 // Host FFT in long double (iterative radix 2, length a power of two): Bluestein's table B.
@@ -2312,6 +2353,8 @@ static void host_fft(std::vector<std::complex<long double>>& a) {
 template <class T>
 static dt_status make_any_tables(dt_flex* s, Lane<T>& L) {
   using C = cplx<T>;
+  L.block_one = any_block_pays<T>(s->block_plan, s->plan, 1, s->sms);
+  L.block_bank = any_block_pays<T>(s->block_plan, s->plan, 3, s->sms);
   const AnyPlan& p = s->plan;
   std::vector<C> tw(p.L);
   for (int t = 0; t < p.L; ++t) {
@@ -2733,9 +2776,9 @@ static void transform_smem_attributes() {
   int big = 200 * 1024;
   cudaFuncSetAttribute(k_any_block_fwd<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
   cudaFuncSetAttribute(k_any_block_fwd<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
+  cudaFuncSetAttribute(k_any_block_bank<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
   cudaFuncSetAttribute(k_any_block_inv<T, INV_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
   cudaFuncSetAttribute(k_any_block_inv<T, INV_STORE_W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
-  cudaFuncSetAttribute(k_any_block_bank<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
   cudaFuncSetAttribute(k_any_block_inv<T, INV_STORE_DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANY_BLOCK_SMEM);
   cudaFuncSetAttribute(k_row_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   for (int l = 0; l < FFT_LOGS; ++l) {
@@ -2800,17 +2843,11 @@ static cplx<T>* any_slot(dt_flex* s, Lane<T>& L, int level) {
   return L.any_buf + (size_t)level * 2 * s->plan.pairs * s->plan.L;
 }
 
-// Whether a row pair of the plan is transformed in one block's shared memory, both ways.
-template <class T>
-static bool any_in_block(const AnyPlan& p) {
-  return any_block_smem<T>(p) <= ANY_BLOCK_SMEM;
-}
-
 template <class T>
 static void any_rows_fwd(dt_flex* s, Lane<T>& L, const T* in, const T* wt, cplx<T>* half, int level, Scalars* S,
                          cudaStream_t st, int levels = 1) {
-  const AnyPlan& p = s->plan;
-  if (any_in_block<T>(p)) {
+  if (wt ? L.block_bank : L.block_one) {  // the weights are the bank's
+    const AnyPlan& p = s->block_plan;
     const dim3 grid(p.pairs, levels);
     const int nt = any_block_threads(p);
     if (wt)
@@ -2822,6 +2859,7 @@ static void any_rows_fwd(dt_flex* s, Lane<T>& L, const T* in, const T* wt, cplx<
     counted();
     return;
   }
+  const AnyPlan& p = s->plan;
   cplx<T>* a = any_slot<T>(s, L, level);
   cplx<T>* b = a + (size_t)p.pairs * p.L;
   const unsigned g = any_grid((size_t)p.pairs * p.L);
@@ -2838,8 +2876,8 @@ static void any_rows_fwd(dt_flex* s, Lane<T>& L, const T* in, const T* wt, cplx<
 template <class T>
 static void any_rows_inv(dt_flex* s, Lane<T>& L, int mode, const cplx<T>* half, T* out, const T* wt, const T* r,
                          Scalars* S, cudaStream_t st) {
-  const AnyPlan& p = s->plan;
-  if (any_in_block<T>(p)) {
+  if (mode == INV_BANK ? L.block_bank : L.block_one) {
+    const AnyPlan& p = s->block_plan;
     const size_t smem = any_block_smem<T>(p);
     const int nt = any_block_threads(p);
     auto go = [&](auto kernel) {
@@ -2856,6 +2894,7 @@ static void any_rows_inv(dt_flex* s, Lane<T>& L, int mode, const cplx<T>* half, 
     counted();
     return;
   }
+  const AnyPlan& p = s->plan;
   const int levels = mode == INV_BANK ? 3 : 1;
   const size_t pl = (size_t)p.pairs * p.L;
   cplx<T>* f0 = nullptr;
@@ -2869,9 +2908,9 @@ static void any_rows_inv(dt_flex* s, Lane<T>& L, int mode, const cplx<T>* half, 
   const unsigned g = std::min<unsigned>(any_grid((size_t)p.pairs * p.w), (unsigned)s->sms * 4);
   const size_t stride = 2 * pl;
   switch (mode) {
+    case INV_BANK: k_any_emit<T, INV_BANK><<<g, 256, 0, st>>>(p, s->h, f0, stride, out, wt, r, L.any_chirp, s->partials, S); break;
     case INV_STORE: k_any_emit<T, INV_STORE><<<g, 256, 0, st>>>(p, s->h, f0, stride, out, wt, r, L.any_chirp, s->partials, S); break;
     case INV_STORE_W: k_any_emit<T, INV_STORE_W><<<g, 256, 0, st>>>(p, s->h, f0, stride, out, wt, r, L.any_chirp, s->partials, S); break;
-    case INV_BANK: k_any_emit<T, INV_BANK><<<g, 256, 0, st>>>(p, s->h, f0, stride, out, wt, r, L.any_chirp, s->partials, S); break;
     default: k_any_emit<T, INV_STORE_DOT><<<g, 256, 0, st>>>(p, s->h, f0, stride, out, wt, r, L.any_chirp, s->partials, S); break;
   }
   counted();
@@ -2981,8 +3020,8 @@ static void launch_spectral(dt_flex* s, Lane<T>& L, const T* in, const T* wt, T*
 // Whether the bank's levels share a launch a pass: where each pass is one kernel (the power-of-two
 // transforms, and along y the cosine transform or k_row_solve).
 template <class T>
-static bool bank_batched(const dt_flex* s) {
-  return s->bank_one_launch && !(s->any && !any_in_block<T>(s->plan)) && !(s->row_solve && row_groups<T>(s->h) < 0);
+static bool bank_batched(const dt_flex* s, const Lane<T>& L) {
+  return s->bank_one_launch && !(s->any && !L.block_bank) && !(s->row_solve && row_groups<T>(s->h) < 0);
 }
 
 // z = M^-1 r with r.z and max|z| reduced into S (finish_precond). levels 1: one spectral solve at
@@ -2999,7 +3038,7 @@ static void launch_precondition(dt_flex* s, Lane<T>& L, const T* r, T* z, int le
   // (their spectra and weights are consecutive); otherwise levels 1 and 2 run on side streams
   // (parallel branches when captured into the loop graph). One inverse pass then takes the
   // three spectra to the weighted sum.
-  if (bank_batched<T>(s)) {
+  if (bank_batched<T>(s, L)) {
     FftGeo g = fft_geometry<T>(s);
     if (s->any) {
       any_rows_fwd<T>(s, L, L.left, L.wt[0], L.half, 0, L.S, st, 3);
@@ -3641,7 +3680,10 @@ dt_status dt_flex_create(int w, int h, double dx, const double* metric_a, const 
   s->h = h;
   s->any = (w & 1) || !is_pow2(w / 2) || w / 2 > 8192;
   s->N = (w + 1) / 2;
-  if (s->any) s->plan = make_any_plan(w, h);
+  if (s->any) {
+    s->plan = make_any_plan(w, h, false);
+    s->block_plan = make_any_plan(w, h, true);
+  }
   s->dx = dx;
   s->n = (size_t)w * h;
   cudaDeviceProp prop;
@@ -4072,7 +4114,7 @@ static dt_status profile_lane(dt_flex* s, Lane<T>& L, int reps, double* ms, doub
   };
   // the bank's column passes and weighted forward row passes as the solve launches them: the
   // three levels in one launch (each level's bytes again) where it does so
-  const bool bank1 = bank_batched<T>(s);
+  const bool bank1 = bank_batched<T>(s, L);
   const double bank_levels = bank1 ? 3.0 : 1.0;
   cudaEvent_t a, b;
   DT_CUDA(cudaEventCreate(&a));

@@ -297,12 +297,12 @@ __global__ void __launch_bounds__(256) k_any_emit(AnyPlan p, int h, const cplx<T
   }
 }
 // ---- the same transform with a row pair in one block's shared memory ----
-// Where two buffers of L values (and for the bank's inverse a row pair of sums) fit one block, each pass
+// For the rows where it is the faster form (any_block_pays in flexure.cu), each pass
 // takes a row pair from the raster to the spectrum or back: the stages alternate between the buffers, a
 // barrier each, and nothing of them goes through global memory. The values of the passes above, stage for
 // stage. Bound by the stages' latency: the block's threads are chosen so that the stages' butterflies
 // fill whole rounds of them (any_block_threads; 256 threads on 300 butterflies of radix 5 leave two
-// thirds of the second round idle), the FP64 plans take radix 8 at most to keep four blocks an SM, and the
+// thirds of the second round idle), the plans take radix 8 at most to keep four FP64 blocks an SM, and the
 // bank's three levels run side by side as a cluster of blocks. FP64 1500 x 750 (radices 4, 3, 5, 5, 5), a
 // bank pass of three levels: forward 44 us and inverse 65 (cold caches), against 21 launches of 6 us each
 // way and a summing one on three streams; the step's solve there 2.43 to 2.10 ms.
@@ -389,9 +389,6 @@ __device__ __forceinline__ cplx<T>* any_block_fft(const AnyPlan& p, cplx<T>* a, 
       case 5: any_block_stage<T, 5>(p, s, a, b, tw); break;
       case 7: any_block_stage<T, 7>(p, s, a, b, tw); break;
       case 8: any_block_stage<T, 8>(p, s, a, b, tw); break;
-      case 16:
-        if constexpr (sizeof(T) == 4) any_block_stage<T, 16>(p, s, a, b, tw);  // FP64 plans: radix 8 at most
-        break;
       default: any_block_prime<T>(p, s, a, b, tw); break;
     }
     __syncthreads();
