@@ -2108,8 +2108,8 @@ struct Lane {
   T* row_transfer = nullptr;
   cplx<T>* row_state = nullptr;
   // widths whose half is not a power of two (rows_any.cuh): whether a row pair's transform takes one block
-  // (any_block_pays), one level's and the bank's; per bank level two buffers of pairs x L complex
-  // values, the passes' twiddles (L), and for Bluestein the chirp (w) and the chirp's transform (L)
+  // (any_block_pays), one level's and the bank's; for the passes, per level two buffers of pairs x L
+  // complex values; the twiddles (L), and for Bluestein the chirp (w) and the chirp's transform (L)
   bool block_one = false, block_bank = false;
   cplx<T>* any_buf = nullptr;
   cplx<T>* any_tw = nullptr;
@@ -2363,7 +2363,9 @@ static dt_status make_any_tables(dt_flex* s, Lane<T>& L) {
   }
   DT_TRY(dalloc(s, &L.any_tw, p.L));
   DT_CUDA(cudaMemcpy(L.any_tw, tw.data(), p.L * sizeof(C), cudaMemcpyHostToDevice));
-  DT_TRY(dalloc(s, &L.any_buf, (size_t)3 * 2 * p.pairs * p.L));
+  // the passes' buffers, for what does not run in blocks: the bank's three levels, or one
+  const size_t slots = !L.block_bank ? 3 : !L.block_one ? 1 : 0;
+  if (slots) DT_TRY(dalloc(s, &L.any_buf, slots * 2 * p.pairs * p.L));
   if (p.bluestein) {
     // c_n = e^(i pi n^2 / w) with n^2 reduced mod 2 w; b_n = c_n, b_(M - n) = c_n; B = FFT_M(b)
     const int w = p.w;

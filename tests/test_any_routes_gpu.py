@@ -43,3 +43,16 @@ def test_long_rows_keep_the_speed_of_the_passes():
                      max_iterations=20)
         times[w] = min(sv.solve_with(d, c, b, p)[1].device_ms for _ in range(4))
     assert times[9000] < 4.4 * times[8192], times
+
+
+def test_blocks_allocate_no_buffers_for_the_passes():
+    # 1500 x 750: the passes' buffers would be 3 levels x 2 x 375 x 1500 complex values in each lane, 81 MB;
+    # the handle without them takes 328 MB (allocations round up to 2 MB)
+    torch = pytest.importorskip("torch")
+    w, h = 1500, 750
+    F.Solver(64, 32, 20_000.0).close()  # the context and the library's modules
+    before = torch.cuda.mem_get_info()[0]
+    sv = F.Solver(w, h, 20_000.0)
+    used = before - torch.cuda.mem_get_info()[0]
+    sv.close()
+    assert used < 370e6, used
