@@ -1765,10 +1765,11 @@ static void launch_tile(dt_diff* s, const DLevel<TM>& L, const DLevel<TM>& C, co
   }
   launch_tile_dot<TM, RB, PRE, false>(s, L, C, zc, zout, nullptr, st);
 }
-// k_mg_tile's 32-bit offsets
+// k_mg_tile's 32-bit offsets, and its rows of tiles (24 cells at the least) on the grid's y extent, which
+// ends at 65535; taller levels take the launches a sweep
 template <class TM>
 static bool tile_fits(const DLevel<TM>& L) {
-  return (size_t)L.w * L.h < ((size_t)1 << 31);
+  return (size_t)L.w * L.h < ((size_t)1 << 31) && ceil_div(L.h, 24) <= 65535;
 }
 
 // One V-cycle from z = 0 on level l with r set; returns the buffer holding the level's z. With `rz` on
