@@ -165,8 +165,10 @@ __device__ __forceinline__ void block_reduce(double* v, const int* kind, double 
 // Writes this block's partials and, in the last block to arrive (an atomic ticket, reset for
 // reuse), reduces all of them in a fixed order; true there, with the results in thread 0. A tail
 // of latencies at the end of every reducing kernel: the components go through the shuffles
-// together, the ticket's atomic carries the release and only the last block fences, and it has two partials a thread in flight
-// (four took the vector kernels past 32 registers, eight blocks an SM). One component after another, a
+// together, the ticket's atomic carries both halves of the order (its release follows this block's
+// partials; its acquire, in the same thread, precedes the barrier that lets the last block's threads
+// read the others'), and two partials a thread are in flight (four took the vector kernels past 32
+// registers, eight blocks an SM). One component after another, a
 // __threadfence and one load at a time made an FP64 512 x 256 update 12.2 us (with the L2 flushed)
 // where a kernel without a reduction took 8.2; this 11.5.
 template <int NV>
@@ -180,13 +182,12 @@ __device__ bool reduce_partials(Acc<NV>& a, const int* kind, double* partials, u
 #pragma unroll
     for (int q = 0; q < NV; ++q) partials[(size_t)q * nblocks + bid] = a.v[q];
     unsigned int t;
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(ticket) : "memory");
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(ticket) : "memory");
     is_last = t == nblocks - 1;
     if (is_last) *ticket = 0u;
   }
   __syncthreads();
   if (!is_last) return false;
-  __threadfence();  // the ticket's releases before the partials' loads
 #pragma unroll
   for (int q = 0; q < NV; ++q) a.v[q] = kind[q] ? -INFINITY : 0.0;
   for (unsigned b = tid; b < nblocks; b += 2 * nthreads) {
