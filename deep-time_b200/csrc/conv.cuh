@@ -100,20 +100,134 @@ __device__ __forceinline__ void conv_store(bf16* dst, int col, float v0, float v
   *d2 = __floats2bfloat162_rn(v0, v1);
 }
 
-// One 3 x 3 convolution (or its input gradient with mirrored, transposed weights): W is [9][Cin][Cout]
-// bf16, tap = ky * 3 + kx reading in[y + ky - 1][x + kx - 1]; image rows of width `w` (a multiple of 64),
-// `h` rows, `nimg` images. A block takes RY rows by 64 pixels of one image and BN output channels, its
+// One 3 x 3 convolution (or its input gradient with mirrored, transposed weights): W is
+// [9][Cin][Cout] bf16, tap = ky * 3 + kx reading in[y + ky - 1][x + kx - 1]. Image rows of width
+// `w` (a multiple of 64), `h` rows, `nimg` images. A block takes 64 pixels of a row by BN output channels,
+// its four warps 32 by BN / 2 each; a step stages one tap's pixels and weights of 32 channels, two steps
+// in flight. Small blocks, so few pixels still reach many SMs; the pixels are staged nine times. Sums in
+// k_conv3x3_res's order, so the same values.
+template <int BN, int EPI>
+__global__ void __launch_bounds__(128) k_conv3x3_line(int nimg, int h, int w, Tensor4 in, const bf16* __restrict__ W,
+                                                 const float* __restrict__ bias, Tensor4 out, Tensor4 mask) {
+  constexpr int BM = 64, BK = 32;
+  __shared__ __align__(128) bf16 sA[2][BM * BK];
+  __shared__ __align__(128) bf16 sB[2][BK * BN];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = warp >> 1, wn = warp & 1;  // warp tile: rows wm*32.., cols wn*(BN/2)..
+  const int tiles_x = w / BM;
+  int bid = blockIdx.x;
+  const int xt = bid % tiles_x;
+  bid /= tiles_x;
+  const int y = bid % h;
+  const int n = bid / h;
+  const int x0 = xt * BM;
+  const int co0 = blockIdx.y * BN;
+  const int cin = in.c;
+  const int kchunks = 9 * (cin / BK);
+  constexpr int NT = BN / 16;  // n8 tiles per warp
+  float acc[2][NT][4];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < NT; ++b)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[a][b][c] = 0.f;
+
+  auto load = [&](int kc, int stage) {
+    int tap = kc / (cin / BK);
+    int ci0 = (kc % (cin / BK)) * BK;
+    int ky = tap / 3, kx = tap % 3;
+    int yy = y + ky - 1;
+    bool yok = yy >= 0 && yy < h;
+    // A: 64 pixels x 32 channels = 256 chunks of 16 B; 2 a thread
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      int cidx = tid + q * 128;
+      int row = cidx >> 2, ch = cidx & 3;
+      int xx = x0 + row + kx - 1;
+      xx = xx < 0 ? xx + w : (xx >= w ? xx - w : xx);
+      const bf16* src = in.p + ((size_t)((size_t)n * h + (yok ? yy : 0)) * w + xx) * in.stride + in.off + ci0 + ch * 8;
+      cp_async16(&sA[stage][swz_a(row, ch)], src, yok);
+    }
+    // B: 32 k-rows x BN channels
+    constexpr int BCH = BK * BN / 8;
+#pragma unroll
+    for (int q = 0; q < (BCH + 127) / 128; ++q) {
+      int cidx = tid + q * 128;
+      if (cidx < BCH) {
+        int row = cidx / (BN / 8), ch = cidx % (BN / 8);
+        const bf16* src = W + ((size_t)tap * cin + ci0 + row) * out.c + co0 + ch * 8;
+        cp_async16(&sB[stage][swz_b<BN>(row, ch)], src, true);
+      }
+    }
+    cp_async_commit();
+  };
+
+  load(0, 0);
+  for (int kc = 0; kc < kchunks; ++kc) {
+    int stage = kc & 1;
+    if (kc + 1 < kchunks) {
+      load(kc + 1, stage ^ 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 16) {
+      unsigned af[2][4];
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) {
+        int row = wm * 32 + mt * 16 + (lane & 15);
+        int chunk = (kk >> 3) + (lane >> 4);
+        ldmatrix_x4(af[mt][0], af[mt][1], af[mt][2], af[mt][3], &sA[stage][swz_a(row, chunk)]);
+      }
+      unsigned bfr[NT][2];
+#pragma unroll
+      for (int nt = 0; nt < NT; nt += 2) {
+        int krow = kk + (lane & 15);
+        int chunk = (wn * (BN / 2) + nt * 8) / 8 + (lane >> 4);
+        unsigned r0, r1, r2, r3;
+        ldmatrix_x4_trans(r0, r1, r2, r3, &sB[stage][swz_b<BN>(krow, chunk)]);
+        bfr[nt][0] = r0;
+        bfr[nt][1] = r1;
+        bfr[nt + 1][0] = r2;
+        bfr[nt + 1][1] = r3;
+      }
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) mma_bf16(acc[mt][nt], af[mt], bfr[nt]);
+    }
+    __syncthreads();
+  }
+  // epilogue: rows = pixels, cols = output channels
+  const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      int row = wm * 32 + mt * 16 + g + half * 8;
+      size_t pix = ((size_t)n * h + y) * w + x0 + row;
+      bf16* dst = out.p + pix * out.stride + out.off + co0;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int col = wn * (BN / 2) + nt * 8 + t4 * 2;
+        conv_store<EPI>(dst, col, acc[mt][nt][half * 2], acc[mt][nt][half * 2 + 1], bias, co0, mask, pix);
+      }
+    }
+}
+
+// The same with the pixels staged once. A block takes RY rows by 64 pixels of one image and BN output channels, its
 // warps 32 pixels each of one row by all BN channels. The region's (RY + 2) x 66 pixels of every input
 // channel are copied once into shared memory (padding and wrap in the copies) and the nine taps read them
 // at shifted addresses; the weights come a tap and 32 channels at a time through a ring of STAGES.
 // Products are summed by tap, then channel, 16 at a time. A pixel's channels are spaced by 16 bytes
 // more than their own, which puts the eight rows of an ldmatrix in distinct banks.
 // 2 RY x COW warps of 32 pixels by NC channels each, BN = NC COW.
-// Bound by the legacy tensor path's issue (mma.sync) and its ldmatrix loads. Staging every tap's 128
-// pixels anew through shared memory (nine times the input traffic) took, at 16 x 512 x 256 cells,
-// 357 us for 32 -> 32 channels (now 253, 153 TFLOP/s), 716 for the gradient 32 -> 96 (522), 265
-// for a masked gradient 32 -> 32 (184), 492 for 64 -> 192 at half the size (430) and 875 for 384 -> 128
-// at a quarter (552).
+// Bound by the legacy tensor path's issue (mma.sync) and its ldmatrix loads: 16 x 512 x 256 pixels, warm,
+// 32 -> 32 channels 166 us (232 TFLOP/s; the line kernel 238), the gradient 32 -> 96 502 (690), a
+// masked gradient 32 -> 32 178 (254), 64 -> 64 at half the size 139 (161).
 __host__ __device__ constexpr size_t conv_res_smem(int cin, int ry, int bn, int stages) {
   return (size_t)(ry + 2) * 66 * (cin * 2 + 16) + (size_t)stages * 32 * bn * 2;
 }

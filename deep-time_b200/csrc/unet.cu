@@ -479,35 +479,55 @@ static bool conv_tc(dt_unet* u, int B, int h, int w, Tensor4 in, const bf16* Bk,
   return true;
 }
 
-// One convolution on the mma.sync path.
-template <int NC, int COW, int RY, int STAGES, int EPI>
-static void conv_res_go(int B, int h, int w, Tensor4 in, const bf16* W, const float* bias, Tensor4 out, Tensor4 mask,
-                        cudaStream_t st) {
-  const dim3 grid((unsigned)((size_t)B * ceil_div(h, RY) * (w / 64)), out.c / (NC * COW));
-  k_conv3x3_res<NC, COW, RY, STAGES, EPI>
-      <<<grid, 64 * RY * COW, conv_res_smem(in.c, RY, NC * COW, STAGES), st>>>(B, h, w, in, W, bias, out, mask);
-}
-// The tile by the input channels, whose region has to stay in shared memory beside the weights' ring:
-// up to 96, 8 warps of 32 pixels and two or more blocks an SM; beyond, one block of 16 warps that
-// share the region over twice the output channels (8 warps and two rows a block took 288 us where
-// this takes 171, 128 -> 128 channels at 16 x 128 x 64 pixels); 384 channels leave room for two rows only.
+// One convolution on the mma.sync path: the resident-region kernel where its tiles, by the input channels,
+// are the faster, else the line kernel. Up to 96 channels 8 warps of 32 pixels and two or more blocks an SM; beyond,
+// one block of 16 warps that share the region over twice the output channels. Warm, resident against
+// line, us:
+// - few tiles leave SMs idle, and a block's chain of taps is longer: 64 -> 64 at 64 x 256 pixels, 64 blocks,
+//   15.5 against 12.4; 128, 16.5 both; 256, 22.7 against 25.7; 256 -> 256 at 32 x 64, 16 blocks, 77.9
+//   against 28.8; 128, 78.0 against 83.9. So from three quarters of the SMs on.
+// - 97 to 192 channels, one block an SM: past one round of blocks the line kernel's smaller ones balance
+//   better, 128 -> 128 128 blocks 43.2 against 45.2, 512 166 against 156; 192 -> 64 35.0 against 40.8, 456
+//   against 439.
+// - more than 256 channels leave room for two rows only: 384 -> 128 525 against 438 at 16 x 64 x 128, slower
+//   at every size.
 template <int EPI>
-static void conv_res(int B, int h, int w, Tensor4 in, const bf16* W, const float* bias, Tensor4 out, Tensor4 mask,
+static void conv_line_go(int B, int h, int w, Tensor4 in, const bf16* W, const float* bias, Tensor4 out, Tensor4 mask,
+                         cudaStream_t st) {
+  const unsigned lines = (unsigned)((size_t)B * h * (w / 64));
+  if (out.c % 64 == 0)
+    k_conv3x3_line<64, EPI><<<dim3(lines, out.c / 64), 128, 0, st>>>(B, h, w, in, W, bias, out, mask);
+  else
+    k_conv3x3_line<32, EPI><<<dim3(lines, out.c / 32), 128, 0, st>>>(B, h, w, in, W, bias, out, mask);
+}
+template <int NC, int COW, int STAGES, int EPI>
+static void conv_go(int sms, int B, int h, int w, Tensor4 in, const bf16* W, const float* bias, Tensor4 out, Tensor4 mask,
+                    cudaStream_t st) {
+  const dim3 grid((unsigned)((size_t)B * ceil_div(h, 4) * (w / 64)), out.c / (NC * COW));
+  const size_t blocks = (size_t)grid.x * grid.y;
+  if (4 * blocks >= 3 * (size_t)sms && (in.c <= 96 || in.c > 192 || blocks <= (size_t)sms))
+    k_conv3x3_res<NC, COW, 4, STAGES, EPI>
+        <<<grid, 256 * COW, conv_res_smem(in.c, 4, NC * COW, STAGES), st>>>(B, h, w, in, W, bias, out, mask);
+  else
+    conv_line_go<EPI>(B, h, w, in, W, bias, out, mask, st);
+}
+template <int EPI>
+static void conv_mma(int sms, int B, int h, int w, Tensor4 in, const bf16* W, const float* bias, Tensor4 out, Tensor4 mask,
                      cudaStream_t st) {
   if (in.c <= 96) {
     if (out.c % 64 == 0)
-      conv_res_go<64, 1, 4, 4, EPI>(B, h, w, in, W, bias, out, mask, st);
+      conv_go<64, 1, 4, EPI>(sms, B, h, w, in, W, bias, out, mask, st);
     else
-      conv_res_go<32, 1, 4, 4, EPI>(B, h, w, in, W, bias, out, mask, st);
+      conv_go<32, 1, 4, EPI>(sms, B, h, w, in, W, bias, out, mask, st);
   } else if (in.c <= 192) {
     if (out.c % 128 == 0)
-      conv_res_go<64, 2, 4, 4, EPI>(B, h, w, in, W, bias, out, mask, st);
+      conv_go<64, 2, 4, EPI>(sms, B, h, w, in, W, bias, out, mask, st);
     else
-      conv_res_go<32, 2, 4, 4, EPI>(B, h, w, in, W, bias, out, mask, st);
+      conv_go<32, 2, 4, EPI>(sms, B, h, w, in, W, bias, out, mask, st);
   } else if (in.c <= 256) {
-    conv_res_go<64, 2, 4, 2, EPI>(B, h, w, in, W, bias, out, mask, st);
+    conv_go<64, 2, 2, EPI>(sms, B, h, w, in, W, bias, out, mask, st);
   } else {
-    conv_res_go<32, 4, 2, 2, EPI>(B, h, w, in, W, bias, out, mask, st);
+    conv_line_go<EPI>(B, h, w, in, W, bias, out, mask, st);
   }
   count_launch();
 }
@@ -529,7 +549,6 @@ static dt_status conv_res_attributes() {
   DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<64, 2, 4, 4, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<32, 2, 4, 4, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<64, 2, 4, 2, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  DT_CUDA(cudaFuncSetAttribute(k_conv3x3_res<32, 4, 2, 2, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   return DT_OK;
 }
 
@@ -541,9 +560,9 @@ static void conv_fwd(dt_unet* u, const ConvLayer& L, int B, int h, int w, Tensor
                    : conv_tc<EPI_BIAS>(u, B, h, w, in, L.WT, L.cout, bias, out, none, st);
   if (done) return;
   if (relu)
-    conv_res<EPI_BIAS_RELU>(B, h, w, in, L.W, bias, out, none, st);
+    conv_mma<EPI_BIAS_RELU>(u->sms, B, h, w, in, L.W, bias, out, none, st);
   else
-    conv_res<EPI_BIAS>(B, h, w, in, L.W, bias, out, none, st);
+    conv_mma<EPI_BIAS>(u->sms, B, h, w, in, L.W, bias, out, none, st);
 }
 
 // input gradient gin = conv(g, WT) (times the ReLU mask of `mask` when given)
@@ -558,9 +577,9 @@ static void conv_dgrad(dt_unet* u, const ConvLayer& L, int B, int h, int w, Tens
                    : conv_tc<EPI_STORE>(u, B, h, w, gg, L.W, cout, nullptr, gout, none, st);
   if (done) return;
   if (mask)
-    conv_res<EPI_MASK>(B, h, w, gg, L.WT, nullptr, gout, *mask, st);
+    conv_mma<EPI_MASK>(u->sms, B, h, w, gg, L.WT, nullptr, gout, *mask, st);
   else
-    conv_res<EPI_STORE>(B, h, w, gg, L.WT, nullptr, gout, none, st);
+    conv_mma<EPI_STORE>(u->sms, B, h, w, gg, L.WT, nullptr, gout, none, st);
 }
 
 // weight and bias gradients of a layer into u->grad
