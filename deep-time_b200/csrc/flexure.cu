@@ -2392,7 +2392,7 @@ static dt_status make_any_tables(dt_flex* s, Lane<T>& L) {
 
 // log2 of the wavenumbers a k_row_solve block takes for rasters of h rows: 8, or 4 where that keeps
 // the block within ROW_THREADS threads and the SM's shared memory; -1 (the chunk passes) where even
-// 4 do not fit, h > 2048 in FP32 and h > 1936 in FP64.
+// 4 do not fit, h > 2048 in FP32 and h > 1952 in FP64.
 template <class T>
 static int row_groups(int h) {
   const int P = (int)ceil_div(h, ROW_CH);
