@@ -71,7 +71,7 @@ __device__ __forceinline__ int swz_b(int row, int chunk) {
   return row * BN + ((chunk ^ (row & 7)) << 3);                       // 128-byte rows
 }
 
-enum { EPI_BIAS_RELU = 0, EPI_BIAS = 1, EPI_STORE = 2, EPI_ACCUM = 3, EPI_MASK = 4 };
+enum { EPI_BIAS_RELU = 0, EPI_BIAS = 1, EPI_STORE = 2, EPI_MASK = 3 };
 
 // Two neighbouring channels of a pixel's output: the bias and ReLU, or the producing ReLU's mask.
 template <int EPI>
@@ -91,11 +91,6 @@ __device__ __forceinline__ void conv_store(bf16* dst, int col, float v0, float v
     __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(mask.p + pix * mask.stride + mask.off + co0 + col);
     if (!(__bfloat162float(m.x) > 0.f)) v0 = 0.f;
     if (!(__bfloat162float(m.y) > 0.f)) v1 = 0.f;
-  }
-  if (EPI == EPI_ACCUM) {
-    __nv_bfloat162 prev = *d2;
-    v0 += __bfloat162float(prev.x);
-    v1 += __bfloat162float(prev.y);
   }
   *d2 = __floats2bfloat162_rn(v0, v1);
 }

@@ -244,15 +244,6 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(int nimg, int h, int w, Tens
           if (!(__bfloat162float(m.y) > 0.f)) v[2 * e + 1] = 0.f;
         }
       }
-      __nv_bfloat162* d2 = reinterpret_cast<__nv_bfloat162*>(dst + c0);
-      if (EPI == EPI_ACCUM) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          __nv_bfloat162 prev = d2[e];
-          v[2 * e] += __bfloat162float(prev.x);
-          v[2 * e + 1] += __bfloat162float(prev.y);
-        }
-      }
       uint4 pk;
       __nv_bfloat162 b0 = __floats2bfloat162_rn(v[0], v[1]), b1 = __floats2bfloat162_rn(v[2], v[3]);
       __nv_bfloat162 b2 = __floats2bfloat162_rn(v[4], v[5]), b3 = __floats2bfloat162_rn(v[6], v[7]);

@@ -1898,7 +1898,7 @@ static TM* cycle_rz(dt_diff* s, CgLane<TC, TM>& C, int kind, cudaStream_t st) {
 // The residual replacement of a reliable-update iteration (the FP32 lane): gated kernels that do
 // nothing unless the iteration's update asked for it. `count`: count their launches (not inside
 // the loop body's IF node, whose runs are counted from the replacements).
-static void launch_reliable_d(dt_diff* s, Hier<float>& H, cudaStream_t st, bool count) {
+static void launch_reliable_d(dt_diff* s, cudaStream_t st, bool count) {
   unsigned int g = dgrid(s, s->n);
   k_d_rel_accumulate<<<g, 256, 0, st>>>(s->n, s->x, s->x32, s->scale, s->S32);
   k_d_apply<double, float, DA_RESID_GATED><<<g, 256, 0, st>>>(s->w, s->h, s->wrap && s->w > 1, s->east, s->south, s->diag, s->x,
@@ -1910,8 +1910,7 @@ static void launch_reliable_d(dt_diff* s, Hier<float>& H, cudaStream_t st, bool 
 
 // While `st` captures a loop body: a conditional IF node, its body the residual replacement
 // (captured on `aside`), so that iterations that replace nothing launch nothing for it.
-static dt_status add_reliable_if_d(dt_diff* s, Hier<float>& H, cudaStream_t st, cudaStream_t aside,
-                                   unsigned long long* handle_out) {
+static dt_status add_reliable_if_d(dt_diff* s, cudaStream_t st, cudaStream_t aside, unsigned long long* handle_out) {
   cudaStreamCaptureStatus cs;
   unsigned long long id = 0;
   cudaGraph_t graph = nullptr;
@@ -1934,7 +1933,7 @@ static dt_status add_reliable_if_d(dt_diff* s, Hier<float>& H, cudaStream_t st, 
   DT_CUDA(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
   DT_CUDA(cudaStreamBeginCaptureToGraph(aside, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                         cudaStreamCaptureModeThreadLocal));
-  launch_reliable_d(s, H, aside, false);
+  launch_reliable_d(s, aside, false);
   cudaGraph_t ifbody;
   DT_CUDA(cudaStreamEndCapture(aside, &ifbody));
   *handle_out = (unsigned long long)h;
@@ -1957,9 +1956,9 @@ static dt_status cg_iteration(dt_diff* s, CgLane<TC, TM>& C, int kind, cudaStrea
   if constexpr (std::is_same<TM, float>::value) {
     if (reliable) {
       if (aside)
-        DT_TRY(add_reliable_if_d(s, *C.H, st, aside, if_handle));
+        DT_TRY(add_reliable_if_d(s, st, aside, if_handle));
       else
-        launch_reliable_d(s, *C.H, st, true);
+        launch_reliable_d(s, st, true);
     }
   }
   TM* z = cycle_rz<TC, TM>(s, C, kind, st);

@@ -2493,28 +2493,29 @@ static bool tensor_map(dt_flex* s, const void* p, int elem, int bw, int bh, CUte
   return true;
 }
 
-// Resident blocks per SM of each TMA stencil instantiation ([double][mode]), set at create.
-static int g_tma_per_sm[2][7];
+// Resident blocks per SM of each TMA stencil mode, set at create.
+static int g_tma_per_sm[7];
 
-template <class T, int MODE>
+template <int MODE>
 static void tma_setup() {
-  using ST = TmaStage<T, MODE>;
-  cudaFuncSetAttribute(k_apply_tma<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST::SMEM);
+  using ST = TmaStage<double, MODE>;
+  cudaFuncSetAttribute(k_apply_tma<double, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST::SMEM);
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_apply_tma<T, MODE>, TBX * TTY, ST::SMEM);
-  g_tma_per_sm[sizeof(T) == 8][MODE] = std::max(nb, 1);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_apply_tma<double, MODE>, TBX * TTY, ST::SMEM);
+  g_tma_per_sm[MODE] = std::max(nb, 1);
 }
-template <class T>
 static void tma_setup_all() {
-  tma_setup<T, RESID>();
-  tma_setup<T, PLAIN>();
-  tma_setup<T, BEND>();
-  tma_setup<T, RESID_GATED>();
+  tma_setup<RESID>();
+  tma_setup<PLAIN>();
+  tma_setup<BEND>();
+  tma_setup<RESID_GATED>();
 }
 
 // The persistent TMA stencil; false (nothing launched) when a buffer cannot be mapped.
-template <class T, int MODE>
-static bool launch_apply_tma(dt_flex* s, const T* v, const T* d, const T* c, const T* rb, T* y, Scalars* S, cudaStream_t st) {
+template <int MODE>
+static bool launch_apply_tma(dt_flex* s, const double* v, const double* d, const double* c, const double* rb, double* y, Scalars* S,
+                             cudaStream_t st) {
+  using T = double;
   using ST = TmaStage<T, MODE>;
   CUtensorMap mv, md, mc, mb;
   if (!tensor_map(s, v, sizeof(T), ST::P, ST::UR, &mv)) return false;
@@ -2523,7 +2524,7 @@ static bool launch_apply_tma(dt_flex* s, const T* v, const T* d, const T* c, con
   if (ST::HAS_C && !tensor_map(s, c, sizeof(T), TBX, ST::TBY, &mc)) return false;
   if (ST::HAS_B && !tensor_map(s, rb, sizeof(T), TBX, ST::TBY, &mb)) return false;
   const int tiles_x = s->w / TBX, ntiles = tiles_x * (int)ceil_div(s->h, ST::TBY);
-  const int grid = std::max(1, std::min(ntiles, g_tma_per_sm[sizeof(T) == 8][MODE] * s->sms));
+  const int grid = std::max(1, std::min(ntiles, g_tma_per_sm[MODE] * s->sms));
   T inv = (T)(1.0 / (s->dx * s->dx));
   k_apply_tma<T, MODE><<<grid, dim3(TBX, TTY), ST::SMEM, st>>>(mv, md, mc, mb, s->w, s->h, inv, v, d, y, s->partials, S, tiles_x,
                                                               ntiles);
@@ -2532,14 +2533,12 @@ static bool launch_apply_tma(dt_flex* s, const T* v, const T* d, const T* c, con
 }
 
 // The operator on the sphere's row metric: the per-block kernel (the TMA stencil has the block
-// metric only), the handle's couplings in the lane's precision.
-template <class T>
-static void launch_apply_metric(dt_flex* s, int mode, dim3 grid, dim3 block, T inv, const T* v, const T* d, const T* c, const T* rb,
-                                T* y, Scalars* S, cudaStream_t st) {
-  const T* ma = metric_a<T>(s);
-  const T* mb = metric_b<T>(s);
+// metric only).
+static void launch_apply_metric(dt_flex* s, int mode, dim3 grid, dim3 block, double inv, const double* v, const double* d,
+                                const double* c, const double* rb, double* y, Scalars* S, cudaStream_t st) {
+  const double *ma = metric_a<double>(s), *mb = metric_b<double>(s);
 #define DT_MET_CASE(M) \
-  case M: k_apply<T, M, true><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S, ma, mb); break;
+  case M: k_apply<double, M, true><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S, ma, mb); break;
   switch (mode) {
     DT_MET_CASE(RESID)
     DT_MET_CASE(PLAIN)
@@ -2587,6 +2586,37 @@ static void launch_tile(dt_flex* s, const T* v, const T* J, const T* part, const
     launch_tile_rows<T, MODE, false, W2, R2>(s, v, J, part, d, c, y, S, st);
 }
 
+// The residual, and the plain and bend forms, which FP64 alone takes.
+static void launch_apply_fp64(dt_flex* s, int mode, const double* v, const double* d, const double* c, const double* rb, double* y,
+                              Scalars* S, cudaStream_t st) {
+  if (s->tma && !s->metric) {
+    bool done = false;
+    switch (mode) {
+      case RESID: done = launch_apply_tma<RESID>(s, v, d, c, rb, y, S, st); break;
+      case PLAIN: done = launch_apply_tma<PLAIN>(s, v, d, c, rb, y, S, st); break;
+      case BEND: done = launch_apply_tma<BEND>(s, v, d, c, rb, y, S, st); break;
+      case RESID_GATED: done = launch_apply_tma<RESID_GATED>(s, v, d, c, rb, y, S, st); break;
+    }
+    if (done) return;
+  }
+  dim3 grid(ceil_div(s->w, TBX), ceil_div(s->h, tile_rows<double>())), block(TBX, TTY);
+  const double inv = 1.0 / (s->dx * s->dx);
+  if (s->metric) {
+    launch_apply_metric(s, mode, grid, block, inv, v, d, c, rb, y, S, st);
+    return;
+  }
+#define DT_APPLY_CASE(M) \
+  case M: k_apply<double, M><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); break;
+  switch (mode) {
+    DT_APPLY_CASE(RESID)
+    DT_APPLY_CASE(PLAIN)
+    DT_APPLY_CASE(BEND)
+    DT_APPLY_CASE(RESID_GATED)
+  }
+#undef DT_APPLY_CASE
+  counted();
+}
+
 template <class T>
 static void launch_apply(dt_flex* s, int mode, const T* v, const T* J, const T* part, const T* d, const T* c, const T* rb, T* y,
                          Scalars* S, cudaStream_t st) {
@@ -2594,29 +2624,8 @@ static void launch_apply(dt_flex* s, int mode, const T* v, const T* J, const T* 
     case AP_DOT: launch_tile<T, AP_DOT>(s, v, nullptr, nullptr, d, c, y, S, st); return;
     case JAC_LEFT: launch_tile<T, JAC_LEFT>(s, rb, J, nullptr, d, c, y, S, st); return;
     case JAC_FINAL: launch_tile<T, JAC_FINAL>(s, rb, J, part, d, c, y, S, st); return;
-    default: break;
-  }
-  if (s->tma && !s->metric) {
-    bool done = false;
-    switch (mode) {
-      case RESID: done = launch_apply_tma<T, RESID>(s, v, d, c, rb, y, S, st); break;
-      case PLAIN: done = launch_apply_tma<T, PLAIN>(s, v, d, c, rb, y, S, st); break;
-      case BEND: done = launch_apply_tma<T, BEND>(s, v, d, c, rb, y, S, st); break;
-      case RESID_GATED: done = launch_apply_tma<T, RESID_GATED>(s, v, d, c, rb, y, S, st); break;
-    }
-    if (done) return;
-  }
-  dim3 grid(ceil_div(s->w, TBX), ceil_div(s->h, tile_rows<T>())), block(TBX, TTY);
-  T inv = (T)(1.0 / (s->dx * s->dx));
-  if (s->metric) {
-    launch_apply_metric<T>(s, mode, grid, block, inv, v, d, c, rb, y, S, st);
-    return;
-  }
-  switch (mode) {
-    case RESID: k_apply<T, RESID><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); counted(); break;
-    case PLAIN: k_apply<T, PLAIN><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); counted(); break;
-    case BEND: k_apply<T, BEND><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); counted(); break;
-    case RESID_GATED: k_apply<T, RESID_GATED><<<grid, block, 0, st>>>(s->w, s->h, inv, v, d, c, rb, y, s->partials, S); counted(); break;
+    default:
+      if constexpr (sizeof(T) == 8) launch_apply_fp64(s, mode, v, d, c, rb, y, S, st);
   }
 }
 
@@ -3748,10 +3757,7 @@ dt_status dt_flex_create(int w, int h, double dx, const double* metric_a, const 
     // the TMA stencil takes rasters whose rows are whole tiles; DT_STENCIL_TMA=0 turns it off
     const char* env = getenv("DT_STENCIL_TMA");
     s->tma = w % TBX == 0 && !s->metric && encode_tiled() != nullptr && !(env && env[0] == '0');
-    if (s->tma) {
-      tma_setup_all<double>();
-      tma_setup_all<float>();
-    }
+    if (s->tma) tma_setup_all();
   }
   for (int k = 0; k < 2; ++k)
     if (cudaStreamCreateWithFlags(&s->side[k], cudaStreamNonBlocking) != cudaSuccess ||

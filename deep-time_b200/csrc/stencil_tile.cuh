@@ -67,108 +67,108 @@ __global__ void __launch_bounds__(32 * FT_WARPS, 2) k_flex_tile(int w, int h, T 
   // a buffer of `edge` is written again only after the next barrier of its other one
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-  const int ty = tile / tiles_x;
-  const int raw = (tile - ty * tiles_x) * FT_TX - FT_H + 2 * lane, j0 = ty * TY - FT_H + warp * RPW;
-  int c0 = raw % w;
-  c0 += c0 < 0 ? w : 0;
-  const int c1 = c0 + 1 == w ? 0 : c0 + 1;
-  const bool tile_cols = lane >= FT_H / 2 && lane < 32 - FT_H / 2 && raw < w;
-  Duo<T> u[RPW], rr[JAC ? RPW : 1], jj[MODE == JAC_FINAL ? RPW : 1], m[RPW], cc[RPW];
+    const int ty = tile / tiles_x;
+    const int raw = (tile - ty * tiles_x) * FT_TX - FT_H + 2 * lane, j0 = ty * TY - FT_H + warp * RPW;
+    int c0 = raw % w;
+    c0 += c0 < 0 ? w : 0;
+    const int c1 = c0 + 1 == w ? 0 : c0 + 1;
+    const bool tile_cols = lane >= FT_H / 2 && lane < 32 - FT_H / 2 && raw < w;
+    Duo<T> u[RPW], rr[JAC ? RPW : 1], jj[MODE == JAC_FINAL ? RPW : 1], m[RPW], cc[RPW];
 #pragma unroll
-  for (int q = 0; q < RPW; ++q) {
-    const int j = j0 + q;
-    const bool in = j >= 0 && j < h;
-    const size_t row = (size_t)(in ? j : 0) * w;
-    u[q] = ft_load<T, VEC>(v, row, c0, c1, in);
-    if constexpr (JAC) {
-      const Duo<T> w_ = ft_load<T, VEC>(J, row, c0, c1, in);
-      rr[q] = u[q];
-      if constexpr (MODE == JAC_FINAL) {
-        jj[q] = w_;
-        u[q] = ft_load<T, VEC>(part, row, c0, c1, in);
-      } else {
-        u[q] = w_;
+    for (int q = 0; q < RPW; ++q) {
+      const int j = j0 + q;
+      const bool in = j >= 0 && j < h;
+      const size_t row = (size_t)(in ? j : 0) * w;
+      u[q] = ft_load<T, VEC>(v, row, c0, c1, in);
+      if constexpr (JAC) {
+        const Duo<T> w_ = ft_load<T, VEC>(J, row, c0, c1, in);
+        rr[q] = u[q];
+        if constexpr (MODE == JAC_FINAL) {
+          jj[q] = w_;
+          u[q] = ft_load<T, VEC>(part, row, c0, c1, in);
+        } else {
+          u[q] = w_;
+        }
       }
+      m[q] = ft_load<T, VEC>(d, row, c0, c1, in);
+      cc[q] = ft_load<T, VEC>(c, row, c0, c1, in && tile_cols);
     }
-    m[q] = ft_load<T, VEC>(d, row, c0, c1, in);
-    cc[q] = ft_load<T, VEC>(c, row, c0, c1, in && tile_cols);
-  }
-  if constexpr (JAC) {
-    // the vector the mode forms: u = J r (+ part)
+    if constexpr (JAC) {
+      // the vector the mode forms: u = J r (+ part)
 #pragma unroll
-    for (int q = 0; q < RPW; ++q)
+      for (int q = 0; q < RPW; ++q)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if constexpr (MODE == JAC_FINAL) {
+            T t = jj[q].v[e] * rr[q].v[e];
+            t += u[q].v[e];
+            u[q].v[e] = t;
+          } else {
+            u[q].v[e] = u[q].v[e] * rr[q].v[e];
+          }
+        }
+    }
+    // L x at the lane's cells of row q; up / down: the rows beyond the lane's own
+    auto lap = [&](const Duo<T>* x, int q, const Duo<T>& up, const Duo<T>& down) {
+      const int j = j0 + q;
+      const RowCoef<T, MET> k = row_coef<T, MET>(ma, mb, j, h);
+      const Duo<T> self = x[q], north = j == 0 ? self : q ? x[q ? q - 1 : 0] : up,
+                   south = j == h - 1 ? self : q + 1 < RPW ? x[q + 1 < RPW ? q + 1 : q] : down;
+      const T right = __shfl_down_sync(0xffffffffu, self.v[0], 1), left = __shfl_up_sync(0xffffffffu, self.v[1], 1);
+      Duo<T> o;
+      o.v[0] = lap5<T, MET>(left, self.v[1], north.v[0], south.v[0], self.v[0], k, inv_dx2);
+      o.v[1] = lap5<T, MET>(self.v[0], right, north.v[1], south.v[1], self.v[1], k, inv_dx2);
+      return o;
+    };
+    auto meet = [&](int b, const Duo<T>* x, Duo<T>& up, Duo<T>& down) {
+      edge[b][0][warp][lane] = x[0];
+      edge[b][1][warp][lane] = x[RPW - 1];
+      __syncthreads();
+      up.v[0] = up.v[1] = down.v[0] = down.v[1] = (T)0;
+      if (warp > 0) up = edge[b][1][warp - 1][lane];
+      if (warp < FT_WARPS - 1) down = edge[b][0][warp + 1][lane];
+    };
+    Duo<T> up, down;
+    meet(0, u, up, down);
+#pragma unroll
+    for (int q = 0; q < RPW; ++q) {
+      const Duo<T> l = lap(u, q, up, down);
+      m[q].v[0] = l.v[0] * m[q].v[0];
+      m[q].v[1] = l.v[1] * m[q].v[1];
+    }
+    meet(1, m, up, down);
+#pragma unroll
+    for (int q = 0; q < RPW; ++q) {
+      const Duo<T> l = lap(m, q, up, down);
+      const int j = j0 + q, rw = warp * RPW + q;
+      if (!tile_cols || rw < FT_H || rw >= R - FT_H || j >= h) continue;
+      Duo<T> o;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        if constexpr (MODE == JAC_FINAL) {
-          T t = jj[q].v[e] * rr[q].v[e];
-          t += u[q].v[e];
-          u[q].v[e] = t;
+        const T uu = u[q].v[e], au = l.v[e] + cc[q].v[e] * uu;
+        const bool on = VEC || e == 0 || raw + 1 < w;
+        if constexpr (MODE == AP_DOT) {
+          o.v[e] = au;
+          if (on) acc.v[0] += (double)uu * (double)au;
+        } else if constexpr (MODE == JAC_LEFT) {
+          o.v[e] = rr[q].v[e] - au;
         } else {
-          u[q].v[e] = u[q].v[e] * rr[q].v[e];
+          const T r = rr[q].v[e], z = uu + jj[q].v[e] * (r - au);
+          o.v[e] = z;
+          if (on) {
+            acc.v[0] += (double)r * (double)z;
+            most = max_num(most, fabs(z));
+          }
         }
       }
-  }
-  // L x at the lane's cells of row q; up / down: the rows beyond the lane's own
-  auto lap = [&](const Duo<T>* x, int q, const Duo<T>& up, const Duo<T>& down) {
-    const int j = j0 + q;
-    const RowCoef<T, MET> k = row_coef<T, MET>(ma, mb, j, h);
-    const Duo<T> self = x[q], north = j == 0 ? self : q ? x[q ? q - 1 : 0] : up,
-                 south = j == h - 1 ? self : q + 1 < RPW ? x[q + 1 < RPW ? q + 1 : q] : down;
-    const T right = __shfl_down_sync(0xffffffffu, self.v[0], 1), left = __shfl_up_sync(0xffffffffu, self.v[1], 1);
-    Duo<T> o;
-    o.v[0] = lap5<T, MET>(left, self.v[1], north.v[0], south.v[0], self.v[0], k, inv_dx2);
-    o.v[1] = lap5<T, MET>(self.v[0], right, north.v[1], south.v[1], self.v[1], k, inv_dx2);
-    return o;
-  };
-  auto meet = [&](int b, const Duo<T>* x, Duo<T>& up, Duo<T>& down) {
-    edge[b][0][warp][lane] = x[0];
-    edge[b][1][warp][lane] = x[RPW - 1];
-    __syncthreads();
-    up.v[0] = up.v[1] = down.v[0] = down.v[1] = (T)0;
-    if (warp > 0) up = edge[b][1][warp - 1][lane];
-    if (warp < FT_WARPS - 1) down = edge[b][0][warp + 1][lane];
-  };
-  Duo<T> up, down;
-  meet(0, u, up, down);
-#pragma unroll
-  for (int q = 0; q < RPW; ++q) {
-    const Duo<T> l = lap(u, q, up, down);
-    m[q].v[0] = l.v[0] * m[q].v[0];
-    m[q].v[1] = l.v[1] * m[q].v[1];
-  }
-  meet(1, m, up, down);
-#pragma unroll
-  for (int q = 0; q < RPW; ++q) {
-    const Duo<T> l = lap(m, q, up, down);
-    const int j = j0 + q, rw = warp * RPW + q;
-    if (!tile_cols || rw < FT_H || rw >= R - FT_H || j >= h) continue;
-    Duo<T> o;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const T uu = u[q].v[e], au = l.v[e] + cc[q].v[e] * uu;
-      const bool on = VEC || e == 0 || raw + 1 < w;
-      if constexpr (MODE == AP_DOT) {
-        o.v[e] = au;
-        if (on) acc.v[0] += (double)uu * (double)au;
-      } else if constexpr (MODE == JAC_LEFT) {
-        o.v[e] = rr[q].v[e] - au;
+      const size_t at = (size_t)j * w + raw;
+      if constexpr (VEC) {
+        *reinterpret_cast<cplx<T>*>(y + at) = mk<cplx<T>>(o.v[0], o.v[1]);
       } else {
-        const T r = rr[q].v[e], z = uu + jj[q].v[e] * (r - au);
-        o.v[e] = z;
-        if (on) {
-          acc.v[0] += (double)r * (double)z;
-          most = max_num(most, fabs(z));
-        }
+        y[at] = o.v[0];
+        if (raw + 1 < w) y[at + 1] = o.v[1];
       }
     }
-    const size_t at = (size_t)j * w + raw;
-    if constexpr (VEC) {
-      *reinterpret_cast<cplx<T>*>(y + at) = mk<cplx<T>>(o.v[0], o.v[1]);
-    } else {
-      y[at] = o.v[0];
-      if (raw + 1 < w) y[at + 1] = o.v[1];
-    }
-  }
   }
   if constexpr (MODE != JAC_LEFT) {
     const int kind[2] = {0, 1};
