@@ -86,9 +86,11 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return __ffma2_rn(make_float2(-a.y, a.y), make_float2(b.y, b.x), __fmul2_rn(make_float2(a.x, a.x), b));
 }
 
-// Reciprocals of normal numbers with no slow-path call: float, the correctly rounded intrinsic;
-// double, of m 2^e, the hardware's float estimate of 1 / m, m in [1, 2), scaled by 2^-e in the exponent bits and refined by two Newton-Raphson steps r <- r + r (1 - x r)
-// (each squares the relative error: 2^-22 -> 2^-44 -> 2^-88, so the last rounding is what is left).
+// Reciprocals with no slow-path call: float, the correctly rounded intrinsic; double, for normal x
+// below 2^1022 (divisors of positive definite systems; 0 and infinity give no number, NaN gives NaN):
+// of x = m 2^e, m in [1, 2), the hardware's float estimate of 1 / m, scaled by 2^-e in the exponent
+// bits and refined by two Newton-Raphson steps r <- r + r (1 - x r) (each squares the relative
+// error: 2^-22 -> 2^-44 -> 2^-88, so the last rounding is what is left).
 __device__ __forceinline__ double recip(double x) {
   const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
   const double m = __hiloint2double(hi - (e << 20), __double2loint(x));

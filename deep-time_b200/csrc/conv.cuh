@@ -8,7 +8,8 @@
 // with the taps mirrored and the weight matrix transposed.
 //
 // Forward / input-gradient: out[p][co] = sum_{tap, ci} in[p + off(tap)][ci] W[tap][ci][co], a GEMM
-// with M = pixels, N = output channels, K = 9 x input channels (k_conv3x3_res). Fragments are loaded with
+// with M = pixels, N = output channels, K = 9 x input channels (k_conv3x3_res, and k_conv3x3_line where
+// that one's larger blocks are too few or do not fit). Fragments are loaded with
 // ldmatrix (x4 for A, x4.trans for B from XOR-swizzled shared memory) and multiplied with
 // mma.sync.m16n8k16.row.col.f32.bf16.bf16.f32.
 //

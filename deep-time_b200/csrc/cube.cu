@@ -595,8 +595,8 @@ __global__ void k_mg_restrict(size_t cells, size_t fine, const uint32_t* __restr
 // with the same arithmetic per cell, a block barrier where a launch ends (the coarsest level, at
 // most 64 cells, in one warp). A chain of some 40 short passes, each bound by the latency of its
 // gathers, so the levels' rows and vectors are brought into shared memory first, by asynchronous
-// copies (rows stored entry by entry read free of bank conflicts). From global memory the 1536-cell level and those below took 56 us a
-// cycle, now 29.
+// copies (rows stored entry by entry read free of bank conflicts): 29 us a cycle for the
+// 1536-cell level and those below, 56 from global memory.
 struct MgLevelDev {
   unsigned cells, entries;  // entries = width cells
   const uint32_t *ptr, *col, *kid_ptr, *kids;

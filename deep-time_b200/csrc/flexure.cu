@@ -5,9 +5,12 @@
 // operator :1546-1624, Spectral :1108-1348, Bank :1352-1402, Preconditioner :1405-1468,
 // Solver::solve :1680-1740) with its own kernels:
 //
-//   k_apply      the 13-point variable-D biharmonic y = L(d L v) + c v over a shared-memory tile
-//                with a 2-cell halo (x wraps, rows clamp), fused with the CG reduction of its
-//                caller (p.Ap, ||b - Ax||^2, or the Jacobi sandwich of the preconditioner);
+//   k_flex_tile  the 13-point variable-D biharmonic y = L(d L v) + c v of an iteration over register
+//                tiles (stencil_tile.cuh; x wraps, rows clamp): with p.Ap, and as the two passes of
+//                the preconditioner's Jacobi sandwich;
+//   k_apply_tma, k_apply  the FP64 residual b - A x with its norm and the operator's plain and bend
+//                forms, over shared-memory tiles fed by bulk tensor copies (stencil_tma.cuh; widths
+//                of whole 64-column tiles on the block metric) or by cp.async;
 //   k_rows_fwd   per row: a real FFT of length w as a complex FFT of length w/2 (even samples
 //                real, odd imaginary) and the usual split, written in a packed half spectrum:
 //                column 0 holds (X[0], X[w/2]), both real;
@@ -2294,8 +2297,9 @@ static AnyPlan make_any_plan(int w, int h, bool block) {
 // blocks against one with the passes:
 // - One level turns with the times of the two forms of a transform. The block: a thread's values through
 //   the stages, 0.13 us each and 0.08 for a term of a prime radix's sum (R terms a value). The passes: a
-//   launch each of 2.2 us (4 in Bluestein's two transforms) and their bytes, and a prime radix's terms at 0.3 us. FP64 1500 x 256 67 us
-//   against 86, 1830 x 256 (radix 61) 263 against 177, 3000 x 16 84 against 73, 3000 x 256 100 against 109.
+//   launch each of 2.2 us (4 in Bluestein's two transforms) and their bytes, and a prime radix's terms at
+//   0.3 us. FP64 1500 x 256 67 us against 86, 1830 x 256 (radix 61) 263 against 177, 3000 x 16 84 against 73,
+//   3000 x 256 100 against 109.
 // - The bank's three levels side by side hide more of the chain, half of the primes' table reads:
 //   FP64 740 x 256 (radix 37) 137 us against 183, 1859 x 16 (11, 13, 13) 181 against 125.
 // - Rows that fill the SMs more than once (the bank with a short chain: twice; FP64 1301 x 100 by Bluestein,
@@ -3028,8 +3032,8 @@ static void launch_spectral(dt_flex* s, Lane<T>& L, const T* in, const T* wt, T*
   launch_rows_inv<T>(s, L, inv_mode, half, out, wt, inv_mode == INV_STORE_DOT ? in : nullptr, g, S, st);
 }
 
-// Whether the bank's levels share a launch a pass: where each pass is one kernel (the power-of-two
-// transforms, and along y the cosine transform or k_row_solve).
+// Whether the bank's levels share a launch a pass: where each pass is one kernel (along x the
+// power-of-two transforms or row pairs in blocks, along y the cosine transform or k_row_solve).
 template <class T>
 static bool bank_batched(const dt_flex* s, const Lane<T>& L) {
   return s->bank_one_launch && !(s->any && !L.block_bank) && !(s->row_solve && row_groups<T>(s->h) < 0);

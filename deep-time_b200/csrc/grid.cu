@@ -194,16 +194,16 @@ __global__ void k_blur_cols(int w, int h, int r, double norm, const double* __re
 }
 
 // The box blur's running sums with the lines streamed through shared memory. A block takes LINES
-// (8, 16 or 32) lines (rows with ROWS, else columns); line line0 + l is lane l's (and l + LINES's, ...): out(k) = acc (1 / (2r + 1)),
-// acc += v(k + r + 1) - v(k - r), with acc started as the sum of v(-r .. r) in order, the
+// (8, 16 or 32) lines (rows with ROWS, else columns); line line0 + l is lane l's (and l + LINES's, ...):
+// out(k) = acc (1 / (2r + 1)), acc += v(k + r + 1) - v(k - r), with acc started as the sum of v(-r .. r) in order, the
 // reference's loop bit for bit. Only the running sum is serial, so six warps split the work, one
 // tile of 32 positions a step, skewed by a step and separated by one block barrier a step:
 //   warp 1  the loader: keeps up to RING / 32 - B - 1 tiles ahead in flight, 8-byte cp.async
 //           copies of one 256-byte row segment per line (ROWS) or per position (columns), into a
 //           ring of RING positions per line;
 //   warps 2-5  the differences d(k) = v(k + r + 1) - v(k - r) of step s's tile (8 positions
-//           each, shared by the lanes of a line) from the ring, or from global memory past the line's ends (wrap, clamp or
-//           reflection); and the stores of step s - 2's sums times 1 / (2r + 1), whole row
+//           each, shared by the lanes of a line) from the ring, or from global memory past the
+//           line's ends (wrap, clamp or reflection); and the stores of step s - 2's sums times 1 / (2r + 1), whole row
 //           segments in both directions;
 //   warp 0  the running sum over step s - 1's differences.
 // The ring is line-major with ROWS (a line's RING positions contiguous, pitch RING + 1) and

@@ -18,6 +18,8 @@
 // (AP_DOT, JAC_LEFT, JAC_FINAL): FP32 4096 x 2048 39.3, 44.0, 54.0 -> 37.9, 37.7, 49.1; FP64 57.7, 75.6,
 // 88.4 -> 59.2, 63.9, 81.9; FP64 1024 x 328 15.6, 14.1, 18.3 -> 13.3, 11.1, 15.3; FP64 1500 x 750 21.6,
 // 19.8, 29.6 -> 17.9, 16.3, 23.5.
+// The one loss, AP_DOT at FP64 4096 x 2048, is not felt: a mean-D iteration there, which has no other
+// stencil, went from 327 to 321 us with the vector kernels' words.
 // Included by flexure.cu after k_apply.
 #pragma once
 
