@@ -414,6 +414,16 @@ __global__ void k_cube_untranspose(int n, const double* __restrict__ t, double* 
 }
 
 // ---- the V-cycle's levels (multigrid.rs:199-363), FP32 without fused multiply-adds ----
+// A level's neighbours from row after row to entry by entry ([width][cells], 0 past a row's end), once a handle. On
+// the device: the host's walk over a strided copy of 12.6 MB made a handle of 6 x 256^2 cells take 69 ms, from 62.
+__global__ void k_mg_by_entry(size_t cells, unsigned width, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ rows,
+                              uint32_t* __restrict__ col) {
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < cells; c += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t at = ptr[c], cnt = ptr[c + 1] - at;
+    for (unsigned e = 0; e < width; ++e) col[e * cells + c] = e < cnt ? rows[at + e] : 0u;
+  }
+}
+
 __global__ void k_mg_val0(size_t cells, const uint32_t* __restrict__ slots, const double* __restrict__ k,
                           const double* __restrict__ mu, const double* __restrict__ diag64, const uint32_t* __restrict__ ptr,
                           float* __restrict__ val, float* __restrict__ ell, float* __restrict__ mass, float* __restrict__ diag) {
@@ -1417,14 +1427,21 @@ dt_status dt_cube_create(int n, const uint32_t* slots, const double* lap, const 
     lv.nnz = p.col.size();
     lv.side = p.side;
     for (size_t c = 0; c < p.cells; ++c) lv.width = std::max<size_t>(lv.width, p.ptr[c + 1] - p.ptr[c]);
-    std::vector<uint32_t> col(lv.width * p.cells, 0);
-    for (size_t c = 0; c < p.cells; ++c)
-      for (uint32_t e = p.ptr[c]; e < p.ptr[c + 1]; ++e) col[(e - p.ptr[c]) * p.cells + c] = p.col[e];
-    if ((st = cube_upload(s, &lv.ptr, p.ptr)) != DT_OK || (st = cube_upload(s, &lv.col, col)) != DT_OK) return fail(st);
+    // the neighbours row after row pass through the buffer of `ell`, whose values a solve writes; on the stream of
+    // the copies
+    if ((st = cube_upload(s, &lv.ptr, p.ptr)) != DT_OK || (st = cube_alloc(s, &lv.col, lv.width * lv.cells)) != DT_OK ||
+        (st = cube_alloc(s, &lv.ell, lv.width * lv.cells + lv.nnz)) != DT_OK)
+      return fail(st);
+    lv.val = lv.ell + lv.width * lv.cells;
+    uint32_t* rows = reinterpret_cast<uint32_t*>(lv.ell);
+    if (cudaMemcpy(rows, p.col.data(), lv.nnz * sizeof(uint32_t), cudaMemcpyHostToDevice) != cudaSuccess) {
+      set_error("dt_cube_create: %s", cudaGetErrorString(cudaGetLastError()));
+      return fail(DT_DEVICE_ERROR);
+    }
+    k_mg_by_entry<<<cube_grid(lv.cells), 256>>>(lv.cells, (unsigned)lv.width, lv.ptr, rows, lv.col);
     if (l > 0 && ((st = cube_upload(s, &lv.src_ptr, p.src_ptr)) != DT_OK || (st = cube_upload(s, &lv.src, p.src)) != DT_OK ||
                   (st = cube_upload(s, &lv.kid_ptr, p.kid_ptr)) != DT_OK || (st = cube_upload(s, &lv.kids, p.kids)) != DT_OK))
       return fail(st);
-    if ((st = cube_alloc(s, &lv.val, lv.nnz)) != DT_OK || (st = cube_alloc(s, &lv.ell, lv.width * lv.cells)) != DT_OK) return fail(st);
     for (float** q : {&lv.mass, &lv.diag, &lv.r, &lv.z, &lv.t})
       if ((st = cube_alloc(s, q, lv.cells)) != DT_OK) return fail(st);
   }
