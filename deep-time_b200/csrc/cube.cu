@@ -899,8 +899,8 @@ struct dt_cube {
   double *kd = nullptr, *h = nullptr;  // staging for the host entry points
   double *k = nullptr, *s = nullptr, *diag = nullptr;
   double *rhs = nullptr, *x = nullptr, *b = nullptr, *tmp = nullptr, *cb = nullptr;
-  double* lodw[7] = {};  // the LOD's row systems (transposed) and column systems
-  // the chunked line solves' scratch: q, r (a value a cell), the chunks' end records (6 a chunk)
+  double* lodw[7] = {};  // the LOD's row systems (transposed) and column systems (the last three in the CG's r, z, ap)
+  // the chunked line solves' scratch: q, r (a value a cell, in the CG's po, pn), the chunks' end records (6 a chunk)
   // and the reduction's (4 a chunk); DT_CUBE_LOD_CHUNKED=0 at create keeps one serial walk a line
   double *lq = nullptr, *lr = nullptr, *ledge = nullptr, *lal = nullptr;
   bool lod_chunked = true;
@@ -1398,12 +1398,16 @@ dt_status dt_cube_create(int n, const uint32_t* slots, const double* lap, const 
   if ((st = cube_alloc(s, &s->k, cells * 8)) != DT_OK) return fail(st);
   for (double** p : {&s->kd, &s->h, &s->s, &s->diag, &s->rhs, &s->x, &s->b, &s->tmp, &s->cb, &s->r, &s->z, &s->po, &s->pn, &s->ap})
     if ((st = cube_alloc(s, p, cells)) != DT_OK) return fail(st);
-  for (double*& p : s->lodw)
-    if ((st = cube_alloc(s, &p, cells)) != DT_OK) return fail(st);
+  for (int q = 0; q < 4; ++q)
+    if ((st = cube_alloc(s, &s->lodw[q], cells)) != DT_OK) return fail(st);
+  // the first guess is done before the CG's vectors are first written
+  s->lodw[4] = s->r;
+  s->lodw[5] = s->z;
+  s->lodw[6] = s->ap;
+  s->lq = s->po;
+  s->lr = s->pn;
   {
     const size_t chunks = (size_t)6 * n * ((n + CUBE_LOD_CHUNK - 1) / CUBE_LOD_CHUNK);
-    for (double** p : {&s->lq, &s->lr})
-      if ((st = cube_alloc(s, p, cells)) != DT_OK) return fail(st);
     if ((st = cube_alloc(s, &s->ledge, chunks * 6)) != DT_OK) return fail(st);
     if ((st = cube_alloc(s, &s->lal, chunks * 4)) != DT_OK) return fail(st);
   }
